@@ -44,6 +44,8 @@ struct Ctx {
   std::vector<PhaseRec> phases;
   // tile reduction of resident T6 heat patterns: on unless ELFEL_TILES=0
   int tiles = 1;
+  // one-launch Krylov iterations: on unless ELFEL_ONE_LAUNCH=0
+  int one_launch = 1;
   // autotuner: on unless ELFEL_TUNE=0; one line per tuned key
   int tune = 1;
   std::vector<std::string> tune_lines;

@@ -35,6 +35,7 @@
 
 #include <chrono>
 
+#include "krylov.cuh"
 #include "solve.cuh"
 
 namespace elfel {
@@ -740,6 +741,43 @@ static Red4 red_area(SolverData* S, int k) {
   return r;
 }
 
+// The division of the slices among the blocks of the one-launch iterations
+// (krylov.cu): out[0], out[1] = the largest number of stored entries in any
+// run of spb0 (cluster), spb1 (grid) consecutive slices.
+__global__ void block_entries_k(int64_t nsl, const int64_t* __restrict__ sptr, int spb0, int spb1, int* out) {
+  for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b * min(spb0, spb1) < nsl;
+       b += (int64_t)gridDim.x * blockDim.x) {
+    if (b * spb0 < nsl) atomicMax(out, (int)(sptr[min((b + 1) * spb0, nsl)] - sptr[b * spb0]));
+    if (b * spb1 < nsl) atomicMax(out + 1, (int)(sptr[min((b + 1) * spb1, nsl)] - sptr[b * spb1]));
+  }
+}
+
+// halo[b] = the first and last block that block b's columns lie in (blocks of
+// spb slices; one CTA each); *most = the largest number of blocks between them.
+__global__ void block_halo_k(int64_t nsl, const int64_t* __restrict__ sptr, int spb, const int32_t* __restrict__ col,
+                             int2* __restrict__ halo, int* __restrict__ most) {
+  __shared__ int lo, hi;
+  const int64_t s0 = (int64_t)blockIdx.x * spb;
+  if (threadIdx.x == 0) {
+    lo = 0x7fffffff;
+    hi = 0;
+  }
+  __syncthreads();
+  int a = 0x7fffffff, z = 0;
+  for (int64_t k = sptr[s0] + threadIdx.x; k < sptr[min(s0 + spb, nsl)]; k += blockDim.x) {
+    a = min(a, col[k]);
+    z = max(z, col[k]);
+  }
+  atomicMin(&lo, (int)__reduce_min_sync(0xffffffffu, (unsigned)a));
+  atomicMax(&hi, (int)__reduce_max_sync(0xffffffffu, (unsigned)z));
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const int2 h = make_int2(min(lo, (int)s0 * 32) / (32 * spb), max(hi, (int)s0 * 32) / (32 * spb));
+    halo[blockIdx.x] = h;
+    atomicMax(most, h.y - h.x + 1);
+  }
+}
+
 static int build_sell(Ctx* c, SolverData* S) {
   const int64_t nu = S->nu;
   Sell& A = S->A;
@@ -769,17 +807,28 @@ static int build_sell(Ctx* c, SolverData* S) {
   const size_t np = (size_t)(A.nnz_pad > 0 ? A.nnz_pad : 1);
   ELFEL_TRY(col.alloc(c, np));
   ELFEL_TRY(A.map.alloc(c, np));
-  ELFEL_TRY(wide.alloc(c, 1));
-  ELFEL_CUDA(c, cudaMemsetAsync(wide.p, 0, sizeof(int), c->stream));
+  ELFEL_TRY(wide.alloc(c, 4));  // a column delta beyond 16 bits; the largest blocks' entries; the widest halo
+  ELFEL_CUDA(c, cudaMemsetAsync(wide.p, 0, 4 * sizeof(int), c->stream));
+  block_entries_k<<<1, 256, 0, c->stream>>>(nsl, A.sptr.p, run_spb_cluster(nsl), run_spb_grid(c, nsl), wide.p + 1);
   sell_fill_k<<<grid_for(nsl * 32, 256, (int64_t)c->sm_count * 16), 256, 0, c->stream>>>(
       nu, nsl, S->ff.rowptr.p, S->ff.col.p, S->ff.map.p, A.perm.p, iperm.p, A.sptr.p, A.sw.p, col.p, A.map.p, wide.p);
   ELFEL_LAUNCH_CHECK(c);
-  int hw = 0;
-  ELFEL_CUDA(c, cudaMemcpyAsync(&hw, wide.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  const int spb = run_spb_grid(c, nsl);
+  const unsigned ngb = (unsigned)((nsl + spb - 1) / spb);
+  ELFEL_TRY(S->run_halo.alloc(c, ngb));
+  if (nu <= kRunGridRows) {
+    block_halo_k<<<ngb, 512, 0, c->stream>>>(nsl, A.sptr.p, spb, col.p, S->run_halo.p, wide.p + 3);
+    ELFEL_LAUNCH_CHECK(c);
+  }
+  int hw[4] = {0, 0, 0, 0};
+  ELFEL_CUDA(c, cudaMemcpyAsync(hw, wide.p, sizeof(hw), cudaMemcpyDeviceToHost, c->stream));
   ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
+  S->run_entries[0] = hw[1];
+  S->run_entries[1] = hw[2];
+  S->run_neighbours = hw[3] >= 1 && hw[3] <= 32;
   wide.release(c);
   iperm.release(c);
-  if (!hw) {
+  if (!hw[0]) {
     A.d16 = 1;
     ELFEL_TRY(A.dcol.alloc(c, np));
     sell_delta_k<<<grid_for(nsl, 8, (int64_t)c->sm_count * 16), 256, 0, c->stream>>>(A.nnz_pad, nu, A.sptr.p, nsl,
@@ -871,6 +920,8 @@ int build_solver(elfel_sysmat* m, int64_t nu) {
   ELFEL_TRY(S->flags.alloc(c, F_COUNT));
   ELFEL_TRY(S->red.alloc(c, (size_t)3 * kMaxRedBlocks * 4));
   ELFEL_TRY(S->tickets.alloc(c, 4));
+  ELFEL_TRY(S->run_slots.alloc(c, (size_t)2 * 3 * kRunMaxBlocks));
+  ELFEL_TRY(S->run_bar.alloc(c, kRunWords));
   ELFEL_CUDA(c, cudaMemsetAsync(S->tickets.p, 0, sizeof(unsigned) * 4, c->stream));
   ELFEL_CUDA(c, cudaMemsetAsync(S->scal.p, 0, sizeof(double) * S_COUNT, c->stream));
   ELFEL_CUDA(c, cudaMemsetAsync(S->flags.p, 0, sizeof(int) * F_COUNT, c->stream));
@@ -982,6 +1033,17 @@ static int set_scal(Ctx* c, SolverData* S, int idx, double v) {
   return ELFEL_OK;
 }
 
+// A one-launch run of iterations was launched: its flags, and an error if a
+// wait inside it ran out.
+static int read_run(Ctx* c, SolverData* S, const RunPlan& P, int* h) {
+  unsigned bar[2] = {0, 0};
+  if (!P.cluster)
+    ELFEL_CUDA(c, cudaMemcpyAsync(bar, S->run_bar.p, sizeof(bar), cudaMemcpyDeviceToHost, c->stream));
+  ELFEL_TRY(read_flags(c, S, h));
+  if (bar[1]) return fail(c, ELFEL_ERR_TIMEOUT, "solve: a barrier of the iteration kernel timed out");
+  return ELFEL_OK;
+}
+
 // Capture kGraphIters iterations of a kernel sequence into an executable graph.
 template <typename F>
 static int capture(Ctx* c, cudaGraphExec_t* out, F&& body) {
@@ -1027,7 +1089,25 @@ int solution_residual(elfel_sysmat* m) {
 }
 
 // ------------------------------------------------------------------ drivers
-static int run_pcg64(elfel_sysmat* m, int maxit, elfel_solve_stats* st) {
+// solution_residual(), its ||b - K x||^2 in *rr, and whether elfel_solve calls
+// that converged.  The drivers ask it before they stop: the residual of the
+// permuted system, added in another order, may pass by a hair where this one
+// does not.
+static int residual_converged(elfel_sysmat* m, double rtol, double* rr, bool* conv) {
+  Ctx* c = &m->h->c;
+  SolverData* S = m->solver;
+  ELFEL_TRY(solution_residual(m));
+  double bn2 = 0.0;
+  ELFEL_CUDA(c, cudaMemcpyAsync(rr, S->scal.p + S_RR, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  ELFEL_CUDA(c, cudaMemcpyAsync(&bn2, S->scal.p + S_BN2, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
+  *conv = sqrt(*rr / bn2) <= rtol;
+  return ELFEL_OK;
+}
+
+// rr: ||b - K x||^2 of the solution in S->xo64 when the driver has formed it
+// (else negative), as solution_residual leaves it.
+static int run_pcg64(elfel_sysmat* m, double rtol, int maxit, elfel_solve_stats* st, double* rr) {
   Ctx* c = &m->h->c;
   SolverData* S = m->solver;
   const int64_t nu = S->nu;
@@ -1039,7 +1119,8 @@ static int run_pcg64(elfel_sysmat* m, int maxit, elfel_solve_stats* st) {
   cg_start_k<double><<<vg, kBlk, 0, c->stream>>>(nu, S->r64.p, S->z64.p, S->p64.p, S->dinv64.p, red_area(S, 0),
                                                  S->scal.p, S->flags.p, 1, 1.0);
   ELFEL_LAUNCH_CHECK(c);
-  ELFEL_TRY(capture(c, &S->g_pcg64, [&]() {
+  const RunPlan run = run_plan(c, S, sizeof(double), 5);
+  if (!run.blocks) ELFEL_TRY(capture(c, &S->g_pcg64, [&]() {
     launch_cg_spmv<double, false, false>(c, S, S->A.v64.p, S->p64.p, S->q64.p, nullptr, red_area(S, 0), S_PQ);
     launch_pdl(cg_update_k<double, false>, vg, kBlk, c->stream, nu, S->x64.p, S->r64.p, S->p64.p, S->q64.p, S->z64.p,
                S->dinv64.p, red_area(S, 1), S->scal.p, S->flags.p);
@@ -1051,19 +1132,24 @@ static int run_pcg64(elfel_sysmat* m, int maxit, elfel_solve_stats* st) {
   // CG restarts from it.
   int replacements = 0;
   while (true) {
-    ELFEL_CUDA(c, cudaGraphLaunch(S->g_pcg64, c->stream));
-    ELFEL_TRY(read_flags(c, S, hf));
+    if (run.blocks) {
+      ELFEL_TRY(run_cg64(c, S, run));
+      ELFEL_TRY(read_run(c, S, run, hf));
+    } else {
+      ELFEL_CUDA(c, cudaGraphLaunch(S->g_pcg64, c->stream));
+      ELFEL_TRY(read_flags(c, S, hf));
+    }
     if (!hf[F_DONE]) continue;
     if (!hf[F_CONV] || hf[F_ITER] >= maxit || replacements >= 50) break;
+    bool conv = false;
+    ELFEL_TRY(residual_converged(m, rtol, rr, &conv));
+    if (conv) break;
     ELFEL_TRY(launch_sell_resid(c, S, S->x64.p, S->b64.p, S->r64.p, red_area(S, 2), S_RR));
-    double hsc[S_COUNT];
-    ELFEL_CUDA(c, cudaMemcpyAsync(hsc, S->scal.p, sizeof(hsc), cudaMemcpyDeviceToHost, c->stream));
-    ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
-    if (hsc[S_RR] <= hsc[S_TOL2] * hsc[S_BN2]) break;
     ++replacements;
     if (c->trace)
       fprintf(stderr, "[elfel pcg64] it %d: true residual %.3e above the recurrence's; restart\n", hf[F_ITER],
-              sqrt(hsc[S_RR] / hsc[S_BN2]));
+              sqrt(*rr));
+    *rr = -1.0;
     hf[F_DONE] = 0;
     hf[F_CONV] = 0;
     ELFEL_CUDA(c, cudaMemcpyAsync(S->flags.p, hf, sizeof(hf), cudaMemcpyHostToDevice, c->stream));
@@ -1076,7 +1162,7 @@ static int run_pcg64(elfel_sysmat* m, int maxit, elfel_solve_stats* st) {
   return ELFEL_OK;
 }
 
-static int run_pcg32(elfel_sysmat* m, int maxit, elfel_solve_stats* st) {
+static int run_pcg32(elfel_sysmat* m, double rtol, int maxit, elfel_solve_stats* st, double* rr) {
   Ctx* c = &m->h->c;
   SolverData* S = m->solver;
   const int64_t nu = S->nu;
@@ -1099,18 +1185,24 @@ static int run_pcg32(elfel_sysmat* m, int maxit, elfel_solve_stats* st) {
   cg_start_k<float><<<vg, kBlk, 0, c->stream>>>(nu, S->r32.p, S->z32.p, S->p32.p, S->dinv32.p, red_area(S, 0),
                                                 S->scal.p, S->flags.p, 1, 1.0f);
   ELFEL_LAUNCH_CHECK(c);
-  ELFEL_TRY(capture(c, &S->g_pcg32, [&]() {
+  const RunPlan run = run_plan(c, S, sizeof(float), 5);
+  if (!run.blocks) ELFEL_TRY(capture(c, &S->g_pcg32, [&]() {
     launch_cg_spmv<float, true, true>(c, S, S->A.v32.p, S->p32.p, S->q32.p, S->r32.p, red_area(S, 0), S_PQ);
     launch_pdl(cg_update_k<float, true>, vg, kBlk, c->stream, nu, S->xa32.p, S->r32.p, S->p32.p, S->q32.p, S->z32.p,
                S->dinv32.p, red_area(S, 1), S->scal.p, S->flags.p);
     launch_pdl(cg_p_k<float>, vg, kBlk, c->stream, nu, S->p32.p, S->z32.p, S->scal.p, S->flags.p);
   }));
-  int refinements = 0;
+  int refinements = 0, late = 0;
   int launches = 0;
   double hsc[S_COUNT];
   while (true) {
-    ELFEL_CUDA(c, cudaGraphLaunch(S->g_pcg32, c->stream));
-    ELFEL_TRY(read_flags(c, S, hf));
+    if (run.blocks) {
+      ELFEL_TRY(run_cg32(c, S, run));
+      ELFEL_TRY(read_run(c, S, run, hf));
+    } else {
+      ELFEL_CUDA(c, cudaGraphLaunch(S->g_pcg32, c->stream));
+      ELFEL_TRY(read_flags(c, S, hf));
+    }
     ++launches;
     if (c->trace && (launches % 256) == 0) {
       ELFEL_CUDA(c, cudaMemcpyAsync(hsc, S->scal.p, sizeof(hsc), cudaMemcpyDeviceToHost, c->stream));
@@ -1137,13 +1229,13 @@ static int run_pcg32(elfel_sysmat* m, int maxit, elfel_solve_stats* st) {
       fprintf(stderr, "[elfel pcg32] it %d replace %d: recurrence %.3e true %.3e (rel %.3e) brk %d restart %d\n",
               hf[F_ITER], refinements, sqrt(rr_rec), sqrt(hsc[S_RR]), sqrt(hsc[S_RR] / hsc[S_BN2]), hf[F_BRK],
               restart);
-    if (!(hsc[S_RR] > 0.0)) {  // exact solution
-      hf[F_CONV] = 1;
-      break;
-    }
-    if (conv || hf[F_ITER] >= maxit) {
-      hf[F_CONV] = conv ? 1 : 0;
-      break;
+    if (!(hsc[S_RR] > 0.0)) break;  // exact solution
+    if (hf[F_ITER] >= maxit) break;
+    if (conv) {
+      bool all = false;
+      ELFEL_TRY(residual_converged(m, rtol, rr, &all));
+      if (all || ++late >= 50) break;
+      *rr = -1.0;
     }
     if (hf[F_BRK]) {
       int z = 0;
@@ -1162,10 +1254,19 @@ static int run_pcg32(elfel_sysmat* m, int maxit, elfel_solve_stats* st) {
   return ELFEL_OK;
 }
 
-// MINRES on A x = b (precision T, permuted order).
+static int run_mr(Ctx* c, SolverData* S, const RunPlan& P, double* x, double* const* h) {
+  return run_mr64(c, S, P, x, h[3], h[0], h[2], h[6], h[8]);
+}
+static int run_mr(Ctx* c, SolverData* S, const RunPlan& P, float* x, float* const* h) {
+  return run_mr32(c, S, P, x, h[3], h[0], h[2], h[6], h[8]);
+}
+
+// MINRES on A x = b (precision T, permuted order).  dp, hp: the nine
+// three-term buffers (v, z, w) as a device and as a host table.
 template <typename T>
-static int run_minres(Ctx* c, SolverData* S, const T* v, const T* minv, const T* b, T* x, T* const* vb, T* const* zb,
-                      T* const* wb, T* q, double rtol, int maxit, cudaGraphExec_t* graph, int* iters, int* conv) {
+static int run_minres(Ctx* c, SolverData* S, const T* v, const T* minv, const T* b, T* x, T* const* dp, T* const* hp,
+                      T* q, double rtol, int maxit, cudaGraphExec_t* graph, int* iters, int* conv) {
+  T *const *vb = dp, *const *zb = dp + 3, *const *wb = dp + 6;
   const int64_t nu = S->nu;
   const unsigned vg = vec_grid(nu);
   int hf[F_COUNT] = {0, 0, 0, maxit, 0, 0, 0};
@@ -1174,15 +1275,21 @@ static int run_minres(Ctx* c, SolverData* S, const T* v, const T* minv, const T*
   mr_start_k<T><<<vg, kBlk, 0, c->stream>>>(nu, b, vb, zb, wb, minv, x, red_area(S, 0), S->scal.p, S->flags.p);
   scale_k<T><<<vg, kBlk, 0, c->stream>>>(nu, zb, S->scal.p);
   ELFEL_LAUNCH_CHECK(c);
-  ELFEL_TRY(capture(c, graph, [&]() {
+  const RunPlan run = run_plan(c, S, sizeof(T), 8);
+  if (!run.blocks) ELFEL_TRY(capture(c, graph, [&]() {
     launch_mr_spmv<T>(c, S, v, zb, q, red_area(S, 0));
     mr_vec_k<T><<<vg, kBlk, 0, c->stream>>>(nu, q, vb, zb, minv, red_area(S, 1), S->scal.p, S->flags.p);
     mr_upd_k<T><<<vg, kBlk, 0, c->stream>>>(nu, zb, wb, x, S->scal.p, S->flags.p);
     mr_tail_k<<<1, 1, 0, c->stream>>>(S->scal.p, S->flags.p);
   }));
   while (true) {
-    ELFEL_CUDA(c, cudaGraphLaunch(*graph, c->stream));
-    ELFEL_TRY(read_flags(c, S, hf));
+    if (run.blocks) {
+      ELFEL_TRY(run_mr(c, S, run, x, hp));
+      ELFEL_TRY(read_run(c, S, run, hf));
+    } else {
+      ELFEL_CUDA(c, cudaGraphLaunch(*graph, c->stream));
+      ELFEL_TRY(read_flags(c, S, hf));
+    }
     if (hf[F_DONE]) break;
   }
   *iters = hf[F_ITER];
@@ -1232,15 +1339,16 @@ extern "C" int elfel_solve(elfel_sysmat* m, const double* Fh, double* T, int64_t
   }
   ELFEL_TRY(set_scal(c, S, S_DELTA, delta));
   int rc = ELFEL_OK;
+  double rr = -1.0;
   if (bn2 == 0.0) {
     ELFEL_CUDA(c, cudaMemsetAsync(S->x64.p, 0, sizeof(double) * nu, c->stream));
     st.converged = 1;
   } else if (method == ELFEL_PCG64) {
     Phase ph(c, "pcg64");
-    rc = run_pcg64(m, maxit, &st);
+    rc = run_pcg64(m, rtol, maxit, &st, &rr);
   } else if (method == ELFEL_PCG32_IR) {
     Phase ph(c, "pcg32_ir");
-    rc = run_pcg32(m, maxit, &st);
+    rc = run_pcg32(m, rtol, maxit, &st, &rr);
   } else if (method == ELFEL_MINRES64) {
     Phase ph(c, "minres64");
     for (int i = 0; i < 3; ++i) {
@@ -1257,8 +1365,8 @@ extern "C" int elfel_solve(elfel_sysmat* m, const double* Fh, double* T, int64_t
       S->g_minres64 = nullptr;
     }
     int it = 0, conv = 0;
-    rc = run_minres<double>(c, S, S->A.v64.p, S->dinv64.p, S->b64.p, S->x64.p, dptr.p, dptr.p + 3, dptr.p + 6,
-                            S->q64.p, rtol, maxit, &S->g_minres64, &it, &conv);
+    rc = run_minres<double>(c, S, S->A.v64.p, S->dinv64.p, S->b64.p, S->x64.p, dptr.p, hp, S->q64.p, rtol, maxit,
+                            &S->g_minres64, &it, &conv);
     ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
     dptr.release(c);
     st.iterations = it;
@@ -1281,26 +1389,26 @@ extern "C" int elfel_solve(elfel_sysmat* m, const double* Fh, double* T, int64_t
     const unsigned vg = vec_grid(nu);
     ELFEL_CUDA(c, cudaMemsetAsync(S->x64.p, 0, sizeof(double) * nu, c->stream));
     ELFEL_CUDA(c, cudaMemcpyAsync(S->r64.p, S->b64.p, sizeof(double) * nu, cudaMemcpyDeviceToDevice, c->stream));
-    double rr = bn2;
+    double r2 = bn2;
     int total = 0, outer = 0;
     const double inner_tol = 1e-5;
     while (true) {
-      const double s = sqrt(rr);  // inner solve on the unit-norm residual
+      const double s = sqrt(r2);  // inner solve on the unit-norm residual
       if (!(s > 0.0)) break;
       demote_k<<<vg, kBlk, 0, c->stream>>>(nu, S->r64.p, S->b32.p, 1.0 / s);
       int it = 0, conv = 0;
-      rc = run_minres<float>(c, S, S->A.v32.p, S->dinv32.p, S->b32.p, S->x32.p, dptr.p, dptr.p + 3, dptr.p + 6,
-                             S->q32.p, inner_tol, maxit - total, &S->g_minres32, &it, &conv);
+      rc = run_minres<float>(c, S, S->A.v32.p, S->dinv32.p, S->b32.p, S->x32.p, dptr.p, hp, S->q32.p, inner_tol,
+                             maxit - total, &S->g_minres32, &it, &conv);
       if (rc != ELFEL_OK) break;
       total += it;
       ++outer;
       add_scaled_k<<<vg, kBlk, 0, c->stream>>>(nu, S->x64.p, S->x32.p, s);
       ELFEL_TRY(launch_sell_resid(c, S, S->x64.p, S->b64.p, S->r64.p, red_area(S, 2), S_RR));
-      ELFEL_CUDA(c, cudaMemcpyAsync(&rr, S->scal.p + S_RR, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+      ELFEL_CUDA(c, cudaMemcpyAsync(&r2, S->scal.p + S_RR, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
       ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
       if (c->trace)
-        fprintf(stderr, "[elfel minres32] outer %d inner %d rel %.3e\n", outer, it, sqrt(rr / bn2));
-      if (rr <= rtol * rtol * bn2 || total >= maxit || outer >= 100) break;
+        fprintf(stderr, "[elfel minres32] outer %d inner %d rel %.3e\n", outer, it, sqrt(r2 / bn2));
+      if (r2 <= rtol * rtol * bn2 || total >= maxit || outer >= 100) break;
     }
     dptr.release(c);
     st.iterations = total;
@@ -1308,9 +1416,10 @@ extern "C" int elfel_solve(elfel_sysmat* m, const double* Fh, double* T, int64_t
   }
   if (rc != ELFEL_OK) return rc;
   // solution back to the original order; final FP64 residual there
-  ELFEL_TRY(solution_residual(m));
-  double rr = 0.0;
-  ELFEL_CUDA(c, cudaMemcpyAsync(&rr, S->scal.p + S_RR, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  if (rr < 0.0) {
+    ELFEL_TRY(solution_residual(m));
+    ELFEL_CUDA(c, cudaMemcpyAsync(&rr, S->scal.p + S_RR, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  }
   ELFEL_CUDA(c, cudaMemcpyAsync(T, S->xo64.p, sizeof(double) * nu, cudaMemcpyDeviceToHost, c->stream));
   ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
   st.relres = bn2 > 0.0 ? sqrt(rr / bn2) : 0.0;

@@ -93,6 +93,13 @@ struct SolverData {
   DBuf<int> flags;
   DBuf<double> red;  // 3 reduction areas
   DBuf<unsigned> tickets;
+  // one-launch iterations (krylov.cu): the largest block's stored entries for
+  // the cluster and the grid division; the grid group's memory (RunGroup)
+  int run_entries[2] = {0, 0};
+  int run_neighbours = 0;
+  DBuf<double> run_slots;
+  DBuf<unsigned> run_bar;
+  DBuf<int2> run_halo;
   cudaGraphExec_t g_pcg64 = nullptr, g_pcg32 = nullptr, g_minres64 = nullptr, g_minres32 = nullptr;
   SellView view() const {
     return SellView{A.nrows, A.nslices, A.sptr.p, A.sw.p, A.d16 ? A.dcol.p : nullptr, A.d16 ? nullptr : A.col.p};
@@ -103,7 +110,7 @@ struct SolverData {
       b->release(c);
     for (DBuf<float>* b : {&dinv32, &r32, &p32, &q32, &z32, &xa32, &zz32, &b32, &x32}) b->release(c);
     for (int i = 0; i < 3; ++i) { v64[i].release(c); w64[i].release(c); v32[i].release(c); w32[i].release(c); }
-    scal.release(c); flags.release(c); red.release(c); tickets.release(c);
+    scal.release(c); flags.release(c); red.release(c); tickets.release(c); run_slots.release(c); run_bar.release(c); run_halo.release(c);
     for (cudaGraphExec_t* g : {&g_pcg64, &g_pcg32, &g_minres64, &g_minres32})
       if (*g) { cudaGraphExecDestroy(*g); *g = nullptr; }
   }
