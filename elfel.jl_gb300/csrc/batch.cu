@@ -19,6 +19,10 @@
 // launch, on how tiles are grouped into items or on the grid size, so a
 // system's iterates are bit-identical alone and in any mix.
 //
+// Small systems do not take part in that: each has a thread-block cluster of
+// its own, which runs its whole state machine (batch_run.cu), side by side
+// with the graphs of the large ones.
+//
 // Methods.  ELFEL_PCG64: Jacobi PCG in FP64.  ELFEL_PCG32_IR: Jacobi CG on the
 // FP32 difference-form copy of K with FP64 residual replacement (reliable
 // updates), flexible step and Polak-Ribiere beta, as the one-system driver;
@@ -36,34 +40,9 @@
 #include <map>
 #include <vector>
 
-#include "solve.cuh"
+#include "batch.cuh"
 
 namespace elfel {
-
-// per-system scalars
-enum { B_RZ = 0, B_PQ, B_ALPHA, B_BETA, B_RR, B_RMAX, B_DELTA, B_TOL2, B_BN2, B_SCALE, B_RRT, B_RREC, B_COUNT = 16 };
-// per-system ints
-enum { I_MODE = 0, I_ITER, I_MAXIT, I_BRK, I_RESTART, I_CONV, I_REPL, I_COUNT = 8 };
-enum { M_IDLE = 0, M_CG, M_FOLD, M_RESTART, M_STARTED, M_DONE };
-
-// One system as the batched kernels see it.
-struct BSys {
-  SellView A;
-  const float* v32;
-  const double* v64;
-  const float* dinv32;
-  const double* dinv64;
-  float *x32, *r32, *z32, *p32, *q32;
-  double *x64, *r64, *z64, *p64, *q64;
-  const double* b64;
-  int64_t ntiles;
-  int sl, pad_;        // row groups of kBlk per tile (1, 4 or 8: fixed per system by its size)
-  double* part;        // ntiles x 4 partial sums
-  unsigned* ticket;    // work items finished in the current kernel
-  const int* nitems;   // work items of this system in the current map
-  double* sc;          // B_COUNT scalars
-  int* st;             // I_COUNT ints
-};
 
 constexpr int kItemMax = 32;  // tiles per work item (bounds the shared staging)
 constexpr int kWarps = kBlk / 32;
@@ -677,9 +656,17 @@ struct Slot {
   int state = 0;  // 0 free, 1 active, 2 done (result not taken)
   int64_t nu = 0, ntiles = 0;
   double rtol = 0.0;
+  BRunPlan run;  // run.blocks > 0: iterated in a cluster of its own
   DBuf<double> part;
   std::chrono::steady_clock::time_point t_add, t_done;
 };
+
+// The active systems of one cluster size: n slots from off in the run list.
+struct RunClass {
+  int blocks = 0, off = 0, n = 0;
+  size_t smem = 0;
+};
+constexpr int kRunClasses = 5;  // clusters of 1, 2, 4, 8, 16 blocks
 
 // grid of one configuration: blocks per SM of the spmv and of the vector kernels
 struct GridCfg {
@@ -702,7 +689,11 @@ struct elfel_batch {
   DBuf<int4> items;
   int64_t items_cap = 0;
   DBuf<int> ntot;
-  DBuf<int> act;  // off[cap + 1], slot[cap], ntiles[cap]
+  DBuf<int> act;  // off[cap + 1], slot[cap], ntiles[cap], run list[cap]
+  RunClass run[kRunClasses];
+  int nrun = 0;  // active systems in clusters
+  cudaStream_t run_stream[kRunClasses] = {};
+  cudaEvent_t run_fork = nullptr, run_join[kRunClasses] = {};
   int64_t total_tiles = 0, total_items = 0;
   bool map_dirty = false;
   std::vector<int> hst;
@@ -769,7 +760,7 @@ int rebuild_map(elfel_batch* b) {
   std::vector<int> sl, ntl;
   int64_t tiles = 0;
   for (int i = 0; i < b->cap; ++i)
-    if (b->slots[i].state == 1) {
+    if (b->slots[i].state == 1 && !b->slots[i].run.blocks) {
       sl.push_back(i);
       ntl.push_back((int)b->slots[i].ntiles);
       tiles += b->slots[i].ntiles;
@@ -777,7 +768,22 @@ int rebuild_map(elfel_batch* b) {
   const int nact = (int)sl.size();
   const int64_t target = 2LL * c->sm_count * std::max(b->occ_spmv, b->occ_vec);
   const int item_tiles = (int)std::min<int64_t>(kItemMax, std::max<int64_t>(1, tiles / std::max<int64_t>(target, 1)));
-  std::vector<int> h(3 * (size_t)b->cap + 1, 0);
+  std::vector<int> h(4 * (size_t)b->cap + 1, 0);
+  int* rl = h.data() + 3 * (size_t)b->cap + 1;
+  b->nrun = 0;
+  for (int k = 0; k < kRunClasses; ++k) {
+    RunClass& R = b->run[k];
+    R = RunClass();
+    R.blocks = 1 << k;
+    R.off = b->nrun;
+    for (int i = 0; i < b->cap; ++i) {
+      const Slot& s = b->slots[i];
+      if (s.state != 1 || s.run.blocks != R.blocks) continue;
+      rl[b->nrun++] = i;
+      ++R.n;
+      R.smem = std::max(R.smem, s.run.smem);
+    }
+  }
   int64_t nit = 0;
   for (int k = 0; k < nact; ++k) {
     h[k] = (int)nit;
@@ -802,6 +808,45 @@ int rebuild_map(elfel_batch* b) {
                          b->ntot.p, b->nitems.p);
   ELFEL_LAUNCH_CHECK(c);
   b->map_dirty = false;
+  return ELFEL_OK;
+}
+
+// The cluster systems' iterations of a step, one launch per cluster size on
+// streams of their own between the events fork and join, so that the sizes
+// and the graphs of the large systems run side by side.
+int run_clusters(elfel_batch* b, int graphs) {
+  Ctx* c = ctx_of(b);
+  int used = 0;
+  for (const RunClass& R : b->run) used += R.n > 0;
+  const bool alone = used == 1 && b->total_tiles == 0;
+  if (!alone && !b->run_fork) ELFEL_CUDA(c, cudaEventCreateWithFlags(&b->run_fork, cudaEventDisableTiming));
+  if (!alone) ELFEL_CUDA(c, cudaEventRecord(b->run_fork, c->stream));
+  const int* list = b->act.p + 3 * (size_t)b->cap + 1;
+  for (int k = kRunClasses - 1; k >= 0; --k) {  // the largest clusters first
+    const RunClass& R = b->run[k];
+    if (!R.n) continue;
+    cudaStream_t st = c->stream;
+    if (!alone) {
+      if (!b->run_stream[k]) {
+        ELFEL_CUDA(c, cudaStreamCreateWithFlags(&b->run_stream[k], cudaStreamNonBlocking));
+        ELFEL_CUDA(c, cudaEventCreateWithFlags(&b->run_join[k], cudaEventDisableTiming));
+      }
+      st = b->run_stream[k];
+      ELFEL_CUDA(c, cudaStreamWaitEvent(st, b->run_fork, 0));
+    }
+    ELFEL_TRY(batch_run_launch(c, st, b->method == ELFEL_PCG32_IR, b->sys.p, list + R.off, R.n, R.blocks, R.smem,
+                               kBRunIters * graphs));
+    if (!alone) ELFEL_CUDA(c, cudaEventRecord(b->run_join[k], st));
+    b->launches++;
+    b->kernel_launches++;
+  }
+  return ELFEL_OK;
+}
+
+int join_clusters(elfel_batch* b) {
+  Ctx* c = ctx_of(b);
+  for (int k = 0; k < kRunClasses; ++k)
+    if (b->run[k].n && b->run_join[k]) ELFEL_CUDA(c, cudaStreamWaitEvent(c->stream, b->run_join[k], 0));
   return ELFEL_OK;
 }
 
@@ -942,6 +987,10 @@ int batch_add_dev(elfel_batch* b, elfel_sysmat* m, const double* F, const double
   d.nitems = b->nitems.p + k;
   d.sc = b->sc.p + (size_t)k * B_COUNT;
   d.st = b->st.p + (size_t)k * I_COUNT;
+  s.run = batch_run_plan(c, S, b->method == ELFEL_PCG32_IR);
+  d.spb = s.run.spb;
+  d.ms = s.run.ms;
+  d.max_entries = s.run.max_entries;
   double hsc[B_COUNT] = {0};
   int hst[I_COUNT] = {0};
   hsc[B_TOL2] = rtol * rtol;
@@ -982,6 +1031,7 @@ int batch_step(elfel_batch* b, int32_t graphs, int32_t* active) {
   Ctx* c = ctx_of(b);
   cudaSetDevice(c->device);
   if (b->map_dirty) ELFEL_TRY(rebuild_map(b));
+  if (b->nrun) ELFEL_TRY(run_clusters(b, graphs));
   for (int gi = 0; b->persist && gi < graphs && b->total_tiles > 0; ++gi) {
     // one cooperative launch of iters iterations (all blocks resident)
     const BSys* sy = b->sys.p;
@@ -1018,6 +1068,7 @@ int batch_step(elfel_batch* b, int32_t graphs, int32_t* active) {
     b->launches++;
     b->kernel_launches += 3LL * b->iters;
   }
+  if (b->nrun) ELFEL_TRY(join_clusters(b));
   ELFEL_TRY(read_states(b));
   if (b->map_dirty) ELFEL_TRY(rebuild_map(b));
   int n = 0;
@@ -1096,7 +1147,7 @@ extern "C" int elfel_batch_create(elfel_ctx* h, int32_t method, int32_t capacity
   if ((rc = b->sys.alloc(c, (size_t)capacity)) || (rc = b->sc.alloc(c, (size_t)capacity * B_COUNT)) ||
       (rc = b->st.alloc(c, (size_t)capacity * I_COUNT)) || (rc = b->tickets.alloc(c, (size_t)capacity)) ||
       (rc = b->nitems.alloc(c, (size_t)capacity)) || (rc = b->ntot.alloc(c, 1)) ||
-      (rc = b->act.alloc(c, 3 * (size_t)capacity + 1))) {
+      (rc = b->act.alloc(c, 4 * (size_t)capacity + 1))) {
     delete b;
     return rc;
   }
@@ -1158,6 +1209,11 @@ extern "C" int elfel_batch_destroy(elfel_batch* b) {
     if (s.m) s.m->busy = 0;
   }
   drop_graphs(b);
+  for (int k = 0; k < kRunClasses; ++k) {
+    if (b->run_stream[k]) cudaStreamDestroy(b->run_stream[k]);
+    if (b->run_join[k]) cudaEventDestroy(b->run_join[k]);
+  }
+  if (b->run_fork) cudaEventDestroy(b->run_fork);
   b->gbar.release(c);
   b->sys.release(c);
   b->sc.release(c);

@@ -1,0 +1,307 @@
+// Small systems of a batch, each iterated by a thread-block cluster of its own:
+// the CG loop of krylov.cu with the whole state machine of the batched engine
+// (batch.cu) inside the kernel, kBRunIters iterations a launch.
+//
+// What bounds it.  In the graphs of three kernels an iteration of a batch of
+// small systems cost 21 us, the latency of three kernels, however little work
+// it held.  A cluster needs no grid-wide barrier: its systems' blocks meet at
+// the hardware cluster barrier (0.2-0.3 us), and the clusters of a launch run
+// side by side and independently.  A system takes 1 to 16 blocks by its size
+// alone, at most 2048 rows a block in FP32 (the vectors, 41 KB, and the
+// matrix, about 140 KB for quadratic triangles, fit a block's shared memory),
+// so that a burst of requests spreads over the SMs, and its sums do not depend
+// on the mix: the same bits alone, in any mix and whenever it joins.
+#include <type_traits>
+
+#include "batch.cuh"
+#include "krylov_dev.cuh"
+
+namespace elfel {
+
+namespace {
+
+// One sum over the cluster (all threads; the totals are valid in warp 0).
+template <int NV, typename T>
+__device__ __forceinline__ void cluster_sum(ClusterGroup& grp, T (&v)[NV], double* part, double* wsum, double (&t)[NV]) {
+  const int wid = threadIdx.x >> 5;
+  block_sums<NV>(v, part, wsum, t);
+  if (wid == 0) grp.publish(t);
+  grp.arrive(wid);
+  grp.wait(wid);
+  grp.collect(wid, wsum, t);
+}
+
+template <bool IR, bool D16, bool MS>
+__device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint8_t* smem, RunMsg& msg, int iters) {
+  typedef typename std::conditional<IR, float, double>::type T;
+  const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
+  double* part = reinterpret_cast<double*>(smem);
+  double* wsum = part + 3 * kRT;
+  T* sx = reinterpret_cast<T*>(part + kRunPart);
+  const int ld = S.spb * 32;
+  T *sr = sx + ld, *sp = sr + ld, *sq = sp + ld, *sd = sq + ld;
+  T* const gx = IR ? (T*)S.x32 : (T*)S.x64;
+  T* const gr = IR ? (T*)S.r32 : (T*)S.r64;
+  T* const gp = IR ? (T*)S.p32 : (T*)S.p64;
+  const T* const gd = IR ? (const T*)S.dinv32 : (const T*)S.dinv64;
+  const RunRows<T, D16, MS> R(S.A, IR ? (const T*)S.v32 : (const T*)S.v64, grp.rank, S.spb, S.max_entries,
+                              reinterpret_cast<int2*>(sd + ld));
+  const int64_t r0 = R.row0;
+  for (int i = tid; i < R.nloc; i += kRT) {
+    sx[i] = gx[r0 + i];
+    sr[i] = gr[r0 + i];
+    sp[i] = gp[r0 + i];
+    sd[i] = gd[r0 + i];
+  }
+  // the system's scalars (warp 0 uses them)
+  const double scale = S.sc[B_SCALE], tol = S.sc[B_TOL2], bn2 = S.sc[B_BN2];
+  const double thr = IR ? tol : tol * bn2, delta2 = S.sc[B_DELTA] * S.sc[B_DELTA];
+  double rz = S.sc[B_RZ], rr = S.sc[B_RR], rmax2 = S.sc[B_RMAX] * S.sc[B_RMAX], pq = 0.0;
+  double inv_rz = 1.0 / rz, low2 = delta2 * rmax2;
+  int it = S.st[I_ITER], brk = S.st[I_BRK], repl = S.st[I_REPL], conv = 0, mode = M_CG;
+  const int maxit = S.st[I_MAXIT];
+  __syncthreads();
+
+  for (int k = 0; k < iters; ++k) {
+    // q = A p; p.q (and r.p) -> alpha
+    constexpr int N1 = IR ? 2 : 1;
+    T d1[N1] = {};
+    for (int n = 0; n * kRW < R.nsl; ++n) {
+      const int s = R.slice(wid, n);
+      const int i = s * 32 + lane;
+      if (i < R.nloc) {
+        const T pi = sp[i];
+        const T acc = R.template row<IR, false>(s, i, gp, gp, (T)0, pi);
+        sq[i] = acc;
+        d1[0] += acc * pi;
+        if (IR) d1[N1 - 1] += sr[i] * pi;
+      }
+    }
+    double t1[N1];
+    cluster_sum<N1>(grp, d1, part, wsum, t1);
+    if (wid == 0) {
+      pq = t1[0];
+      const double alpha = pos_finite(pq) ? fast_div(IR ? t1[N1 - 1] : rz, pq, fast_rcp(pq)) : 0.0;
+      if (lane == 0) msg.c[0] = alpha;
+    }
+    __syncthreads();
+    // r -= alpha q, z = D r (kept in q); r.z, r.r (and z.r_old) -> beta
+    constexpr int N2 = IR ? 3 : 2;
+    const T al = (T)msg.c[0];
+    T d2[N2] = {};
+    for (int i = tid; i < R.nloc; i += kRT) {
+      const T ro = sr[i];
+      const T ri = ro - al * sq[i];
+      sr[i] = ri;
+      const T zi = sd[i] * ri;
+      sq[i] = zi;
+      d2[0] += ri * zi;
+      d2[1] += ri * ri;
+      if (IR) d2[N2 - 1] += zi * ro;
+    }
+    double t2[N2];
+    block_sums<N2>(d2, part, wsum, t2);
+    if (wid == 0) grp.publish(t2);
+    grp.arrive(wid);
+    for (int i = tid; i < R.nloc; i += kRT) sx[i] += al * sp[i];
+    if (wid == 0) inv_rz = fast_rcp(rz);
+    grp.wait(wid);
+    grp.collect(wid, wsum, t2);
+    if (wid == 0) {
+      const double beta = (IR ? t2[0] - t2[N2 - 1] : t2[0]) * inv_rz;
+      rz = t2[0];
+      rr = t2[1];
+      ++it;
+      conv = le_pos(rr, thr);
+      const bool bad = !pos_finite(pq) || !finite(rz) || !finite(rr);
+      if (IR) {
+        if (bad) {
+          brk = 1;
+          mode = M_FOLD;
+        } else {
+          if (lt_pos(rmax2, rr)) {
+            rmax2 = rr;
+            low2 = delta2 * rmax2;
+          }
+          if (conv) brk = 2;  // spent directions: restart from p = z
+          if (conv || it >= maxit || lt_pos(rr, low2)) mode = M_FOLD;
+        }
+      } else if (conv && !bad && it < maxit) {
+        mode = M_FOLD;  // the recurrence says converged: check the true residual
+      } else if (conv || bad || it >= maxit) {
+        conv = conv && !bad;
+        mode = M_DONE;
+      }
+      if (lane == 0) {
+        msg.c[0] = beta;
+        msg.stop = mode;
+      }
+    }
+    __syncthreads();
+    mode = msg.stop;
+    if (mode == M_DONE) break;
+    const T be = (T)msg.c[0];
+    for (int i = tid; i < R.nloc; i += kRT) {
+      const T pn = axpy<T>(be, sp[i], sq[i]);
+      sp[i] = pn;
+      if (mode == M_CG) gp[r0 + i] = pn;
+    }
+    if (mode == M_FOLD) {
+      // x64 += s x32 (FP32), then the true residual b - K x64 in FP64
+      for (int i = tid; i < R.nloc; i += kRT) {
+        if (IR) {
+          S.x64[r0 + i] += scale * (double)sx[i];
+          sx[i] = 0;
+        } else {
+          S.x64[r0 + i] = (double)sx[i];
+        }
+      }
+      grp.arrive(wid);
+      grp.wait(wid);
+      double d[1] = {0.0};
+      for (int s = wid; s < R.nsl; s += kRW) {
+        const int i = s * 32 + lane;
+        const double acc = sell_row_resid<D16, true>(S.A, S.v64, S.x64, r0 / 32 + s, lane);
+        if (i < R.nloc) {
+          const double rv = S.b64[r0 + i] - acc;
+          S.r64[r0 + i] = rv;
+          d[0] += rv * rv;
+        }
+      }
+      double t[1];
+      cluster_sum<1>(grp, d, part, wsum, t);
+      if (wid == 0) {
+        const double rrt = t[0];
+        ++repl;
+        conv = (!(rrt > 0.0) && finite(rrt)) || rrt <= tol * bn2;
+        if (conv || !finite(rrt) || it >= maxit || (!IR && repl > 50)) {
+          mode = M_DONE;
+        } else {
+          // FP32: keep the direction unless the recurrence broke down or its
+          // residual drifted far below the true one; FP64: restart
+          const double rrec = rr * scale * scale;
+          const int restart = !IR || brk || !(rrec > 0.0) || !(rrec >= 1e-6 * rrt);
+          brk = 0;
+          mode = restart ? M_RESTART : M_STARTED;
+          rmax2 = IR ? rrt / (scale * scale) : rmax2;
+          low2 = delta2 * rmax2;
+        }
+        if (lane == 0) {
+          msg.c[0] = rrt;
+          msg.stop = mode;
+        }
+      }
+      __syncthreads();
+      mode = msg.stop;
+      if (mode == M_DONE) break;
+      const double inv = 1.0 / scale;
+      T dz[1] = {0};
+      for (int s = wid; s < R.nsl; s += kRW) {
+        const int i = s * 32 + lane;
+        if (i < R.nloc) {
+          const T ri = IR ? (T)(S.r64[r0 + i] * inv) : (T)S.r64[r0 + i];
+          sr[i] = ri;
+          const T zi = sd[i] * ri;
+          const T pi = mode == M_RESTART ? zi : sp[i];
+          sp[i] = pi;
+          gp[r0 + i] = pi;
+          dz[0] += ri * zi;
+        }
+      }
+      double t3[1];
+      cluster_sum<1>(grp, dz, part, wsum, t3);
+      if (wid == 0) rz = t3[0];
+      mode = M_CG;
+      __syncthreads();
+      continue;  // the sum's barrier has made the direction visible
+    }
+    grp.arrive(wid);
+    grp.wait(wid);
+  }
+  __syncthreads();
+  for (int i = tid; i < R.nloc; i += kRT) {
+    gx[r0 + i] = sx[i];
+    gr[r0 + i] = sr[i];
+  }
+  if (grp.rank == 0 && tid == 0) {
+    S.sc[B_RZ] = rz;
+    S.sc[B_RR] = rr;
+    S.sc[B_PQ] = pq;
+    S.sc[B_RMAX] = sqrt(rmax2);
+    S.st[I_ITER] = it;
+    S.st[I_BRK] = brk;
+    S.st[I_REPL] = repl;
+    S.st[I_CONV] = conv;
+    S.st[I_MODE] = mode;
+  }
+}
+
+template <bool IR>
+__global__ void __launch_bounds__(kRT, 1) batch_run_k(const BSys* __restrict__ sys, const int* __restrict__ list,
+                                                     int iters) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ ClusterGroup::Shared gsh;
+  __shared__ RunMsg msg;
+  __shared__ BSys S;
+  ClusterGroup grp(RunGroup(), &gsh);
+  static_assert(sizeof(BSys) % 8 == 0 && sizeof(BSys) / 8 <= kRT, "descriptor staging");
+  if (threadIdx.x < sizeof(BSys) / 8)
+    reinterpret_cast<uint64_t*>(&S)[threadIdx.x] =
+        reinterpret_cast<const uint64_t*>(sys + list[blockIdx.x / grp.n])[threadIdx.x];
+  __syncthreads();
+  if (S.st[I_MODE] == M_CG) {
+    if (S.A.d16) {
+      if (S.ms) batch_run<IR, true, true>(S, grp, smem, msg, iters);
+      else batch_run<IR, true, false>(S, grp, smem, msg, iters);
+    } else {
+      if (S.ms) batch_run<IR, false, true>(S, grp, smem, msg, iters);
+      else batch_run<IR, false, false>(S, grp, smem, msg, iters);
+    }
+  }
+  grp.arrive(0);  // no block leaves while another may still write its shared memory
+  grp.wait(0);
+}
+
+}  // namespace
+
+BRunPlan batch_run_plan(const Ctx* c, const SolverData* S, int ir) {
+  BRunPlan P;
+  if (!c->one_launch || S->nu < 1) return P;
+  const int elem = ir ? 4 : 8;
+  const int spb = run_spb_batch(S->A.nslices, elem);
+  const int entries = S->run_entries[ir ? 2 : 3];
+  const size_t sv = run_smem(spb, elem, 5, 0, S->A.d16), sm = run_smem(spb, elem, 5, entries, S->A.d16);
+  // a system whose matrix does not fit iterates from L2 as long as its rows
+  // are few; larger ones are left to the graphs, which use the whole device
+  if (sv > (size_t)kRunSmem || spb * 32 > (ir ? kRunBatchRows32 : kRunBatchRows64) * 5 / 4) return P;
+  P.ms = sm <= (size_t)kRunSmem;
+  P.spb = spb;
+  P.blocks = 1;
+  while ((int64_t)P.blocks * spb < S->A.nslices) P.blocks *= 2;
+  P.max_entries = entries;
+  P.smem = P.ms ? sm : sv;
+  return P;
+}
+
+int batch_run_launch(Ctx* c, cudaStream_t st, int ir, const BSys* sys, const int* list, int n, int blocks, size_t smem,
+                     int iters) {
+  auto k = ir ? batch_run_k<true> : batch_run_k<false>;
+  ELFEL_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kRunSmem));
+  if (blocks > 8) ELFEL_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)(n * blocks));
+  cfg.blockDim = dim3(kRT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)blocks;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  ELFEL_CUDA(c, cudaLaunchKernelEx(&cfg, k, sys, list, iters));
+  return ELFEL_OK;
+}
+
+}  // namespace elfel

@@ -13,6 +13,8 @@ constexpr int64_t kRunClusterRows64 = 16384, kRunClusterRows32 = 32768;
 // Beyond this no grid group holds the vectors (226 KB of 20 bytes a row, 160 blocks).
 constexpr int64_t kRunGridRows = (int64_t)kRunMaxBlocks * 12000;
 constexpr int64_t kRunTwoRows64 = 65536;  // FP64: two barriers an iteration up to here (cg_run_k)
+// A batched system takes the smallest cluster whose blocks hold this many rows each.
+constexpr int kRunBatchRows32 = 2048, kRunBatchRows64 = 1024;
 constexpr int kRunIters = 4096;     // iterations of one launch at most
 constexpr int kRunSmem = 227 * 1024 - 1024;  // dynamic shared memory of a block (the kernels' static part apart)
 
@@ -68,9 +70,14 @@ struct RunPlan {
 };
 
 // The slices-per-block values whose largest block entry counts build_sell
-// records in SolverData::run_entries: [0] cluster, [1] grid.
+// records in SolverData::run_entries: [0] cluster, [1] grid, and of a batched
+// system [2] FP32, [3] FP64.
 int run_spb_cluster(int64_t nslices);
 int run_spb_grid(const Ctx* c, int64_t nslices);
+int run_spb_batch(int64_t nslices, int elem);
+// Shared memory of a block of spb slices: vecs vectors of elem-byte values
+// and, with entries > 0, that many entries of the matrix.
+size_t run_smem(int spb, int elem, int vecs, int entries, int d16);
 // vecs: vectors of the iteration kept in shared memory (5 for CG, 8 for MINRES).
 RunPlan run_plan(Ctx* c, const SolverData* S, int elem, int vecs);
 

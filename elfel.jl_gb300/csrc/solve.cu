@@ -741,14 +741,17 @@ static Red4 red_area(SolverData* S, int k) {
   return r;
 }
 
-// The division of the slices among the blocks of the one-launch iterations
-// (krylov.cu): out[0], out[1] = the largest number of stored entries in any
-// run of spb0 (cluster), spb1 (grid) consecutive slices.
-__global__ void block_entries_k(int64_t nsl, const int64_t* __restrict__ sptr, int spb0, int spb1, int* out) {
-  for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b * min(spb0, spb1) < nsl;
-       b += (int64_t)gridDim.x * blockDim.x) {
-    if (b * spb0 < nsl) atomicMax(out, (int)(sptr[min((b + 1) * spb0, nsl)] - sptr[b * spb0]));
-    if (b * spb1 < nsl) atomicMax(out + 1, (int)(sptr[min((b + 1) * spb1, nsl)] - sptr[b * spb1]));
+// out[q] = the largest number of stored entries in any run of spb.v[q]
+// consecutive slices (the blocks of the one-launch iterations).
+struct SpbList {
+  int v[4];
+};
+__global__ void block_entries_k(int64_t nsl, const int64_t* __restrict__ sptr, const SpbList spb, int* out) {
+  for (int q = 0; q < 4; ++q) {
+    const int n = spb.v[q];
+    for (int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * n; s < nsl;
+         s += (int64_t)gridDim.x * blockDim.x * n)
+      atomicMax(out + q, (int)(sptr[min(s + n, nsl)] - sptr[s]));
   }
 }
 
@@ -807,9 +810,11 @@ static int build_sell(Ctx* c, SolverData* S) {
   const size_t np = (size_t)(A.nnz_pad > 0 ? A.nnz_pad : 1);
   ELFEL_TRY(col.alloc(c, np));
   ELFEL_TRY(A.map.alloc(c, np));
-  ELFEL_TRY(wide.alloc(c, 4));  // a column delta beyond 16 bits; the largest blocks' entries; the widest halo
-  ELFEL_CUDA(c, cudaMemsetAsync(wide.p, 0, 4 * sizeof(int), c->stream));
-  block_entries_k<<<1, 256, 0, c->stream>>>(nsl, A.sptr.p, run_spb_cluster(nsl), run_spb_grid(c, nsl), wide.p + 1);
+  // a column delta beyond 16 bits; the widest halo; the largest blocks' entries
+  ELFEL_TRY(wide.alloc(c, 6));
+  ELFEL_CUDA(c, cudaMemsetAsync(wide.p, 0, 6 * sizeof(int), c->stream));
+  const SpbList spbs{{run_spb_cluster(nsl), run_spb_grid(c, nsl), run_spb_batch(nsl, 4), run_spb_batch(nsl, 8)}};
+  block_entries_k<<<1, 256, 0, c->stream>>>(nsl, A.sptr.p, spbs, wide.p + 2);
   sell_fill_k<<<grid_for(nsl * 32, 256, (int64_t)c->sm_count * 16), 256, 0, c->stream>>>(
       nu, nsl, S->ff.rowptr.p, S->ff.col.p, S->ff.map.p, A.perm.p, iperm.p, A.sptr.p, A.sw.p, col.p, A.map.p, wide.p);
   ELFEL_LAUNCH_CHECK(c);
@@ -817,15 +822,14 @@ static int build_sell(Ctx* c, SolverData* S) {
   const unsigned ngb = (unsigned)((nsl + spb - 1) / spb);
   ELFEL_TRY(S->run_halo.alloc(c, ngb));
   if (nu <= kRunGridRows) {
-    block_halo_k<<<ngb, 512, 0, c->stream>>>(nsl, A.sptr.p, spb, col.p, S->run_halo.p, wide.p + 3);
+    block_halo_k<<<ngb, 512, 0, c->stream>>>(nsl, A.sptr.p, spb, col.p, S->run_halo.p, wide.p + 1);
     ELFEL_LAUNCH_CHECK(c);
   }
-  int hw[4] = {0, 0, 0, 0};
+  int hw[6] = {0, 0, 0, 0, 0, 0};
   ELFEL_CUDA(c, cudaMemcpyAsync(hw, wide.p, sizeof(hw), cudaMemcpyDeviceToHost, c->stream));
   ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
-  S->run_entries[0] = hw[1];
-  S->run_entries[1] = hw[2];
-  S->run_neighbours = hw[3] >= 1 && hw[3] <= 32;
+  for (int q = 0; q < 4; ++q) S->run_entries[q] = hw[2 + q];
+  S->run_neighbours = hw[1] >= 1 && hw[1] <= 32;
   wide.release(c);
   iperm.release(c);
   if (!hw[0]) {

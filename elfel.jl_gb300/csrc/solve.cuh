@@ -93,9 +93,9 @@ struct SolverData {
   DBuf<int> flags;
   DBuf<double> red;  // 3 reduction areas
   DBuf<unsigned> tickets;
-  // one-launch iterations (krylov.cu): the largest block's stored entries for
-  // the cluster and the grid division; the grid group's memory (RunGroup)
-  int run_entries[2] = {0, 0};
+  // one-launch iterations (krylov.cu): the largest block's stored entries of
+  // each division (run_spb_*); the grid group's memory (RunGroup)
+  int run_entries[4] = {0, 0, 0, 0};
   int run_neighbours = 0;
   DBuf<double> run_slots;
   DBuf<unsigned> run_bar;

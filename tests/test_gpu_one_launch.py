@@ -131,3 +131,40 @@ def test_two_contexts_at_once(E, O, gpu):
     for t in th:
         t.join()
     assert len(errs) == 40 and all(isinstance(e, float) and e <= TOL for e in errs), errs[:4]
+
+
+BATCH = {"pcg32_ir": [1, 33, 2048, 2049, 4097, 8193, 16385, 32768, 40960, 40993],
+         "pcg64": [1, 33, 1024, 1025, 2049, 4097, 8193, 16384, 20480, 20513]}
+
+
+@pytest.mark.parametrize("method", sorted(BATCH))
+def test_batched_clusters(E, O, gpu, method):
+    """Batched systems on both sides of every cluster size (1 to 16 blocks) and
+    beyond the largest, one of them with 32-bit columns: the direct solution
+    within TOL, and the same bits alone and in the mix."""
+    probs = []
+    for i, n in enumerate(BATCH[method] + [36000 if method == "pcg32_ir" else 20000]):
+        A = laplacian(n, shuffle=5 if i == len(BATCH[method]) else None)
+        c = A.tocoo()
+        a = E.start(E.SysmatAssemblerSparse(), n, n)
+        a._chunks.append((c.row.astype(np.int64) + 1, c.col.astype(np.int64) + 1, c.data.astype(np.float64)))
+        E.finish(a)
+        F = np.random.default_rng(n).standard_normal(n)
+        probs.append((A, a, F))
+
+    def run(which):
+        b = E.BatchSolver(method, capacity=len(which))
+        slots = [b.add(probs[i][1], np.zeros(probs[i][0].shape[0]), probs[i][0].shape[0], F=probs[i][2], rtol=1e-11)
+                 for i in which]
+        out = b.run()
+        b.close()
+        return [out[s] for s in slots]
+
+    mixed = run(list(range(len(probs))))
+    for i, (A, a, F) in enumerate(probs):
+        T, st = mixed[i]
+        assert st["converged"] and st["relres"] <= 1e-11
+        T0 = O.solve_lifted(A, F, np.zeros(A.shape[0]), A.shape[0])
+        assert np.linalg.norm(T - T0) <= TOL * np.linalg.norm(T0), A.shape
+        (Ta, sta), = run([i])
+        assert np.array_equal(T, Ta) and st["iterations"] == sta["iterations"], A.shape
