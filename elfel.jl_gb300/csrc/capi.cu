@@ -288,6 +288,14 @@ extern "C" int elfel_sysmat_csc(elfel_sysmat* m, int64_t* colptr, int64_t* rowva
   cudaSetDevice(c->device);
   const int64_t nnz = m->P.nnz, ncol = m->P.ncol;
   const unsigned grid = grid_for(nnz > ncol + 1 ? nnz : ncol + 1, 256, (int64_t)c->sm_count * 16);
+  if (!colptr && !rowval) {
+    // the values of a pattern the caller has already: no index arrays are formed
+    // (2M quadratic triangles: 0.12 ms of a 2.6 ms re-assembly and download)
+    if (nzval && nnz)
+      ELFEL_CUDA(c, cudaMemcpyAsync(nzval, m->vals.p, sizeof(double) * nnz, cudaMemcpyDeviceToHost, c->stream));
+    ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
+    return ELFEL_OK;
+  }
   int pin_c = 0, pin_r = 0;
   int64_t* cpd = colptr ? (int64_t*)host_device_ptr(c, colptr, &pin_c) : nullptr;
   int64_t* rvd = rowval ? (int64_t*)host_device_ptr(c, rowval, &pin_r) : nullptr;
