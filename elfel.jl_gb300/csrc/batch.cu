@@ -969,6 +969,7 @@ int batch_add_dev(elfel_batch* b, elfel_sysmat* m, const double* F, const double
   d.v64 = S->A.v64.p;
   d.dinv32 = S->dinv32.p;
   d.dinv64 = S->dinv64.p;
+  d.rowsum = S->rowsum32.p;
   d.x32 = S->xa32.p;
   d.r32 = S->r32.p;
   d.z32 = S->z32.p;
@@ -990,7 +991,9 @@ int batch_add_dev(elfel_batch* b, elfel_sysmat* m, const double* F, const double
   s.run = batch_run_plan(c, S, b->method == ELFEL_PCG32_IR);
   d.spb = s.run.spb;
   d.ms = s.run.ms;
-  d.max_entries = s.run.max_entries;
+  d.window = s.run.window;
+  d.room = s.run.room;
+  d.win = s.run.win;
   double hsc[B_COUNT] = {0};
   int hst[I_COUNT] = {0};
   hsc[B_TOL2] = rtol * rtol;

@@ -17,6 +17,7 @@ struct BSys {
   const double* v64;
   const float* dinv32;
   const double* dinv64;
+  const float* rowsum;  // the FP32 matrix's row sums
   float *x32, *r32, *z32, *p32, *q32;
   double *x64, *r64, *z64, *p64, *q64;
   const double* b64;
@@ -27,14 +28,16 @@ struct BSys {
   const int* nitems;   // work items of this system in the current map
   double* sc;          // B_COUNT scalars
   int* st;             // I_COUNT ints
-  int spb, ms, max_entries, pad2_;  // its division in a cluster (batch_run.cu)
+  int spb, ms, window, room;  // its division in a cluster (batch_run.cu): see RunPlan
+  const int4* win;
 };
 
 // How a system runs in the batch: in a cluster of `blocks` thread blocks of its
 // own (batch_run.cu), or with the others in the graphs (blocks = 0).  A
 // function of the system alone, so that its result does not depend on the mix.
 struct BRunPlan {
-  int blocks = 0, spb = 0, ms = 0, max_entries = 0;
+  int blocks = 0, spb = 0, ms = 0, window = 0, room = 0;
+  const int4* win = nullptr;
   size_t smem = 0;
 };
 BRunPlan batch_run_plan(const Ctx* c, const SolverData* S, int ir);

@@ -39,19 +39,23 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
   double* wsum = part + 3 * kRT;
   T* sx = reinterpret_cast<T*>(part + kRunPart);
   const int ld = S.spb * 32;
-  T *sr = sx + ld, *sp = sr + ld, *sq = sp + ld, *sd = sq + ld;
+  T *sr = sx + ld, *sq = sr + ld, *sd = sq + ld, *ss = sd + ld, *pw = ss + (IR ? ld : 0);
   T* const gx = IR ? (T*)S.x32 : (T*)S.x64;
   T* const gr = IR ? (T*)S.r32 : (T*)S.r64;
   T* const gp = IR ? (T*)S.p32 : (T*)S.p64;
   const T* const gd = IR ? (const T*)S.dinv32 : (const T*)S.dinv64;
-  const RunRows<T, D16, MS> R(S.A, IR ? (const T*)S.v32 : (const T*)S.v64, grp.rank, S.spb, S.max_entries,
-                              reinterpret_cast<int2*>(sd + ld));
+  T* const gz = IR ? (T*)S.z32 : (T*)S.z64;
+  const RunRows<T, D16, MS> R(S.A, IR ? (const T*)S.v32 : (const T*)S.v64, grp.rank, S.spb, S.room,
+                              reinterpret_cast<int2*>(pw + S.window));
   const int64_t r0 = R.row0;
+  Window<T> W(pw, S.win[grp.rank], false, (int)r0, R.nloc);
+  T* const sp = pw + W.own;
+  W.load(gp);
   for (int i = tid; i < R.nloc; i += kRT) {
     sx[i] = gx[r0 + i];
     sr[i] = gr[r0 + i];
-    sp[i] = gp[r0 + i];
     sd[i] = gd[r0 + i];
+    if (IR) ss[i] = (T)S.rowsum[r0 + i];
   }
   // the system's scalars (warp 0 uses them)
   const double scale = S.sc[B_SCALE], tol = S.sc[B_TOL2], bn2 = S.sc[B_BN2];
@@ -62,7 +66,14 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
   const int maxit = S.st[I_MAXIT];
   __syncthreads();
 
+  T be = 0;
+  bool keep = true;  // the window holds the direction already
   for (int k = 0; k < iters; ++k) {
+    if (!keep) {  // p = z + beta p
+      W.template advance<true>(sq, gz, be);
+      __syncthreads();
+    }
+    keep = false;
     // q = A p; p.q (and r.p) -> alpha
     constexpr int N1 = IR ? 2 : 1;
     T d1[N1] = {};
@@ -71,7 +82,8 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
       const int i = s * 32 + lane;
       if (i < R.nloc) {
         const T pi = sp[i];
-        const T acc = R.template row<IR, false>(s, i, gp, gp, (T)0, pi);
+        T acc = R.template row<IR>(s, i, W.by_row(), pi);
+        if (IR) acc += ss[i] * pi;
         sq[i] = acc;
         d1[0] += acc * pi;
         if (IR) d1[N1 - 1] += sr[i] * pi;
@@ -95,6 +107,7 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
       sr[i] = ri;
       const T zi = sd[i] * ri;
       sq[i] = zi;
+      gz[r0 + i] = zi;
       d2[0] += ri * zi;
       d2[1] += ri * ri;
       if (IR) d2[N2 - 1] += zi * ro;
@@ -140,15 +153,12 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
     __syncthreads();
     mode = msg.stop;
     if (mode == M_DONE) break;
-    const T be = (T)msg.c[0];
-    for (int i = tid; i < R.nloc; i += kRT) {
-      const T pn = axpy<T>(be, sp[i], sq[i]);
-      sp[i] = pn;
-      if (mode == M_CG) gp[r0 + i] = pn;
-    }
+    be = (T)msg.c[0];
     if (mode == M_FOLD) {
-      // x64 += s x32 (FP32), then the true residual b - K x64 in FP64
+      // the next direction, x64 += s x32 (FP32), then the true residual
+      // b - K x64 in FP64
       for (int i = tid; i < R.nloc; i += kRT) {
+        sp[i] = axpy<T>(be, sp[i], sq[i]);
         if (IR) {
           S.x64[r0 + i] += scale * (double)sx[i];
           sx[i] = 0;
@@ -202,9 +212,7 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
           const T ri = IR ? (T)(S.r64[r0 + i] * inv) : (T)S.r64[r0 + i];
           sr[i] = ri;
           const T zi = sd[i] * ri;
-          const T pi = mode == M_RESTART ? zi : sp[i];
-          sp[i] = pi;
-          gp[r0 + i] = pi;
+          gp[r0 + i] = mode == M_RESTART ? zi : sp[i];
           dz[0] += ri * zi;
         }
       }
@@ -212,16 +220,16 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
       cluster_sum<1>(grp, dz, part, wsum, t3);
       if (wid == 0) rz = t3[0];
       mode = M_CG;
+      W.load(gp);  // the sum's barrier has made it visible
+      keep = true;
       __syncthreads();
-      continue;  // the sum's barrier has made the direction visible
     }
-    grp.arrive(wid);
-    grp.wait(wid);
   }
   __syncthreads();
   for (int i = tid; i < R.nloc; i += kRT) {
     gx[r0 + i] = sx[i];
     gr[r0 + i] = sr[i];
+    if (mode == M_CG) gp[r0 + i] = keep ? sp[i] : axpy<T>(be, sp[i], sq[i]);
   }
   if (grp.rank == 0 && tid == 0) {
     S.sc[B_RZ] = rz;
@@ -270,7 +278,10 @@ BRunPlan batch_run_plan(const Ctx* c, const SolverData* S, int ir) {
   const int elem = ir ? 4 : 8;
   const int spb = run_spb_batch(S->A.nslices, elem);
   const int entries = S->run_entries[ir ? 2 : 3];
-  const size_t sv = run_smem(spb, elem, 5, 0, S->A.d16), sm = run_smem(spb, elem, 5, entries, S->A.d16);
+  const int window = S->run_window[ir ? 2 : 3] + (S->run_window[ir ? 2 : 3] & 1);
+  if (window == 0) return P;  // too large for the division
+  const size_t sv = run_smem(spb, elem, ir ? 5 : 4, window, 0, S->A.d16);
+  const size_t sm = run_smem(spb, elem, ir ? 5 : 4, window, entries, S->A.d16);
   // a system whose matrix does not fit iterates from L2 as long as its rows
   // are few; larger ones are left to the graphs, which use the whole device
   if (sv > (size_t)kRunSmem || spb * 32 > (ir ? kRunBatchRows32 : kRunBatchRows64) * 5 / 4) return P;
@@ -278,7 +289,9 @@ BRunPlan batch_run_plan(const Ctx* c, const SolverData* S, int ir) {
   P.spb = spb;
   P.blocks = 1;
   while ((int64_t)P.blocks * spb < S->A.nslices) P.blocks *= 2;
-  P.max_entries = entries;
+  P.room = P.ms ? entries : 0;
+  P.window = window;
+  P.win = S->run_win.p + (ir ? kRunWinBatch32 : kRunWinBatch64);
   P.smem = P.ms ? sm : sv;
   return P;
 }

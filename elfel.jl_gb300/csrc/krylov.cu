@@ -7,21 +7,28 @@
 // waited for its flags and scalars, re-read the vectors of its rows, and ended
 // in a last-block reduction, each a chain of memory round trips and of FP64
 // adds (64 cycles apiece).  Here
-//   - a thread block keeps the same rows for the whole solve: x, r, p, q and
-//     the preconditioner stay in shared memory, and the matrix too when it
-//     fits (MS); only what is gathered goes through global memory;
+//   - a thread block keeps the same rows for the whole solve: x, r, q and the
+//     preconditioner stay in shared memory, the matrix too when it fits (MS),
+//     and the gathered direction of all rows that the block's columns touch
+//     (Window), which the block advances itself: only z of the rows around its
+//     own travels between blocks;
 //   - the sums go thread -> warp -> block -> group, and one warp of every
 //     block forms alpha, beta and the convergence test from the group totals
 //     (the same partials in the same order: the same bits in every block);
 //   - x is advanced between the arrival at and the wait for the second sum.
 // Per iteration, quadratic heat, FP64 and FP32 (graphs, then one launch):
-//       961 unknowns  21.3 ->  6.3 us   25.8 ->  9.6 us (12 replacements incl.)
-//     14161           21.1 -> 10.1      21.9 ->  7.5
-//    128881           26.2 -> 13.8      22.2 ->  9.4
-//    358801           40.2 -> 23.2      32.0 -> 13.9
-//    808201           62.7 -> 46.6      45.9 -> 21.1
-// MINRES (Taylor-Hood cavity) 27.2 -> 12.5 us at 9026 unknowns.  What is left
-// is the barriers (about 4 us of the 13.8) and the FP64 unit (6 us of them).
+//       961 unknowns  21.3 ->  6.4 us   25.8 ->  9.5 us (12 replacements incl.)
+//     14161           21.1 ->  8.9      21.9 ->  6.5
+//    128881           26.2 -> 12.7      22.2 ->  8.6
+//    358801           40.2 -> 23.5      32.0 -> 11.9
+//    808201           62.7 -> 47.9      45.9 -> 16.2
+// MINRES (Taylor-Hood cavity) 27.2 -> 11.9 us at 9026 unknowns.  What is left
+// at 128881: the two sums over the grid (2.0 us each with their barriers), in
+// FP64 the FP64 unit (6 us).  Measured and not kept: the direction gathered
+// from global memory after a barrier of its own (FP32 9.4 us at 128881, 21.1 at
+// 808201: gathers that miss L1), 1024 threads a block (17.5 at 808201), the
+// next chunk of the matrix prefetched into registers (no change: the product
+// is bound by instruction issue).
 // Two groups are provided:
 //   ClusterGroup  one cluster of up to 16 blocks: sums through distributed
 //                 shared memory, the hardware cluster barrier (0.2-0.3 us);
@@ -29,9 +36,6 @@
 //                 in global memory (1.1 us per barrier at 152 blocks).  Every
 //                 wait is bounded; a wait that runs out marks the error word
 //                 and ends the kernel.
-// FP64 work grows with 1 / blocks, so a cluster of 16 SMs serves systems up to
-// 16k unknowns in FP64 (at 14k: 10.1 us, at 22k in a grid 9.2) and, bound by
-// its barriers instead, 32k in FP32.
 #include <algorithm>
 
 #include "krylov_dev.cuh"
@@ -45,12 +49,10 @@ namespace {
 // replacement), else FP64 Jacobi PCG.  The recurrences and stopping rules are
 // those of the graph kernels (sell_cg_spmv_k, cg_update_k, cg_p_k).
 //
-// The direction p = z + beta p needs beta, which needs every block: written
-// out and gathered after a third barrier; or (TWO) z is written before the
-// second sum, and the product gathers z + beta p with the p of the iteration
-// before, one multiply-add more per entry instead of the barrier.  p then
-// alternates between two buffers.
-template <typename T, bool D16, bool IR, bool MS, bool TWO, class Group>
+// WIN: the direction of the block's column window lies in shared memory
+// (Window), two sums an iteration.  Otherwise (columns from everywhere) it is
+// gathered from global memory, where a third barrier completes it.
+template <typename T, bool D16, bool IR, bool MS, bool WIN, class Group>
 __global__ void __launch_bounds__(kRT, 1) cg_run_k(const CgRun<T> a, const RunGroup rg) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ typename Group::Shared gsh;
@@ -60,16 +62,19 @@ __global__ void __launch_bounds__(kRT, 1) cg_run_k(const CgRun<T> a, const RunGr
   double* wsum = part + 3 * kRT;
   T* sx = reinterpret_cast<T*>(part + kRunPart);
   const int ld = a.spb * 32;
-  T *sr = sx + ld, *sp = sr + ld, *sq = sp + ld, *sd = sq + ld;
-  const RunRows<T, D16, MS> R(a.A, a.v, (int)blockIdx.x, a.spb, a.max_entries, reinterpret_cast<int2*>(sd + ld));
+  T *sr = sx + ld, *sq = sr + ld, *sd = sq + ld, *ss = sd + ld, *pw = ss + (a.own_sums ? ld : 0);
+  const RunRows<T, D16, MS> R(a.A, a.v, (int)blockIdx.x, a.spb, a.room, reinterpret_cast<int2*>(pw + a.window));
+  const int r1 = (int)R.row0 + R.nloc;
+  Window<T> W(pw, WIN ? a.win[blockIdx.x] : make_int4((int)R.row0, r1, r1, r1), false, (int)R.row0, R.nloc);
+  T* const sp = pw + W.own;
+  W.load(a.p);
   for (int i = tid; i < R.nloc; i += kRT) {
     sx[i] = a.x[R.row0 + i];
     sr[i] = a.r[R.row0 + i];
-    const T p = a.p[R.row0 + i];
-    sp[i] = TWO ? 0 : p;
-    if (TWO) sq[i] = p;  // the first direction is z + 0 p
     sd[i] = a.dinv[R.row0 + i];
+    if (IR && a.own_sums) ss[i] = a.rowsum[R.row0 + i];
   }
+  const T* const rs = IR && !a.own_sums ? a.rowsum + R.row0 : ss;  // row sums: of the own rows, or where they are
   // the loop's scalars (warp 0 uses them)
   double rz = a.scal[S_RZ], rr = a.scal[S_RR], pq = 0.0, alpha = 0.0, beta = 0.0, inv_rz = 1.0 / rz;
   const double thr = a.scal[S_TOL2] * (IR ? a.scal[S_BN2S] : a.scal[S_BN2]);
@@ -81,25 +86,39 @@ __global__ void __launch_bounds__(kRT, 1) cg_run_k(const CgRun<T> a, const RunGr
   Group grp(rg, &gsh);
   __syncthreads();
 
-  // what the product gathers: (z, p of the iteration before), first (p, p) with beta = 0
-  const T *zg = a.p, *pold = a.p;
-  T* pnew = TWO ? a.p2 : a.p;
   T be = 0;
   for (int k = 0; k < a.max_iters; ++k) {
-    // (p = z + beta p) q = A p; p.q (and r.p) -> alpha
+    if (k > 0) {  // p = z + beta p
+      if (WIN) {
+        W.template advance<true>(sq, a.z, be);
+        __syncthreads();
+      } else {
+        for (int i = tid; i < R.nloc; i += kRT) {
+          const T pn = axpy<T>(be, sp[i], sq[i]);
+          sp[i] = pn;
+          a.p[R.row0 + i] = pn;
+        }
+        // the new direction is complete before the gathers
+        if (!Group::kCluster) __syncthreads();
+        grp.arrive(wid);
+        const bool ok = grp.wait(wid);
+        if (!Group::kCluster) {
+          if (tid == 0) msg.stop = ok ? 0 : 2;
+          __syncthreads();
+          if (msg.stop) break;
+        }
+      }
+    }
+    // q = A p; p.q (and r.p) -> alpha
     constexpr int N1 = IR ? 2 : 1;
     T d1[N1] = {};
     for (int n = 0; n * kRW < R.nsl; ++n) {
       const int s = R.slice(wid, n);
       const int i = s * 32 + lane;
       if (i < R.nloc) {
-        T pi = sp[i];
-        if (TWO) {
-          pi = axpy<T>(be, pi, sq[i]);
-          sp[i] = pi;
-          pnew[R.row0 + i] = pi;
-        }
-        const T acc = R.template row<IR, TWO>(s, i, pold, zg, be, pi);
+        const T pi = sp[i];
+        T acc = R.template row<IR>(s, i, WIN ? W.by_row() : (const T*)a.p, pi);
+        if (IR) acc += rs[i] * pi;
         sq[i] = acc;
         d1[0] += acc * pi;
         if (IR) d1[N1 - 1] += sr[i] * pi;
@@ -131,7 +150,7 @@ __global__ void __launch_bounds__(kRT, 1) cg_run_k(const CgRun<T> a, const RunGr
       sr[i] = ri;
       const T zi = sd[i] * ri;
       sq[i] = zi;
-      if (TWO) a.z[R.row0 + i] = zi;
+      if (WIN) a.z[R.row0 + i] = zi;
       d2[0] += ri * zi;
       d2[1] += ri * ri;
       if (IR) d2[N2 - 1] += zi * ro;
@@ -173,37 +192,14 @@ __global__ void __launch_bounds__(kRT, 1) cg_run_k(const CgRun<T> a, const RunGr
       }
     }
     __syncthreads();
-    const int stop = msg.stop;
-    if (stop == 2) break;
     be = (T)msg.c[0];
-    if (TWO) {
-      if (stop) break;
-      zg = a.z;
-      pold = pnew;
-      pnew = pnew == a.p2 ? a.p : a.p2;
-      continue;
-    }
-    for (int i = tid; i < R.nloc; i += kRT) {
-      const T pn = axpy<T>(be, sp[i], sq[i]);
-      sp[i] = pn;
-      pnew[R.row0 + i] = pn;
-    }
-    if (stop) break;
-    // the new direction is complete before the next gathers
-    if (!Group::kCluster) __syncthreads();
-    grp.arrive_halo(wid);
-    ok = grp.wait_halo(wid);
-    if (!Group::kCluster) {
-      if (tid == 0) msg.stop = ok ? 0 : 2;
-      __syncthreads();
-      if (msg.stop) break;
-    }
+    if (msg.stop) break;
   }
   __syncthreads();
   for (int i = tid; i < R.nloc; i += kRT) {
     a.x[R.row0 + i] = sx[i];
     a.r[R.row0 + i] = sr[i];
-    if (TWO) a.p[R.row0 + i] = axpy<T>(be, sp[i], sq[i]);
+    a.p[R.row0 + i] = axpy<T>(be, sp[i], sq[i]);  // the recurrence's next direction
   }
   if (blockIdx.x == 0 && tid == 0) {
     a.scal[S_RZ] = rz;
@@ -228,10 +224,11 @@ __global__ void __launch_bounds__(kRT, 1) cg_run_k(const CgRun<T> a, const RunGr
 
 // Preconditioned MINRES, the three steps of mr_spmv_k / mr_vec_k / mr_upd_k /
 // mr_tail_k.  The scalar chain of a step (two square roots and five
-// divisions) runs in warp 0 with the divisions side by side in its lanes; w
-// and x are advanced between the arrival at and the wait for the barrier that
-// ends the iteration.
-template <typename T, bool D16, bool MS, class Group>
+// divisions) runs in warp 0 with the divisions side by side in its lanes.
+// WIN: the normalised z of the block's column window is in shared memory, and
+// what travels is z' before its normalisation, written ahead of the sum that
+// gives its norm; otherwise z is gathered from global memory after a barrier.
+template <typename T, bool D16, bool MS, bool WIN, class Group>
 __global__ void __launch_bounds__(kRT, 1) mr_run_k(const MrRun<T> a, const RunGroup rg) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ typename Group::Shared gsh;
@@ -241,12 +238,15 @@ __global__ void __launch_bounds__(kRT, 1) mr_run_k(const MrRun<T> a, const RunGr
   double* wsum = part + 3 * kRT;
   T* sx = reinterpret_cast<T*>(part + kRunPart);
   const int ld = a.spb * 32;
-  T *sz = sx + ld, *sq = sz + ld, *sm = sq + ld, *sv = sm + ld, *svm = sv + ld, *sw = svm + ld, *swm = sw + ld;
-  const RunRows<T, D16, MS> R(a.A, a.v, (int)blockIdx.x, a.spb, a.max_entries, reinterpret_cast<int2*>(swm + ld));
+  T *sq = sx + ld, *sm = sq + ld, *sv = sm + ld, *svm = sv + ld, *sw = svm + ld, *swm = sw + ld, *zw = swm + ld;
+  const RunRows<T, D16, MS> R(a.A, a.v, (int)blockIdx.x, a.spb, a.room, reinterpret_cast<int2*>(zw + a.window));
   const int64_t r0 = R.row0;
+  const int r1 = (int)r0 + R.nloc;
+  Window<T> W(zw, WIN ? a.win[blockIdx.x] : make_int4((int)r0, r1, r1, r1), true, (int)r0, R.nloc);
+  T* const sz = zw + W.own;
+  W.load(a.z);
   for (int i = tid; i < R.nloc; i += kRT) {
     sx[i] = a.x[r0 + i];
-    sz[i] = a.z[r0 + i];
     sm[i] = a.minv[r0 + i];
     sv[i] = a.vj[r0 + i];
     svm[i] = a.vjm[r0 + i];
@@ -262,8 +262,30 @@ __global__ void __launch_bounds__(kRT, 1) mr_run_k(const MrRun<T> a, const RunGr
   Group grp(rg, &gsh);
   __syncthreads();
 
-  for (int k = 0; k < a.max_iters; ++k) {
-    if (done && k == 0) break;  // nothing to do (zero right-hand side)
+  T zs = 0;
+  bool moved = false;  // sq holds the next z, not normalised yet
+  for (int k = 0; k < a.max_iters && !done; ++k) {
+    if (k > 0) {  // z = z' / gamn
+      moved = false;
+      if (WIN) {
+        W.template advance<false>(sq, a.z, zs);
+        __syncthreads();
+      } else {
+        for (int i = tid; i < R.nloc; i += kRT) {
+          const T zn = sq[i] * zs;
+          sz[i] = zn;
+          a.z[r0 + i] = zn;
+        }
+        if (!Group::kCluster) __syncthreads();
+        grp.arrive(wid);
+        const bool ok = grp.wait(wid);
+        if (!Group::kCluster) {
+          if (tid == 0) msg.stop = ok ? 0 : 2;
+          __syncthreads();
+          if (msg.stop) break;
+        }
+      }
+    }
     // q = A z, delta = q.z
     T d1[1] = {0};
     for (int n = 0; n * kRW < R.nsl; ++n) {
@@ -271,7 +293,8 @@ __global__ void __launch_bounds__(kRT, 1) mr_run_k(const MrRun<T> a, const RunGr
       const int i = sl * 32 + lane;
       if (i < R.nloc) {
         const T zi = sz[i];
-        const T acc = R.template row<false, false>(sl, i, a.z, a.z, (T)0, zi);
+        const T acc = WIN ? R.template row<false>(sl, i, W.by_row_split(), zi)
+                          : R.template row<false>(sl, i, (const T*)a.z, zi);
         sq[i] = acc;
         d1[0] += acc * zi;
       }
@@ -281,12 +304,13 @@ __global__ void __launch_bounds__(kRT, 1) mr_run_k(const MrRun<T> a, const RunGr
     if (wid == 0) grp.publish(t);
     grp.arrive(wid);
     bool ok = grp.wait(wid);
-    double delta = 0.0;
     grp.collect(wid, wsum, t);
+    double delta = 0.0;
     if (wid == 0) {
       delta = t[0];
+      const double ca = fast_div(delta, gam, fast_rcp(gam));
       if (lane == 0) {
-        msg.c[0] = delta / gam;
+        msg.c[0] = ca;
         msg.c[1] = bcoef;
         msg.stop = ok ? 0 : 2;
       }
@@ -301,6 +325,7 @@ __global__ void __launch_bounds__(kRT, 1) mr_run_k(const MrRun<T> a, const RunGr
       svm[i] = vv;
       const T zz = sm[i] * vv;
       sq[i] = zz;
+      if (WIN) a.z[r0 + i] = zz;
       d2[0] += zz * vv;
     }
     block_sums<1>(d2, part, wsum, t);
@@ -346,18 +371,13 @@ __global__ void __launch_bounds__(kRT, 1) mr_run_k(const MrRun<T> a, const RunGr
     __syncthreads();
     const int stop = msg.stop;
     if (stop == 2) break;
-    const T zs = (T)msg.c[0], ca3 = (T)msg.c[1], ca2 = (T)msg.c[2], cia = (T)msg.c[3], cce = (T)msg.c[4];
-    // w' = (z - a3 w_{j-1} - a2 w_j) / a1, x += c eta w', z = z' / gamn
+    done = stop;
+    zs = (T)msg.c[0];
+    moved = true;
+    const T ca3 = (T)msg.c[1], ca2 = (T)msg.c[2], cia = (T)msg.c[3], cce = (T)msg.c[4];
+    // w' = (z - a3 w_{j-1} - a2 w_j) / a1, x += c eta w'
     for (int i = tid; i < R.nloc; i += kRT) {
-      const T zi = sz[i], zn = sq[i] * zs;
-      sz[i] = zn;
-      a.z[r0 + i] = zn;
-      sq[i] = zi;
-    }
-    if (!Group::kCluster) __syncthreads();
-    if (!stop) grp.arrive_halo(wid);
-    for (int i = tid; i < R.nloc; i += kRT) {
-      const T w = (sq[i] - ca3 * swm[i] - ca2 * sw[i]) * cia;
+      const T w = (sz[i] - ca3 * swm[i] - ca2 * sw[i]) * cia;
       swm[i] = w;
       sx[i] += cce * w;
     }
@@ -367,17 +387,11 @@ __global__ void __launch_bounds__(kRT, 1) mr_run_k(const MrRun<T> a, const RunGr
     T* tw = sw;
     sw = swm;
     swm = tw;
-    if (stop) break;
-    ok = grp.wait_halo(wid);
-    if (!Group::kCluster) {
-      if (tid == 0) msg.stop = ok ? 0 : 2;
-      __syncthreads();
-      if (msg.stop) break;
-    }
   }
   __syncthreads();
   for (int i = tid; i < R.nloc; i += kRT) {
     a.x[r0 + i] = sx[i];
+    if (moved) a.z[r0 + i] = sq[i] * zs;
     a.vj[r0 + i] = sv[i];
     a.vjm[r0 + i] = svm[i];
     a.wj[r0 + i] = sw[i];
@@ -403,7 +417,7 @@ __global__ void __launch_bounds__(kRT, 1) mr_run_k(const MrRun<T> a, const RunGr
 
 template <class Args>
 int run_launch(Ctx* c, SolverData* S, const RunPlan& P, void (*k)(const Args, const RunGroup), const Args& a) {
-  RunGroup rg{S->run_slots.p, S->run_bar.p, S->run_halo.p, S->run_neighbours};
+  RunGroup rg{S->run_slots.p, S->run_bar.p};
   ELFEL_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem));
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
@@ -418,7 +432,7 @@ int run_launch(Ctx* c, SolverData* S, const RunPlan& P, void (*k)(const Args, co
     at[0].val.clusterDim.x = (unsigned)P.blocks;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   } else {
-    ELFEL_CUDA(c, cudaMemsetAsync(S->run_bar.p, 0, sizeof(unsigned) * kRunWords, c->stream));
+    ELFEL_CUDA(c, cudaMemsetAsync(S->run_bar.p, 0, 2 * sizeof(unsigned), c->stream));
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
   }
@@ -430,27 +444,26 @@ int run_launch(Ctx* c, SolverData* S, const RunPlan& P, void (*k)(const Args, co
 
 template <typename T, bool D16, bool IR>
 int cg_launch(Ctx* c, SolverData* S, const RunPlan& P, const CgRun<T>& a) {
+  if (P.cluster && P.window) return run_launch(c, S, P, cg_run_k<T, D16, IR, true, true, ClusterGroup>, a);
   if (P.cluster) return run_launch(c, S, P, cg_run_k<T, D16, IR, true, false, ClusterGroup>, a);
-  // FP64: the extra multiply-add per entry pays for the barrier in small systems only
-  if (sizeof(T) == 4 || S->nu <= kRunTwoRows64) {
-    if (P.ms) return run_launch(c, S, P, cg_run_k<T, D16, IR, true, true, GridGroup>, a);
-    return run_launch(c, S, P, cg_run_k<T, D16, IR, false, true, GridGroup>, a);
-  }
-  if (P.ms) return run_launch(c, S, P, cg_run_k<T, D16, IR, true, false, GridGroup>, a);
+  if (P.window && P.ms) return run_launch(c, S, P, cg_run_k<T, D16, IR, true, true, GridGroup>, a);
+  if (P.window) return run_launch(c, S, P, cg_run_k<T, D16, IR, false, true, GridGroup>, a);
   return run_launch(c, S, P, cg_run_k<T, D16, IR, false, false, GridGroup>, a);
 }
 
 template <typename T, bool D16>
 int mr_launch(Ctx* c, SolverData* S, const RunPlan& P, const MrRun<T>& a) {
-  if (P.cluster) return run_launch(c, S, P, mr_run_k<T, D16, true, ClusterGroup>, a);
-  if (P.ms) return run_launch(c, S, P, mr_run_k<T, D16, true, GridGroup>, a);
-  return run_launch(c, S, P, mr_run_k<T, D16, false, GridGroup>, a);
+  if (P.cluster && P.window) return run_launch(c, S, P, mr_run_k<T, D16, true, true, ClusterGroup>, a);
+  if (P.cluster) return run_launch(c, S, P, mr_run_k<T, D16, true, false, ClusterGroup>, a);
+  if (P.window && P.ms) return run_launch(c, S, P, mr_run_k<T, D16, true, true, GridGroup>, a);
+  if (P.window) return run_launch(c, S, P, mr_run_k<T, D16, false, true, GridGroup>, a);
+  return run_launch(c, S, P, mr_run_k<T, D16, false, false, GridGroup>, a);
 }
 
 }  // namespace
 
-size_t run_smem(int spb, int elem, int vecs, int entries, int d16) {
-  return sizeof(double) * kRunPart + (size_t)spb * 32 * elem * vecs + (size_t)spb * sizeof(int2) +
+size_t run_smem(int spb, int elem, int vecs, int window, int entries, int d16) {
+  return sizeof(double) * kRunPart + ((size_t)spb * 32 * vecs + window) * elem + (size_t)spb * sizeof(int2) +
          (size_t)entries * (elem + (d16 ? 2 : 4));
 }
 
@@ -474,60 +487,77 @@ int run_spb_batch(int64_t nslices, int elem) {
   return (int)((nslices + cl - 1) / cl);
 }
 
-RunPlan run_plan(Ctx* c, const SolverData* S, int elem, int vecs) {
-  RunPlan P;
+RunPlan run_plan(Ctx* c, const SolverData* S, int elem, int vecs, int least_vecs, int split) {
   const Sell& A = S->A;
-  if (!c->one_launch || S->nu < 1 || !S->run_slots.p) return P;
-  const int64_t limit = elem == 8 ? kRunClusterRows64 : kRunClusterRows32;
-  if (S->nu <= limit) {
-    const int spb = run_spb_cluster(A.nslices);
-    const size_t sm = run_smem(spb, elem, vecs, S->run_entries[0], A.d16);
-    if (sm <= (size_t)kRunSmem) {
-      P.spb = spb;
-      int cl = 1;
-      while ((int64_t)cl * spb < A.nslices) cl *= 2;
-      P.blocks = cl;
-      P.cluster = P.ms = 1;
-      P.max_entries = S->run_entries[0];
-      P.smem = sm;
-      return P;
-    }
+  if (!c->one_launch || S->nu < 1 || !S->run_slots.p) return RunPlan();
+  // A cluster saves about 5000 cycles an iteration at its barriers and sums; in
+  // FP64 its 16 SMs take half a cycle over 16 per multiply-add (entries, and
+  // about 8 per row for the vectors), which makes that up at 180k of them.
+  const bool small = elem == 8 ? A.nnz_pad + 8 * S->nu <= kRunClusterWork64 : S->nu <= kRunClusterRows32;
+  for (int cluster = small ? 1 : 0; cluster >= 0; --cluster) {
+    RunPlan P;
+    const int q = cluster ? 1 : 0;
+    P.cluster = cluster;
+    P.spb = cluster ? run_spb_cluster(A.nslices) : run_spb_grid(c, A.nslices);
+    P.blocks = 1;
+    if (cluster)
+      while ((int64_t)P.blocks * P.spb < A.nslices) P.blocks *= 2;
+    else
+      P.blocks = (int)((A.nslices + P.spb - 1) / P.spb);
+    // Every row of a window that is not the block's own costs a multiply-add a
+    // product (FP64: half a cycle of the SM), which pays for the barrier that
+    // the window saves up to these widths.
+    const int wide = S->run_window[split ? 4 + q : q];
+    const int most = P.spb * 32 + (cluster ? 2000 : 8000) * (elem == 8 ? 1 : 2);
+    P.window = wide > 0 && wide <= most ? wide + (wide & 1) : 0;  // even: 8-byte alignment of what follows
+    auto smem = [&](int entries) {
+      return run_smem(P.spb, elem, P.vecs, P.window ? P.window : P.spb * 32, entries, A.d16);
+    };
+    P.vecs = vecs;
+    if (smem(0) > (size_t)kRunSmem) P.vecs = std::min(vecs, least_vecs);
+    if (smem(0) > (size_t)kRunSmem) P.window = 0;
+    const size_t sv = smem(0), sm = smem(S->run_entries[q]);
+    P.ms = sm <= (size_t)kRunSmem;
+    if (cluster && !P.ms) continue;  // a grid has room
+    if (!P.ms && sv > (size_t)kRunSmem) return RunPlan();
+    if (!P.window) P.ms = cluster;  // (the grid's form without a window reads the matrix from L2)
+    P.room = P.ms ? S->run_entries[q] : 0;
+    P.smem = P.ms ? sm : sv;
+    return P;
   }
-  const int spb = run_spb_grid(c, A.nslices);
-  const size_t sv = run_smem(spb, elem, vecs, 0, A.d16);
-  if (sv > (size_t)kRunSmem) return P;
-  const size_t sm = run_smem(spb, elem, vecs, S->run_entries[1], A.d16);
-  P.spb = spb;
-  P.blocks = (int)((A.nslices + spb - 1) / spb);
-  P.ms = sm <= (size_t)kRunSmem ? 1 : 0;
-  P.max_entries = S->run_entries[1];
-  P.smem = P.ms ? sm : sv;
-  return P;
+  return RunPlan();
+}
+
+// The window argument of a launch: the room for it (without one, for the own
+// rows of the direction), and the blocks' windows.
+static int run_window_arg(const RunPlan& P) { return P.window ? P.window : P.spb * 32; }
+static const int4* run_win_arg(const SolverData* S, const RunPlan& P) {
+  return S->run_win.p + (P.cluster ? 0 : kRunWinGrid);
 }
 
 int run_cg64(Ctx* c, SolverData* S, const RunPlan& P) {
-  const CgRun<double> a{S->view(), S->A.v64.p, S->dinv64.p, S->x64.p, S->r64.p, S->p64.p, S->y64.p, S->z64.p,
-                        S->scal.p, S->flags.p, P.spb,       P.max_entries, kRunIters};
+  const CgRun<double> a{S->view(), S->A.v64.p, S->dinv64.p, nullptr, S->x64.p, S->r64.p, S->p64.p, S->z64.p,
+                        S->scal.p, S->flags.p, P.spb, run_window_arg(P), P.room, kRunIters, run_win_arg(S, P), P.vecs > 4};
   return S->A.d16 ? cg_launch<double, true, false>(c, S, P, a) : cg_launch<double, false, false>(c, S, P, a);
 }
 
 int run_cg32(Ctx* c, SolverData* S, const RunPlan& P) {
-  const CgRun<float> a{S->view(), S->A.v32.p, S->dinv32.p, S->xa32.p, S->r32.p, S->p32.p, S->zz32.p, S->z32.p,
-                       S->scal.p, S->flags.p, P.spb,       P.max_entries, kRunIters};
+  const CgRun<float> a{S->view(), S->A.v32.p, S->dinv32.p, S->rowsum32.p, S->xa32.p, S->r32.p, S->p32.p, S->z32.p,
+                       S->scal.p, S->flags.p, P.spb, run_window_arg(P), P.room, kRunIters, run_win_arg(S, P), P.vecs > 4};
   return S->A.d16 ? cg_launch<float, true, true>(c, S, P, a) : cg_launch<float, false, true>(c, S, P, a);
 }
 
 int run_mr64(Ctx* c, SolverData* S, const RunPlan& P, double* x, double* z, double* vj, double* vjm, double* wj,
              double* wjm) {
   const MrRun<double> a{S->view(), S->A.v64.p, S->dinv64.p, x,     z,             vj,       vjm, wj, wjm,
-                        S->scal.p, S->flags.p, P.spb,       P.max_entries, kRunIters};
+                        S->scal.p, S->flags.p, P.spb, run_window_arg(P), P.room, kRunIters, run_win_arg(S, P)};
   return S->A.d16 ? mr_launch<double, true>(c, S, P, a) : mr_launch<double, false>(c, S, P, a);
 }
 
 int run_mr32(Ctx* c, SolverData* S, const RunPlan& P, float* x, float* z, float* vj, float* vjm, float* wj,
              float* wjm) {
   const MrRun<float> a{S->view(), S->A.v32.p, S->dinv32.p, x,     z,             vj,       vjm, wj, wjm,
-                       S->scal.p, S->flags.p, P.spb,       P.max_entries, kRunIters};
+                       S->scal.p, S->flags.p, P.spb, run_window_arg(P), P.room, kRunIters, run_win_arg(S, P)};
   return S->A.d16 ? mr_launch<float, true>(c, S, P, a) : mr_launch<float, false>(c, S, P, a);
 }
 

@@ -7,16 +7,17 @@ namespace elfel {
 constexpr int kRunThreads = 512;
 constexpr int kRunMaxBlocks = 160;  // blocks of a grid group (one per SM)
 // Cluster groups: slices per block that a cluster is grown for (up to 16
-// blocks), and the largest systems that run in one.
+// blocks), and the largest systems that run in one (FP64: entries + 8 rows).
 constexpr int kRunClusterSlices = 2;
-constexpr int64_t kRunClusterRows64 = 16384, kRunClusterRows32 = 32768;
-// Beyond this no grid group holds the vectors (226 KB of 20 bytes a row, 160 blocks).
+constexpr int64_t kRunClusterWork64 = 180000, kRunClusterRows32 = 32768;
+// Beyond this no grid group holds the vectors (20 bytes a row).
 constexpr int64_t kRunGridRows = (int64_t)kRunMaxBlocks * 12000;
-constexpr int64_t kRunTwoRows64 = 65536;  // FP64: two barriers an iteration up to here (cg_run_k)
 // A batched system takes the smallest cluster whose blocks hold this many rows each.
 constexpr int kRunBatchRows32 = 2048, kRunBatchRows64 = 1024;
+// Systems up to this size may run in a cluster (of the batch too).
+constexpr int64_t kRunSmallRows = 65536;
 constexpr int kRunIters = 4096;     // iterations of one launch at most
-constexpr int kRunSmem = 227 * 1024 - 1024;  // dynamic shared memory of a block (the kernels' static part apart)
+constexpr int kRunSmem = 227 * 1024 - 2048;  // dynamic shared memory of a block (the kernels' static part apart)
 
 template <bool D16>
 struct ColType {
@@ -28,26 +29,29 @@ struct ColType<false> {
 };
 
 // A grid group's memory: partial sums [parity][value][block]; words (cleared
-// before each launch): arrival counter, error flag, and a flag per block, set
-// to the iteration whose rows of the direction are written.  halo: the blocks
-// (first, last) that each block gathers from; neighbours: they are at most 32.
-constexpr int kRunFlag0 = 32, kRunFlagStride = 8, kRunWords = kRunFlag0 + kRunMaxBlocks * kRunFlagStride;
+// before each launch): arrival counter, error flag.
 struct RunGroup {
   double* slots;
   unsigned* words;
-  const int2* halo;
-  int neighbours;
 };
+
+// Blocks' column windows in SolverData::run_win: of the cluster division, the
+// grid's, and a batched system's (FP32, FP64).
+constexpr int kRunWinGrid = 16, kRunWinBatch32 = kRunWinGrid + kRunMaxBlocks, kRunWinBatch64 = kRunWinBatch32 + 16,
+              kRunWins = kRunWinBatch64 + 16;
 
 template <typename T>
 struct CgRun {
   SellView A;
   const T* v;
   const T* dinv;
-  T *x, *r, *p, *p2, *z;  // p2: the second direction buffer
+  const T* rowsum;  // FP32 (difference form): the row sums
+  T *x, *r, *p, *z;
   double* scal;
   int* flags;
-  int spb, max_entries, max_iters;
+  int spb, window, room, max_iters;  // slices, window rows and matrix entries of a block's shared memory
+  const int4* win;
+  int own_sums;  // FP32: a copy of the row sums in shared memory
 };
 
 template <typename T>
@@ -58,28 +62,33 @@ struct MrRun {
   T *x, *z, *vj, *vjm, *wj, *wjm;
   double* scal;
   int* flags;
-  int spb, max_entries, max_iters;
+  int spb, window, room, max_iters;  // slices, window rows and matrix entries of a block's shared memory
+  const int4* win;
 };
 
 // How a system of nslices slices runs: blocks of the group, slices per
-// block, cluster or grid, matrix in shared memory.  blocks = 0: not at all
+// block, cluster or grid, what lies in shared memory.  blocks = 0: not at all
 // (too large for the blocks' shared memory).
 struct RunPlan {
-  int blocks = 0, spb = 0, cluster = 0, ms = 0, max_entries = 0;
+  int blocks = 0, spb = 0, cluster = 0, vecs = 0;
+  int window = 0;        // rows of the largest column window (0: the direction is gathered from global memory)
+  int ms = 0, room = 0;  // matrix in shared memory: entries of the largest block
   size_t smem = 0;
 };
 
-// The slices-per-block values whose largest block entry counts build_sell
-// records in SolverData::run_entries: [0] cluster, [1] grid, and of a batched
-// system [2] FP32, [3] FP64.
+// The slices a block takes in each division q of a system: 0 grid, 1 cluster,
+// and of a batched system 2 FP32, 3 FP64.  build_sell records the largest
+// block's matrix entries (SolverData::run_entries[q]) and the rows of the
+// widest column window as one range (run_window[q]) and as two (run_window[4 + q]).
 int run_spb_cluster(int64_t nslices);
 int run_spb_grid(const Ctx* c, int64_t nslices);
 int run_spb_batch(int64_t nslices, int elem);
-// Shared memory of a block of spb slices: vecs vectors of elem-byte values
-// and, with entries > 0, that many entries of the matrix.
-size_t run_smem(int spb, int elem, int vecs, int entries, int d16);
-// vecs: vectors of the iteration kept in shared memory (5 for CG, 8 for MINRES).
-RunPlan run_plan(Ctx* c, const SolverData* S, int elem, int vecs);
+// Shared memory of a block of spb slices: vecs vectors of elem-byte values, a
+// window of that many, and `entries` entries of the matrix.
+size_t run_smem(int spb, int elem, int vecs, int window, int entries, int d16);
+// vecs: vectors of the iteration kept for a block's own rows (4 for FP64 CG, 5 for FP32 CG, which does with 4 where those do not fit, 7 for MINRES).
+// split: the window may be in two ranges (MINRES).
+RunPlan run_plan(Ctx* c, const SolverData* S, int elem, int vecs, int least_vecs, int split);
 
 // Up to kRunIters iterations of the FP64 CG, the FP32 CG of the refinement,
 // or MINRES in one launch on the context stream; the state is that of the

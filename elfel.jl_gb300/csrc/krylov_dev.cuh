@@ -122,24 +122,17 @@ struct ClusterGroup {
     }
     par ^= 1;
   }
-  // barrier that ends an iteration: the blocks' slices of the direction are visible
-  __device__ __forceinline__ void arrive_halo(int wid) { arrive(wid); }
-  __device__ __forceinline__ bool wait_halo(int wid) { return wait(wid); }
   static constexpr bool kCluster = true;
 };
 
 struct GridGroup {
   RunGroup g;
   int n, par;
-  unsigned target, epoch;
-  int2 halo;  // blocks whose rows this block's columns lie in
+  unsigned target;
   struct Shared {
     int dummy;
   };
-  __device__ GridGroup(const RunGroup& rg, Shared*) : g(rg), par(0), target(0), epoch(0) {
-    n = (int)gridDim.x;
-    halo = rg.neighbours ? rg.halo[blockIdx.x] : make_int2(0, 0);
-  }
+  __device__ GridGroup(const RunGroup& rg, Shared*) : g(rg), par(0), target(0) { n = (int)gridDim.x; }
   template <int NV>
   __device__ __forceinline__ void publish(const double (&v)[NV]) {
     if ((threadIdx.x & 31) == 0) {
@@ -156,26 +149,24 @@ struct GridGroup {
       atomicAdd(g.words, 1u);
     }
   }
-  // Polls word w until it has reached v (warp 0, by lane; inactive lanes pass).
-  __device__ __forceinline__ bool poll(const unsigned* w, unsigned v, bool active) {
-    bool ok = true, here = !active;
-    for (unsigned spins = 0; !__all_sync(0xffffffffu, here); ++spins) {
-      if (!here) {
-        unsigned x;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(w) : "memory");
-        here = (int)(x - v) >= 0;
+  __device__ __forceinline__ bool wait(int wid) {
+    if (wid) return true;
+    int ok = 1;
+    if (threadIdx.x == 0) {
+      unsigned spins = 0, v;
+      for (;;) {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(g.words) : "memory");
+        if ((int)(v - target) >= 0) break;
+        if (++spins > kRunSpins || ((spins & 1023u) == 0 && *(volatile unsigned*)(g.words + 1))) {
+          atomicExch(g.words + 1, 1u);
+          ok = 0;
+          break;
+        }
       }
-      const bool out = spins > kRunSpins || ((spins & 1023u) == 1023u && *(volatile unsigned*)(g.words + 1));
-      if (__any_sync(0xffffffffu, out)) {
-        if (threadIdx.x == 0) atomicExch(g.words + 1, 1u);
-        ok = false;
-        break;
-      }
+      __threadfence();
     }
-    __threadfence();
-    return ok;
+    return __shfl_sync(0xffffffffu, ok, 0) != 0;
   }
-  __device__ __forceinline__ bool wait(int wid) { return wid ? true : poll(g.words, target, threadIdx.x == 0); }
   template <int NV>
   __device__ __forceinline__ void collect(int wid, double* wsum, double (&t)[NV]) {
     if (wid < 4) {
@@ -195,28 +186,6 @@ struct GridGroup {
       quad_total<NV>(lanes_sum<L>(s), wsum, t);
     }
     par ^= 1;
-  }
-  // The barrier that ends an iteration, before the next gathers: where a
-  // block gathers from at most 32 blocks around its own it waits for those
-  // alone (a flag each); a block rewrites its rows of the direction only after
-  // two more sums, which every block enters after its gathers.
-  __device__ __forceinline__ void arrive_halo(int wid) {
-    if (!g.neighbours) {
-      arrive(wid);
-      return;
-    }
-    ++epoch;
-    if (threadIdx.x == 0) {
-      __threadfence();
-      asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(g.words + kRunFlag0 + blockIdx.x * kRunFlagStride), "r"(epoch)
-                   : "memory");
-    }
-  }
-  __device__ __forceinline__ bool wait_halo(int wid) {
-    if (!g.neighbours) return wait(wid);
-    if (wid) return true;
-    const int b = halo.x + (int)threadIdx.x;
-    return poll(g.words + kRunFlag0 + b * kRunFlagStride, epoch, b <= halo.y);
   }
   static constexpr bool kCluster = false;
 };
@@ -264,69 +233,59 @@ __device__ __forceinline__ void block_sums(T (&v)[NV], double* part, double* wsu
   }
 }
 
-// A gathered entry of the direction: x[c], or z[c] + beta x[c] when the new
-// direction is formed where it is gathered (TWO).  Plain loads: other blocks
-// rewrite both between the group's barriers, whose acquire refreshes L1.
 template <typename T>
 __device__ __forceinline__ T axpy(T b, T x, T z) {
   return sizeof(T) == 4 ? (T)fmaf((float)b, (float)x, (float)z) : (T)fma((double)b, (double)x, (double)z);
 }
-template <typename T, bool TWO>
-__device__ __forceinline__ T gather(const T* x, const T* z, T beta, int c) {
-  return TWO ? axpy<T>(beta, x[c], z[c]) : x[c];
-}
 
 // U entries of a row from entry j on: the columns and values of all of them
-// are loaded before the gathers, so that U gathers are in flight.  With TAIL
-// the entries beyond w are left out (w is the same in all lanes).
-template <typename T, bool D16, bool DIFF, bool MS, bool TWO, int U, bool TAIL, typename C>
-__device__ __forceinline__ void run_part(const T* v, const C* cols, int base, int j, int w, int64_t row, const T* x,
-                                         const T* z, T beta, T xi, T (&a)[4]) {
+// are loaded before the gathers, so that U gathers are in flight.  DIFF: each
+// term is a_ij (x_j - x_i) (the diagonal slot, which holds the row sum, adds
+// nothing: the caller adds it times x_i).
+template <typename T, bool D16, bool DIFF, bool MS, int U, typename C, class X>
+__device__ __forceinline__ void run_part(const T* v, const C* cols, int row, const X& x, T xi, T (&a)[4]) {
   int cc[U];
   T vv[U], xx[U];
 #pragma unroll
-  for (int u = 0; u < U; ++u)
-    if (!TAIL || j + u < w) {
-      const C c = MS ? cols[base + 32 * (j + u)] : __ldcg(cols + base + 32 * (j + u));
-      cc[u] = D16 ? (int)row + (int)c : (int)c;
-    }
+  for (int u = 0; u < U; ++u) {
+    const C c = MS ? cols[32 * u] : __ldcg(cols + 32 * u);
+    cc[u] = D16 ? row + (int)c : (int)c;
+  }
 #pragma unroll
-  for (int u = 0; u < U; ++u)
-    if (!TAIL || j + u < w) vv[u] = MS ? v[base + 32 * (j + u)] : __ldcg(v + base + 32 * (j + u));
+  for (int u = 0; u < U; ++u) vv[u] = MS ? v[32 * u] : __ldcg(v + 32 * u);
 #pragma unroll
-  for (int u = 0; u < U; ++u)
-    if (!TAIL || j + u < w) xx[u] = xterm<T, DIFF>(gather<T, TWO>(x, z, beta, cc[u]), cc[u], row, xi);
+  for (int u = 0; u < U; ++u) xx[u] = DIFF ? x[cc[u]] - xi : x[cc[u]];
 #pragma unroll
-  for (int u = 0; u < U; ++u)
-    if (!TAIL || j + u < w) a[u & 3] += vv[u] * xx[u];
+  for (int u = 0; u < U; ++u) a[u & 3] += vv[u] * xx[u];
 }
 
-// One row of a slice, the matrix in shared memory (MS: v, cols and base are
-// the block's copies) or in global memory.  FP32 takes a predicated tail; an
-// FP64 multiply-add costs the same left out by a predicate, so FP64 takes the
-// tail in parts of 4, 2 and 1 (N = 180 quadratic heat: 8.0k cycles a product
-// with the predicated tail, 6.4k so).
-template <typename T, bool D16, bool DIFF, bool MS, bool TWO, typename C>
-__device__ __forceinline__ T run_row(const T* v, const C* cols, int base, int w, int64_t row, const T* x, const T* z,
-                                     T beta, T xi) {
+// One row of a slice (its lane's first entry at v, cols; w entries 32 apart),
+// the matrix in shared memory (MS) or in global memory.  x is addressed by row
+// numbers as they are stored (for a window in shared memory, by its address
+// less the window's first row); other blocks rewrite a global x between the
+// group's barriers, whose acquire refreshes L1 (plain loads).  X: a pointer,
+// or SplitX.  The tail goes in parts of 4, 2 and 1 without predicates: the
+// product is bound by instruction issue (and in FP64 a multiply-add left out
+// by a predicate costs what it costs).
+template <typename T>
+struct SplitX {  // the two parts of a window: rows below and from `lo2` on
+  const T *a, *b;
+  int lo2;
+  __device__ __forceinline__ T operator[](int c) const { return (c < lo2 ? a : b)[c]; }
+};
+template <typename T, bool D16, bool DIFF, bool MS, typename C, class X>
+__device__ __forceinline__ T run_row(const T* v, const C* cols, int w, int row, const X& x, T xi) {
   T a[4] = {0, 0, 0, 0};
-  constexpr int U = sizeof(T) == 4 ? 10 : 8;
-  int j = 0;
-#define RUN_PART(n, tail) run_part<T, D16, DIFF, MS, TWO, n, tail, C>(v, cols, base, j, w, row, x, z, beta, xi, a)
-  for (; j + U <= w; j += U) RUN_PART(U, false);
-  if (sizeof(T) == 4) {
-    if (j < w) RUN_PART(U, true);
-  } else {
-    if ((w - j) & 4) {
-      RUN_PART(4, false);
-      j += 4;
-    }
-    if ((w - j) & 2) {
-      RUN_PART(2, false);
-      j += 2;
-    }
-    if ((w - j) & 1) RUN_PART(1, false);
-  }
+#define RUN_PART(n)                                           \
+  do {                                                        \
+    run_part<T, D16, DIFF, MS, n, C, X>(v, cols, row, x, xi, a); \
+    v += 32 * n;                                              \
+    cols += 32 * n;                                           \
+  } while (0)
+  for (int j = w >> 3; j > 0; --j) RUN_PART(8);
+  if (w & 4) RUN_PART(4);
+  if (w & 2) RUN_PART(2);
+  if (w & 1) RUN_PART(1);
 #undef RUN_PART
   return (a[0] + a[1]) + (a[2] + a[3]);
 }
@@ -347,8 +306,8 @@ struct RunRows {
   const T* mv;
   const C* mc;
   const int2* sbw;
-  // sbw_sh: room for spb slices, followed by the matrix (MS)
-  __device__ __forceinline__ RunRows(const SellView& A, const T* v, int block, int spb, int max_entries, int2* sbw_sh) {
+  // sbw_sh: spb slices, followed by `room` entries of the matrix (MS)
+  __device__ __forceinline__ RunRows(const SellView& A, const T* v, int block, int spb, int room, int2* sbw_sh) {
     const int tid = threadIdx.x;
     const int64_t s0 = (int64_t)block * spb;
     nsl = (int)max((int64_t)0, min((int64_t)spb, A.nslices - s0));
@@ -363,7 +322,7 @@ struct RunRows {
     mc = gc;
     if (MS) {
       T* sv = reinterpret_cast<T*>(sbw_sh + spb);
-      C* sc = reinterpret_cast<C*>(sv + max_entries);
+      C* sc = reinterpret_cast<C*>(sv + room);
       const int ne = nsl > 0 ? (int)(A.sptr[s0 + nsl] - e0) : 0;
       for (int k = tid; k < ne; k += kRT) {
         sv[k] = gv[k];
@@ -380,11 +339,62 @@ struct RunRows {
     const int win = n * (kRW / 8) + (wid >> 3);
     return win * 8 + ((wid - 2 * win) & 7);
   }
-  // (A p)_i of local row i in slice s; p = x, or z + beta x (TWO); xi: p_i
-  template <bool DIFF, bool TWO>
-  __device__ __forceinline__ T row(int s, int i, const T* x, const T* z, T beta, T xi) const {
+  // (A x)_i of local row i in slice s; xi: x_i (DIFF: less the row sum times x_i)
+  template <bool DIFF, class X>
+  __device__ __forceinline__ T row(int s, int i, const X& x, T xi) const {
     const int2 bw = sbw[s];
-    return run_row<T, D16, DIFF, MS, TWO, C>(mv, mc, bw.x + (i & 31), bw.y, row0 + i, x, z, beta, xi);
+    const int k = bw.x + (i & 31);
+    return run_row<T, D16, DIFF, MS, C, X>(mv + k, mc + k, bw.y, (int)row0 + i, x, xi);
+  }
+};
+
+// The gathered vector of a block: the rows that its columns lie in (its own
+// among them), in shared memory: one range, or two with a gap between them
+// (velocity and pressure unknowns).  The block advances all of them itself:
+// x = z + beta x (CG) or x = beta z (MINRES), with z of its own rows from
+// shared memory and of the others from global memory, where their owners have
+// put it before the group's last sum.  The same operations on the same
+// operands as the owner's: the same bits.  So only z travels, a product
+// gathers from shared memory alone, and the vector needs no barrier of its own.
+template <typename T>
+struct Window {
+  T* x;
+  int lo1, n1, lo2, n, own, nown;  // rows [lo1, lo1 + n1), then [lo2, lo2 + n - n1); own rows from x[own] on
+  // w: both ranges (see WinArgs in solve.cu); split: keep them apart
+  __device__ __forceinline__ Window(T* sh, int4 w, bool split, int row0, int nloc) : x(sh), nown(nloc) {
+    lo1 = w.x;
+    n1 = (split ? w.y : w.w) - w.x;
+    lo2 = split ? w.z : w.w;
+    n = n1 + w.w - lo2;
+    own = row0 < lo1 + n1 ? row0 - lo1 : n1 + row0 - lo2;
+    if (nloc == 0) n = n1 = own = 0;
+  }
+  __device__ __forceinline__ const T* by_row() const { return x - lo1; }
+  __device__ __forceinline__ SplitX<T> by_row_split() const { return SplitX<T>{x - lo1, x + n1 - lo2, lo2}; }
+  __device__ __forceinline__ int row(int j) const { return j < n1 ? lo1 + j : lo2 + (j - n1); }
+  __device__ __forceinline__ void load(const T* g) {
+    for (int j = threadIdx.x; j < n; j += kRT) x[j] = g[row(j)];
+  }
+  // mine: z of the own rows; g: z of all rows; CG: x = z + beta x, else x = beta z
+  template <bool CG>
+  __device__ __forceinline__ void advance(const T* mine, const T* g, T beta) {
+    const int nh = n - nown;  // rows of others: x[0, own) and x[own + nown, n)
+    constexpr int U = 4;
+    for (int h0 = threadIdx.x; h0 < nh; h0 += U * kRT) {
+      T zz[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int h = h0 + u * kRT, j = h < own ? h : h + nown;
+        if (h < nh) zz[u] = g[row(j)];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int h = h0 + u * kRT, j = h < own ? h : h + nown;
+        if (h < nh) x[j] = CG ? axpy<T>(beta, x[j], zz[u]) : zz[u] * beta;
+      }
+    }
+    for (int i = threadIdx.x; i < nown; i += kRT)
+      x[own + i] = CG ? axpy<T>(beta, x[own + i], mine[i]) : mine[i] * beta;
   }
 };
 

@@ -660,11 +660,12 @@ __global__ void sell_vals_k(int64_t npad, const int32_t* __restrict__ map, const
   }
 }
 
-// FP32 values in difference form: each row's diagonal slot gets the row sum
-// s_i = sum_j a_ij (added in FP64, rounded once); the other slots keep a_ij.
+// FP32 values in difference form: each row's diagonal slot, and rowsum, get the
+// row sum s_i = sum_j a_ij (added in FP64, rounded once); the other slots keep
+// a_ij.
 template <bool D16>
 __global__ void sell_rowsum_k(SellView A, const int32_t* __restrict__ map, const double* __restrict__ v64,
-                              float* __restrict__ v32) {
+                              float* __restrict__ v32, float* __restrict__ rowsum) {
   for (int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; row < A.nrows;
        row += (int64_t)gridDim.x * blockDim.x) {
     const int64_t s = row >> 5;
@@ -680,6 +681,7 @@ __global__ void sell_rowsum_k(SellView A, const int32_t* __restrict__ map, const
       if ((int64_t)c == row) dpos = k;
     }
     if (dpos >= 0) v32[dpos] = (float)sum;
+    rowsum[row] = dpos >= 0 ? (float)sum : 0.0f;
   }
 }
 
@@ -755,29 +757,71 @@ __global__ void block_entries_k(int64_t nsl, const int64_t* __restrict__ sptr, c
   }
 }
 
-// halo[b] = the first and last block that block b's columns lie in (blocks of
-// spb slices; one CTA each); *most = the largest number of blocks between them.
-__global__ void block_halo_k(int64_t nsl, const int64_t* __restrict__ sptr, int spb, const int32_t* __restrict__ col,
-                             int2* __restrict__ halo, int* __restrict__ most) {
-  __shared__ int lo, hi;
-  const int64_t s0 = (int64_t)blockIdx.x * spb;
+// Column windows of the blocks of the divisions (krylov.cuh): win[off[q] + b] =
+// {lo1, hi1, lo2, hi2}: the rows that the columns and rows of block b of
+// division q lie in, [lo1, hi2) in one range, or [lo1, hi1) and [lo2, hi2) with
+// the widest gap left out (to a 256th of the range); widest[q], widest[4 + q] =
+// the most rows of one, of two.  One CTA per block (blockIdx.y: q).
+struct WinArgs {
+  int spb[4], off[4];
+};
+__global__ void __launch_bounds__(256) block_window_k(int64_t nu, int64_t nsl, const int64_t* __restrict__ sptr,
+                                                      const int32_t* __restrict__ sw, const int32_t* __restrict__ col,
+                                                      const WinArgs w, int4* __restrict__ win, int* widest) {
+  constexpr int B = 256;
+  __shared__ unsigned lo, hi, first[B], last[B];
+  const int q = blockIdx.y, spb = w.spb[q];
+  const int64_t s0 = (int64_t)blockIdx.x * spb, s1 = min(s0 + spb, nsl);
+  if (s0 >= nsl) return;
+  const unsigned own0 = (unsigned)(s0 * 32), own1 = (unsigned)min(s1 * 32, nu);  // own rows
+  const int lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    lo = 0x7fffffff;
-    hi = 0;
+    lo = own0;
+    hi = own1 - 1;
+  }
+  first[threadIdx.x] = 0xffffffffu;
+  last[threadIdx.x] = 0;
+  __syncthreads();
+  unsigned a = 0xffffffffu, z = 0;
+  for (int64_t s = s0 + (threadIdx.x >> 5); s < s1; s += blockDim.x / 32)
+    if (s * 32 + lane < nu)
+      for (int j = 0; j < sw[s]; ++j) {
+        const unsigned c = (unsigned)col[sptr[s] + lane + (int64_t)j * 32];
+        a = min(a, c);
+        z = max(z, c);
+      }
+  a = __reduce_min_sync(0xffffffffu, a);
+  z = __reduce_max_sync(0xffffffffu, z);
+  if (lane == 0) {
+    atomicMin(&lo, a);
+    atomicMax(&hi, z);
   }
   __syncthreads();
-  int a = 0x7fffffff, z = 0;
-  for (int64_t k = sptr[s0] + threadIdx.x; k < sptr[min(s0 + spb, nsl)]; k += blockDim.x) {
-    a = min(a, col[k]);
-    z = max(z, col[k]);
-  }
-  atomicMin(&lo, (int)__reduce_min_sync(0xffffffffu, (unsigned)a));
-  atomicMax(&hi, (int)__reduce_max_sync(0xffffffffu, (unsigned)z));
+  // the rows of each 256th of the range that occur
+  const unsigned l0 = lo, len = hi + 1 - lo, bin = (len + B - 1) / B;
+  auto mark = [&](unsigned c) {
+    const unsigned k = (c - l0) / bin;
+    if (c < first[k]) atomicMin(&first[k], c);
+    if (c > last[k]) atomicMax(&last[k], c);
+  };
+  for (unsigned r = own0 + threadIdx.x; r < own1; r += B) mark(r);
+  for (int64_t s = s0 + (threadIdx.x >> 5); s < s1; s += blockDim.x / 32)
+    if (s * 32 + lane < nu)
+      for (int j = 0; j < sw[s]; ++j) mark((unsigned)col[sptr[s] + lane + (int64_t)j * 32]);
   __syncthreads();
   if (threadIdx.x == 0) {
-    const int2 h = make_int2(min(lo, (int)s0 * 32) / (32 * spb), max(hi, (int)s0 * 32) / (32 * spb));
-    halo[blockIdx.x] = h;
-    atomicMax(most, h.y - h.x + 1);
+    unsigned end = l0, hi1 = hi + 1, lo2 = hi + 1;  // end: the rows seen so far
+    for (int k = 0; k < B; ++k) {
+      if (first[k] == 0xffffffffu) continue;
+      if (end > l0 && first[k] - end > lo2 - hi1) {
+        hi1 = end;
+        lo2 = first[k];
+      }
+      end = last[k] + 1;
+    }
+    win[w.off[q] + blockIdx.x] = make_int4((int)l0, (int)hi1, (int)lo2, (int)hi + 1);
+    atomicMax(widest + q, (int)len);
+    atomicMax(widest + 4 + q, (int)(len - (lo2 - hi1)));
   }
 }
 
@@ -810,26 +854,27 @@ static int build_sell(Ctx* c, SolverData* S) {
   const size_t np = (size_t)(A.nnz_pad > 0 ? A.nnz_pad : 1);
   ELFEL_TRY(col.alloc(c, np));
   ELFEL_TRY(A.map.alloc(c, np));
-  // a column delta beyond 16 bits; the widest halo; the largest blocks' entries
-  ELFEL_TRY(wide.alloc(c, 6));
-  ELFEL_CUDA(c, cudaMemsetAsync(wide.p, 0, 6 * sizeof(int), c->stream));
-  const SpbList spbs{{run_spb_cluster(nsl), run_spb_grid(c, nsl), run_spb_batch(nsl, 4), run_spb_batch(nsl, 8)}};
-  block_entries_k<<<1, 256, 0, c->stream>>>(nsl, A.sptr.p, spbs, wide.p + 2);
+  // a column delta beyond 16 bits; the largest blocks' entries; the widest windows
+  ELFEL_TRY(wide.alloc(c, 13));
+  ELFEL_CUDA(c, cudaMemsetAsync(wide.p, 0, 13 * sizeof(int), c->stream));
+  const SpbList spbs{{run_spb_grid(c, nsl), run_spb_cluster(nsl), run_spb_batch(nsl, 4), run_spb_batch(nsl, 8)}};
+  block_entries_k<<<1, 256, 0, c->stream>>>(nsl, A.sptr.p, spbs, wide.p + 1);
   sell_fill_k<<<grid_for(nsl * 32, 256, (int64_t)c->sm_count * 16), 256, 0, c->stream>>>(
       nu, nsl, S->ff.rowptr.p, S->ff.col.p, S->ff.map.p, A.perm.p, iperm.p, A.sptr.p, A.sw.p, col.p, A.map.p, wide.p);
   ELFEL_LAUNCH_CHECK(c);
-  const int spb = run_spb_grid(c, nsl);
-  const unsigned ngb = (unsigned)((nsl + spb - 1) / spb);
-  ELFEL_TRY(S->run_halo.alloc(c, ngb));
   if (nu <= kRunGridRows) {
-    block_halo_k<<<ngb, 512, 0, c->stream>>>(nsl, A.sptr.p, spb, col.p, S->run_halo.p, wide.p + 1);
+    // the cluster and batch divisions serve small systems only
+    const bool small = nu <= kRunSmallRows;
+    const WinArgs wa{{spbs.v[0], spbs.v[1], spbs.v[2], spbs.v[3]}, {kRunWinGrid, 0, kRunWinBatch32, kRunWinBatch64}};
+    block_window_k<<<dim3(kRunMaxBlocks, small ? 4 : 1), 256, 0, c->stream>>>(nu, nsl, A.sptr.p, A.sw.p, col.p, wa,
+                                                                              S->run_win.p, wide.p + 5);
     ELFEL_LAUNCH_CHECK(c);
   }
-  int hw[6] = {0, 0, 0, 0, 0, 0};
+  int hw[13] = {0};
   ELFEL_CUDA(c, cudaMemcpyAsync(hw, wide.p, sizeof(hw), cudaMemcpyDeviceToHost, c->stream));
   ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
-  for (int q = 0; q < 4; ++q) S->run_entries[q] = hw[2 + q];
-  S->run_neighbours = hw[1] >= 1 && hw[1] <= 32;
+  for (int q = 0; q < 4; ++q) S->run_entries[q] = hw[1 + q];
+  for (int q = 0; q < 8; ++q) S->run_window[q] = hw[5 + q];
   wide.release(c);
   iperm.release(c);
   if (!hw[0]) {
@@ -912,12 +957,14 @@ int build_solver(elfel_sysmat* m, int64_t nu) {
   R.release(c);
   nff.release(c); nfd.release(c); pff.release(c); pfd.release(c);
   S->nu = nu;
+  ELFEL_TRY(S->run_win.alloc(c, kRunWins));
   if (nu > 0) ELFEL_TRY(build_sell(c, S));
   const size_t vn = (size_t)(nu > 0 ? nu : 1);
   for (DBuf<double>* b : {&S->bo64, &S->xo64, &S->ro64, &S->dinvo, &S->dinv64, &S->b64, &S->x64, &S->r64, &S->z64,
                           &S->p64, &S->q64, &S->y64})
     ELFEL_TRY(b->alloc(c, vn));
-  for (DBuf<float>* b : {&S->dinv32, &S->r32, &S->p32, &S->q32, &S->z32, &S->xa32, &S->zz32, &S->b32, &S->x32})
+  for (DBuf<float>* b : {&S->dinv32, &S->r32, &S->p32, &S->q32, &S->z32, &S->xa32, &S->zz32, &S->b32, &S->x32,
+                        &S->rowsum32})
     ELFEL_TRY(b->alloc(c, vn));
   ELFEL_TRY(S->T64.alloc(c, (size_t)(n > 0 ? n : 1)));
   ELFEL_TRY(S->scal.alloc(c, S_COUNT));
@@ -925,7 +972,7 @@ int build_solver(elfel_sysmat* m, int64_t nu) {
   ELFEL_TRY(S->red.alloc(c, (size_t)3 * kMaxRedBlocks * 4));
   ELFEL_TRY(S->tickets.alloc(c, 4));
   ELFEL_TRY(S->run_slots.alloc(c, (size_t)2 * 3 * kRunMaxBlocks));
-  ELFEL_TRY(S->run_bar.alloc(c, kRunWords));
+  ELFEL_TRY(S->run_bar.alloc(c, 2));
   ELFEL_CUDA(c, cudaMemsetAsync(S->tickets.p, 0, sizeof(unsigned) * 4, c->stream));
   ELFEL_CUDA(c, cudaMemsetAsync(S->scal.p, 0, sizeof(double) * S_COUNT, c->stream));
   ELFEL_CUDA(c, cudaMemsetAsync(S->flags.p, 0, sizeof(int) * F_COUNT, c->stream));
@@ -956,10 +1003,10 @@ int refresh_values(elfel_sysmat* m, int abs_diag, int diff32) {
     const SellView V = S->view();
     if (S->A.d16)
       sell_rowsum_k<true><<<grid_for(nu, 256, (int64_t)c->sm_count * 16), 256, 0, c->stream>>>(
-          V, S->A.map.p, S->A.v64.p, S->A.v32.p);
+          V, S->A.map.p, S->A.v64.p, S->A.v32.p, S->rowsum32.p);
     else
       sell_rowsum_k<false><<<grid_for(nu, 256, (int64_t)c->sm_count * 16), 256, 0, c->stream>>>(
-          V, S->A.map.p, S->A.v64.p, S->A.v32.p);
+          V, S->A.map.p, S->A.v64.p, S->A.v32.p, S->rowsum32.p);
   }
   const double* aux = (m->fused && m->F.physics == ELFEL_STOKES) ? m->F.pmass_diag.p : nullptr;
   if (nu > 0) {
@@ -1123,7 +1170,7 @@ static int run_pcg64(elfel_sysmat* m, double rtol, int maxit, elfel_solve_stats*
   cg_start_k<double><<<vg, kBlk, 0, c->stream>>>(nu, S->r64.p, S->z64.p, S->p64.p, S->dinv64.p, red_area(S, 0),
                                                  S->scal.p, S->flags.p, 1, 1.0);
   ELFEL_LAUNCH_CHECK(c);
-  const RunPlan run = run_plan(c, S, sizeof(double), 5);
+  const RunPlan run = run_plan(c, S, sizeof(double), 4, 4, 0);
   if (!run.blocks) ELFEL_TRY(capture(c, &S->g_pcg64, [&]() {
     launch_cg_spmv<double, false, false>(c, S, S->A.v64.p, S->p64.p, S->q64.p, nullptr, red_area(S, 0), S_PQ);
     launch_pdl(cg_update_k<double, false>, vg, kBlk, c->stream, nu, S->x64.p, S->r64.p, S->p64.p, S->q64.p, S->z64.p,
@@ -1189,7 +1236,7 @@ static int run_pcg32(elfel_sysmat* m, double rtol, int maxit, elfel_solve_stats*
   cg_start_k<float><<<vg, kBlk, 0, c->stream>>>(nu, S->r32.p, S->z32.p, S->p32.p, S->dinv32.p, red_area(S, 0),
                                                 S->scal.p, S->flags.p, 1, 1.0f);
   ELFEL_LAUNCH_CHECK(c);
-  const RunPlan run = run_plan(c, S, sizeof(float), 5);
+  const RunPlan run = run_plan(c, S, sizeof(float), 5, 4, 0);
   if (!run.blocks) ELFEL_TRY(capture(c, &S->g_pcg32, [&]() {
     launch_cg_spmv<float, true, true>(c, S, S->A.v32.p, S->p32.p, S->q32.p, S->r32.p, red_area(S, 0), S_PQ);
     launch_pdl(cg_update_k<float, true>, vg, kBlk, c->stream, nu, S->xa32.p, S->r32.p, S->p32.p, S->q32.p, S->z32.p,
@@ -1279,7 +1326,7 @@ static int run_minres(Ctx* c, SolverData* S, const T* v, const T* minv, const T*
   mr_start_k<T><<<vg, kBlk, 0, c->stream>>>(nu, b, vb, zb, wb, minv, x, red_area(S, 0), S->scal.p, S->flags.p);
   scale_k<T><<<vg, kBlk, 0, c->stream>>>(nu, zb, S->scal.p);
   ELFEL_LAUNCH_CHECK(c);
-  const RunPlan run = run_plan(c, S, sizeof(T), 8);
+  const RunPlan run = run_plan(c, S, sizeof(T), 7, 7, 1);
   if (!run.blocks) ELFEL_TRY(capture(c, graph, [&]() {
     launch_mr_spmv<T>(c, S, v, zb, q, red_area(S, 0));
     mr_vec_k<T><<<vg, kBlk, 0, c->stream>>>(nu, q, vb, zb, minv, red_area(S, 1), S->scal.p, S->flags.p);

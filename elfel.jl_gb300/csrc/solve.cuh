@@ -86,20 +86,21 @@ struct SolverData {
   DBuf<double> T64, bo64, xo64, ro64, dinvo;
   // permuted order
   DBuf<double> dinv64, b64, x64, r64, z64, p64, q64, y64;
-  DBuf<float> dinv32, r32, p32, q32, z32, xa32, zz32, b32, x32;
+  DBuf<float> dinv32, r32, p32, q32, z32, xa32, zz32, b32, x32, rowsum32;
   DBuf<double> v64[3], w64[3];
   DBuf<float> v32[3], w32[3];
   DBuf<double> scal;
   DBuf<int> flags;
   DBuf<double> red;  // 3 reduction areas
   DBuf<unsigned> tickets;
-  // one-launch iterations (krylov.cu): the largest block's stored entries of
-  // each division (run_spb_*); the grid group's memory (RunGroup)
+  // one-launch iterations (krylov.cu): the largest block's stored entries and
+  // column window of each division (run_spb_*); the grid group's memory
+  // (RunGroup) and the blocks' windows
   int run_entries[4] = {0, 0, 0, 0};
-  int run_neighbours = 0;
+  int run_window[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   DBuf<double> run_slots;
   DBuf<unsigned> run_bar;
-  DBuf<int2> run_halo;
+  DBuf<int4> run_win;
   cudaGraphExec_t g_pcg64 = nullptr, g_pcg32 = nullptr, g_minres64 = nullptr, g_minres32 = nullptr;
   SellView view() const {
     return SellView{A.nrows, A.nslices, A.sptr.p, A.sw.p, A.d16 ? A.dcol.p : nullptr, A.d16 ? nullptr : A.col.p};
@@ -108,9 +109,9 @@ struct SolverData {
     ff.release(c); fd.release(c); A.release(c);
     for (DBuf<double>* b : {&T64, &bo64, &xo64, &ro64, &dinvo, &dinv64, &b64, &x64, &r64, &z64, &p64, &q64, &y64})
       b->release(c);
-    for (DBuf<float>* b : {&dinv32, &r32, &p32, &q32, &z32, &xa32, &zz32, &b32, &x32}) b->release(c);
+    for (DBuf<float>* b : {&dinv32, &r32, &p32, &q32, &z32, &xa32, &zz32, &b32, &x32, &rowsum32}) b->release(c);
     for (int i = 0; i < 3; ++i) { v64[i].release(c); w64[i].release(c); v32[i].release(c); w32[i].release(c); }
-    scal.release(c); flags.release(c); red.release(c); tickets.release(c); run_slots.release(c); run_bar.release(c); run_halo.release(c);
+    scal.release(c); flags.release(c); red.release(c); tickets.release(c); run_slots.release(c); run_bar.release(c); run_win.release(c);
     for (cudaGraphExec_t* g : {&g_pcg64, &g_pcg32, &g_minres64, &g_minres32})
       if (*g) { cudaGraphExecDestroy(*g); *g = nullptr; }
   }
