@@ -84,6 +84,9 @@ struct ShapeTab {
   double G[kMaxQP][4][2];  // Q4 only (T4 gradients are constant)
   double P[4];
   double W;
+  // Q4: the rule is the 2 x 2 one at (+-g, +-g) with equal weights w[0]
+  int gauss2;
+  double g;
 };
 int make_shape_tables(int shape, int npts, const double* pc, const double* w, ShapeTab* t);
 // Element records of the heat weak form on Q4 (xy: nnodes x 2) or T4 (xy:

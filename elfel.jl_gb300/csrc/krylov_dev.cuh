@@ -4,6 +4,7 @@
 #pragma once
 #include <cooperative_groups.h>
 
+#include "fastdiv64.cuh"
 #include "krylov.cuh"
 
 namespace elfel {
@@ -29,24 +30,6 @@ __device__ __forceinline__ double lanes_sum(double s) {
 #pragma unroll
   for (int o = L / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   return s;
-}
-
-// 1 / x by Newton's iteration from the hardware's 20-bit estimate (four FP64
-// operations; the compiler's division takes about twelve, 64 cycles each).
-// x of extreme exponent goes through the division.
-__device__ __forceinline__ double fast_rcp(double x) {
-  const int e = (int)((__double_as_longlong(x) >> 52) & 0x7ff);
-  if (e < 60 || e > 1980) return 1.0 / x;
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = fma(y, fma(-x, y, 1.0), y);
-  return fma(y, fma(-x, y, 1.0), y);
-}
-
-// a / x, y = fast_rcp(x): the quotient corrected by its remainder.
-__device__ __forceinline__ double fast_div(double a, double x, double y) {
-  const double q = a * y;
-  return fma(fma(-x, q, a), y, q);
 }
 
 // x > 0 and finite, a <= b, a < b for nonnegative a, b (and NaN above all of
