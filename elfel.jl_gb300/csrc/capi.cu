@@ -1,6 +1,8 @@
 // C ABI: SysmatAssemblerSparse (COO mode), SysvecAssembler, fused assembly.
 #include <math.h>
 
+#include <algorithm>
+
 #include "integrate.cuh"
 #include "solve.cuh"
 #include "sysmat.cuh"
@@ -162,6 +164,7 @@ static void release_all(elfel_sysmat* m) {
   m->fused = 0;
   m->finished = 0;
   m->pattern_recorded = 0;
+  m->head.nnz = 0;
 }
 
 // Marks m->P complete at this point of the context stream.
@@ -181,6 +184,7 @@ extern "C" int elfel_sysmat_destroy(elfel_sysmat* m) {
     release_all(m);
     cudaStreamSynchronize(m->h->c.stream);
     if (m->ev_pattern) cudaEventDestroy(m->ev_pattern);
+    if (m->head.ev) cudaEventDestroy(m->head.ev);
   }
   delete stage_of(m);
   delete m;
@@ -291,8 +295,20 @@ extern "C" int elfel_sysmat_csc(elfel_sysmat* m, int64_t* colptr, int64_t* rowva
   if (!colptr && !rowval) {
     // the values of a pattern the caller has already: no index arrays are formed
     // (2M quadratic triangles: 0.12 ms of a 2.6 ms re-assembly and download)
-    if (nzval && nnz)
+    int pin_v = 0;
+    const int64_t head = nzval && host_device_ptr(c, nzval, &pin_v) && pin_v ? std::min(m->head.nnz, nnz) : 0;
+    if (head) {
+      // the head of the values leaves on the auxiliary stream as soon as it is
+      // reduced, the rest behind it once the context stream has come so far
+      cudaStream_t s;
+      ELFEL_TRY(aux_after(c, m->head.ev, &s));
+      ELFEL_CUDA(c, cudaMemcpyAsync(nzval, m->vals.p, sizeof(double) * head, cudaMemcpyDeviceToHost, s));
+      ELFEL_CUDA(c, cudaMemcpyAsync(nzval + head, m->vals.p + head, sizeof(double) * (nnz - head),
+                                    cudaMemcpyDeviceToHost, c->stream));
+      ELFEL_TRY(aux_join(c));
+    } else if (nzval && nnz) {
       ELFEL_CUDA(c, cudaMemcpyAsync(nzval, m->vals.p, sizeof(double) * nnz, cudaMemcpyDeviceToHost, c->stream));
+    }
     ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
     return ELFEL_OK;
   }
@@ -850,12 +866,22 @@ int elfel::ensure_fpat(elfel_sysmat* m) {
   return ELFEL_OK;
 }
 
+// The head of the system's next reduction (its event is created once).
+static int head_of(elfel_sysmat* m, Head** h) {
+  if (!m->head.ev) ELFEL_CUDA(&m->h->c, cudaEventCreateWithFlags(&m->head.ev, cudaEventDisableTiming));
+  m->head.nnz = 0;
+  *h = &m->head;
+  return ELFEL_OK;
+}
+
 // rhs_done: the integration kernel already added the load vector into rhs.
 static int finish_values(elfel_sysmat* m, bool rhs_done = false) {
   Ctx* c = &m->h->c;
   {
+    Head* head;
+    ELFEL_TRY(head_of(m, &head));
     Phase ph(c, "reduce_K");
-    ELFEL_TRY(reduce_values(c, m->P, m->F.kstore.p, m->vals.p));
+    ELFEL_TRY(reduce_values(c, m->P, m->F.kstore.p, m->vals.p, head));
   }
   if (!rhs_done) {
     ELFEL_TRY(ensure_fpat(m));
@@ -896,8 +922,10 @@ extern "C" int elfel_fused_heat(elfel_sysmat* m, const double* kappa, double Q) 
                                   fdirect ? F.dofs_u.p : nullptr, fdirect ? m->rhs.p : nullptr));
     }
     {
+      Head* head;
+      ELFEL_TRY(head_of(m, &head));
       Phase ph(c, "reduce_K");
-      ELFEL_TRY(tile_reduce(c, m->P, F.kstore.p, 1, m->vals.p));
+      ELFEL_TRY(tile_reduce(c, m->P, F.kstore.p, 1, m->vals.p, head));
     }
     m->P.reductions++;
     if (!fdirect) {
@@ -1015,8 +1043,10 @@ extern "C" int elfel_fused_stokes(elfel_sysmat* m, double mu) {
     ELFEL_TRY(launch_stokes(c, F.nel, F.conn_u.p, F.xy_u.p, mu, F.ncurved, F.tab, F.kstore.p, F.pmass_store.p));
   }
   {
+    Head* head;
+    ELFEL_TRY(head_of(m, &head));
     Phase ph(c, "reduce_K");
-    ELFEL_TRY(reduce_values(c, m->P, F.kstore.p, m->vals.p));
+    ELFEL_TRY(reduce_values(c, m->P, F.kstore.p, m->vals.p, head));
   }
   ELFEL_CUDA(c, cudaMemsetAsync(m->rhs.p, 0, sizeof(double) * m->nrow, c->stream));
   ELFEL_TRY(reduce_dense(c, F.pmpat, F.pmass_store.p, F.pmass_diag.p));

@@ -243,12 +243,20 @@ extern "C" int elfel_ctx_create(int device, int64_t mem_budget_bytes, elfel_ctx*
 
 namespace elfel {
 
+// The auxiliary stream's blocks go first where both streams have some waiting:
+// what it does (uploads, the head of the values) is what something waits for.
+static int aux_create(Ctx* c) {
+  if (c->aux) return ELFEL_OK;
+  int least = 0, greatest = 0;
+  ELFEL_CUDA(c, cudaDeviceGetStreamPriorityRange(&least, &greatest));
+  ELFEL_CUDA(c, cudaStreamCreateWithPriority(&c->aux, cudaStreamNonBlocking, greatest));
+  ELFEL_CUDA(c, cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
+  ELFEL_CUDA(c, cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
+  return ELFEL_OK;
+}
+
 int aux_fork(Ctx* c, cudaStream_t* aux) {
-  if (!c->aux) {
-    ELFEL_CUDA(c, cudaStreamCreateWithFlags(&c->aux, cudaStreamNonBlocking));
-    ELFEL_CUDA(c, cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
-    ELFEL_CUDA(c, cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
-  }
+  ELFEL_TRY(aux_create(c));
   ELFEL_CUDA(c, cudaEventRecord(c->ev_fork, c->stream));
   ELFEL_CUDA(c, cudaStreamWaitEvent(c->aux, c->ev_fork, 0));
   *aux = c->aux;
@@ -256,11 +264,7 @@ int aux_fork(Ctx* c, cudaStream_t* aux) {
 }
 
 int aux_after(Ctx* c, cudaEvent_t ev, cudaStream_t* aux) {
-  if (!c->aux) {
-    ELFEL_CUDA(c, cudaStreamCreateWithFlags(&c->aux, cudaStreamNonBlocking));
-    ELFEL_CUDA(c, cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
-    ELFEL_CUDA(c, cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
-  }
+  ELFEL_TRY(aux_create(c));
   ELFEL_CUDA(c, cudaStreamWaitEvent(c->aux, ev, 0));
   *aux = c->aux;
   return ELFEL_OK;

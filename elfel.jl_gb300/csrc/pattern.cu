@@ -671,7 +671,8 @@ int reduce_batch(Ctx* c, const RedJob* jobs_dev, int njobs, int64_t blocks) {
   return ELFEL_OK;
 }
 
-int reduce_values(Ctx* c, Pattern& P, const double* store, double* vals_out) {
+int reduce_values(Ctx* c, Pattern& P, const double* store, double* vals_out, Head* head) {
+  if (head) head->nnz = 0;
   if (P.nnz == 0) return ELFEL_OK;
   // The count order (window_order_k) pays for itself from a pattern's second
   // reduction on; a pattern reduced once (an end-to-end call) does without it.
@@ -684,15 +685,29 @@ int reduce_values(Ctx* c, Pattern& P, const double* store, double* vals_out) {
     ELFEL_LAUNCH_CHECK(c);
   }
   P.reductions++;
-  if (P.perm.p) {
-    const int64_t nwin = (P.nnz + kReduceWindow - 1) / kReduceWindow;
-    reduce_win_k<<<grid_for(nwin, 8, (int64_t)c->sm_count * 16), 256, 0, c->stream>>>(
-        P.cptr.p, P.contrib.p, P.perm.p, store, P.nnz, vals_out);
-  } else {
-    reduce_k<<<grid_for(P.nnz, 256, (int64_t)c->sm_count * 16), 256, 0, c->stream>>>(P.cptr.p, P.contrib.p, store,
-                                                                                     P.nnz, vals_out);
-  }
-  ELFEL_LAUNCH_CHECK(c);
+  // (a first assembly is followed by a call for the whole CSC, whose indices
+  // have the link first, and the auxiliary stream)
+  const int64_t hd = head && P.reductions > 1 ? values_head(P.nnz) / kReduceWindow * kReduceWindow : 0;
+  auto range = [&](cudaStream_t st, int64_t k0, int64_t n) -> int {  // k0: a multiple of kReduceWindow
+    if (P.perm.p) {
+      const int64_t nwin = (n + kReduceWindow - 1) / kReduceWindow;
+      reduce_win_k<<<grid_for(nwin, 8, (int64_t)c->sm_count * 16), 256, 0, st>>>(
+          P.cptr.p + k0, P.contrib.p, P.perm.p + k0, store, n, vals_out + k0);
+    } else {
+      reduce_k<<<grid_for(n, 256, (int64_t)c->sm_count * 16), 256, 0, st>>>(P.cptr.p + k0, P.contrib.p, store, n,
+                                                                            vals_out + k0);
+    }
+    ELFEL_LAUNCH_CHECK(c);
+    return ELFEL_OK;
+  };
+  if (head) head->nnz = hd;
+  if (!hd) return range(c->stream, 0, P.nnz);
+  cudaStream_t aux;
+  ELFEL_TRY(aux_fork(c, &aux));
+  ELFEL_TRY(range(aux, 0, hd));
+  ELFEL_CUDA(c, cudaEventRecord(head->ev, aux));
+  ELFEL_TRY(range(c->stream, hd, P.nnz - hd));
+  ELFEL_CUDA(c, cudaStreamWaitEvent(c->stream, head->ev, 0));
   return ELFEL_OK;
 }
 

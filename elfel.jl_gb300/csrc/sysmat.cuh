@@ -215,6 +215,7 @@ struct TilePlan {
   // limits), at most runlen tiles each: (first tile, tiles)
   int64_t nruns = 0;
   int runlen = 0;
+  int64_t head_runs = 0, head_nnz = 0;  // the first runs and the nonzeros they cover (values_head)
   DBuf<int2> runs;
   DBuf<TileHdr> hdr;
   // the distinct programs, each 16-byte aligned: count-class starts (uint16),
@@ -250,8 +251,21 @@ struct Pattern {
 // Build the CSC pattern of the slots of `g` (nrow x ncol matrix).
 int build_pattern(Ctx* c, const SlotGen& g, int64_t nrow, int64_t ncol, Pattern* P);
 
+// A head of the nonzeros, reduced on the auxiliary stream beside the rest and
+// followed by an event, so that a download of the values (elfel_sysmat_csc)
+// starts while the rest is being reduced.  The reduction is about ten times as fast as the
+// host link (2M quadratic triangles: 204 us against 1930): the transfer of an
+// eighth covers the reduction of the others.  Small systems do without: their
+// whole reduction takes less than the extra launch saves.
+constexpr int64_t kHeadMinNnz = 1 << 22;
+inline int64_t values_head(int64_t nnz) { return nnz < kHeadMinNnz ? 0 : nnz / 8; }
+struct Head {
+  cudaEvent_t ev = nullptr;
+  int64_t nnz = 0;  // nonzeros complete at ev (0: none was reduced apart)
+};
+
 // vals_out[k] = sum of store[contrib[t]] over t in [cptr[k], cptr[k+1]), in order.
-int reduce_values(Ctx* c, Pattern& P, const double* store, double* vals_out);
+int reduce_values(Ctx* c, Pattern& P, const double* store, double* vals_out, Head* head = nullptr);
 // Dense vector of a 1 x n pattern (the rhs): out[c] = contributions of column c.
 int reduce_dense(Ctx* c, const Pattern& P, const double* store, double* out);
 
@@ -261,7 +275,7 @@ int build_tile_plan(Ctx* c, Pattern& P, int S, int V, const uint8_t* map);
 // vals = the K values of P from element records (src: nel x S doubles), or,
 // with t6r_bases, from the 8 bases per element of the exact-rational T6
 // heat record; the same bits as reduce_values.
-int tile_reduce(Ctx* c, const Pattern& P, const double* src, int t6r_bases, double* vals);
+int tile_reduce(Ctx* c, const Pattern& P, const double* src, int t6r_bases, double* vals, Head* head = nullptr);
 
 // One reduction of a batched launch (device array ordered by blk0).
 constexpr int kRedJobThreads = 256;
@@ -350,6 +364,7 @@ struct elfel_sysmat {
   // recorded on the context stream when P (its colptr and rowval) is complete
   cudaEvent_t ev_pattern = nullptr;
   int pattern_recorded = 0;
+  elfel::Head head;  // of the last assembly
 };
 
 namespace elfel {

@@ -501,6 +501,7 @@ void TilePlan::release(Ctx* c) {
   runs.release(c);
   nruns = 0;
   runlen = 0;
+  head_runs = head_nnz = 0;
   hdr.release(c);
   blob.release(c);
   ntiles = 0;
@@ -696,6 +697,13 @@ int build_tile_plan(Ctx* c, Pattern& P, int S, int V, const uint8_t* map) {
       t = u;
     }
     T.nruns = (int64_t)runs.size();
+    const int64_t want = values_head(P.nnz);
+    for (int64_t r = 0; r < T.nruns && want > 0; ++r) {
+      const int64_t p0 = tiles[(size_t)runs[(size_t)r].x].p0;  // run r starts here
+      if (p0 > want) break;
+      T.head_runs = r;
+      T.head_nnz = p0;
+    }
     T.runlen = run_max;
     ELFEL_TRY(T.runs.alloc(c, runs.size()));
     ELFEL_CUDA(c, cudaMemcpyAsync(T.runs.p, runs.data(), sizeof(int2) * runs.size(), cudaMemcpyHostToDevice, c->stream));
@@ -733,15 +741,27 @@ static int tile_reduce_runs(Ctx* c, const Pattern& P, const double* bases, doubl
   return ELFEL_OK;
 }
 
-int tile_reduce(Ctx* c, const Pattern& P, const double* src, int t6r_bases, double* vals) {
+int tile_reduce(Ctx* c, const Pattern& P, const double* src, int t6r_bases, double* vals, Head* head) {
   const TilePlan& T = P.tiles;
+  if (head) head->nnz = 0;
   if (!T.built) return fail(c, ELFEL_ERR_STATE, "tile reduction without a plan");
   if (T.ntiles == 0) return ELFEL_OK;
   const size_t sm = tile_smem(T);
   if (t6r_bases) {
     if (T.V != kT6RTable || T.S != 21) return fail(c, ELFEL_ERR_STATE, "tile plan is not for T6 bases");
     RecT6R r{src};
-    if (tile_runs_ok(T)) return tile_reduce_runs(c, P, src, vals, 0, T.nruns, c->stream);
+    if (tile_runs_ok(T)) {
+      const int64_t r0 = head ? T.head_runs : 0;
+      if (!r0) return tile_reduce_runs(c, P, src, vals, 0, T.nruns, c->stream);
+      cudaStream_t aux;
+      ELFEL_TRY(aux_fork(c, &aux));
+      ELFEL_TRY(tile_reduce_runs(c, P, src, vals, 0, r0, aux));
+      ELFEL_CUDA(c, cudaEventRecord(head->ev, aux));
+      ELFEL_TRY(tile_reduce_runs(c, P, src, vals, r0, T.nruns - r0, c->stream));
+      ELFEL_CUDA(c, cudaStreamWaitEvent(c->stream, head->ev, 0));
+      head->nnz = T.head_nnz;
+      return ELFEL_OK;
+    }
     ELFEL_CUDA(c, cudaFuncSetAttribute(tile_reduce_k<RecT6R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     tile_reduce_k<RecT6R><<<(unsigned)T.ntiles, kRT, sm, c->stream>>>(T.hdr.p, T.maxnel, T.V, T.maxblob, T.blob.p,
                                                                        P.cptr.p, P.contrib.p, r, vals);

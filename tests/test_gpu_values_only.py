@@ -33,3 +33,41 @@ def test_partial_csc(E, gpu, pinned, which):
     nnz = ctypes.c_int64()
     gpu.check(gpu.lib.elfel_sysmat_dims(am._hd.h, None, None, ctypes.byref(nnz)))
     assert nnz.value == K.nnz
+
+
+@pytest.mark.parametrize("kind", ["T6", "T3", "elasticity"])
+def test_head_of_the_values(E, gpu, kind):
+    """A system of more than 4M nonzeros, whose values are reduced and copied
+    in two parts on two streams: every assembly's values arrive whole (the
+    staged copy into pageable arrays is the yardstick), also when the
+    coefficient changes between assemblies that nothing waits for."""
+    import torch
+
+    from problems import elasticity_setup
+
+    N = E._native
+    if kind == "elasticity":
+        mesh, fesp, bforce, right = elasticity_setup(E, 300, 150)
+        n = E.ndofs(fesp)
+        am = E.start(E.SysmatAssemblerGPU(), n, n)
+        elit, qpit = E.FEIterator(fesp), E.QPIterator(fesp, {"npts": 3})
+        E.assemble_elasticity(am, elit, qpit, 1.0, 0.3, True, bforce)
+        again = lambda s: am.elasticity(s, 0.3, True, bforce)  # noqa: E731
+    else:
+        k = 310 if kind == "T6" else 780
+        mesh = (E.T6block if kind == "T6" else E.T3block)(1.0, 1.0, k, k)
+        fesp = E.FESpace(float, mesh, E.FEH1_T6() if kind == "T6" else E.FEH1_T3())
+        E.numberdofs(fesp)
+        n = E.ndofs(fesp)
+        am = E.start(E.SysmatAssemblerGPU(), n, n)
+        E.assemble_heat(am, E.FEIterator(fesp), E.QPIterator(fesp, {"npts": 3}), 1.0, -6.0)
+        again = lambda s: am.heat(s, -6.0)  # noqa: E731
+    nnz = ctypes.c_int64()
+    gpu.check(gpu.lib.elfel_sysmat_dims(am._hd.h, None, None, ctypes.byref(nnz)))
+    assert nnz.value >= 1 << 22
+    v = torch.full((nnz.value,), -7.0, dtype=torch.float64).pin_memory().numpy()
+    for s in (1.0, 3.0, 0.7):
+        again(2.0 * s)
+        again(s)
+        gpu.check(gpu.lib.elfel_sysmat_csc(am._hd.h, None, None, N.ptr(v)))
+        assert np.array_equal(v, am.csc().data), s
