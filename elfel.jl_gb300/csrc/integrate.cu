@@ -1320,13 +1320,151 @@ __global__ void __launch_bounds__(kIntThreads) elast_straight_k(int64_t nel, con
   write_records<NT>(fa, ND, e0, nel, fstore);
 }
 
+// ------------------------------------------------------------------ exact T6 forms
+// For rules that integrate the products of the T6 gradients exactly
+// (kPatT6R), a bilinear form of straight-sided elements with the constant
+// 2 x 2 tensor Phi has closed-form entries: with m_ab = grad l_a^T Phi grad l_b of
+// the barycentric coordinates (rows and columns of m add up to zero),
+//   vertex a, vertex b       m_aa / 2, -m_ab / 6
+//   vertex p, edge (p, q)    2/3 m_pq (0 for an edge that p is not on)
+//   edge (p, q) with itself  4/3 (m_pp + m_qq) + 2/3 (m_pq + m_qp)
+//   edge (s, x), edge (s, y) 4/3 m_xy + 2/3 (m_sy - m_ys)
+// (integrals of l_a l_b over the triangle: area / 12 for a != b, area / 6 for a == b; edge
+// node 3 + p lies between vertices p and p + 1 mod 3).
+struct BaryForm {
+  double m[3][3];
+};
+
+template <bool SYM>
+__device__ __forceinline__ double t6_entry(const BaryForm& F, int a, int b) {
+  const auto& m = F.m;
+  constexpr double k23 = 2.0 / 3.0, k43 = 4.0 / 3.0, k16 = -1.0 / 6.0;
+  if (a < 3 && b < 3) return a == b ? __dmul_rn(0.5, m[a][a]) : __dmul_rn(k16, m[a][b]);
+  if (a < 3 || b < 3) {
+    const int v = a < 3 ? a : b, p = (a < 3 ? b : a) - 3, q = (p + 1) % 3;
+    if (v != p && v != q) return 0.0;
+    const int o = v == p ? q : p;
+    return __dmul_rn(k23, a < 3 ? m[v][o] : m[o][v]);
+  }
+  const int p = a - 3, q = (p + 1) % 3, r = b - 3, u = (r + 1) % 3;
+  if (a == b) {
+    if (SYM) return __dmul_rn(k43, __dadd_rn(__dadd_rn(m[p][p], m[q][q]), m[p][q]));
+    return __fma_rn(k43, __dadd_rn(m[p][p], m[q][q]), __dmul_rn(k23, __dadd_rn(m[p][q], m[q][p])));
+  }
+  const int s = (p == r || p == u) ? p : q, x = p + q - s, y = r + u - s;
+  if (SYM) return __dmul_rn(k43, m[x][y]);
+  return __fma_rn(k43, m[x][y], __dmul_rn(k23, __dsub_rn(m[s][y], m[y][s])));
+}
+
+// m from Phi = [f00 f01; f10 f11] (grad l_1 = (1, 0), grad l_2 = (0, 1)).
+__device__ __forceinline__ BaryForm bary_form(double f00, double f01, double f10, double f11) {
+  BaryForm F;
+  auto& m = F.m;
+  m[1][1] = f00;
+  m[1][2] = f01;
+  m[2][1] = f10;
+  m[2][2] = f11;
+  const double r1 = __dadd_rn(f00, f01), r2 = __dadd_rn(f10, f11);
+  m[1][0] = -r1;
+  m[2][0] = -r2;
+  m[0][1] = -__dadd_rn(f00, f10);
+  m[0][2] = -__dadd_rn(f01, f11);
+  m[0][0] = __dadd_rn(r1, r2);
+  return F;
+}
+
+// Entries K0 .. K0 + NK - 1 of a record (column-packed upper triangle of 12 x 12)
+// staged as acc[(k - K0) * LD].
+template <int K0, int NK, int LD>
+__device__ __forceinline__ void stage_elast_part(double* acc, const BaryForm& A, const BaryForm& B, const BaryForm& C) {
+#pragma unroll
+  for (int j = 0; j < 12; ++j)
+#pragma unroll
+    for (int i = 0; i <= j; ++i) {
+      const int k = j * (j + 1) / 2 + i;
+      if (k < K0 || k >= K0 + NK) continue;
+      const int a = i >> 1, b = j >> 1;
+      double v;
+      if ((i & 1) == (j & 1)) v = t6_entry<true>((i & 1) ? B : A, a, b);
+      else if (i & 1) v = t6_entry<false>(C, b, a);  // (1, 0): the transpose of (0, 1)
+      else v = t6_entry<false>(C, a, b);
+      acc[(k - K0) * LD] = v;
+    }
+}
+
+// Elasticity on straight-sided T6 meshes with an exact rule: isotropic D
+// (D02 = D12 = 0), the three forms Phi^00, Phi^11, Phi^01 of elast_straight_k, the
+// closed-form entries, about 160 FP64 operations per element instead of 380, and
+// the records written in six parts through a 13-entry buffer (13 KB a CTA
+// instead of 93: the staging had limited the kernel to two CTAs an SM).
+// 250,000 elements, the copy of 4 MB of forces included: 228 us in
+// elast_straight_k, 84 us here; the FP64 unit (16 cycles an SM and warp
+// instruction) takes about 65 of them, the 180 MB of records 27.
+__global__ void __launch_bounds__(kIntThreads) elast_t6_exact_k(int64_t nel, const int32_t* __restrict__ conn,
+                                                               const double2* __restrict__ xy, double D00, double D11,
+                                                               double D01, double D22,
+                                                               const double* __restrict__ bforce,
+                                                               double* __restrict__ kstore,
+                                                               double* __restrict__ fstore) {
+  constexpr int NS = 78, NT = kIntThreads, LD = NT + 1, NK = 13;
+  __shared__ double acc[NK * LD];
+  const int t = threadIdx.x;
+  const int64_t e0 = (int64_t)blockIdx.x * NT, e = e0 + t;
+  BaryForm A, B, C;
+  double f0 = 0.0, f1 = 0.0;
+  const bool in = e < nel;
+  if (in) {
+    const double2 p0 = __ldg(xy + __ldg(conn + e * 6)), p1 = __ldg(xy + __ldg(conn + e * 6 + 1)),
+                  p2 = __ldg(xy + __ldg(conn + e * 6 + 2));
+    // rows of adj(J): r0 = (J22, -J12), r1 = (-J21, J11)
+    const double r0x = p2.y - p0.y, r0y = p0.x - p2.x, r1x = p0.y - p1.y, r1y = p1.x - p0.x;
+    const double det = __fma_rn(r1y, r0x, -__dmul_rn(r1x, r0y));
+    const double rd = fast_rcp(det);
+    const double s0x = r0x * rd, s0y = r0y * rd, s1x = r1x * rd, s1y = r1y * rd;
+    const double xx0 = r0x * s0x, yy0 = r0y * s0y, xx1 = r1x * s1x, yy1 = r1y * s1y, xx = r0x * s1x, yy = r0y * s1y;
+    const double a01 = __fma_rn(D00, xx, D22 * yy), b01 = __fma_rn(D22, xx, D11 * yy);
+    A = bary_form(__fma_rn(D00, xx0, D22 * yy0), a01, a01, __fma_rn(D00, xx1, D22 * yy1));
+    B = bary_form(__fma_rn(D22, xx0, D11 * yy0), b01, b01, __fma_rn(D22, xx1, D11 * yy1));
+    const double xy01 = r0x * s1y, yx01 = r0y * s1x, Ds = D01 + D22;
+    C = bary_form(r0x * s0y * Ds, __fma_rn(D01, xy01, D22 * yx01), __fma_rn(D01, yx01, D22 * xy01), r1x * s1y * Ds);
+    if (bforce) {
+      f0 = __ldg(bforce + 2 * e) * det * (1.0 / 6.0);
+      f1 = __ldg(bforce + 2 * e + 1) * det * (1.0 / 6.0);
+    }
+  }
+#define ELAST_PART(K0)                                                       \
+  do {                                                                       \
+    if (in) stage_elast_part<K0, NK, LD>(acc + t, A, B, C);                  \
+    write_records_fixed<NT, NS, NK>(acc, K0, e0, nel, kstore);               \
+    __syncthreads();                                                         \
+  } while (0)
+  ELAST_PART(0);
+  ELAST_PART(13);
+  ELAST_PART(26);
+  ELAST_PART(39);
+  ELAST_PART(52);
+  ELAST_PART(65);
+#undef ELAST_PART
+  // load vector: 0 at the vertices, det b / 6 at the midside nodes
+  if (in) {
+#pragma unroll
+    for (int k = 0; k < 12; ++k) acc[k * LD + t] = k < 6 ? 0.0 : (k & 1) ? f1 : f0;
+  }
+  write_records_fixed<NT, 12, 12>(acc, 0, e0, nel, fstore);
+}
+
 int launch_elasticity(Ctx* c, int nn, int64_t nel, const int32_t* conn, const double* xy, const Mat3& D,
                       const double* bforce, int64_t ncurved, const QPTab& tab, double* kstore, double* fstore) {
   if (nel == 0) return ELFEL_OK;
   const unsigned grid = grid_for(nel, kIntThreads);
   if (ncurved == 0) {
     const size_t sm = (size_t)(nn == 3 ? 21 + 6 : 78 + 12) * (kIntThreads + 1) * sizeof(double);
-    if (nn == 3) {
+    const bool iso = D.a[0][2] == 0.0 && D.a[1][2] == 0.0 && D.a[2][0] == 0.0 && D.a[2][1] == 0.0 &&
+                     D.a[0][1] == D.a[1][0];
+    if (nn == 6 && iso && heat_pattern(6, tab) == kPatT6R) {
+      elast_t6_exact_k<<<grid, kIntThreads, 0, c->stream>>>(nel, conn, (const double2*)xy, D.a[0][0], D.a[1][1],
+                                                            D.a[0][1], D.a[2][2], bforce, kstore, fstore);
+    } else if (nn == 3) {
       elast_straight_k<3><<<grid, kIntThreads, sm, c->stream>>>(nel, conn, (const double2*)xy, D, bforce, tab,
                                                                  kstore, fstore);
     } else {
@@ -1550,6 +1688,109 @@ __global__ void __launch_bounds__(kIntThreads) stokes_straight_k(int64_t nel, co
   write_records<NT>(pa, 3, e0, nel, pmass);
 }
 
+// Stokes on straight-sided T6 meshes with an exact rule.  uu: the heat bases
+// with kappa = mu (the same bits as stokes_straight_k), zero across components;
+// up: kup_(a,c),j = -(T^0_aj adj_0c + T^1_aj adj_1c), T the exact integrals of l_j grad N_a:
+//   vertex a: grad l_a / 6 for j = a, else 0
+//   edge (p, q): grad l_q / 3 + grad l_p / 6 for j = p (p, q exchanged for j = q), -grad l_j / 6 else
+// written in six parts through a 19-entry buffer (the 144-entry staging of
+// stokes_straight_k allows one CTA of 128 threads an SM).
+// 105,800 elements: 87 us in stokes_straight_k, 43 us here (99 MB of records: 15 us).
+template <int K0, int NK, int LD>
+__device__ __forceinline__ void stage_stokes_part(double* acc, const double (&v)[kT6RTable], const double (&g)[3][2]) {
+#pragma unroll
+  for (int j = 0; j < 12; ++j)
+#pragma unroll
+    for (int i = 0; i <= j; ++i) {
+      const int k = j * (j + 1) / 2 + i;
+      if (k < K0 || k >= K0 + NK) continue;
+      const int a = i >> 1, b = j >> 1;
+      acc[(k - K0) * LD] = (i & 1) == (j & 1) ? v[t6r_entry(b * (b + 1) / 2 + a)] : 0.0;
+    }
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+#pragma unroll
+    for (int d = 0; d < 12; ++d) {
+      const int k = 78 + d + 12 * j;
+      if (k < K0 || k >= K0 + NK) continue;
+      const int a = d >> 1, c = d & 1;
+      double x = 0.0;
+      if (a < 3) {
+        if (a == j) x = -(1.0 / 6.0) * g[a][c];
+      } else {
+        const int p = a - 3, q = (p + 1) % 3;
+        if (j != p && j != q) x = (1.0 / 6.0) * g[j][c];
+        else x = -__fma_rn(1.0 / 3.0, g[j == p ? q : p][c], (1.0 / 6.0) * g[j][c]);
+      }
+      acc[(k - K0) * LD] = x;
+    }
+}
+
+__global__ void __launch_bounds__(kIntThreads) stokes_t6_exact_k(int64_t nel, const int32_t* __restrict__ conn,
+                                                                const double2* __restrict__ xy, double mu, double P6,
+                                                                double Mp0, double Mp1, double Mp2,
+                                                                double* __restrict__ kstore,
+                                                                double* __restrict__ pmass) {
+  constexpr int NR = 114, NT = kIntThreads, LD = NT + 1, NK = 19;
+  __shared__ double acc[NK * LD];
+  const int t = threadIdx.x;
+  const int64_t e0 = (int64_t)blockIdx.x * NT, e = e0 + t;
+  const bool in = e < nel;
+  double v[kT6RTable], g[3][2], det = 0.0;
+  if (in) {
+    const double2 p0 = __ldg(xy + __ldg(conn + e * 6)), p1 = __ldg(xy + __ldg(conn + e * 6 + 1)),
+                  p2 = __ldg(xy + __ldg(conn + e * 6 + 2));
+    const double J11 = __dsub_rn(p1.x, p0.x), J12 = __dsub_rn(p2.x, p0.x);
+    const double J21 = __dsub_rn(p1.y, p0.y), J22 = __dsub_rn(p2.y, p0.y);
+    double b[8];
+    t6r_bases(J11, J12, J21, J22, mu, 0.0, P6, b);
+    t6r_table(b, v);
+    det = J11 * J22 - J21 * J12;
+    // det J times the gradients of l_1, l_2, l_0
+    g[1][0] = J22;
+    g[1][1] = -J12;
+    g[2][0] = -J21;
+    g[2][1] = J11;
+    g[0][0] = J21 - J22;
+    g[0][1] = J12 - J11;
+  }
+#define STOKES_PART(K0)                                              \
+  do {                                                               \
+    if (in) stage_stokes_part<K0, NK, LD>(acc + t, v, g);            \
+    write_records_fixed<NT, NR, NK>(acc, K0, e0, nel, kstore);       \
+    __syncthreads();                                                 \
+  } while (0)
+  STOKES_PART(0);
+  STOKES_PART(19);
+  STOKES_PART(38);
+  STOKES_PART(57);
+  STOKES_PART(76);
+  STOKES_PART(95);
+#undef STOKES_PART
+  if (in) {
+    acc[t] = det * Mp0;
+    acc[LD + t] = det * Mp1;
+    acc[2 * LD + t] = det * Mp2;
+  }
+  write_records_fixed<NT, 3, 3>(acc, 0, e0, nel, pmass);
+}
+
+// True when the rule's velocity-pressure integrals T are the exact ones.
+static bool stokes_exact(const QPTab& tab) {
+  static const double gl[3][2] = {{-1.0, -1.0}, {1.0, 0.0}, {0.0, 1.0}};
+  for (int a = 0; a < 6; ++a)
+    for (int j = 0; j < 3; ++j)
+      for (int c = 0; c < 2; ++c) {
+        double x = a == j ? gl[a][c] / 6.0 : 0.0;
+        if (a >= 3) {
+          const int p = a - 3, q = (p + 1) % 3;
+          x = j == p ? gl[q][c] / 3.0 + gl[p][c] / 6.0 : j == q ? gl[p][c] / 3.0 + gl[q][c] / 6.0 : -gl[j][c] / 6.0;
+        }
+        if (fabs(tab.T[c][a * 3 + j] - x) > 1e-14) return false;
+      }
+  return true;
+}
+
 int launch_stokes(Ctx* c, int64_t nel, const int32_t* conn, const double* xy, double mu, int64_t ncurved,
                   const QPTab& tab, double* kstore, double* pmass) {
   if (nel == 0) return ELFEL_OK;
@@ -1557,7 +1798,10 @@ int launch_stokes(Ctx* c, int64_t nel, const int32_t* conn, const double* xy, do
     const size_t sm = (size_t)(78 + 36 + 3 + 21 + 6) * (kIntThreads + 1) * sizeof(double);
     const int pat = heat_pattern(6, tab);
     const unsigned grid = grid_for(nel, kIntThreads);
-    if (pat == kPatT6R) {
+    if (pat == kPatT6R && stokes_exact(tab)) {
+      stokes_t6_exact_k<<<grid, kIntThreads, 0, c->stream>>>(nel, conn, (const double2*)xy, mu, tab.P[3], tab.Mp[0],
+                                                             tab.Mp[1], tab.Mp[2], kstore, pmass);
+    } else if (pat == kPatT6R) {
       ELFEL_CUDA(c, cudaFuncSetAttribute(stokes_straight_k<kPatT6R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)sm));
       stokes_straight_k<kPatT6R><<<grid, kIntThreads, sm, c->stream>>>(nel, conn, (const double2*)xy, mu, tab,
