@@ -540,8 +540,8 @@ extern "C" int elfel_fused_setup(elfel_sysmat* m, const elfel_fused_desc* d) {
     if (stokes) ELFEL_TRY(upload_direct_rest(c, d->p, 2, &F.conn_p, nullptr, bad.p + 2, aux));
     ELFEL_TRY(fused_build(m, d->ndofs));  // joins the auxiliary stream before using conn / xy
     int hb[4] = {0, 0, 0, 0};
-    ELFEL_CUDA(c, cudaMemcpyAsync(hb, bad.p, sizeof(hb), cudaMemcpyDeviceToHost, c->stream));
-    ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
+    ELFEL_CUDA(c, cudaMemcpyAsync(hb, bad.p, sizeof(hb), cudaMemcpyDeviceToHost, aux));
+    ELFEL_CUDA(c, cudaStreamSynchronize(aux));
     static const char* what[4] = {"primary connectivity", "primary eldofs", "pressure connectivity",
                                   "pressure eldofs"};
     const int64_t lim[4] = {u.nnodes, d->ndofs, stokes ? d->p.nnodes : 0, d->ndofs};
@@ -561,9 +561,13 @@ extern "C" int elfel_fused_setup(elfel_sysmat* m, const elfel_fused_desc* d) {
 
 namespace elfel {
 
-// Slot generators, patterns and value buffers of a fused system whose tables
-// (connectivity, coordinates, element DOFs) are already on the device.
-int fused_build(elfel_sysmat* m, int64_t ndofs) {
+// The checks of a fused system's tables that run beside its pattern build.
+struct TableChecks {
+  DBuf<int32_t> cnt;  // element contributions of each DOF as a midside node
+  DBuf<unsigned long long> res;  // curved elements; (32 bits) a DOF has more than two such contributions
+};
+
+static int fused_build_in(elfel_sysmat* m, int64_t ndofs, TableChecks* chk) {
   Ctx* c = &m->h->c;
   Fused& F = m->F;
   const int nedof = F.nn_u * F.ncomp_u;
@@ -592,6 +596,29 @@ int fused_build(elfel_sysmat* m, int64_t ndofs) {
     g.store_per_elem = 78 + 36;
   }
   m->nrow = m->ncol = ndofs;
+  // checks of the tables, on the auxiliary stream beside the pattern build: the
+  // T6 load vector may be added atomically (launch_heat) when no DOF collects
+  // more than two nonzero element contributions; curved elements are counted
+  const bool midside =
+      F.physics == ELFEL_HEAT && F.shape == ELFEL_SHAPE_TRIANGLE && F.nn_u == 6 && F.ncomp_u == 1 && F.nel > 0;
+  const bool triangles = F.shape == ELFEL_SHAPE_TRIANGLE && F.nel > 0;
+  DBuf<int32_t>& cnt = chk->cnt;
+  DBuf<unsigned long long>& res = chk->res;
+  ELFEL_TRY(F.straight.alloc(c, (size_t)(F.nel > 0 ? F.nel : 1)));
+  if (midside) ELFEL_TRY(cnt.alloc(c, (size_t)ndofs + 1));
+  if (triangles) {
+    ELFEL_TRY(res.alloc(c, 2));
+    cudaStream_t aux;
+    ELFEL_TRY(aux_fork(c, &aux));
+    ELFEL_CUDA(c, cudaMemsetAsync(res.p, 0, 2 * sizeof(unsigned long long), aux));
+    if (midside) {
+      ELFEL_CUDA(c, cudaMemsetAsync(cnt.p, 0, sizeof(int32_t) * (ndofs + 1), aux));
+      midside_count_k<<<grid_for(F.nel * 3, 256, (int64_t)c->sm_count * 16), 256, 0, aux>>>(
+          F.dofs_u.p, F.nel, cnt.p, reinterpret_cast<int32_t*>(res.p + 1));
+      ELFEL_LAUNCH_CHECK(c);
+    }
+    ELFEL_TRY(launch_straight_count(c, aux, F.nn_u, F.nel, F.conn_u.p, F.xy_u.p, F.straight.p, res.p));
+  }
   {
     Phase ph(c, "pattern_K");
     ELFEL_TRY(build_pattern(c, g, ndofs, ndofs, &m->P));
@@ -623,41 +650,37 @@ int fused_build(elfel_sysmat* m, int64_t ndofs) {
     ELFEL_TRY(F.pmass_store.alloc(c, (size_t)(F.nel * 3 > 0 ? F.nel * 3 : 1)));
     ELFEL_TRY(F.pmass_diag.alloc(c, (size_t)(ndofs > 0 ? ndofs : 1)));
   }
-  ELFEL_TRY(aux_join(c));  // tables uploaded on the auxiliary stream
-  F.f_direct_ok = 0;
-  if (F.physics == ELFEL_HEAT && F.shape == ELFEL_SHAPE_TRIANGLE && F.nn_u == 6 && F.ncomp_u == 1 && F.nel > 0) {
-    // the T6 load vector may be added atomically (launch_heat) when no DOF
-    // collects more than two nonzero element contributions
-    DBuf<int32_t> cnt;  // ndofs counters, then the flag
-    int h_many = 1;
-    auto count = [&]() -> int {
-      ELFEL_TRY(cnt.alloc(c, (size_t)ndofs + 1));
-      ELFEL_CUDA(c, cudaMemsetAsync(cnt.p, 0, sizeof(int32_t) * (ndofs + 1), c->stream));
-      midside_count_k<<<grid_for(F.nel * 3, 256, (int64_t)c->sm_count * 16), 256, 0, c->stream>>>(
-          F.dofs_u.p, F.nel, cnt.p, cnt.p + ndofs);
-      ELFEL_LAUNCH_CHECK(c);
-      ELFEL_CUDA(c, cudaMemcpyAsync(&h_many, cnt.p + ndofs, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-      ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
-      return ELFEL_OK;
-    };
-    const int rc = count();
-    cnt.release(c);
-    if (rc != ELFEL_OK) return rc;
-    F.f_direct_ok = h_many == 0;
-  }
-  ELFEL_TRY(F.straight.alloc(c, (size_t)(F.nel > 0 ? F.nel : 1)));
-  if (F.shape == ELFEL_SHAPE_TRIANGLE)
-    ELFEL_TRY(launch_straight(c, F.nn_u, F.nel, F.conn_u.p, F.xy_u.p, F.straight.p, &F.ncurved));
+  ELFEL_TRY(aux_join(c));  // tables uploaded and checked on the auxiliary stream
   ELFEL_TRY(F.kstore.alloc(c, (size_t)(F.nel * g.store_per_elem > 0 ? F.nel * g.store_per_elem : 1)));
   ELFEL_TRY(F.fstore.alloc(c, (size_t)(F.nel * nedof > 0 ? F.nel * nedof : 1)));
   ELFEL_TRY(m->vals.alloc(c, (size_t)(m->P.nnz > 0 ? m->P.nnz : 1)));
   ELFEL_TRY(m->rhs.alloc(c, (size_t)(ndofs > 0 ? ndofs : 1)));
   ELFEL_TRY(F.coef.alloc(c, (size_t)(F.nel > 0 ? 2 * F.nel : 1)));
-  ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
+  // the results of the checks are read on their own stream: the last kernel of the
+  // pattern build runs on while the caller goes on (the tables have left the host)
+  unsigned long long h[2] = {0, 1};
+  cudaStream_t rs = triangles ? c->aux : c->stream;
+  if (triangles) ELFEL_CUDA(c, cudaMemcpyAsync(h, res.p, sizeof(h), cudaMemcpyDeviceToHost, rs));
+  ELFEL_CUDA(c, cudaStreamSynchronize(rs));
+  F.f_direct_ok = midside && h[1] == 0;
+  F.ncurved = (int64_t)h[0];
   m->fused = 1;
   m->started = 1;
   m->finished = 0;
   return ELFEL_OK;
+}
+
+// Slot generators, patterns and value buffers of a fused system whose tables
+// (connectivity, coordinates, element DOFs) are already on the device or on their
+// way there on the auxiliary stream.
+int fused_build(elfel_sysmat* m, int64_t ndofs) {
+  Ctx* c = &m->h->c;
+  TableChecks chk;
+  const int rc = fused_build_in(m, ndofs, &chk);
+  if (rc != ELFEL_OK) aux_join(c);  // the buffers are freed behind the auxiliary stream's work
+  chk.cnt.release(c);
+  chk.res.release(c);
+  return rc;
 }
 
 }  // namespace elfel

@@ -60,8 +60,10 @@ int red_scratch(Ctx* c, int nslots, int nblocks, RedSlot* slots) {
 }
 
 // ------------------------------------------------------------------ scan
-// Three-phase exclusive scan: per-block totals, recursive scan of the totals,
-// then a block-local scan with the block offset added.
+// Exclusive scan: per-block totals, recursive scan of the totals, then a
+// block-local scan with the block offset added; one launch up to a tile of
+// 4096 items, three up to 4096 tiles (a pattern build of a few hundred columns
+// is launches only).
 constexpr int kScanBlock = 512;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanBlock * kScanItems;
@@ -88,7 +90,8 @@ __global__ void scan_block_totals_k(const TIn* in, int64_t n, int64_t* totals) {
 }
 
 // Block-local exclusive scan of a tile; each thread owns kScanItems
-// consecutive items.  offsets = exclusive scan of the block totals.
+// consecutive items.  offsets = exclusive scan of the block totals (nullptr: one
+// block); the last item's thread writes the total to out[n].
 template <typename TIn>
 __global__ void scan_tile_k(const TIn* in, int64_t n, const int64_t* offsets, int64_t* out) {
   __shared__ int64_t warp_tot[kScanBlock / 32];
@@ -123,16 +126,13 @@ __global__ void scan_tile_k(const TIn* in, int64_t n, const int64_t* offsets, in
     if (lane < kScanBlock / 32) warp_tot[lane] = wi - w;
   }
   __syncthreads();
-  int64_t excl = incl - run + warp_tot[wid] + offsets[blockIdx.x];
+  int64_t excl = incl - run + warp_tot[wid] + (offsets ? offsets[blockIdx.x] : 0);
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
     int64_t i = base + k;
     if (i < n) out[i] = v[k] + excl;
   }
-}
-
-__global__ void write_total_k(const int64_t* offsets, int64_t nblocks, const int64_t* totals, int64_t* out_total) {
-  *out_total = offsets[nblocks - 1] + totals[nblocks - 1];
+  if (base < n && n <= base + kScanItems) out[n] = excl + run;
 }
 
 template <typename TIn>
@@ -143,18 +143,14 @@ static int scan_impl(Ctx* c, const TIn* in, int64_t n, int64_t* out) {
   }
   int64_t nb = (n + kScanTile - 1) / kScanTile;
   DBuf<int64_t> totals, offsets;
-  ELFEL_TRY(totals.alloc(c, (size_t)nb));
-  ELFEL_TRY(offsets.alloc(c, (size_t)nb + 1));
-  scan_block_totals_k<TIn><<<(unsigned)nb, kScanBlock, 0, c->stream>>>(in, n, totals.p);
-  ELFEL_LAUNCH_CHECK(c);
-  if (nb == 1) {
-    ELFEL_CUDA(c, cudaMemsetAsync(offsets.p, 0, sizeof(int64_t), c->stream));
-  } else {
+  if (nb > 1) {
+    ELFEL_TRY(totals.alloc(c, (size_t)nb));
+    ELFEL_TRY(offsets.alloc(c, (size_t)nb + 1));
+    scan_block_totals_k<TIn><<<(unsigned)nb, kScanBlock, 0, c->stream>>>(in, n, totals.p);
+    ELFEL_LAUNCH_CHECK(c);
     ELFEL_TRY(scan_impl<int64_t>(c, totals.p, nb, offsets.p));
   }
   scan_tile_k<TIn><<<(unsigned)nb, kScanBlock, 0, c->stream>>>(in, n, offsets.p, out);
-  ELFEL_LAUNCH_CHECK(c);
-  write_total_k<<<1, 1, 0, c->stream>>>(offsets.p, nb, totals.p, out + n);
   ELFEL_LAUNCH_CHECK(c);
   totals.release(c);
   offsets.release(c);

@@ -246,6 +246,15 @@ __global__ void straight_k(int64_t nel, const int32_t* __restrict__ conn, const 
   if ((threadIdx.x & 31) == 0 && curved) atomicAdd(ncurved, curved);
 }
 
+int launch_straight_count(Ctx* c, cudaStream_t st, int nn, int64_t nel, const int32_t* conn, const double* xy,
+                          uint8_t* flag, unsigned long long* ncurved) {
+  const unsigned grid = grid_for(nel, 256, (int64_t)c->sm_count * 16);
+  if (nn == 3) straight_k<3><<<grid, 256, 0, st>>>(nel, conn, (const double2*)xy, flag, ncurved);
+  else straight_k<6><<<grid, 256, 0, st>>>(nel, conn, (const double2*)xy, flag, ncurved);
+  ELFEL_LAUNCH_CHECK(c);
+  return ELFEL_OK;
+}
+
 int launch_straight(Ctx* c, int nn, int64_t nel, const int32_t* conn, const double* xy, uint8_t* flag,
                     int64_t* ncurved) {
   *ncurved = 0;
@@ -253,10 +262,7 @@ int launch_straight(Ctx* c, int nn, int64_t nel, const int32_t* conn, const doub
   DBuf<unsigned long long> cnt;
   ELFEL_TRY(cnt.alloc(c, 1));
   ELFEL_CUDA(c, cudaMemsetAsync(cnt.p, 0, sizeof(unsigned long long), c->stream));
-  const unsigned grid = grid_for(nel, 256, (int64_t)c->sm_count * 16);
-  if (nn == 3) straight_k<3><<<grid, 256, 0, c->stream>>>(nel, conn, (const double2*)xy, flag, cnt.p);
-  else straight_k<6><<<grid, 256, 0, c->stream>>>(nel, conn, (const double2*)xy, flag, cnt.p);
-  ELFEL_LAUNCH_CHECK(c);
+  ELFEL_TRY(launch_straight_count(c, c->stream, nn, nel, conn, xy, flag, cnt.p));
   unsigned long long h = 0;
   ELFEL_CUDA(c, cudaMemcpyAsync(&h, cnt.p, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
   ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));

@@ -57,6 +57,9 @@ bool heat_f_direct(int nn, int64_t ncurved, const QPTab& tab);
 // recomputed whenever the coordinates change.  Synchronises the stream.
 int launch_straight(Ctx* c, int nn, int64_t nel, const int32_t* conn, const double* xy, uint8_t* flag,
                     int64_t* ncurved);
+// The same on stream st, the count added to *ncurved on the device (nel > 0).
+int launch_straight_count(Ctx* c, cudaStream_t st, int nn, int64_t nel, const int32_t* conn, const double* xy,
+                          uint8_t* flag, unsigned long long* ncurved);
 
 // One mesh of a batched heat integration (device array, ordered by blk0).
 struct HeatJob {

@@ -11,35 +11,60 @@
 //   1. column counts (one int32 atomic per column group in block mode, per
 //      slot in COO mode)
 //   2. exclusive scan -> column starts
-//   3. bucket each slot's key (row << 32 | slot) into its column (one cursor
-//      atomic per run of equal columns within a warp; the order inside a
-//      column does not matter, the keys carry the slot)
-//   4. sort each column's keys in registers (bitonic networks sized to the
-//      column, 32-bit packed keys where the spans fit, 33-64 keys merged by
-//      rank), count its distinct rows, write the storage index of every
-//      contribution (contrib) in sorted order and the column's row starts
-//   5. scan -> colptr; compact the row starts into rowval and the first
+//   3. bucket the column groups' numbers (block mode) or each slot's key
+//      (row << 32 | slot) (COO mode) into their columns; the order inside a
+//      column does not matter, groups and keys carry the slot order
+//   4. sort each column's keys in the registers of one thread (merge-exchange
+//      networks sized to the longest of the warp's 32 columns; long columns by
+//      the whole warp), count its distinct rows, write the storage index of every
+//      contribution (contrib) in sorted order and the warp's row starts
+//   5. scan -> colptr; copy the row starts to rowval and the first
 //      contribution of each nonzero (cptr)
 //   6. (at a pattern's second value reduction) the contributor-count order
 //      of each window of 128 nonzeros (window_order_k).
+#include <type_traits>
+
 #include "pack32.cuh"
 #include "sysmat.cuh"
 
 namespace elfel {
 
-constexpr int kSortThreads = 256;           // 8 warps
-constexpr int kSortCap = 256;               // keys per warp sorted in shared memory
+constexpr int kWideThreads = 256;  // 8 warps
+constexpr int kSortCap = 256;      // keys of a long column sorted in shared memory
+constexpr int kColBatch = 32;      // columns of a warp: one per thread
+
+// The sort of a batch of columns by threads, for columns of up to NK keys.
+template <int NK>
+struct Net {
+  static constexpr int kThreads = NK > 48 ? 32 : 128;
+  static constexpr int kBlocks = NK > 48 ? 8 : NK == 48 ? 4 : 3;  // an SM
+  static constexpr int kGroups = NK > 48 ? 32 : 16;               // column groups of a column (block mode)
+  static constexpr int kBatch = NK > 48 ? 3072 : 1240;            // keys of a batch
+  static constexpr int kArea = NK > 48 ? 3168 : 1320;             // words of a shared area: kBatch and its padding
+  static constexpr int kBits = NK > 64 ? 7 : 6;                   // of a key's place among its column's
+  static constexpr uint32_t kSpan = (1u << (32 - kBits)) - 2;     // row span that fits beside it in 32 bits
+};
+constexpr int kNet = 48;    // block mode, on average at most kNetMean slots a column
+constexpr int kNetL = 96;   // block mode, more
+constexpr int kNet64 = 40;  // COO mode: 64-bit keys (48 spill)
+// Slots per column: 16 to 18 on T3, T6 and Q4 meshes (vertices of a T6 mesh 36), 36 in
+// plane elasticity on T6 (24 and 72), 48 in Taylor-Hood, 96 on T4.  The larger form keeps
+// eight warps an SM instead of 16 and is taken where the other would leave most
+// batches to sort_wide_k.  Set-up to CSC with the smaller and the larger form: T6 500 x 500
+// 1765 and 2005 us, Q4 700 x 700 1196 and 1287; elasticity 250 x 125 1264 and 1130,
+// Taylor-Hood 60 x 60 529 and 455, T4 40^3 920 and 837.
+constexpr int kNetMean = 24;
 
 // Block mode: one thread per column group (one atomic per group instead of
 // one per slot).  The row tables are the uploaded element DOF tables, range
 // checked on upload; the column is checked here.
-__global__ void count_groups_k(SlotGen g, int G, int64_t ngroups, int32_t* colcnt, int64_t ncol, int* bad) {
+__global__ void count_groups_k(SlotGen g, int64_t ngroups, int32_t* colcnt, int64_t ncol, int* bad) {
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < ngroups; q += (int64_t)gridDim.x * blockDim.x) {
     int32_t c;
     int64_t s0;
     int len;
     const int32_t* rt;
-    group_info(g, G, q, c, s0, len, rt);
+    group_info(g, (uint32_t)q, c, s0, len, rt);
     if (c < 0 || c >= ncol) {
       atomicExch(bad, 1);
       continue;
@@ -61,32 +86,51 @@ __global__ void count_cols_k(SlotGen g, int64_t n, int32_t* colcnt, int64_t ncol
   }
 }
 
-// Consecutive slots mostly share their column (a local column of an element
-// matrix, a run of COO triplets): the lanes of a warp with equal columns in a
+// Block mode: each group's number into its column, gk[colstart + i] (a column of n
+// slots has at most n groups).  A group's rows and slots follow from its number,
+// so 4 bytes per group are written and read back instead of 8 per slot
+// (500,000 T6 elements: 90 us for the 18M slot keys, 32 us here).
+__global__ void bucket_groups_k(SlotGen g, int64_t ngroups, const int64_t* __restrict__ colstart, int64_t ncol,
+                                int32_t* cursor, uint32_t* gk) {
+  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < ngroups; q += (int64_t)gridDim.x * blockDim.x) {
+    int32_t c;
+    int64_t s0;
+    int len;
+    const int32_t* rt;
+    group_info(g, (uint32_t)q, c, s0, len, rt);
+    if (c < 0 || c >= ncol) continue;
+    gk[colstart[c] + atomicAdd(&cursor[c], 1)] = (uint32_t)q;
+  }
+}
+
+// COO mode.  Consecutive triplets mostly share their column (a local column of
+// an element matrix): the lanes of a warp with equal columns in a
 // row form a run whose first lane reserves the run's positions with one
 // atomic and hands them out by shuffle.
-__global__ void bucket_k(SlotGen g, int64_t n, const int64_t* colstart, int32_t* cursor, uint64_t* keys) {
+__global__ void bucket_k(SlotGen g, int64_t n, const int64_t* colstart, int64_t nrow, int64_t ncol, int32_t* cursor,
+                         uint64_t* keys) {
   const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t s0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); s0 < n; s0 += stride) {
     const int64_t s = s0 + lane;
-    const bool valid = s < n;
+    bool valid = s < n;
     int32_t r = 0, c = -1;
     int64_t st;
     if (valid) slot_rc(g, s, r, c, st);
+    valid = valid && r >= 0 && r < nrow && c >= 0 && c < ncol;  // as counted
+    if (!valid) c = -1;
     const int32_t cprev = __shfl_up_sync(0xffffffffu, c, 1);
-    const bool head = valid && (lane == 0 || c != cprev);
+    const bool head = lane == 0 || c != cprev;  // lanes without a triplet form runs (c = -1) of their own
     const unsigned heads = __ballot_sync(0xffffffffu, head);
-    const unsigned vmask = __ballot_sync(0xffffffffu, valid);
     const unsigned upto = lane == 31 ? 0xffffffffu : ((2u << lane) - 1u);
     const int start = 31 - __clz(heads & upto);  // first lane of this lane's run
     int32_t base = 0;
-    if (head) {
+    if (head && valid) {
       const unsigned after = heads & ~upto;  // heads of later runs
-      const int end = after ? __ffs(after) - 1 : 32 - __clz(vmask);
+      const int end = after ? __ffs(after) - 1 : 32;
       base = atomicAdd(&cursor[c], end - lane);
     }
-    base = __shfl_sync(0xffffffffu, base, valid ? start : 0);
+    base = __shfl_sync(0xffffffffu, base, start);
     if (valid) keys[colstart[c] + base + (lane - start)] = ((uint64_t)(uint32_t)r << 32) | (uint64_t)(uint32_t)s;
   }
 }
@@ -180,44 +224,36 @@ __device__ __forceinline__ bool pack_warp(uint32_t rlo, uint32_t rhi, uint32_t s
   return true;
 }
 
-// The same for each half warp separately (xor partners below 16).
-__device__ __forceinline__ bool pack_half(uint32_t rlo, uint32_t rhi, uint32_t slo, uint32_t shi, Pack32* p) {
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1) {
-    rlo = min(rlo, __shfl_xor_sync(0xffffffffu, rlo, o));
-    rhi = max(rhi, __shfl_xor_sync(0xffffffffu, rhi, o));
-    slo = min(slo, __shfl_xor_sync(0xffffffffu, slo, o));
-    shi = max(shi, __shfl_xor_sync(0xffffffffu, shi, o));
-  }
-  if (rhi < rlo || shi < slo) return false;
-  const int sb = bit_length(shi - slo);
-  if (bit_length(rhi - rlo) + sb > 31) return false;
-  *p = Pack32{rlo, slo, sb};
-  return true;
-}
-
-// Output of a sorted column: each key's storage index goes to contrib[b + t]
-// (t = its place in the column), and each key that starts a row (its
-// predecessor has another row) to nzkey[b + i] as (row << 32 | b + t), i =
-// the number of rows before it in the column.  compact_k moves the latter to
-// rowval / cptr once the column's first nonzero is known.
+// Output of the sorted columns: each key's storage index goes to contrib[b + t]
+// (b = the column's first slot, t = the key's place in it), and the keys that
+// start a row (their predecessor has another row) to nzrow / nzpos = (row, b + t):
+// in a batch of 32 columns sorted by threads one after the other from the
+// batch's first slot, in a batch marked wide[] from each column's first slot.
+// compact_k moves them to rowval / cptr once the first nonzeros are known.
 struct ColOut {
   int32_t* contrib;
-  uint64_t* nzkey;
+  int32_t* nzrow;
+  int32_t* nzpos;
+  int32_t* wide;   // of each batch: its columns are sorted by warps
+  int32_t* list;   // the batches that are
+  int32_t* nlist;  // their number
 };
 
 __device__ __forceinline__ void put_key(const SlotGen& g, const ColOut& o, int64_t b, uint64_t key, int t, bool first,
                                         int li) {
   o.contrib[b + t] = (int32_t)slot_store(g, (int64_t)(key & 0xffffffffull));
-  if (first) o.nzkey[b + li] = (key & 0xffffffff00000000ull) | (uint64_t)(uint32_t)(b + t);
+  if (first) {
+    o.nzrow[b + li] = (int32_t)(key >> 32);
+    o.nzpos[b + li] = (int32_t)(b + t);
+  }
 }
 
 // Sort 32 < n <= 64 keys (keys[b + lane], keys[b + 32 + lane]) by merging:
 // the first 32 and the other n - 32 are sorted in registers separately, each
 // key's place is its index plus the number of keys of the other sequence
 // below it; the keys are placed in sh and read back in order.
-__device__ __forceinline__ void sort_column_merge(const SlotGen& g, const ColOut& o, int64_t b, int n,
-                                                  const uint64_t* keys, int32_t* cnt_out, uint64_t* sh, int lane) {
+__device__ __forceinline__ int sort_column_merge(const SlotGen& g, const ColOut& o, int64_t b, int n,
+                                                 const uint64_t* keys, uint64_t* sh, int lane) {
   uint64_t v0 = keys[b + lane];
   uint64_t v1 = lane + 32 < n ? keys[b + lane + 32] : ~0ull;
   const int m = n - 32;
@@ -260,17 +296,17 @@ __device__ __forceinline__ void sort_column_merge(const SlotGen& g, const ColOut
   const unsigned below = (1u << lane) - 1u;
   put_key(g, o, b, s0, lane, f0, __popc(m0 & below));
   if (lane + 32 < n) put_key(g, o, b, s1, lane + 32, f1, __popc(m0) + __popc(m1 & below));
-  if (lane == 0) *cnt_out = __popc(m0) + __popc(m1);
   __syncwarp();  // sh is reused by the warp's next column
+  return __popc(m0) + __popc(m1);
 }
 
-// Sort one column's keys by (row, slot), write its output (ColOut) and its
+// Sort one column's keys by (row, slot), write its output (ColOut) and return its
 // number of distinct rows (one warp).  Columns of up to 32 keys are sorted in
 // registers, up to 64 by sort_column_merge; longer ones with the bitonic
 // network in shared memory (up to kSortCap keys, in sh) or in place in global
 // memory.
-__device__ void sort_column(const SlotGen& g, const ColOut& o, int64_t b, int n, uint64_t* keys, int32_t* cnt_out,
-                            uint64_t* sh, int lane) {
+__device__ int sort_column(const SlotGen& g, const ColOut& o, int64_t b, int n, uint64_t* keys,
+                           uint64_t* sh, int lane) {
   const unsigned below = (1u << lane) - 1u;
   if (n <= 32) {
     const bool has = lane < n;
@@ -295,13 +331,9 @@ __device__ void sort_column(const SlotGen& g, const ColOut& o, int64_t b, int n,
     const bool first = lane < n && (lane == 0 || (v >> 32) != (pv >> 32));
     const unsigned m = __ballot_sync(0xffffffffu, first);
     if (lane < n) put_key(g, o, b, v, lane, first, __popc(m & below));
-    if (lane == 0) *cnt_out = __popc(m);
-    return;
+    return __popc(m);
   }
-  if (n <= 64) {
-    sort_column_merge(g, o, b, n, keys, cnt_out, sh, lane);
-    return;
-  }
+  if (n <= 64) return sort_column_merge(g, o, b, n, keys, sh, lane);
   uint64_t* a;
   if (n <= kSortCap) {
     for (int t = lane; t < n; t += 32) sh[t] = keys[b + t];
@@ -324,97 +356,302 @@ __device__ void sort_column(const SlotGen& g, const ColOut& o, int64_t b, int n,
     if (t < n) put_key(g, o, b, key, t, first, cnt + __popc(m & below));
     cnt += __popc(m);
   }
-  if (lane == 0) *cnt_out = cnt;
   __syncwarp();
+  return cnt;
 }
 
-// A warp takes four consecutive columns.  When each has at most 8 keys (the
-// rhs pattern, where a column holds a node's element contributions), the
-// four are sorted at once, one per group of 8 lanes; when each has at most
-// 16 (T6 midside columns), two at a time; otherwise one after the other by
-// the whole warp.
-constexpr int kColsPerWarp = 4;
-
-__global__ void __launch_bounds__(kSortThreads) sort_cols_k(SlotGen g, ColOut o, const int64_t* colstart,
-                                                           int64_t ncol, uint64_t* keys, int32_t* nnzcnt) {
-  __shared__ uint64_t sh[kSortThreads / 32][kSortCap];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int grp = lane >> 3, gl = lane & 7;
-  const unsigned below = (1u << lane) - 1u;
-  const int64_t warps = (int64_t)gridDim.x * (kSortThreads / 32);
-  for (int64_t c0 = ((int64_t)blockIdx.x * (kSortThreads / 32) + wid) * kColsPerWarp; c0 < ncol;
-       c0 += warps * kColsPerWarp) {
-    const int64_t cg = c0 + grp;
-    int64_t bg = 0;
-    int ng = 0;
-    if (cg < ncol) {
-      bg = colstart[cg];
-      ng = (int)(colstart[cg + 1] - bg);
-    }
-    if (__all_sync(0xffffffffu, ng <= 8)) {
-      uint64_t v = gl < ng ? keys[bg + gl] : ~0ull;
-      v = reg_sort<8>(v, gl);  // partners lane ^ j (j < 8) stay inside the group
-      const uint64_t pv = __shfl_up_sync(0xffffffffu, v, 1, 8);
-      const bool first = gl < ng && (gl == 0 || (v >> 32) != (pv >> 32));
-      const unsigned group = 0xffu << (grp * 8);
-      const unsigned m = __ballot_sync(0xffffffffu, first) & group;
-      if (gl < ng) put_key(g, o, bg, v, gl, first, __popc(m & below));
-      if (gl == 0 && cg < ncol) nnzcnt[cg] = __popc(m);
-      continue;
-    }
-    if (__all_sync(0xffffffffu, ng <= 16)) {
-      // two columns at a time, one per half warp (T6 midside columns: 12 keys)
-      const int h = lane >> 4, hl = lane & 15;
-      const unsigned half = 0xffffu << (h * 16);
+// Merge exchange (Knuth, The Art of Computer Programming 3, 5.2.2, algorithm M)
+// of N keys in registers: the smaller key of every comparator at the lower
+// index, so keys of ~0 after the column's own stay behind them.
+template <int N, typename K>
+__device__ __forceinline__ void net_sort(K (&k)[N]) {
+  constexpr int LG = N <= 2 ? 1 : N <= 4 ? 2 : N <= 8 ? 3 : N <= 16 ? 4 : N <= 32 ? 5 : N <= 64 ? 6 : 7;
 #pragma unroll
-      for (int r = 0; r < kColsPerWarp / 2; ++r) {
-        const int q = 2 * r + h;
-        const int64_t b = __shfl_sync(0xffffffffu, bg, q * 8);
-        const int n = __shfl_sync(0xffffffffu, ng, q * 8);
-        const bool has = hl < n;
-        uint64_t v = has ? keys[b + hl] : ~0ull;
-        const uint32_t rv = (uint32_t)(v >> 32), sv = (uint32_t)v;
-        Pack32 pk;
-        // partners lane ^ j (j < 16) stay inside the half; both halves take
-        // the same branch only when both packings fit
-        const bool fit = pack_half(has ? rv : ~0u, has ? rv : 0u, has ? sv : ~0u, has ? sv : 0u, &pk);
-        if (__all_sync(0xffffffffu, fit || n <= 1)) {
-          uint32_t k = has && n > 1 ? pack32(v, pk) : ~0u;
-          k = reg_sort<16>(k, hl);
-          if (n > 1) v = has ? unpack32(k, pk) : ~0ull;
-        } else {
-          v = reg_sort<16>(v, hl);
+  for (int lp = LG - 1; lp >= 0; --lp) {
+    const int p = 1 << lp;
+#pragma unroll
+    for (int lq = LG - 1; lq >= lp; --lq) {
+      const int r = lq == LG - 1 ? 0 : p, d = lq == LG - 1 ? p : (2 << lq) - p;
+#pragma unroll
+      for (int i = 0; i < N; ++i)
+        if (i + d < N && (i & p) == r) {
+          const K x = k[i], y = k[i + d];
+          k[i] = min(x, y);
+          k[i + d] = max(x, y);
         }
-        const uint64_t pv = __shfl_up_sync(0xffffffffu, v, 1, 16);
-        const bool first = hl < n && (hl == 0 || (v >> 32) != (pv >> 32));
-        const unsigned m = __ballot_sync(0xffffffffu, first) & half;
-        if (hl < n) put_key(g, o, b, v, hl, first, __popc(m & below));
-        if (hl == 0 && c0 + q < ncol) nnzcnt[c0 + q] = __popc(m);
-      }
-      continue;
-    }
-    for (int q = 0; q < kColsPerWarp; ++q) {
-      const int64_t col = c0 + q;
-      if (col >= ncol) break;
-      const int64_t b = colstart[col];
-      sort_column(g, o, b, (int)(colstart[col + 1] - b), keys, nnzcnt + col, sh[wid], lane);
     }
   }
 }
 
-// rowval / cptr of every column from its row starts (ColOut.nzkey): one half
-// warp per column.
-__global__ void compact_k(const int64_t* __restrict__ colstart, const int64_t* __restrict__ colptr, int64_t ncol,
-                          const uint64_t* __restrict__ nzkey, int32_t* __restrict__ rowval,
-                          int32_t* __restrict__ cptr) {
-  const int hl = threadIdx.x & 15;
-  const int64_t halves = (int64_t)gridDim.x * (blockDim.x / 16);
-  for (int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 4; c < ncol; c += halves) {
-    const int64_t k0 = colptr[c], cnt = colptr[c + 1] - k0, b = colstart[c];
-    for (int64_t i = hl; i < cnt; i += 16) {
-      const uint64_t v = nzkey[b + i];
-      rowval[k0 + i] = (int32_t)(v >> 32);
-      cptr[k0 + i] = (int32_t)(uint32_t)v;
+// Shared-memory index of word a of a batch: the columns of a warp start n words
+// apart, and one word of padding in 32 spreads the usual n (12, 16, 36) over the
+// banks.  64-bit keys: one in 16.
+__device__ __forceinline__ int pad32(int a) { return a + (a >> 5); }
+__device__ __forceinline__ int pad64(int a) { return a + (a >> 4); }
+
+// The batch of columns of a warp, one per lane.
+struct Batch {
+  int64_t b0;   // first slot
+  int total;    // slots
+  int off, n;   // of the lane's column: slots before it in the batch, its slots
+  int ng;       // its column groups (block mode)
+  int nmax, ngmax;
+};
+
+// Rows and storage indices of the lane's column, groups in order, to the shared
+// areas (T: storage indices, R: rows); returns the column's smallest row and
+// whether the row span fits the 32-bit keys.
+template <int NG>
+__device__ __forceinline__ bool fill_groups(const SlotGen& g, const Batch& B, const uint32_t* gk, int32_t* T, int32_t* R,
+                                            uint32_t span, uint32_t* row0) {
+  int32_t* Q = T;  // the sorted groups wait at the end of the column's part of T: a group's
+                   // entries end at or before its own number, as every later group has one at least
+  {
+    uint32_t q[NG];
+#pragma unroll
+    for (int i = 0; i < NG; ++i) q[i] = i < B.ng ? gk[B.b0 + B.off + i] : ~0u;
+    net_sort<NG>(q);
+#pragma unroll
+    for (int i = 0; i < NG; ++i)
+      if (i < B.ng) Q[pad32(B.off + B.n - B.ng + i)] = (int32_t)q[i];
+  }
+  uint32_t lo = ~0u, hi = 0u;
+  int p = B.off;
+  for (int i = 0; i < B.ng; ++i) {
+    const GroupPos G = group_pos(g, (uint32_t)Q[pad32(B.off + B.n - B.ng + i)]);
+    const SlotBlock& K = g.b[G.bi];
+    const int len = K.transposed ? K.nc : K.nr;
+    const int32_t* rt = K.transposed ? K.C + (int64_t)G.e * K.nc : (K.R ? K.R + (int64_t)G.e * K.nr : nullptr);
+    const int32_t st = (int32_t)((int64_t)G.e * g.store_per_elem + K.store_off);
+    constexpr int U = 6;
+    for (int k0 = 0; k0 < len; k0 += U) {
+      uint32_t row[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) row[u] = rt && k0 + u < len ? (uint32_t)__ldg(rt + k0 + u) : 0u;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (k0 + u < len) {
+          const int k = k0 + u, a = K.transposed ? G.lg : k, b = K.transposed ? k : G.lg;
+          T[pad32(p)] = st + (K.sym ? sym_index(a, b) : a + b * K.nr);
+          R[pad32(p)] = (int32_t)row[u];
+          lo = min(lo, row[u]);
+          hi = max(hi, row[u]);
+          ++p;
+        }
+    }
+  }
+  *row0 = lo;
+  return B.ng == 0 || hi - lo <= span;
+}
+
+// Row starts of the batch from each lane's sorted rows (row(i), i < n), then
+// both shared areas to the output; the batch's contrib has left R.
+template <int N, typename F>
+__device__ __forceinline__ int put_starts(const ColOut& o, const Batch& B, int lane, int32_t* T, int32_t* R, F row) {
+  uint32_t first[(N + 31) / 32] = {};
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (i < B.n && (i == 0 || row(i) != row(i - 1))) first[i / 32] |= 1u << (i % 32);
+  int cnt = 0;
+#pragma unroll
+  for (int w = 0; w < (N + 31) / 32; ++w) cnt += __popc(first[w]);
+  int end = cnt;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, end, d);
+    if (lane >= d) end += v;
+  }
+  const int tot = __shfl_sync(0xffffffffu, end, 31);
+  int j = end - cnt;
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (first[i / 32] >> (i % 32) & 1) {
+      T[pad32(j)] = (int32_t)row(i);
+      R[pad32(j)] = (int32_t)(B.b0 + B.off + i);
+      ++j;
+    }
+  __syncwarp();
+  for (int t = lane; t < tot; t += 32) {
+    o.nzrow[B.b0 + t] = T[pad32(t)];
+    o.nzpos[B.b0 + t] = R[pad32(t)];
+  }
+  __syncwarp();  // the areas are reused by the warp's next batch
+  return cnt;
+}
+
+__device__ __forceinline__ void put_contrib(const ColOut& o, const Batch& B, int lane, const int32_t* R) {
+  __syncwarp();
+  for (int t = lane; t < B.total; t += 32) o.contrib[B.b0 + t] = R[pad32(t)];
+  __syncwarp();
+}
+
+// Block mode: keys (row - row0) << BITS | place in slot order.
+template <int N, int BITS>
+__device__ __forceinline__ int net_groups(const ColOut& o, const Batch& B, int lane, int32_t* T, int32_t* R,
+                                          uint32_t row0) {
+  uint32_t k[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) k[i] = i < B.n ? ((uint32_t)R[pad32(B.off + i)] - row0) << BITS | (uint32_t)i : ~0u;
+  net_sort<N>(k);
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (i < B.n) R[pad32(B.off + i)] = T[pad32(B.off + (int)(k[i] & ((1u << BITS) - 1u)))];
+  put_contrib(o, B, lane, R);
+  return put_starts<N>(o, B, lane, T, R, [&](int i) { return (k[i] >> BITS) + row0; });
+}
+
+// COO mode: keys row << 32 | slot, the slot being the storage index.
+template <int N>
+__device__ __forceinline__ int net_keys(const ColOut& o, const Batch& B, int lane, int32_t* T, int32_t* R,
+                                        const uint64_t* keys) {
+  uint64_t* K = reinterpret_cast<uint64_t*>(T);  // both areas
+  for (int t = lane; t < B.total; t += 32) K[pad64(t)] = keys[B.b0 + t];
+  __syncwarp();
+  uint64_t k[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) k[i] = i < B.n ? K[pad64(B.off + i)] : ~0ull;
+  __syncwarp();
+  net_sort<N>(k);
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (i < B.n) R[pad32(B.off + i)] = (int32_t)(uint32_t)k[i];
+  put_contrib(o, B, lane, R);
+  return put_starts<N>(o, B, lane, T, R, [&](int i) { return (uint32_t)(k[i] >> 32); });
+}
+
+// The keys of a column of block mode (one warp), for sort_column.
+__device__ __forceinline__ void expand_groups(const SlotGen& g, int64_t b, int ng, const uint32_t* gk, uint64_t* keys,
+                                              int lane) {
+  int64_t at = b;
+  for (int i0 = 0; i0 < ng; i0 += 32) {
+    int32_t c;
+    int64_t s0 = 0;
+    int len = 0;
+    const int32_t* rt = nullptr;
+    if (i0 + lane < ng) group_info(g, gk[b + i0 + lane], c, s0, len, rt);
+    int end = len;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, end, d);
+      if (lane >= d) end += v;
+    }
+    for (int k = 0; k < len; ++k)
+      keys[at + end - len + k] = (uint64_t)(rt ? (uint32_t)rt[k] : 0u) << 32 | (uint64_t)(uint32_t)(s0 + k);
+    at += __shfl_sync(0xffffffffu, end, 31);
+  }
+  __syncwarp();
+}
+
+// A warp sorts 32 columns, one per thread, in registers: a network of N keys is
+// 2 (32-bit keys) or 6 (64-bit) instructions a comparator and thread, so a column
+// of 12 costs about 3 warp instructions and one of 36 about 16 (bitonic sorts across the
+// lanes: about 100 and 300).  All global reads and writes of sorted data are
+// whole-batch copies through shared memory.  Batches with a longer column,
+// more groups, or a row span beyond 26 bits are left to sort_wide_k.
+// Measured (500,000 T6 elements, 18M slots): 279 us with one column per warp or
+// half warp, 150 us here (60 % of the issue slots idle on instruction fetch of the
+// unrolled networks and shared-memory latency at 16 warps an SM).
+template <bool COO, int NK>
+__global__ void __launch_bounds__(Net<NK>::kThreads, Net<NK>::kBlocks)
+    sort_cols_k(SlotGen g, ColOut o, const int64_t* colstart, const int32_t* gcnt, const uint32_t* gk, int64_t ncol,
+                const uint64_t* keys, int32_t* nnzcnt) {
+  using D = Net<NK>;
+  constexpr int W = D::kThreads / 32;
+  __shared__ __align__(8) int32_t areas[W][2 * D::kArea];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int32_t *T = areas[wid], *R = areas[wid] + D::kArea;
+  const int64_t warps = (int64_t)gridDim.x * W;
+  for (int64_t c0 = ((int64_t)blockIdx.x * W + wid) * kColBatch; c0 < ncol;
+       c0 += warps * kColBatch) {
+    const int64_t c = c0 + lane, c1 = min(c0 + kColBatch, ncol);
+    Batch B;
+    B.b0 = colstart[c0];
+    const int64_t tot = colstart[c1] - B.b0;
+    B.off = (int)((c < c1 ? colstart[c] : colstart[c1]) - B.b0);
+    B.n = c < c1 ? (int)(colstart[c + 1] - B.b0) - B.off : 0;
+    B.ng = !COO && c < c1 ? gcnt[c] : 0;
+    B.nmax = __reduce_max_sync(0xffffffffu, B.n);
+    B.ngmax = COO ? 0 : __reduce_max_sync(0xffffffffu, B.ng);
+    B.total = (int)min(tot, (int64_t)D::kBatch + 1);
+    int cnt = 0;
+    bool done = false;
+    if (B.total <= D::kBatch && B.nmax <= NK && B.ngmax <= D::kGroups) {
+      uint32_t row0 = 0;
+      bool fit = true;
+      if (!COO) {
+        if (B.ngmax <= 2) fit = fill_groups<2>(g, B, gk, T, R, D::kSpan, &row0);
+        else if (B.ngmax <= 8) fit = fill_groups<8>(g, B, gk, T, R, D::kSpan, &row0);
+        else fit = fill_groups<D::kGroups>(g, B, gk, T, R, D::kSpan, &row0);
+      }
+      if (__all_sync(0xffffffffu, fit)) {
+#define NET_COLUMNS(N)                                     \
+  do {                                                     \
+    if constexpr (COO) cnt = net_keys<N>(o, B, lane, T, R, keys); \
+    else cnt = net_groups<N, D::kBits>(o, B, lane, T, R, row0);   \
+  } while (0)
+        if constexpr (NK <= 48) {
+          if (B.nmax <= 6) NET_COLUMNS(6);
+          else if (B.nmax <= 12) NET_COLUMNS(12);
+          else if (B.nmax <= 18) NET_COLUMNS(18);
+          else if (B.nmax <= 24) NET_COLUMNS(24);
+          else if (B.nmax <= 36) NET_COLUMNS(36);
+          else NET_COLUMNS(NK);
+        } else {
+          if (B.nmax <= 24) NET_COLUMNS(24);
+          else if (B.nmax <= 36) NET_COLUMNS(36);
+          else if (B.nmax <= 48) NET_COLUMNS(48);
+          else if (B.nmax <= 72) NET_COLUMNS(72);
+          else NET_COLUMNS(NK);
+        }
+#undef NET_COLUMNS
+        if (c < c1) nnzcnt[c] = cnt;
+        done = true;
+      }
+    }
+    __syncwarp();
+    if (lane == 0) {
+      const int32_t k = (int32_t)(c0 / kColBatch);
+      o.wide[k] = !done;
+      if (!done) o.list[atomicAdd(o.nlist, 1)] = k;
+    }
+  }
+}
+
+// The columns of the batches left by sort_cols_k, a warp each: one block per batch.
+template <bool COO>
+__global__ void __launch_bounds__(kWideThreads) sort_wide_k(SlotGen g, ColOut o, const int64_t* colstart,
+                                                           const int32_t* gcnt, const uint32_t* gk, int64_t ncol,
+                                                           uint64_t* keys, int32_t* nnzcnt) {
+  __shared__ uint64_t sh[kWideThreads / 32][kSortCap];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int n = *o.nlist;
+  for (int i = blockIdx.x; i < n; i += gridDim.x) {
+    const int64_t k = o.list[i];
+    const int64_t c1 = min((k + 1) * kColBatch, ncol);
+    for (int64_t c = k * kColBatch + wid; c < c1; c += kWideThreads / 32) {
+      const int64_t b = colstart[c];
+      if (!COO) expand_groups(g, b, gcnt[c], gk, keys, lane);
+      const int cnt = sort_column(g, o, b, (int)(colstart[c + 1] - b), keys, sh[wid], lane);
+      if (lane == 0) nnzcnt[c] = cnt;
+    }
+  }
+}
+
+// rowval / cptr from the row starts (ColOut): one warp per batch.
+__global__ void compact_k(ColOut o, const int64_t* __restrict__ colstart, const int64_t* __restrict__ colptr,
+                          int64_t ncol, int32_t* __restrict__ rowval, int32_t* __restrict__ cptr) {
+  const int lane = threadIdx.x & 31;
+  const int64_t stride = ((int64_t)gridDim.x * blockDim.x >> 5) * kColBatch;
+  for (int64_t c0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kColBatch; c0 < ncol; c0 += stride) {
+    const int64_t c1 = min(c0 + kColBatch, ncol);
+    const bool wide = o.wide[c0 / kColBatch];
+    for (int64_t c = c0; c < c1; c = wide ? c + 1 : c1) {
+      const int64_t k0 = colptr[c], cnt = colptr[wide ? c + 1 : c1] - k0, b = colstart[c];
+#pragma unroll 4
+      for (int64_t i = lane; i < cnt; i += 32) {
+        rowval[k0 + i] = o.nzrow[b + i];
+        cptr[k0 + i] = o.nzpos[b + i];
+      }
     }
   }
 }
@@ -482,68 +719,89 @@ int build_pattern(Ctx* c, const SlotGen& g0, int64_t nrow, int64_t ncol, Pattern
   DBuf<int32_t> colcnt, cursor;
   DBuf<int64_t> colstart;
   DBuf<uint64_t> keys;
-  DBuf<int> bad;
-  ELFEL_TRY(colcnt.alloc(c, (size_t)ncol + 1));
-  ELFEL_TRY(cursor.alloc(c, (size_t)ncol + 1));
+  // counts, the flag of slots out of range, the number of wide batches, their marks and list (ColOut)
+  const int64_t nbatch = (ncol + kColBatch - 1) / kColBatch;
+  ELFEL_TRY(colcnt.alloc(c, (size_t)(ncol + 2 + 2 * nbatch)));
+  ELFEL_TRY(cursor.alloc(c, (size_t)(ncol > 0 ? ncol : 1)));
   ELFEL_TRY(colstart.alloc(c, (size_t)ncol + 1));
-  ELFEL_TRY(bad.alloc(c, 1));
-  ELFEL_CUDA(c, cudaMemsetAsync(colcnt.p, 0, sizeof(int32_t) * (ncol + 1), st));
-  ELFEL_CUDA(c, cudaMemsetAsync(cursor.p, 0, sizeof(int32_t) * (ncol + 1), st));
-  ELFEL_CUDA(c, cudaMemsetAsync(bad.p, 0, sizeof(int), st));
+  int* bad = colcnt.p + ncol;
+  ELFEL_CUDA(c, cudaMemsetAsync(colcnt.p, 0, sizeof(int32_t) * (ncol + 2), st));
+  if (ncol > 0) ELFEL_CUDA(c, cudaMemsetAsync(cursor.p, 0, sizeof(int32_t) * ncol, st));
   const unsigned gs = grid_for(M, 256, (int64_t)c->sm_count * 16);
-  const int G = groups_per_elem(g);
-  const int64_t ngroups = g.nblocks ? g.nel * (int64_t)G : 0;
+  const int64_t ngroups = g.nblocks ? g.nel * (int64_t)g.groups : 0;
+  const unsigned gg = grid_for(ngroups, 256, (int64_t)c->sm_count * 16);
   if (M > 0) {
-    if (g.nblocks)
-      count_groups_k<<<grid_for(ngroups, 256, (int64_t)c->sm_count * 16), 256, 0, st>>>(g, G, ngroups, colcnt.p,
-                                                                                        ncol, bad.p);
-    else
-      count_cols_k<<<gs, 256, 0, st>>>(g, M, colcnt.p, ncol, nrow, bad.p);
+    if (g.nblocks) count_groups_k<<<gg, 256, 0, st>>>(g, ngroups, colcnt.p, ncol, bad);
+    else count_cols_k<<<gs, 256, 0, st>>>(g, M, colcnt.p, ncol, nrow, bad);
     ELFEL_LAUNCH_CHECK(c);
   }
-  int hbad = 0;
-  ELFEL_CUDA(c, cudaMemcpyAsync(&hbad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-  ELFEL_CUDA(c, cudaStreamSynchronize(st));
-  if (hbad) return fail(c, ELFEL_ERR_ARG, "assembled row or column number out of range (1..%lld, 1..%lld)",
-                        (long long)nrow, (long long)ncol);
   ELFEL_TRY(scan_counts_i32(c, colcnt.p, ncol, colstart.p));
-  ELFEL_TRY(keys.alloc(c, (size_t)(M > 0 ? M : 1)));
+  const size_t m1 = (size_t)(M > 0 ? M : 1);
+  ELFEL_TRY(keys.alloc(c, m1));
+  // row starts (ColOut), compacted after the scan; the group numbers share the
+  // array of the positions (a batch's groups are read before its first row start
+  // is written, those of a wide batch's column before the column's)
+  DBuf<int32_t> nzrow, nzpos;
+  ELFEL_TRY(nzrow.alloc(c, m1));
+  ELFEL_TRY(nzpos.alloc(c, m1));
+  uint32_t* gk = reinterpret_cast<uint32_t*>(nzpos.p);
   if (M > 0) {
-    bucket_k<<<gs, 256, 0, st>>>(g, M, colstart.p, cursor.p, keys.p);
+    if (g.nblocks) bucket_groups_k<<<gg, 256, 0, st>>>(g, ngroups, colstart.p, ncol, cursor.p, gk);
+    else bucket_k<<<gs, 256, 0, st>>>(g, M, colstart.p, nrow, ncol, cursor.p, keys.p);
+    ELFEL_LAUNCH_CHECK(c);
+  }
+  // sort + distinct counts (reuse colcnt as per-column nonzero counts)
+  ELFEL_TRY(P->contrib.alloc(c, m1));
+  int32_t* marks = colcnt.p + ncol + 2;
+  const ColOut out{P->contrib.p, nzrow.p, nzpos.p, marks, marks + nbatch, colcnt.p + ncol + 1};
+  if (ncol > 0) {
+    const unsigned gwide = grid_for(nbatch, 1, (int64_t)c->sm_count * 8);
+    auto sort = [&](auto coo, auto nk) {
+      constexpr bool COO = decltype(coo)::value;
+      using D = Net<decltype(nk)::value>;
+      const unsigned grid = grid_for(nbatch, D::kThreads / 32, (int64_t)c->sm_count * 32);
+      sort_cols_k<COO, decltype(nk)::value>
+          <<<grid, D::kThreads, 0, st>>>(g, out, colstart.p, cursor.p, gk, ncol, keys.p, colcnt.p);
+      sort_wide_k<COO><<<gwide, kWideThreads, 0, st>>>(g, out, colstart.p, cursor.p, gk, ncol, keys.p, colcnt.p);
+    };
+    if (!g.nblocks) sort(std::true_type{}, std::integral_constant<int, kNet64>{});
+    else if (M <= kNetMean * ncol) sort(std::false_type{}, std::integral_constant<int, kNet>{});
+    else sort(std::false_type{}, std::integral_constant<int, kNetL>{});
     ELFEL_LAUNCH_CHECK(c);
   }
   cursor.release(c);
-  // sort + distinct counts (reuse colcnt as per-column nonzero counts)
-  const unsigned gsort = grid_for((ncol + kColsPerWarp - 1) / kColsPerWarp, kSortThreads / 32,
-                                  (int64_t)c->sm_count * 32);
-  DBuf<uint64_t> nzkey;  // row starts of each column (ColOut), compacted after the scan
-  ELFEL_TRY(nzkey.alloc(c, (size_t)(M > 0 ? M : 1)));
-  ELFEL_TRY(P->contrib.alloc(c, (size_t)(M > 0 ? M : 1)));
-  if (ncol > 0) {
-    sort_cols_k<<<gsort, kSortThreads, 0, st>>>(g, ColOut{P->contrib.p, nzkey.p}, colstart.p, ncol, keys.p,
-                                               colcnt.p);
-    ELFEL_LAUNCH_CHECK(c);
-  }
+  keys.release(c);
   ELFEL_TRY(P->colptr.alloc(c, (size_t)ncol + 1));
   ELFEL_TRY(scan_counts_i32(c, colcnt.p, ncol, P->colptr.p));
   int64_t nnz = 0;
+  int hbad = 0;
   ELFEL_CUDA(c, cudaMemcpyAsync(&nnz, P->colptr.p + ncol, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  ELFEL_CUDA(c, cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, st));
   ELFEL_CUDA(c, cudaStreamSynchronize(st));
+  if (hbad) {
+    // slots out of range were left out of every step
+    nzrow.release(c);
+    nzpos.release(c);
+    colcnt.release(c);
+    colstart.release(c);
+    P->release(c);
+    return fail(c, ELFEL_ERR_ARG, "assembled row or column number out of range (1..%lld, 1..%lld)", (long long)nrow,
+                (long long)ncol);
+  }
   P->nnz = nnz;
   ELFEL_TRY(P->rowval.alloc(c, (size_t)(nnz > 0 ? nnz : 1)));
   ELFEL_TRY(P->cptr.alloc(c, (size_t)nnz + 1));
   if (ncol > 0) {
-    compact_k<<<grid_for(ncol, 16, (int64_t)c->sm_count * 32), 256, 0, st>>>(colstart.p, P->colptr.p, ncol,
-                                                                            nzkey.p, P->rowval.p, P->cptr.p);
+    compact_k<<<grid_for(nbatch, 8, (int64_t)c->sm_count * 32), 256, 0, st>>>(out, colstart.p, P->colptr.p, ncol,
+                                                                             P->rowval.p, P->cptr.p);
     ELFEL_LAUNCH_CHECK(c);
   }
-  nzkey.release(c);
+  nzrow.release(c);
+  nzpos.release(c);
   set_last_k<<<1, 1, 0, st>>>(P->cptr.p, nnz, M);
   ELFEL_LAUNCH_CHECK(c);
-  keys.release(c);
   colcnt.release(c);
   colstart.release(c);
-  bad.release(c);
   return ELFEL_OK;
 }
 
@@ -723,27 +981,49 @@ __global__ void to_index32_k(const int64_t* src, int64_t n, int64_t limit, int32
   }
 }
 
-// The same conversion reading the (device-readable) host array directly:
-// four independent loads per thread keep enough bytes in flight over the
-// host link with a small grid, which leaves most of the SMs to the work on
-// other streams.
-__global__ void to_index32_host_k(const int64_t* __restrict__ src, int64_t n, int64_t limit, int32_t* __restrict__ dst,
-                                  int* __restrict__ bad) {
-  constexpr int U = 4;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i0 < n; i0 += U * stride) {
-    int64_t v[U];
+// The same conversion reading the (device-readable) host array directly.  Beside
+// the pattern build (the auxiliary stream) one block of 64 threads for two SMs, each
+// thread with eight 16-byte loads in flight (0.6 MB in all), leaves registers, block
+// slots and issue to it; alone on the link, four an SM.  Set-up to CSC of 500,000 T6
+// elements: 1698 us; 4 and 1 an SM 1720, 8 and 2 1765, 8 and 8 1814.
+constexpr int kHostThreads = 64;
+
+__device__ __forceinline__ int32_t index32(int64_t v, int64_t limit, bool* bad) {
+  const bool out = v < 1 || v > limit;
+  *bad |= out;
+  return out ? 0 : (int32_t)(v - 1);
+}
+
+__global__ void __launch_bounds__(kHostThreads) to_index32_host_k(const int64_t* __restrict__ src, int64_t n,
+                                                                  int64_t limit, int32_t* __restrict__ dst,
+                                                                  int* __restrict__ bad) {
+  constexpr int U = 8;
+  const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+  bool b = false;
+  const int64_t pairs = ((uintptr_t)src & 15) ? 0 : n / 2;  // 16-byte loads where the array allows them
+  const longlong2* s2 = reinterpret_cast<const longlong2*>(src);
+  int2* d2 = reinterpret_cast<int2*>(dst);
+  for (int64_t i0 = tid; i0 < pairs; i0 += U * stride) {
+    longlong2 v[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) v[u] = i0 + u * stride < n ? src[i0 + u * stride] : 1;
-    bool b = false;
+    for (int u = 0; u < U; ++u) v[u] = i0 + u * stride < pairs ? __ldcs(s2 + i0 + u * stride) : longlong2{1, 1};
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const bool out = v[u] < 1 || v[u] > limit;
-      b |= out;
-      if (i0 + u * stride < n) dst[i0 + u * stride] = out ? 0 : (int32_t)(v[u] - 1);
+      const int2 r{index32(v[u].x, limit, &b), index32(v[u].y, limit, &b)};
+      if (i0 + u * stride < pairs) d2[i0 + u * stride] = r;
     }
-    if (b) atomicExch(bad, 1);
   }
+  for (int64_t i0 = 2 * pairs + tid; i0 < n; i0 += U * stride) {
+    int64_t v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = i0 + u * stride < n ? __ldcs((const long long*)src + i0 + u * stride) : 1;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int32_t r = index32(v[u], limit, &b);
+      if (i0 + u * stride < n) dst[i0 + u * stride] = r;
+    }
+  }
+  if (b) atomicExch(bad, 1);
 }
 
 __global__ void copy_host_f64_k(const double* __restrict__ src, int64_t n, double* __restrict__ dst) {
@@ -761,7 +1041,8 @@ __global__ void copy_host_f64_k(const double* __restrict__ src, int64_t n, doubl
 
 int to_index32_direct(Ctx* c, cudaStream_t st, const int64_t* src, int64_t n, int64_t limit, int32_t* dst, int* bad) {
   if (n == 0) return ELFEL_OK;
-  to_index32_host_k<<<grid_for(n, 256 * 4, (int64_t)c->sm_count * 2), 256, 0, st>>>(src, n, limit, dst, bad);
+  const int64_t cap = st == c->stream ? 4 * (int64_t)c->sm_count : (c->sm_count + 1) / 2;
+  to_index32_host_k<<<grid_for(n, kHostThreads * 2, cap), kHostThreads, 0, st>>>(src, n, limit, dst, bad);
   ELFEL_LAUNCH_CHECK(c);
   return ELFEL_OK;
 }

@@ -57,11 +57,15 @@ struct SlotGen {
   const int32_t* J = nullptr;
   int64_t ncoo = 0;
   int64_t total() const { return nblocks ? nel * (int64_t)slots_per_elem : ncoo; }
-  // divisions of slot_rc (prepare() sets them; build_pattern does)
-  FastDiv spe_div, nr_div[kMaxBlocks], nc_div[kMaxBlocks];
+  // divisions of slot_rc and group_pos (prepare() sets them; build_pattern does)
+  FastDiv spe_div, grp_div, nr_div[kMaxBlocks], nc_div[kMaxBlocks];
+  int groups = 0;  // groups_per_elem
   void prepare() {
     if (!nblocks) return;
+    groups = 0;
+    for (int k = 0; k < nblocks; ++k) groups += b[k].transposed ? b[k].nr : b[k].nc;
     spe_div.init((uint32_t)slots_per_elem);
+    grp_div.init((uint32_t)(groups > 0 ? groups : 1));
     for (int k = 0; k < nblocks; ++k) {
       nr_div[k].init((uint32_t)(b[k].nr > 0 ? b[k].nr : 1));
       nc_div[k].init((uint32_t)(b[k].nc > 0 ? b[k].nc : 1));
@@ -102,32 +106,39 @@ __device__ __forceinline__ int64_t slot_store(const SlotGen& g, int64_t s) {
 
 // Block mode: the slots of one element come in runs that share a column --
 // the nr slots of a local column of a plain block, the nc slots of a parent
-// row of a transposed one ("column groups", groups_per_elem() per element).
-__host__ __device__ __forceinline__ int groups_per_elem(const SlotGen& g) {
-  int n = 0;
-  for (int k = 0; k < g.nblocks; ++k) n += g.b[k].transposed ? g.b[k].nr : g.b[k].nc;
-  return n;
-}
+// row of a transposed one ("column groups", SlotGen::groups per element).
+struct GroupPos {
+  uint32_t e;  // element
+  int bi, lg;  // block, the group's number in it
+};
 
-// Column group q: its column, first slot, length, and the element's row table
-// (rows of the group's slots: rtab[k], k < len; nullptr: all rows 0).
-__device__ __forceinline__ void group_info(const SlotGen& g, int G, int64_t q, int32_t& col, int64_t& s0, int& len,
-                                           const int32_t*& rtab) {
-  const int64_t e = q / G;
-  int lg = (int)(q - e * G);
-  int bi = 0;
+// Column group q (numbered element by element, in slot order).
+__device__ __forceinline__ GroupPos group_pos(const SlotGen& g, uint32_t q) {
+  GroupPos p;
+  p.e = g.grp_div.div(q);
+  p.lg = (int)(q - p.e * (uint32_t)g.groups);
+  p.bi = 0;
 #pragma unroll
   for (int k = 0; k < kMaxBlocks; ++k) {
     if (k >= g.nblocks) break;
     const int ng = g.b[k].transposed ? g.b[k].nr : g.b[k].nc;
-    if (lg < ng) {
-      bi = k;
+    if (p.lg < ng) {
+      p.bi = k;
       break;
     }
-    lg -= ng;
+    p.lg -= ng;
   }
-  const SlotBlock& B = g.b[bi];
-  const int64_t base = e * (int64_t)g.slots_per_elem + B.slot_off;
+  return p;
+}
+
+// Column group q: its column, first slot, length, and the element's row table
+// (rows of the group's slots: rtab[k], k < len; nullptr: all rows 0).
+__device__ __forceinline__ void group_info(const SlotGen& g, uint32_t q, int32_t& col, int64_t& s0, int& len,
+                                           const int32_t*& rtab) {
+  const GroupPos p = group_pos(g, q);
+  const SlotBlock& B = g.b[p.bi];
+  const int64_t e = p.e, base = e * (int64_t)g.slots_per_elem + B.slot_off;
+  const int lg = p.lg;
   if (!B.transposed) {  // local column lg: slots lg*nr + i, rows R[e][i]
     col = B.C[e * B.nc + lg];
     s0 = base + (int64_t)lg * B.nr;
