@@ -120,7 +120,14 @@ struct CooStage {
   DBuf<int64_t> I, J;
   DBuf<double> V;
   int64_t n = 0;
+  cudaEvent_t indices = nullptr;  // the row and column numbers of n_indices triplets are on the device
+  int64_t n_indices = 0;
 };
+
+// From here on the pattern of triplets is built on the auxiliary stream while
+// the values, a third of the upload, still cross the host link (2 MB take about
+// 10 us, the event and the join 4).  3.7M triplets to CSC: 942 -> 851 us.
+constexpr int64_t kCooOverlap = 1 << 18;
 
 static CooStage* stage_of(elfel_sysmat* m) {
   static_assert(sizeof(CooStage) > 0, "");
@@ -154,7 +161,7 @@ static void release_all(elfel_sysmat* m) {
   s->I.release(c);
   s->J.release(c);
   s->V.release(c);
-  s->n = 0;
+  s->n = s->n_indices = 0;
   m->P.release(c);
   m->vals.release(c);
   m->rhs.release(c);
@@ -185,6 +192,7 @@ extern "C" int elfel_sysmat_destroy(elfel_sysmat* m) {
     cudaStreamSynchronize(m->h->c.stream);
     if (m->ev_pattern) cudaEventDestroy(m->ev_pattern);
     if (m->head.ev) cudaEventDestroy(m->head.ev);
+    if (stage_of(m)->indices) cudaEventDestroy(stage_of(m)->indices);
   }
   delete stage_of(m);
   delete m;
@@ -217,9 +225,53 @@ extern "C" int elfel_sysmat_assemble_coo(elfel_sysmat* m, const int64_t* rows, c
   ELFEL_TRY(ensure_cap(c, &s->V, (size_t)s->n, (size_t)(s->n + n)));
   ELFEL_CUDA(c, cudaMemcpyAsync(s->I.p + s->n, rows, sizeof(int64_t) * n, cudaMemcpyHostToDevice, c->stream));
   ELFEL_CUDA(c, cudaMemcpyAsync(s->J.p + s->n, cols, sizeof(int64_t) * n, cudaMemcpyHostToDevice, c->stream));
+  if (s->n + n >= kCooOverlap) {
+    if (!s->indices) ELFEL_CUDA(c, cudaEventCreateWithFlags(&s->indices, cudaEventDisableTiming));
+    ELFEL_CUDA(c, cudaEventRecord(s->indices, c->stream));
+    s->n_indices = s->n + n;
+  }
   ELFEL_CUDA(c, cudaMemcpyAsync(s->V.p + s->n, vals, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
   s->n += n;
   m->finished = 0;
+  return ELFEL_OK;
+}
+
+// The pattern of the n staged triplets, on the context stream.
+static int coo_pattern(elfel_sysmat* m, int64_t n) {
+  Ctx* c = &m->h->c;
+  CooStage* s = stage_of(m);
+  DBuf<int32_t> I, J;
+  DBuf<int> bad;
+  ELFEL_TRY(I.alloc(c, (size_t)(n > 0 ? n : 1)));
+  ELFEL_TRY(J.alloc(c, (size_t)(n > 0 ? n : 1)));
+  ELFEL_TRY(bad.alloc(c, 1));
+  ELFEL_CUDA(c, cudaMemsetAsync(bad.p, 0, sizeof(int), c->stream));
+  if (n > 0) {
+    const unsigned g = grid_for(n, 256, (int64_t)c->sm_count * 16);
+    coo_index_k<<<g, 256, 0, c->stream>>>(s->I.p, n, m->nrow, I.p, bad.p);
+    coo_index_k<<<g, 256, 0, c->stream>>>(s->J.p, n, m->ncol, J.p, bad.p);
+    ELFEL_LAUNCH_CHECK(c);
+  }
+  int hbad = 0;
+  ELFEL_CUDA(c, cudaMemcpyAsync(&hbad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
+  bad.release(c);
+  if (hbad) {
+    I.release(c);
+    J.release(c);
+    return fail(c, ELFEL_ERR_ARG, "assemble!: row/column number outside 1..%lld / 1..%lld", (long long)m->nrow,
+                (long long)m->ncol);
+  }
+  SlotGen g;
+  g.I = I.p;
+  g.J = J.p;
+  g.ncoo = n;
+  {
+    Phase ph(c, "pattern_coo");
+    ELFEL_TRY(build_pattern(c, g, m->nrow, m->ncol, &m->P));
+  }
+  I.release(c);
+  J.release(c);
   return ELFEL_OK;
 }
 
@@ -230,40 +282,20 @@ extern "C" int elfel_sysmat_finish(elfel_sysmat* m, int64_t* nnz) {
   cudaSetDevice(c->device);
   if (!m->fused) {
     CooStage* s = stage_of(m);
-    const int64_t n = s->n;
-    DBuf<int32_t> I, J;
-    DBuf<int> bad;
-    ELFEL_TRY(I.alloc(c, (size_t)(n > 0 ? n : 1)));
-    ELFEL_TRY(J.alloc(c, (size_t)(n > 0 ? n : 1)));
-    ELFEL_TRY(bad.alloc(c, 1));
-    ELFEL_CUDA(c, cudaMemsetAsync(bad.p, 0, sizeof(int), c->stream));
-    if (n > 0) {
-      const unsigned g = grid_for(n, 256, (int64_t)c->sm_count * 16);
-      coo_index_k<<<g, 256, 0, c->stream>>>(s->I.p, n, m->nrow, I.p, bad.p);
-      coo_index_k<<<g, 256, 0, c->stream>>>(s->J.p, n, m->ncol, J.p, bad.p);
-      ELFEL_LAUNCH_CHECK(c);
+    cudaStream_t main = c->stream, aux;
+    if (s->n >= kCooOverlap && s->n_indices == s->n) {
+      // the build's work and buffers on the auxiliary stream, behind the indices
+      ELFEL_TRY(aux_after(c, s->indices, &aux));
+      c->stream = aux;
     }
-    int hbad = 0;
-    ELFEL_CUDA(c, cudaMemcpyAsync(&hbad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
-    bad.release(c);
-    if (hbad) {
-      I.release(c);
-      J.release(c);
-      return fail(c, ELFEL_ERR_ARG, "assemble!: row/column number outside 1..%lld / 1..%lld", (long long)m->nrow,
-                  (long long)m->ncol);
+    s->n_indices = 0;  // a second finish! releases the pattern in the context stream's order
+    const int rc = coo_pattern(m, s->n);
+    if (c->stream != main) {
+      c->stream = main;
+      ELFEL_TRY(aux_join(c));
     }
-    SlotGen g;
-    g.I = I.p;
-    g.J = J.p;
-    g.ncoo = n;
-    {
-      Phase ph(c, "pattern_coo");
-      ELFEL_TRY(build_pattern(c, g, m->nrow, m->ncol, &m->P));
-      ELFEL_TRY(record_pattern(m));
-    }
-    I.release(c);
-    J.release(c);
+    ELFEL_TRY(rc);
+    ELFEL_TRY(record_pattern(m));
     ELFEL_TRY(m->vals.alloc(c, (size_t)(m->P.nnz > 0 ? m->P.nnz : 1)));
     {
       Phase ph(c, "reduce_coo");

@@ -65,6 +65,57 @@ def test_triplets(E, gpu, n, ncol, rows):
     assert np.array_equal(x[: nnz.value], ex)
 
 
+@pytest.mark.parametrize("n", [(1 << 18) - 1, 1 << 18, (1 << 18) + 333])
+@pytest.mark.parametrize("pinned", [False, True])
+def test_values_behind_the_indices(E, gpu, n, pinned):
+    """From 2^18 triplets on the pattern is built while the values are uploaded: one
+    and two appends, finish! twice, an index out of range, and a new start!."""
+    import torch
+
+    rng = np.random.default_rng(n)
+    ndof = 20000
+    host = lambda a: torch.from_numpy(a).pin_memory().numpy() if pinned else a  # noqa: E731
+    I, J = (host(rng.integers(1, ndof + 1, n)) for _ in range(2))
+    V = host(rng.standard_normal(n))
+    ctx = E.default_context()
+    N = __import__("importlib").import_module(E.__name__ + "._native")
+    L, ip = ctx.lib, lambda a: N.ptr(a, N._i64p)  # noqa: E731
+    h = ctypes.c_void_p()
+    ctx.check(L.elfel_sysmat_create(ctx.h, ctypes.byref(h)))
+
+    def append(sl):
+        i, j, v = I[sl], J[sl], V[sl]
+        ctx.check(L.elfel_sysmat_assemble_coo(h, ip(i), ip(j), N.ptr(v), i.size))
+
+    def result():
+        nnz = ctypes.c_int64()
+        ctx.check(L.elfel_sysmat_finish(h, ctypes.byref(nnz)))
+        cp, rv, x = np.zeros(ndof + 1, np.int64), np.zeros(nnz.value, np.int64), np.zeros(nnz.value)
+        ctx.check(L.elfel_sysmat_csc(h, ip(cp), ip(rv), N.ptr(x)))
+        return cp - 1, rv, x
+
+    try:
+        want = expected(I, J, V, ndof, ndof)
+        for cuts in ([0, n], [0, 1000, n], [0, n - 10, n]):
+            ctx.check(L.elfel_sysmat_start(h, ndof, ndof))
+            for a, b in zip(cuts[:-1], cuts[1:]):
+                append(slice(a, b))
+            for _ in range(2):
+                assert all(np.array_equal(p, q) for p, q in zip(result(), want))
+            append(slice(0, 500))  # append after finish!
+            again = expected(*(np.r_[a, a[:500]] for a in (I, J, V)), ndof, ndof)
+            assert all(np.array_equal(p, q) for p, q in zip(result(), again))
+        wrong = host(np.full(7, ndof + 1))
+        ctx.check(L.elfel_sysmat_assemble_coo(h, ip(wrong), ip(J[:7]), N.ptr(V[:7]), 7))
+        nnz = ctypes.c_int64()
+        assert L.elfel_sysmat_finish(h, ctypes.byref(nnz)) != 0
+        ctx.check(L.elfel_sysmat_start(h, ndof, ndof))
+        append(slice(0, n))
+        assert all(np.array_equal(p, q) for p, q in zip(result(), want))
+    finally:
+        L.elfel_sysmat_destroy(h)
+
+
 def fused(E, dofs, ndofs, conn, xy):
     """K of the heat form on T3 elements with the given element DOFs."""
     N = __import__("importlib").import_module(E.__name__ + "._native")
