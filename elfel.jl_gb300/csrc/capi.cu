@@ -12,21 +12,17 @@ using namespace elfel;
 
 namespace elfel {
 
-// Dense vector from a 1 x n pattern: out[c] = 0 + the contributions of
-// column c in slot order, as SysvecAssembler adds element vectors into a
-// zeroed vector (Assemblers.jl:194-207; the leading +0 turns a sum of
-// negative zeros into +0, as there).
-__global__ void reduce_row0_dense_k(const int64_t* __restrict__ colptr, const int32_t* __restrict__ cptr,
-                                    const int32_t* __restrict__ contrib, const double* __restrict__ store, int64_t n,
-                                    double* __restrict__ out) {
+// Dense vector from a vector pattern: out[c] = 0 + the contributions of column c
+// in slot order, as SysvecAssembler adds element vectors into a zeroed vector
+// (Assemblers.jl:194-207; the leading +0 turns a sum of negative zeros into
+// +0, as there).
+__global__ void reduce_vector_k(const int32_t* __restrict__ cptr, const int32_t* __restrict__ contrib,
+                                const double* __restrict__ store, int64_t n, double* __restrict__ out) {
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t k0 = colptr[c], k1 = colptr[c + 1];
+    const int32_t b = cptr[c], e = cptr[c + 1];
     double s = 0.0;
-    if (k1 > k0) {
-      const int32_t b = cptr[k0], e = cptr[k0 + 1];
-      s = __dadd_rn(0.0, store[contrib[b]]);
-      for (int32_t t = b + 1; t < e; ++t) s += store[contrib[t]];
-    }
+    if (b < e) s = __dadd_rn(0.0, store[contrib[b]]);
+    for (int32_t t = b + 1; t < e; ++t) s += store[contrib[t]];
     out[c] = s;
   }
 }
@@ -43,8 +39,8 @@ __global__ void midside_count_k(const int32_t* __restrict__ dofs, int64_t nel, i
 
 int reduce_dense(Ctx* c, const Pattern& P, const double* store, double* out) {
   if (P.ncol == 0) return ELFEL_OK;
-  reduce_row0_dense_k<<<grid_for(P.ncol, 256, (int64_t)c->sm_count * 16), 256, 0, c->stream>>>(
-      P.colptr.p, P.cptr.p, P.contrib.p, store, P.ncol, out);
+  reduce_vector_k<<<grid_for(P.ncol, 256, (int64_t)c->sm_count * 16), 256, 0, c->stream>>>(P.cptr.p, P.contrib.p,
+                                                                                           store, P.ncol, out);
   ELFEL_LAUNCH_CHECK(c);
   return ELFEL_OK;
 }
@@ -413,7 +409,7 @@ extern "C" int elfel_sysvec_assemble(elfel_ctx* h, int64_t nrow, const int64_t* 
   g.b[0].nr = 1;
   g.b[0].nc = 1;
   Pattern P;
-  ELFEL_TRY(build_pattern(c, g, 1, nrow, &P));
+  ELFEL_TRY(build_vector_pattern(c, g, nrow, &P));
   ELFEL_TRY(dense.alloc(c, (size_t)(nrow > 0 ? nrow : 1)));
   ELFEL_TRY(reduce_dense(c, P, V.p, dense.p));
   if (nrow) ELFEL_CUDA(c, cudaMemcpyAsync(out, dense.p, sizeof(double) * nrow, cudaMemcpyDeviceToHost, c->stream));
@@ -678,7 +674,7 @@ static int fused_build_in(elfel_sysmat* m, int64_t ndofs, TableChecks* chk) {
     pg.b[0].nc = 3;
     pg.slots_per_elem = 3;
     pg.store_per_elem = 3;
-    ELFEL_TRY(build_pattern(c, pg, 1, ndofs, &F.pmpat));
+    ELFEL_TRY(build_vector_pattern(c, pg, ndofs, &F.pmpat));
     ELFEL_TRY(F.pmass_store.alloc(c, (size_t)(F.nel * 3 > 0 ? F.nel * 3 : 1)));
     ELFEL_TRY(F.pmass_diag.alloc(c, (size_t)(ndofs > 0 ? ndofs : 1)));
   }
@@ -916,7 +912,7 @@ int elfel::ensure_fpat(elfel_sysmat* m) {
   if (F.fpat_built) return ELFEL_OK;
   Ctx* c = &m->h->c;
   Phase ph(c, "pattern_F");
-  ELFEL_TRY(build_pattern(c, F.fgen, 1, m->ncol, &F.fpat));
+  ELFEL_TRY(build_vector_pattern(c, F.fgen, m->ncol, &F.fpat));
   F.fpat_built = 1;
   return ELFEL_OK;
 }
@@ -1071,7 +1067,7 @@ extern "C" int elfel_fused_elasticity(elfel_sysmat* m, double E, double nu, int3
     tg.slots_per_elem = nen * 2;
     tg.store_per_elem = nen * 2;
     Pattern tp;
-    ELFEL_TRY(build_pattern(c, tg, 1, m->nrow, &tp));
+    ELFEL_TRY(build_vector_pattern(c, tg, m->nrow, &tp));
     ELFEL_TRY(tvec.alloc(c, (size_t)m->nrow));
     ELFEL_TRY(reduce_dense(c, tp, tstore.p, tvec.p));
     add_k<<<grid_for(m->nrow, 256, (int64_t)c->sm_count * 16), 256, 0, c->stream>>>(m->rhs.p, tvec.p, m->nrow);

@@ -703,9 +703,24 @@ __global__ void window_order_k(const int32_t* __restrict__ cptr, int64_t nnz, ui
   }
 }
 
-int build_pattern(Ctx* c, const SlotGen& g0, int64_t nrow, int64_t ncol, Pattern* P) {
-  SlotGen g = g0;
-  g.prepare();
+// Buffers of a build and its steps up to the sorted columns.
+struct Build {
+  DBuf<int32_t> colcnt, cursor, nzrow, nzpos;
+  DBuf<int64_t> colstart;
+  DBuf<uint64_t> keys;
+  ColOut out;
+  int64_t nbatch = 0;
+  void release(Ctx* c) {
+    colcnt.release(c);
+    cursor.release(c);
+    nzrow.release(c);
+    nzpos.release(c);
+    colstart.release(c);
+    keys.release(c);
+  }
+};
+
+static int sort_slots(Ctx* c, const SlotGen& g, int64_t nrow, int64_t ncol, Pattern* P, Build* B) {
   P->release(c);
   const int64_t M = g.total();
   if (M >= (int64_t)0x7fffffff)
@@ -716,44 +731,42 @@ int build_pattern(Ctx* c, const SlotGen& g0, int64_t nrow, int64_t ncol, Pattern
   P->ncol = ncol;
   P->nslots = M;
   cudaStream_t st = c->stream;
-  DBuf<int32_t> colcnt, cursor;
-  DBuf<int64_t> colstart;
-  DBuf<uint64_t> keys;
   // counts, the flag of slots out of range, the number of wide batches, their marks and list (ColOut)
-  const int64_t nbatch = (ncol + kColBatch - 1) / kColBatch;
-  ELFEL_TRY(colcnt.alloc(c, (size_t)(ncol + 2 + 2 * nbatch)));
-  ELFEL_TRY(cursor.alloc(c, (size_t)(ncol > 0 ? ncol : 1)));
-  ELFEL_TRY(colstart.alloc(c, (size_t)ncol + 1));
-  int* bad = colcnt.p + ncol;
-  ELFEL_CUDA(c, cudaMemsetAsync(colcnt.p, 0, sizeof(int32_t) * (ncol + 2), st));
-  if (ncol > 0) ELFEL_CUDA(c, cudaMemsetAsync(cursor.p, 0, sizeof(int32_t) * ncol, st));
+  const int64_t nbatch = B->nbatch = (ncol + kColBatch - 1) / kColBatch;
+  ELFEL_TRY(B->colcnt.alloc(c, (size_t)(ncol + 2 + 2 * nbatch)));
+  ELFEL_TRY(B->cursor.alloc(c, (size_t)(ncol > 0 ? ncol : 1)));
+  ELFEL_TRY(B->colstart.alloc(c, (size_t)ncol + 1));
+  int32_t *colcnt = B->colcnt.p, *cursor = B->cursor.p, *bad = colcnt + ncol, *marks = colcnt + ncol + 2;
+  int64_t* colstart = B->colstart.p;
+  ELFEL_CUDA(c, cudaMemsetAsync(colcnt, 0, sizeof(int32_t) * (ncol + 2), st));
+  if (ncol > 0) ELFEL_CUDA(c, cudaMemsetAsync(cursor, 0, sizeof(int32_t) * ncol, st));
   const unsigned gs = grid_for(M, 256, (int64_t)c->sm_count * 16);
   const int64_t ngroups = g.nblocks ? g.nel * (int64_t)g.groups : 0;
   const unsigned gg = grid_for(ngroups, 256, (int64_t)c->sm_count * 16);
   if (M > 0) {
-    if (g.nblocks) count_groups_k<<<gg, 256, 0, st>>>(g, ngroups, colcnt.p, ncol, bad);
-    else count_cols_k<<<gs, 256, 0, st>>>(g, M, colcnt.p, ncol, nrow, bad);
+    if (g.nblocks) count_groups_k<<<gg, 256, 0, st>>>(g, ngroups, colcnt, ncol, bad);
+    else count_cols_k<<<gs, 256, 0, st>>>(g, M, colcnt, ncol, nrow, bad);
     ELFEL_LAUNCH_CHECK(c);
   }
-  ELFEL_TRY(scan_counts_i32(c, colcnt.p, ncol, colstart.p));
+  ELFEL_TRY(scan_counts_i32(c, colcnt, ncol, colstart));
   const size_t m1 = (size_t)(M > 0 ? M : 1);
-  ELFEL_TRY(keys.alloc(c, m1));
+  ELFEL_TRY(B->keys.alloc(c, m1));
   // row starts (ColOut), compacted after the scan; the group numbers share the
   // array of the positions (a batch's groups are read before its first row start
   // is written, those of a wide batch's column before the column's)
-  DBuf<int32_t> nzrow, nzpos;
-  ELFEL_TRY(nzrow.alloc(c, m1));
-  ELFEL_TRY(nzpos.alloc(c, m1));
-  uint32_t* gk = reinterpret_cast<uint32_t*>(nzpos.p);
+  ELFEL_TRY(B->nzrow.alloc(c, m1));
+  ELFEL_TRY(B->nzpos.alloc(c, m1));
+  uint32_t* gk = reinterpret_cast<uint32_t*>(B->nzpos.p);
+  uint64_t* keys = B->keys.p;
   if (M > 0) {
-    if (g.nblocks) bucket_groups_k<<<gg, 256, 0, st>>>(g, ngroups, colstart.p, ncol, cursor.p, gk);
-    else bucket_k<<<gs, 256, 0, st>>>(g, M, colstart.p, nrow, ncol, cursor.p, keys.p);
+    if (g.nblocks) bucket_groups_k<<<gg, 256, 0, st>>>(g, ngroups, colstart, ncol, cursor, gk);
+    else bucket_k<<<gs, 256, 0, st>>>(g, M, colstart, nrow, ncol, cursor, keys);
     ELFEL_LAUNCH_CHECK(c);
   }
   // sort + distinct counts (reuse colcnt as per-column nonzero counts)
   ELFEL_TRY(P->contrib.alloc(c, m1));
-  int32_t* marks = colcnt.p + ncol + 2;
-  const ColOut out{P->contrib.p, nzrow.p, nzpos.p, marks, marks + nbatch, colcnt.p + ncol + 1};
+  const ColOut out = B->out =
+      ColOut{P->contrib.p, B->nzrow.p, B->nzpos.p, marks, marks + nbatch, colcnt + ncol + 1};
   if (ncol > 0) {
     const unsigned gwide = grid_for(nbatch, 1, (int64_t)c->sm_count * 8);
     auto sort = [&](auto coo, auto nk) {
@@ -761,48 +774,75 @@ int build_pattern(Ctx* c, const SlotGen& g0, int64_t nrow, int64_t ncol, Pattern
       using D = Net<decltype(nk)::value>;
       const unsigned grid = grid_for(nbatch, D::kThreads / 32, (int64_t)c->sm_count * 32);
       sort_cols_k<COO, decltype(nk)::value>
-          <<<grid, D::kThreads, 0, st>>>(g, out, colstart.p, cursor.p, gk, ncol, keys.p, colcnt.p);
-      sort_wide_k<COO><<<gwide, kWideThreads, 0, st>>>(g, out, colstart.p, cursor.p, gk, ncol, keys.p, colcnt.p);
+          <<<grid, D::kThreads, 0, st>>>(g, out, colstart, cursor, gk, ncol, keys, colcnt);
+      sort_wide_k<COO><<<gwide, kWideThreads, 0, st>>>(g, out, colstart, cursor, gk, ncol, keys, colcnt);
     };
     if (!g.nblocks) sort(std::true_type{}, std::integral_constant<int, kNet64>{});
     else if (M <= kNetMean * ncol) sort(std::false_type{}, std::integral_constant<int, kNet>{});
     else sort(std::false_type{}, std::integral_constant<int, kNetL>{});
     ELFEL_LAUNCH_CHECK(c);
   }
-  cursor.release(c);
-  keys.release(c);
+  B->cursor.release(c);
+  B->keys.release(c);
+  return ELFEL_OK;
+}
+
+static int finish_pattern(Ctx* c, int64_t nrow, int64_t ncol, Pattern* P, Build* B) {
+  cudaStream_t st = c->stream;
   ELFEL_TRY(P->colptr.alloc(c, (size_t)ncol + 1));
-  ELFEL_TRY(scan_counts_i32(c, colcnt.p, ncol, P->colptr.p));
+  ELFEL_TRY(scan_counts_i32(c, B->colcnt.p, ncol, P->colptr.p));
   int64_t nnz = 0;
   int hbad = 0;
   ELFEL_CUDA(c, cudaMemcpyAsync(&nnz, P->colptr.p + ncol, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-  ELFEL_CUDA(c, cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, st));
+  ELFEL_CUDA(c, cudaMemcpyAsync(&hbad, B->colcnt.p + ncol, sizeof(int), cudaMemcpyDeviceToHost, st));
   ELFEL_CUDA(c, cudaStreamSynchronize(st));
-  if (hbad) {
-    // slots out of range were left out of every step
-    nzrow.release(c);
-    nzpos.release(c);
-    colcnt.release(c);
-    colstart.release(c);
-    P->release(c);
+  if (hbad)  // slots out of range were left out of every step
     return fail(c, ELFEL_ERR_ARG, "assembled row or column number out of range (1..%lld, 1..%lld)", (long long)nrow,
                 (long long)ncol);
-  }
   P->nnz = nnz;
   ELFEL_TRY(P->rowval.alloc(c, (size_t)(nnz > 0 ? nnz : 1)));
   ELFEL_TRY(P->cptr.alloc(c, (size_t)nnz + 1));
   if (ncol > 0) {
-    compact_k<<<grid_for(nbatch, 8, (int64_t)c->sm_count * 32), 256, 0, st>>>(out, colstart.p, P->colptr.p, ncol,
-                                                                             P->rowval.p, P->cptr.p);
+    compact_k<<<grid_for(B->nbatch, 8, (int64_t)c->sm_count * 32), 256, 0, st>>>(B->out, B->colstart.p, P->colptr.p,
+                                                                                ncol, P->rowval.p, P->cptr.p);
     ELFEL_LAUNCH_CHECK(c);
   }
-  nzrow.release(c);
-  nzpos.release(c);
-  set_last_k<<<1, 1, 0, st>>>(P->cptr.p, nnz, M);
+  set_last_k<<<1, 1, 0, st>>>(P->cptr.p, nnz, P->nslots);
   ELFEL_LAUNCH_CHECK(c);
-  colcnt.release(c);
-  colstart.release(c);
   return ELFEL_OK;
+}
+
+int build_pattern(Ctx* c, const SlotGen& g0, int64_t nrow, int64_t ncol, Pattern* P) {
+  SlotGen g = g0;
+  g.prepare();
+  Build B;
+  int rc = sort_slots(c, g, nrow, ncol, P, &B);
+  if (rc == ELFEL_OK) rc = finish_pattern(c, nrow, ncol, P, &B);
+  B.release(c);
+  if (rc != ELFEL_OK) P->release(c);
+  return rc;
+}
+
+__global__ void to32_k(int64_t n, const int64_t* a, int32_t* b) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    b[i] = (int32_t)a[i];
+}
+
+int build_vector_pattern(Ctx* c, const SlotGen& g0, int64_t ncol, Pattern* P) {
+  SlotGen g = g0;
+  g.prepare();
+  Build B;
+  auto run = [&]() -> int {
+    ELFEL_TRY(sort_slots(c, g, 1, ncol, P, &B));
+    ELFEL_TRY(P->cptr.alloc(c, (size_t)ncol + 1));
+    to32_k<<<grid_for(ncol + 1, 256, (int64_t)c->sm_count * 16), 256, 0, c->stream>>>(ncol + 1, B.colstart.p, P->cptr.p);
+    ELFEL_LAUNCH_CHECK(c);
+    return ELFEL_OK;
+  };
+  const int rc = run();
+  B.release(c);
+  if (rc != ELFEL_OK) P->release(c);
+  return rc;
 }
 
 // One thread per nonzero; its contributions are summed left to right, in the
@@ -893,8 +933,8 @@ __global__ void __launch_bounds__(256) reduce_win_k(const int32_t* __restrict__ 
 }
 
 // Many reductions in one launch: CTA b serves job k with jobs[k].blk0 <= b <
-// jobs[k+1].blk0, items (b - blk0) * blockDim.x onwards.  A job with colptr
-// reduces a 1 x n pattern into a dense vector (the rhs), else the nnz values.
+// jobs[k+1].blk0, items (b - blk0) * blockDim.x onwards.  A dense job
+// reduces a vector pattern into the vector (the rhs), else the nnz values.
 // Each item adds its contributions in slot order, as reduce_k.
 __global__ void reduce_batch_k(const RedJob* __restrict__ jobs, int njobs) {
   int lo = 0, hi = njobs - 1;
@@ -905,18 +945,13 @@ __global__ void reduce_batch_k(const RedJob* __restrict__ jobs, int njobs) {
   const RedJob J = jobs[lo];
   const int64_t k = ((int64_t)blockIdx.x - J.blk0) * blockDim.x + threadIdx.x;
   if (k >= J.n) return;
-  int64_t slot = k;
-  if (J.colptr) {
-    const int64_t k0 = J.colptr[k], k1 = J.colptr[k + 1];
-    if (k1 == k0) {
-      J.out[k] = 0.0;
-      return;
-    }
-    slot = k0;
+  const int32_t b = J.cptr[k], e = J.cptr[k + 1];
+  if (J.dense && b == e) {
+    J.out[k] = 0.0;
+    return;
   }
-  const int32_t b = J.cptr[slot], e = J.cptr[slot + 1];
   double s = J.store[J.contrib[b]];
-  if (J.colptr) s = __dadd_rn(0.0, s);  // a vector starts from a zeroed one (SysvecAssembler)
+  if (J.dense) s = __dadd_rn(0.0, s);  // a vector starts from a zeroed one (SysvecAssembler)
   for (int32_t t = b + 1; t < e; ++t) s += J.store[J.contrib[t]];
   J.out[k] = s;
 }

@@ -295,7 +295,7 @@ int assemble_batch(elfel_server* s, const std::vector<Sys*>& ys) {
     RedJob a;
     a.blk0 = blk;
     a.n = m->P.nnz;
-    a.colptr = nullptr;
+    a.dense = 0;
     a.cptr = m->P.cptr.p;
     a.contrib = m->P.contrib.p;
     a.store = m->F.kstore.p;
@@ -307,7 +307,7 @@ int assemble_batch(elfel_server* s, const std::vector<Sys*>& ys) {
     RedJob f;
     f.blk0 = blk;
     f.n = m->F.fpat.ncol;
-    f.colptr = m->F.fpat.colptr.p;
+    f.dense = 1;
     f.cptr = m->F.fpat.cptr.p;
     f.contrib = m->F.fpat.contrib.p;
     f.store = m->F.fstore.p;

@@ -261,6 +261,10 @@ struct Pattern {
 
 // Build the CSC pattern of the slots of `g` (nrow x ncol matrix).
 int build_pattern(Ctx* c, const SlotGen& g, int64_t nrow, int64_t ncol, Pattern* P);
+// The pattern of a vector's slots (block mode, every row table null, columns in
+// range): contrib, and cptr with one list per entry of the vector (ncol + 1
+// offsets; empty lists stay); colptr and rowval are not formed.  Does not synchronise.
+int build_vector_pattern(Ctx* c, const SlotGen& g, int64_t ncol, Pattern* P);
 
 // A head of the nonzeros, reduced on the auxiliary stream beside the rest and
 // followed by an event, so that a download of the values (elfel_sysmat_csc)
@@ -293,7 +297,7 @@ constexpr int kRedJobThreads = 256;
 struct RedJob {
   int64_t blk0;            // first CTA of this job
   int64_t n;               // items: nnz, or columns of a dense rhs
-  const int64_t* colptr;   // dense rhs: the 1 x n pattern's column pointers; else null
+  int dense;               // a dense rhs from a vector pattern
   const int32_t* cptr;
   const int32_t* contrib;
   const double* store;
