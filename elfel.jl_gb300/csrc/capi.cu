@@ -249,8 +249,7 @@ static int coo_pattern(elfel_sysmat* m, int64_t n) {
     ELFEL_LAUNCH_CHECK(c);
   }
   int hbad = 0;
-  ELFEL_CUDA(c, cudaMemcpyAsync(&hbad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
+  ELFEL_TRY(read_back(c, c->stream, {{&hbad, bad.p, sizeof(hbad)}}));
   bad.release(c);
   if (hbad) {
     I.release(c);
@@ -568,8 +567,7 @@ extern "C" int elfel_fused_setup(elfel_sysmat* m, const elfel_fused_desc* d) {
     if (stokes) ELFEL_TRY(upload_direct_rest(c, d->p, 2, &F.conn_p, nullptr, bad.p + 2, aux));
     ELFEL_TRY(fused_build(m, d->ndofs));  // joins the auxiliary stream before using conn / xy
     int hb[4] = {0, 0, 0, 0};
-    ELFEL_CUDA(c, cudaMemcpyAsync(hb, bad.p, sizeof(hb), cudaMemcpyDeviceToHost, aux));
-    ELFEL_CUDA(c, cudaStreamSynchronize(aux));
+    ELFEL_TRY(read_back(c, aux, {{hb, bad.p, sizeof(hb)}}));
     static const char* what[4] = {"primary connectivity", "primary eldofs", "pressure connectivity",
                                   "pressure eldofs"};
     const int64_t lim[4] = {u.nnodes, d->ndofs, stokes ? d->p.nnodes : 0, d->ndofs};
@@ -688,8 +686,8 @@ static int fused_build_in(elfel_sysmat* m, int64_t ndofs, TableChecks* chk) {
   // pattern build runs on while the caller goes on (the tables have left the host)
   unsigned long long h[2] = {0, 1};
   cudaStream_t rs = triangles ? c->aux : c->stream;
-  if (triangles) ELFEL_CUDA(c, cudaMemcpyAsync(h, res.p, sizeof(h), cudaMemcpyDeviceToHost, rs));
-  ELFEL_CUDA(c, cudaStreamSynchronize(rs));
+  if (triangles) ELFEL_TRY(read_back(c, rs, {{h, res.p, sizeof(h)}}));
+  else ELFEL_CUDA(c, cudaStreamSynchronize(rs));
   F.f_direct_ok = midside && h[1] == 0;
   F.ncurved = (int64_t)h[0];
   m->fused = 1;

@@ -6,6 +6,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -29,6 +30,7 @@ struct Ctx {
   cudaStream_t aux = nullptr;         // second stream for uploads that overlap work on `stream` (lazy)
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   int pageable_access = 0;            // kernels may read pageable host memory in place (ATS)
+  char* host = nullptr;  // page-locked memory for small results (read_back)
   cudaMemPool_t pool = nullptr;  // the context's stream-ordered pool (keeps freed memory for reuse)
   int64_t budget = 0;       // bytes the context may hold on the device (0 = unlimited)
   int64_t in_use = 0;       // bytes currently held
@@ -105,6 +107,16 @@ int fail(Ctx* c, int code, const char* fmt, ...);
 // c->stream so far (fork); join() makes c->stream wait for it.
 int aux_fork(Ctx* c, cudaStream_t* aux);
 int aux_join(Ctx* c);
+// Small device values to the host: every copy of the list is issued on st
+// through page-locked memory before one synchronisation of st (a copy to pageable
+// memory synchronises by itself, about 10 us each).
+struct HostRead {
+  void* dst;
+  const void* src;
+  size_t bytes;
+};
+constexpr size_t kHostBytes = 4096;  // of a list
+int read_back(Ctx* c, cudaStream_t st, std::initializer_list<HostRead> reads);
 // The auxiliary stream, made to wait only for the event ev (recorded on
 // c->stream earlier); join with aux_join.
 int aux_after(Ctx* c, cudaEvent_t ev, cudaStream_t* aux);

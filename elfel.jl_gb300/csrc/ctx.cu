@@ -273,6 +273,23 @@ int aux_join(Ctx* c) {
   return ELFEL_OK;
 }
 
+int read_back(Ctx* c, cudaStream_t st, std::initializer_list<HostRead> reads) {
+  if (!c->host) ELFEL_CUDA(c, cudaMallocHost((void**)&c->host, kHostBytes));
+  size_t at = 0;
+  for (const HostRead& r : reads) {
+    if (at + r.bytes > kHostBytes) return fail(c, ELFEL_ERR_ARG, "read_back: %zu bytes", at + r.bytes);
+    ELFEL_CUDA(c, cudaMemcpyAsync(c->host + at, r.src, r.bytes, cudaMemcpyDeviceToHost, st));
+    at += (r.bytes + 15) / 16 * 16;
+  }
+  ELFEL_CUDA(c, cudaStreamSynchronize(st));
+  at = 0;
+  for (const HostRead& r : reads) {
+    memcpy(r.dst, c->host + at, r.bytes);
+    at += (r.bytes + 15) / 16 * 16;
+  }
+  return ELFEL_OK;
+}
+
 const void* host_device_ptr(Ctx* c, const void* host, int* pinned) {
   if (pinned) *pinned = 0;
   if (!host) return nullptr;
@@ -385,6 +402,7 @@ extern "C" int elfel_ctx_destroy(elfel_ctx* h) {
     cudaStreamSynchronize(h->c.aux);
     cudaStreamDestroy(h->c.aux);
   }
+  if (h->c.host) cudaFreeHost(h->c.host);
   if (h->c.ev_fork) cudaEventDestroy(h->c.ev_fork);
   if (h->c.ev_join) cudaEventDestroy(h->c.ev_join);
   // memory still held by live systems is released once they free it

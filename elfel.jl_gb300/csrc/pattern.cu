@@ -793,9 +793,7 @@ static int finish_pattern(Ctx* c, int64_t nrow, int64_t ncol, Pattern* P, Build*
   ELFEL_TRY(scan_counts_i32(c, B->colcnt.p, ncol, P->colptr.p));
   int64_t nnz = 0;
   int hbad = 0;
-  ELFEL_CUDA(c, cudaMemcpyAsync(&nnz, P->colptr.p + ncol, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-  ELFEL_CUDA(c, cudaMemcpyAsync(&hbad, B->colcnt.p + ncol, sizeof(int), cudaMemcpyDeviceToHost, st));
-  ELFEL_CUDA(c, cudaStreamSynchronize(st));
+  ELFEL_TRY(read_back(c, st, {{&nnz, P->colptr.p + ncol, sizeof(nnz)}, {&hbad, B->colcnt.p + ncol, sizeof(hbad)}}));
   if (hbad)  // slots out of range were left out of every step
     return fail(c, ELFEL_ERR_ARG, "assembled row or column number out of range (1..%lld, 1..%lld)", (long long)nrow,
                 (long long)ncol);

@@ -40,7 +40,8 @@ namespace elfel {
 int batch_add_dev(elfel_batch* b, elfel_sysmat* m, const double* F, const double* T, int t_dev, int64_t nu,
                   double rtol, int32_t maxit, int32_t* slot_out);
 int batch_step(elfel_batch* b, int32_t graphs, int32_t* active);
-int batch_take(elfel_batch* b, int32_t k, double* T_out, int t_dev, elfel_solve_stats* stats);
+int batch_take_many(elfel_batch* b, const std::vector<int32_t>& ks, const std::vector<char>& want,
+                    std::vector<std::vector<double>>* T, std::vector<elfel_solve_stats>* stats);
 int batch_counts(elfel_batch* b, int64_t* launches, int64_t* kernels);
 }  // namespace elfel
 
@@ -460,21 +461,22 @@ int step_batched(elfel_server* s, int32_t* active) {
   int32_t nd = 0;
   std::vector<int32_t> ready(s->cfg.max_active);
   ELFEL_TRY(elfel_batch_done(s->batch, ready.data(), (int32_t)ready.size(), &nd));
+  std::vector<int32_t> slots;
+  std::vector<char> want;
   for (int i = 0; i < std::min<int>(nd, (int)ready.size()); ++i) {
-    const int32_t slot = ready[i];
-    auto it = s->by_slot.find(slot);
+    auto it = s->by_slot.find(ready[i]);
     if (it == s->by_slot.end()) continue;
+    slots.push_back(ready[i]);
+    want.push_back(it->second->req.r.keep_solution ? 1 : 0);
+  }
+  std::vector<std::vector<double>> sols;
+  std::vector<elfel_solve_stats> sst;
+  if (!slots.empty()) ELFEL_TRY(batch_take_many(s->batch, slots, want, &sols, &sst));
+  for (size_t i = 0; i < slots.size(); ++i) {
+    auto it = s->by_slot.find(slots[i]);
     Sys* y = it->second;
-    std::vector<double> sol;
-    double* dst = nullptr;
-    if (y->req.r.keep_solution) {
-      sol.resize((size_t)y->n);
-      dst = sol.data();
-    }
-    elfel_solve_stats sst;
-    const int rc = batch_take(s->batch, slot, dst, 0, &sst);
     s->by_slot.erase(it);
-    ELFEL_TRY(finish_request(s, y, sst, rc, &sol));
+    ELFEL_TRY(finish_request(s, y, sst[i], ELFEL_OK, &sols[i]));
   }
   if (active) *active = (int32_t)s->by_slot.size();
   return ELFEL_OK;

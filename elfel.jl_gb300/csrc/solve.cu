@@ -693,16 +693,6 @@ __global__ void sell_delta_k(int64_t npad, int64_t nu, const int64_t* sptr, int6
   }
 }
 
-__global__ void sell_vals_k(int64_t npad, const int32_t* __restrict__ map, const double* __restrict__ vals,
-                            double* __restrict__ v64, float* __restrict__ v32) {
-  FOR4(k, npad) {
-    const int32_t m = map[k];
-    const double v = m >= 0 ? vals[m] : 0.0;
-    v64[k] = v;
-    v32[k] = (float)v;
-  }
-}
-
 // FP32 values in difference form: each row's diagonal slot, and rowsum, get the
 // row sum s_i = sum_j a_ij (added in FP64, rounded once); the other slots keep
 // a_ij.
@@ -728,17 +718,29 @@ __global__ void sell_rowsum_k(SellView A, const int32_t* __restrict__ map, const
   }
 }
 
-__global__ void gather_vals_k(int64_t n, const int32_t* map, const double* src, double* d64) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    d64[i] = src[map[i]];
+// The values of the three matrices: CSR parts ff and fd, SELL (padding: map -1).
+__global__ void refresh_vals_k(int64_t nff, const int32_t* __restrict__ mff, double* __restrict__ ff, int64_t nfd,
+                               const int32_t* __restrict__ mfd, double* __restrict__ fd, int64_t npad,
+                               const int32_t* __restrict__ map, double* __restrict__ v64, float* __restrict__ v32,
+                               const double* __restrict__ vals) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = t; i < nff; i += stride) ff[i] = vals[mff[i]];
+  for (int64_t i = t; i < nfd; i += stride) fd[i] = vals[mfd[i]];
+  FOR4(k, npad) {
+    const int32_t m = map[k];
+    const double v = m >= 0 ? vals[m] : 0.0;
+    v64[k] = v;
+    v32[k] = (float)v;
+  }
 }
 
-// Preconditioner diagonal in the original order: 1/K_ii where K_ii != 0, else
-// 1/aux_i where aux_i > 0 (pressure mass diagonal), else 1.  abs_diag selects
-// |K_ii| (MINRES needs an SPD preconditioner).
-__global__ void diag_k(int64_t nu, const int32_t* rp, const int32_t* ci, const double* v, const double* aux,
-                       int abs_diag, double* d) {
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < nu; r += (int64_t)gridDim.x * blockDim.x) {
+// Preconditioner diagonal in the permuted order: 1/K_rr where K_rr != 0, else
+// 1/aux_r where aux_r > 0 (pressure mass diagonal), else 1.  abs_diag selects
+// |K_rr| (MINRES needs an SPD preconditioner).
+__global__ void diag_k(int64_t nu, const int32_t* perm, const int32_t* rp, const int32_t* ci, const double* v,
+                       const double* aux, int abs_diag, double* d64, float* d32) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nu; i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t r = perm[i];
     double dv = 0.0;
     int32_t lo = rp[r], hi = rp[r + 1] - 1;
     while (lo <= hi) {
@@ -751,15 +753,8 @@ __global__ void diag_k(int64_t nu, const int32_t* rp, const int32_t* ci, const d
     if (dv != 0.0) inv = 1.0 / dv;
     else if (aux && aux[r] > 0.0) inv = 1.0 / aux[r];
     else inv = 1.0;
-    d[r] = inv;
-  }
-}
-
-__global__ void permute_diag_k(int64_t n, const int32_t* perm, const double* in, double* d64, float* d32) {
-  FOR4(i, n) {
-    const double v = in[perm[i]];
-    d64[i] = v;
-    d32[i] = (float)v;
+    d64[i] = inv;
+    d32[i] = (float)inv;
   }
 }
 
@@ -891,8 +886,7 @@ static int build_sell(Ctx* c, SolverData* S) {
   ELFEL_LAUNCH_CHECK(c);
   ELFEL_TRY(scan_counts_i32(c, w32.p, nsl, A.sptr.p));
   w32.release(c);
-  ELFEL_CUDA(c, cudaMemcpyAsync(&A.nnz_pad, A.sptr.p + nsl, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
-  ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
+  ELFEL_TRY(read_back(c, c->stream, {{&A.nnz_pad, A.sptr.p + nsl, sizeof(int64_t)}}));
   if (A.nnz_pad >= (int64_t)0x7fffffff) return fail(c, ELFEL_ERR_ARG, "solver matrix too large for 32-bit offsets");
   const size_t np = (size_t)(A.nnz_pad > 0 ? A.nnz_pad : 1);
   ELFEL_TRY(col.alloc(c, np));
@@ -914,8 +908,7 @@ static int build_sell(Ctx* c, SolverData* S) {
     ELFEL_LAUNCH_CHECK(c);
   }
   int hw[13] = {0};
-  ELFEL_CUDA(c, cudaMemcpyAsync(hw, wide.p, sizeof(hw), cudaMemcpyDeviceToHost, c->stream));
-  ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
+  ELFEL_TRY(read_back(c, c->stream, {{hw, wide.p, sizeof(hw)}}));
   for (int q = 0; q < 4; ++q) S->run_entries[q] = hw[1 + q];
   for (int q = 0; q < 8; ++q) S->run_window[q] = hw[5 + q];
   wide.release(c);
@@ -962,10 +955,7 @@ int build_solver(elfel_sysmat* m, int64_t nu) {
   int64_t tot[2] = {0, 0}, tff = 0;
   auto totals = [&]() -> int {
     ELFEL_TRY(scan_counts_i32(c, cnt.p, 2 * nu, off.p));
-    ELFEL_CUDA(c, cudaMemcpyAsync(tot, off.p + 2 * nu, sizeof(tot), cudaMemcpyDeviceToHost, c->stream));
-    ELFEL_CUDA(c, cudaMemcpyAsync(&tff, off.p + nu, sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
-    ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
-    return ELFEL_OK;
+    return read_back(c, c->stream, {{tot, off.p + 2 * nu, sizeof(tot)}, {&tff, off.p + nu, sizeof(tff)}});
   };
   const unsigned gr = grid_for(nu + 1, 256, (int64_t)c->sm_count * 16);
   ELFEL_TRY(src.alloc(c, (size_t)(m->P.nnz > 0 ? m->P.nnz : 1)));
@@ -1018,13 +1008,7 @@ int build_solver(elfel_sysmat* m, int64_t nu) {
   S->nu = nu;
   ELFEL_TRY(S->run_win.alloc(c, kRunWins));
   if (nu > 0) ELFEL_TRY(build_sell(c, S));
-  const size_t vn = (size_t)(nu > 0 ? nu : 1);
-  for (DBuf<double>* b : {&S->bo64, &S->xo64, &S->ro64, &S->dinvo, &S->dinv64, &S->b64, &S->x64, &S->r64, &S->z64,
-                          &S->p64, &S->q64, &S->y64})
-    ELFEL_TRY(b->alloc(c, vn));
-  for (DBuf<float>* b : {&S->dinv32, &S->r32, &S->p32, &S->q32, &S->z32, &S->xa32, &S->zz32, &S->b32, &S->x32,
-                        &S->rowsum32})
-    ELFEL_TRY(b->alloc(c, vn));
+  ELFEL_TRY(S->alloc_vectors(c, nu));
   ELFEL_TRY(S->T64.alloc(c, (size_t)(n > 0 ? n : 1)));
   ELFEL_TRY(S->scal.alloc(c, S_COUNT));
   ELFEL_TRY(S->flags.alloc(c, F_COUNT));
@@ -1038,7 +1022,6 @@ int build_solver(elfel_sysmat* m, int64_t nu) {
   S->group = pick_group(tff, nu);
   S->pattern_id = m->P.rowval.p;
   S->pattern_nnz = m->P.nnz;
-  ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
   return ELFEL_OK;
 }
 
@@ -1049,15 +1032,10 @@ int refresh_values(elfel_sysmat* m, int abs_diag, int diff32) {
   SolverData* S = m->solver;
   const int64_t nu = S->nu;
   Phase ph(c, "solver_values");
-  if (S->ff.nnz)
-    gather_vals_k<<<grid_for(S->ff.nnz, 256, (int64_t)c->sm_count * 16), 256, 0, c->stream>>>(
-        S->ff.nnz, S->ff.map.p, m->vals.p, S->ff.v64.p);
-  if (S->fd.nnz)
-    gather_vals_k<<<grid_for(S->fd.nnz, 256, (int64_t)c->sm_count * 16), 256, 0, c->stream>>>(
-        S->fd.nnz, S->fd.map.p, m->vals.p, S->fd.v64.p);
-  if (S->A.nnz_pad)
-    sell_vals_k<<<vec_grid(S->A.nnz_pad), kBlk, 0, c->stream>>>(S->A.nnz_pad, S->A.map.p, m->vals.p, S->A.v64.p,
-                                                                 S->A.v32.p);
+  if (S->A.nnz_pad || S->ff.nnz || S->fd.nnz)
+    refresh_vals_k<<<vec_grid(std::max(S->A.nnz_pad, std::max(S->ff.nnz, S->fd.nnz))), kBlk, 0, c->stream>>>(
+        S->ff.nnz, S->ff.map.p, S->ff.v64.p, S->fd.nnz, S->fd.map.p, S->fd.v64.p, S->A.nnz_pad, S->A.map.p,
+        S->A.v64.p, S->A.v32.p, m->vals.p);
   if (diff32 && nu > 0) {
     const SellView V = S->view();
     if (S->A.d16)
@@ -1068,12 +1046,9 @@ int refresh_values(elfel_sysmat* m, int abs_diag, int diff32) {
           V, S->A.map.p, S->A.v64.p, S->A.v32.p, S->rowsum32.p);
   }
   const double* aux = (m->fused && m->F.physics == ELFEL_STOKES) ? m->F.pmass_diag.p : nullptr;
-  if (nu > 0) {
-    diag_k<<<grid_for(nu, 256, (int64_t)c->sm_count * 16), 256, 0, c->stream>>>(nu, S->ff.rowptr.p, S->ff.col.p,
-                                                                                S->ff.v64.p, aux, abs_diag,
-                                                                                S->dinvo.p);
-    permute_diag_k<<<vec_grid(nu), kBlk, 0, c->stream>>>(nu, S->A.perm.p, S->dinvo.p, S->dinv64.p, S->dinv32.p);
-  }
+  if (nu > 0)
+    diag_k<<<grid_for(nu, 256, (int64_t)c->sm_count * 16), 256, 0, c->stream>>>(
+        nu, S->A.perm.p, S->ff.rowptr.p, S->ff.col.p, S->ff.v64.p, aux, abs_diag, S->dinv64.p, S->dinv32.p);
   ELFEL_LAUNCH_CHECK(c);
   return ELFEL_OK;
 }
@@ -1131,25 +1106,44 @@ static void launch_mr_spmv(Ctx* c, SolverData* S, const T* v, T* const* zb, T* q
     mr_spmv_k<T, false><<<sell_grid<T>(S), kBlk, 0, c->stream>>>(V, v, zb, q, red, S->scal.p, S->flags.p);
 }
 
-static int read_flags(Ctx* c, SolverData* S, int* h) {
-  ELFEL_CUDA(c, cudaMemcpyAsync(h, S->flags.p, sizeof(int) * F_COUNT, cudaMemcpyDeviceToHost, c->stream));
-  ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
+// Scalars of a solve by value, and (maxit >= 0) its flags at the start.
+struct ScalSet {
+  int n = 0, maxit = -1;
+  int idx[4];
+  double v[4];
+  ScalSet& set(int i, double x) {
+    idx[n] = i;
+    v[n++] = x;
+    return *this;
+  }
+  ScalSet& start(int it) {
+    maxit = it;
+    return *this;
+  }
+};
+
+__global__ void set_scal_k(double* scal, int* flags, ScalSet s) {
+  if (threadIdx.x < s.n) scal[s.idx[threadIdx.x]] = s.v[threadIdx.x];
+  if (s.maxit >= 0 && threadIdx.x < F_COUNT) flags[threadIdx.x] = threadIdx.x == F_MAXIT ? s.maxit : 0;
+}
+
+static int set_scal(Ctx* c, SolverData* S, const ScalSet& s) {
+  set_scal_k<<<1, 32, 0, c->stream>>>(S->scal.p, S->flags.p, s);
+  ELFEL_LAUNCH_CHECK(c);
   return ELFEL_OK;
 }
 
-static int set_scal(Ctx* c, SolverData* S, int idx, double v) {
-  ELFEL_CUDA(c, cudaMemcpyAsync(S->scal.p + idx, &v, sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
-  return ELFEL_OK;
-}
-
-// A one-launch run of iterations was launched: its flags, and an error if a
-// wait inside it ran out.
-static int read_run(Ctx* c, SolverData* S, const RunPlan& P, int* h) {
+// Iterations were launched (bar: a one-launch run's barrier words): the flags
+// and the scalars (S_COUNT), and an error if a wait inside ran out.
+static int read_run(Ctx* c, SolverData* S, const RunPlan& P, int* h, double* scal) {
   unsigned bar[2] = {0, 0};
-  if (!P.cluster)
-    ELFEL_CUDA(c, cudaMemcpyAsync(bar, S->run_bar.p, sizeof(bar), cudaMemcpyDeviceToHost, c->stream));
-  ELFEL_TRY(read_flags(c, S, h));
+  if (P.blocks && !P.cluster)
+    ELFEL_TRY(read_back(c, c->stream, {{h, S->flags.p, sizeof(int) * F_COUNT},
+                                       {scal, S->scal.p, sizeof(double) * S_COUNT},
+                                       {bar, S->run_bar.p, sizeof(bar)}}));
+  else
+    ELFEL_TRY(read_back(c, c->stream, {{h, S->flags.p, sizeof(int) * F_COUNT},
+                                       {scal, S->scal.p, sizeof(double) * S_COUNT}}));
   if (bar[1]) return fail(c, ELFEL_ERR_TIMEOUT, "solve: a barrier of the iteration kernel timed out");
   return ELFEL_OK;
 }
@@ -1208,9 +1202,7 @@ static int residual_converged(elfel_sysmat* m, double rtol, double* rr, bool* co
   SolverData* S = m->solver;
   ELFEL_TRY(solution_residual(m));
   double bn2 = 0.0;
-  ELFEL_CUDA(c, cudaMemcpyAsync(rr, S->scal.p + S_RR, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  ELFEL_CUDA(c, cudaMemcpyAsync(&bn2, S->scal.p + S_BN2, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
+  ELFEL_TRY(read_back(c, c->stream, {{rr, S->scal.p + S_RR, sizeof(double)}, {&bn2, S->scal.p + S_BN2, sizeof(double)}}));
   *conv = sqrt(*rr / bn2) <= rtol;
   return ELFEL_OK;
 }
@@ -1224,8 +1216,9 @@ static int run_pcg64(elfel_sysmat* m, double rtol, int maxit, elfel_solve_stats*
   const unsigned vg = vec_grid(nu);
   ELFEL_CUDA(c, cudaMemsetAsync(S->x64.p, 0, sizeof(double) * nu, c->stream));
   ELFEL_CUDA(c, cudaMemcpyAsync(S->r64.p, S->b64.p, sizeof(double) * nu, cudaMemcpyDeviceToDevice, c->stream));
-  int hf[F_COUNT] = {0, 0, 0, maxit, 0, 0, 0};
-  ELFEL_CUDA(c, cudaMemcpyAsync(S->flags.p, hf, sizeof(hf), cudaMemcpyHostToDevice, c->stream));
+  int hf[F_COUNT];
+  double hsc[S_COUNT];
+  ELFEL_TRY(set_scal(c, S, ScalSet().start(maxit)));
   cg_start_k<double><<<vg, kBlk, 0, c->stream>>>(nu, S->r64.p, S->z64.p, S->p64.p, S->dinv64.p, red_area(S, 0),
                                                  S->scal.p, S->flags.p, 1, 1.0);
   ELFEL_LAUNCH_CHECK(c);
@@ -1242,13 +1235,9 @@ static int run_pcg64(elfel_sysmat* m, double rtol, int maxit, elfel_solve_stats*
   // CG restarts from it.
   int replacements = 0;
   while (true) {
-    if (run.blocks) {
-      ELFEL_TRY(run_cg64(c, S, run));
-      ELFEL_TRY(read_run(c, S, run, hf));
-    } else {
-      ELFEL_CUDA(c, cudaGraphLaunch(S->g_pcg64, c->stream));
-      ELFEL_TRY(read_flags(c, S, hf));
-    }
+    if (run.blocks) ELFEL_TRY(run_cg64(c, S, run));
+    else ELFEL_CUDA(c, cudaGraphLaunch(S->g_pcg64, c->stream));
+    ELFEL_TRY(read_run(c, S, run, hf, hsc));
     if (!hf[F_DONE]) continue;
     if (!hf[F_CONV] || hf[F_ITER] >= maxit || replacements >= 50) break;
     bool conv = false;
@@ -1272,7 +1261,7 @@ static int run_pcg64(elfel_sysmat* m, double rtol, int maxit, elfel_solve_stats*
   return ELFEL_OK;
 }
 
-static int run_pcg32(elfel_sysmat* m, double rtol, int maxit, elfel_solve_stats* st, double* rr) {
+static int run_pcg32(elfel_sysmat* m, double bn2, double rtol, int maxit, elfel_solve_stats* st, double* rr) {
   Ctx* c = &m->h->c;
   SolverData* S = m->solver;
   const int64_t nu = S->nu;
@@ -1282,16 +1271,10 @@ static int run_pcg32(elfel_sysmat* m, double rtol, int maxit, elfel_solve_stats*
   ELFEL_CUDA(c, cudaMemcpyAsync(S->r64.p, S->b64.p, sizeof(double) * nu, cudaMemcpyDeviceToDevice, c->stream));
   // the FP32 recurrence works on r / s with s = ||b||: the initial residual
   // has unit norm whatever the scale of the problem (no FP32 under/overflow)
-  double hsc0[S_COUNT];
-  ELFEL_CUDA(c, cudaMemcpyAsync(hsc0, S->scal.p, sizeof(hsc0), cudaMemcpyDeviceToHost, c->stream));
-  ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
-  const double s = sqrt(hsc0[S_BN2]);
+  const double s = sqrt(bn2);
   demote_k<<<vg, kBlk, 0, c->stream>>>(nu, S->r64.p, S->r32.p, 1.0 / s);
-  ELFEL_TRY(set_scal(c, S, S_SCALE, s));
-  ELFEL_TRY(set_scal(c, S, S_BN2S, 1.0));
-  ELFEL_TRY(set_scal(c, S, S_RMAX, 1.0));
-  int hf[F_COUNT] = {0, 0, 0, maxit, 0, 0, 0};
-  ELFEL_CUDA(c, cudaMemcpyAsync(S->flags.p, hf, sizeof(hf), cudaMemcpyHostToDevice, c->stream));
+  ELFEL_TRY(set_scal(c, S, ScalSet().set(S_SCALE, s).set(S_BN2S, 1.0).set(S_RMAX, 1.0).start(maxit)));
+  int hf[F_COUNT];
   cg_start_k<float><<<vg, kBlk, 0, c->stream>>>(nu, S->r32.p, S->z32.p, S->p32.p, S->dinv32.p, red_area(S, 0),
                                                 S->scal.p, S->flags.p, 1, 1.0f);
   ELFEL_LAUNCH_CHECK(c);
@@ -1306,30 +1289,20 @@ static int run_pcg32(elfel_sysmat* m, double rtol, int maxit, elfel_solve_stats*
   int launches = 0;
   double hsc[S_COUNT];
   while (true) {
-    if (run.blocks) {
-      ELFEL_TRY(run_cg32(c, S, run));
-      ELFEL_TRY(read_run(c, S, run, hf));
-    } else {
-      ELFEL_CUDA(c, cudaGraphLaunch(S->g_pcg32, c->stream));
-      ELFEL_TRY(read_flags(c, S, hf));
-    }
+    if (run.blocks) ELFEL_TRY(run_cg32(c, S, run));
+    else ELFEL_CUDA(c, cudaGraphLaunch(S->g_pcg32, c->stream));
+    ELFEL_TRY(read_run(c, S, run, hf, hsc));
     ++launches;
     if (c->trace && (launches % 256) == 0) {
-      ELFEL_CUDA(c, cudaMemcpyAsync(hsc, S->scal.p, sizeof(hsc), cudaMemcpyDeviceToHost, c->stream));
-      ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
       fprintf(stderr, "[elfel pcg32] it %d recurrence %.3e rmax %.3e flags ru %d brk %d\n", hf[F_ITER],
               sqrt(hsc[S_RR]), hsc[S_RMAX], hf[F_RU], hf[F_BRK]);
     }
     if (!hf[F_RU]) continue;
-    // recurrence residual before the replacement
-    ELFEL_CUDA(c, cudaMemcpyAsync(hsc, S->scal.p, sizeof(hsc), cudaMemcpyDeviceToHost, c->stream));
-    ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
-    const double rr_rec = hsc[S_RR] * s * s;  // recurrence residual, unscaled
+    const double rr_rec = hsc[S_RR] * s * s;  // recurrence residual before the replacement, unscaled
     // FP64 residual replacement
     fold_k<<<vg, kBlk, 0, c->stream>>>(nu, S->x64.p, S->xa32.p, s);
     ELFEL_TRY(launch_sell_resid(c, S, S->x64.p, S->b64.p, S->r64.p, red_area(S, 2), S_RR));
-    ELFEL_CUDA(c, cudaMemcpyAsync(hsc, S->scal.p, sizeof(hsc), cudaMemcpyDeviceToHost, c->stream));
-    ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
+    ELFEL_TRY(read_back(c, c->stream, {{hsc, S->scal.p, sizeof(hsc)}}));
     ++refinements;
     const bool conv = hsc[S_RR] <= hsc[S_TOL2] * hsc[S_BN2];
     // keep the search direction unless the FP32 recurrence broke down or its
@@ -1347,17 +1320,14 @@ static int run_pcg32(elfel_sysmat* m, double rtol, int maxit, elfel_solve_stats*
       if (all || ++late >= 50) break;
       *rr = -1.0;
     }
-    if (hf[F_BRK]) {
-      int z = 0;
-      ELFEL_CUDA(c, cudaMemcpyAsync(S->flags.p + F_BRK, &z, sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    }
+    if (hf[F_BRK]) ELFEL_CUDA(c, cudaMemsetAsync(S->flags.p + F_BRK, 0, sizeof(int), c->stream));
     // the units stay those of the start (s = ||b||) for the whole solve, so
     // the kept direction p needs no conversion
     demote_k<<<vg, kBlk, 0, c->stream>>>(nu, S->r64.p, S->r32.p, 1.0 / s);
     cg_start_k<float><<<vg, kBlk, 0, c->stream>>>(nu, S->r32.p, S->z32.p, S->p32.p, S->dinv32.p, red_area(S, 0),
                                                   S->scal.p, S->flags.p, restart, 1.0f);
     ELFEL_LAUNCH_CHECK(c);
-    ELFEL_TRY(set_scal(c, S, S_RMAX, sqrt(hsc[S_RR]) / s));
+    ELFEL_TRY(set_scal(c, S, ScalSet().set(S_RMAX, sqrt(hsc[S_RR]) / s)));
   }
   st->iterations = hf[F_ITER];
   st->refinements = refinements;
@@ -1379,9 +1349,9 @@ static int run_minres(Ctx* c, SolverData* S, const T* v, const T* minv, const T*
   T *const *vb = dp, *const *zb = dp + 3, *const *wb = dp + 6;
   const int64_t nu = S->nu;
   const unsigned vg = vec_grid(nu);
-  int hf[F_COUNT] = {0, 0, 0, maxit, 0, 0, 0};
-  ELFEL_CUDA(c, cudaMemcpyAsync(S->flags.p, hf, sizeof(hf), cudaMemcpyHostToDevice, c->stream));
-  ELFEL_TRY(set_scal(c, S, S_TOL2, rtol * rtol));
+  int hf[F_COUNT];
+  double hsc[S_COUNT];
+  ELFEL_TRY(set_scal(c, S, ScalSet().set(S_TOL2, rtol * rtol).start(maxit)));
   mr_start_k<T><<<vg, kBlk, 0, c->stream>>>(nu, b, vb, zb, wb, minv, x, red_area(S, 0), S->scal.p, S->flags.p);
   scale_k<T><<<vg, kBlk, 0, c->stream>>>(nu, zb, S->scal.p);
   ELFEL_LAUNCH_CHECK(c);
@@ -1393,13 +1363,9 @@ static int run_minres(Ctx* c, SolverData* S, const T* v, const T* minv, const T*
     mr_tail_k<<<1, 1, 0, c->stream>>>(S->scal.p, S->flags.p);
   }));
   while (true) {
-    if (run.blocks) {
-      ELFEL_TRY(run_mr(c, S, run, x, hp));
-      ELFEL_TRY(read_run(c, S, run, hf));
-    } else {
-      ELFEL_CUDA(c, cudaGraphLaunch(*graph, c->stream));
-      ELFEL_TRY(read_flags(c, S, hf));
-    }
+    if (run.blocks) ELFEL_TRY(run_mr(c, S, run, x, hp));
+    else ELFEL_CUDA(c, cudaGraphLaunch(*graph, c->stream));
+    ELFEL_TRY(read_run(c, S, run, hf, hsc));
     if (hf[F_DONE]) break;
   }
   *iters = hf[F_ITER];
@@ -1437,17 +1403,14 @@ extern "C" int elfel_solve(elfel_sysmat* m, const double* Fh, double* T, int64_t
   // lifted right-hand side: b = F_f - K_ff T_f - K_fd T_d
   ELFEL_TRY(lift_rhs(m, Fh, T, 0));
   double bn2 = 0.0;
-  ELFEL_CUDA(c, cudaMemcpyAsync(&bn2, S->scal.p + S_BN2, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
-  ELFEL_TRY(set_scal(c, S, S_TOL2, rtol * rtol));
-  ELFEL_TRY(set_scal(c, S, S_RMAX, sqrt(bn2)));
+  ELFEL_TRY(read_back(c, c->stream, {{&bn2, S->scal.p + S_BN2, sizeof(double)}}));
   // residual-replacement threshold of the FP32 refinement (tuning knob)
   double delta = 0.1;
   if (const char* e = getenv("ELFEL_RU_DELTA")) {
     const double d = atof(e);
     if (d > 0.0 && d < 1.0) delta = d;
   }
-  ELFEL_TRY(set_scal(c, S, S_DELTA, delta));
+  ELFEL_TRY(set_scal(c, S, ScalSet().set(S_TOL2, rtol * rtol).set(S_RMAX, sqrt(bn2)).set(S_DELTA, delta)));
   int rc = ELFEL_OK;
   double rr = -1.0;
   if (bn2 == 0.0) {
@@ -1458,7 +1421,7 @@ extern "C" int elfel_solve(elfel_sysmat* m, const double* Fh, double* T, int64_t
     rc = run_pcg64(m, rtol, maxit, &st, &rr);
   } else if (method == ELFEL_PCG32_IR) {
     Phase ph(c, "pcg32_ir");
-    rc = run_pcg32(m, rtol, maxit, &st, &rr);
+    rc = run_pcg32(m, bn2, rtol, maxit, &st, &rr);
   } else if (method == ELFEL_MINRES64) {
     Phase ph(c, "minres64");
     for (int i = 0; i < 3; ++i) {
@@ -1528,7 +1491,7 @@ extern "C" int elfel_solve(elfel_sysmat* m, const double* Fh, double* T, int64_t
   // solution back to the original order; final FP64 residual there
   if (rr < 0.0) {
     ELFEL_TRY(solution_residual(m));
-    ELFEL_CUDA(c, cudaMemcpyAsync(&rr, S->scal.p + S_RR, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    ELFEL_TRY(read_back(c, c->stream, {{&rr, S->scal.p + S_RR, sizeof(double)}}));
   }
   ELFEL_CUDA(c, cudaMemcpyAsync(T, S->xo64.p, sizeof(double) * nu, cudaMemcpyDeviceToHost, c->stream));
   ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));

@@ -75,6 +75,12 @@ struct SellView {
   const int32_t* c32;
 };
 
+// A vector inside a larger allocation.
+template <typename T>
+struct DBufView {
+  T* p = nullptr;
+};
+
 struct SolverData {
   int64_t nu = -1;
   const void* pattern_id = nullptr;
@@ -83,10 +89,13 @@ struct SolverData {
   Csr ff, fd;
   Sell A;
   // original order
-  DBuf<double> T64, bo64, xo64, ro64, dinvo;
+  DBuf<double> T64;
+  DBufView<double> bo64, xo64, ro64;
   // permuted order
-  DBuf<double> dinv64, b64, x64, r64, z64, p64, q64, y64;
-  DBuf<float> dinv32, r32, p32, q32, z32, xa32, zz32, b32, x32, rowsum32;
+  DBufView<double> dinv64, b64, x64, r64, z64, p64, q64, y64;
+  DBufView<float> dinv32, r32, p32, q32, z32, xa32, zz32, b32, x32, rowsum32;
+  DBuf<double> slab64;  // the vectors above, 128-byte aligned
+  DBuf<float> slab32;
   DBuf<double> v64[3], w64[3];
   DBuf<float> v32[3], w32[3];
   DBuf<double> scal;
@@ -105,11 +114,28 @@ struct SolverData {
   SellView view() const {
     return SellView{A.nrows, A.nslices, A.sptr.p, A.sw.p, A.d16 ? A.dcol.p : nullptr, A.d16 ? nullptr : A.col.p};
   }
+  // The vectors of nu entries: two allocations instead of 21.
+  int alloc_vectors(Ctx* c, int64_t nu) {
+    const size_t n = (size_t)(nu > 0 ? nu : 1), ld = (n + 31) / 32 * 32;
+    DBufView<double>* d[] = {&bo64, &xo64, &ro64, &dinv64, &b64, &x64, &r64, &z64, &p64, &q64, &y64};
+    DBufView<float>* f[] = {&dinv32, &r32, &p32, &q32, &z32, &xa32, &zz32, &b32, &x32, &rowsum32};
+    ELFEL_TRY(slab64.alloc(c, ld * (sizeof(d) / sizeof(d[0]))));
+    ELFEL_TRY(slab32.alloc(c, ld * (sizeof(f) / sizeof(f[0]))));
+    double* pd = slab64.p;
+    for (auto* v : d) {
+      v->p = pd;
+      pd += ld;
+    }
+    float* pf = slab32.p;
+    for (auto* v : f) {
+      v->p = pf;
+      pf += ld;
+    }
+    return ELFEL_OK;
+  }
   void release(Ctx* c) {
     ff.release(c); fd.release(c); A.release(c);
-    for (DBuf<double>* b : {&T64, &bo64, &xo64, &ro64, &dinvo, &dinv64, &b64, &x64, &r64, &z64, &p64, &q64, &y64})
-      b->release(c);
-    for (DBuf<float>* b : {&dinv32, &r32, &p32, &q32, &z32, &xa32, &zz32, &b32, &x32, &rowsum32}) b->release(c);
+    T64.release(c); slab64.release(c); slab32.release(c);
     for (int i = 0; i < 3; ++i) { v64[i].release(c); w64[i].release(c); v32[i].release(c); w32[i].release(c); }
     scal.release(c); flags.release(c); red.release(c); tickets.release(c); run_slots.release(c); run_bar.release(c); run_win.release(c);
     for (cudaGraphExec_t* g : {&g_pcg64, &g_pcg32, &g_minres64, &g_minres32})
