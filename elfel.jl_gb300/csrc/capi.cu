@@ -943,14 +943,25 @@ static int finish_values(elfel_sysmat* m, bool rhs_done = false) {
   return ELFEL_OK;
 }
 
+// The n conductivities of a call: page-locked ones are left to the integration
+// kernel (HostCoef), others are copied to dst.
+static int host_coef(Ctx* c, const double* coef, int64_t n, double* dst, HostCoef* host) {
+  if (!coef || n == 0) return ELFEL_OK;
+  int pinned = 0;
+  const void* p = host_device_ptr(c, coef, &pinned);
+  if (pinned) host->p = static_cast<const double*>(p);
+  else ELFEL_CUDA(c, cudaMemcpyAsync(dst, coef, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
+  return ELFEL_OK;
+}
+
 extern "C" int elfel_fused_heat(elfel_sysmat* m, const double* kappa, double Q) {
   CHECK_FREE(m);
   Ctx* c = &m->h->c;
   if (!m->fused || m->F.physics != ELFEL_HEAT) return fail(c, ELFEL_ERR_STATE, "heat: fused_setup(ELFEL_HEAT) first");
   cudaSetDevice(c->device);
   Fused& F = m->F;
-  if (kappa && F.nel)
-    ELFEL_CUDA(c, cudaMemcpyAsync(F.coef.p, kappa, sizeof(double) * F.nel, cudaMemcpyHostToDevice, c->stream));
+  HostCoef host;
+  ELFEL_TRY(host_coef(c, kappa, F.nel, F.coef.p, &host));
   const bool fdirect = F.shape == ELFEL_SHAPE_TRIANGLE && F.f_direct_ok && heat_f_direct(F.nn_u, F.ncurved, F.tab);
   // From a pattern's second assembly on, an exact-rule straight-sided T6 mesh
   // writes 8 bases per element and the tile reduction expands and sums them
@@ -968,7 +979,7 @@ extern "C" int elfel_fused_heat(elfel_sysmat* m, const double* kappa, double Q) 
       Phase ph(c, "integrate_heat");
       if (fdirect) ELFEL_CUDA(c, cudaMemsetAsync(m->rhs.p, 0, sizeof(double) * m->ncol, c->stream));
       ELFEL_TRY(launch_heat_bases(c, F.nel, F.conn_u.p, F.xy_u.p, F.coef.p, Q, F.tab, F.kstore.p, F.fstore.p,
-                                  fdirect ? F.dofs_u.p : nullptr, fdirect ? m->rhs.p : nullptr));
+                                  fdirect ? F.dofs_u.p : nullptr, fdirect ? m->rhs.p : nullptr, host));
     }
     {
       Head* head;
@@ -992,12 +1003,12 @@ extern "C" int elfel_fused_heat(elfel_sysmat* m, const double* kappa, double Q) 
     if (fdirect) {
       ELFEL_CUDA(c, cudaMemsetAsync(m->rhs.p, 0, sizeof(double) * m->ncol, c->stream));
       ELFEL_TRY(launch_heat(c, F.nn_u, F.nel, F.conn_u.p, F.xy_u.p, F.coef.p, Q, F.straight.p, F.ncurved, F.tab,
-                            F.kstore.p, F.fstore.p, F.dofs_u.p, m->rhs.p));
+                            F.kstore.p, F.fstore.p, F.dofs_u.p, m->rhs.p, host));
     } else if (F.shape == ELFEL_SHAPE_TRIANGLE) {
       ELFEL_TRY(launch_heat(c, F.nn_u, F.nel, F.conn_u.p, F.xy_u.p, F.coef.p, Q, F.straight.p, F.ncurved, F.tab,
-                            F.kstore.p, F.fstore.p));
+                            F.kstore.p, F.fstore.p, nullptr, nullptr, host));
     } else {
-      ELFEL_TRY(launch_heat_shape(c, F.stab, F.nel, F.conn_u.p, F.xy_u.p, F.coef.p, Q, F.kstore.p, F.fstore.p));
+      ELFEL_TRY(launch_heat_shape(c, F.stab, F.nel, F.conn_u.p, F.xy_u.p, F.coef.p, Q, F.kstore.p, F.fstore.p, host));
     }
   }
   return finish_values(m, fdirect);

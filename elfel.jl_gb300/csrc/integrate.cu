@@ -552,7 +552,8 @@ __global__ void __launch_bounds__(kIntThreads) heat_t6s_k(int64_t nel, const int
                                                          const __grid_constant__ QPTab tab,
                                                          double* __restrict__ kstore, double* __restrict__ fstore,
                                                          const int32_t* __restrict__ dofs = nullptr,
-                                                         double* __restrict__ fglob = nullptr) {
+                                                         double* __restrict__ fglob = nullptr,
+                                                         double* __restrict__ keep = nullptr) {
   constexpr int NN = 6, NS = 21, NT = kIntThreads, LD = NT + 1;
   extern __shared__ double acc[];  // (NS + NN) * LD
   __shared__ int32_t sconn[NT * NN];
@@ -560,6 +561,8 @@ __global__ void __launch_bounds__(kIntThreads) heat_t6s_k(int64_t nel, const int
   if (PAT != kPatT6R) stage_tensors<NN, NT>(tab, sS);  // the exact-rational form needs no tensors
   const int64_t e0 = (int64_t)blockIdx.x * NT;
   const int64_t base = e0 * NN, lim = nel * NN;
+  // the conductivity first: it may come over the host link (HostCoef)
+  const double kap = PAT == kPatT6R && e0 + threadIdx.x < nel ? __ldcs(kappa + e0 + threadIdx.x) : 0.0;
   for (int k = threadIdx.x; k < NT * NN; k += NT) {
     const int64_t gi = base + k;
     sconn[k] = gi < lim ? __ldg(conn + gi) : 0;
@@ -575,8 +578,9 @@ __global__ void __launch_bounds__(kIntThreads) heat_t6s_k(int64_t nel, const int
     if (e < nel) {
       const double2 p0 = __ldg(xy + sconn[t * NN]), p1 = __ldg(xy + sconn[t * NN + 1]),
                     p2 = __ldg(xy + sconn[t * NN + 2]);
-      t6r_bases(__dsub_rn(p1.x, p0.x), __dsub_rn(p2.x, p0.x), __dsub_rn(p1.y, p0.y), __dsub_rn(p2.y, p0.y), kappa[e],
+      t6r_bases(__dsub_rn(p1.x, p0.x), __dsub_rn(p2.x, p0.x), __dsub_rn(p1.y, p0.y), __dsub_rn(p2.y, p0.y), kap,
                 Q, tab.P[3], bs);
+      if (FDIRECT && keep) keep[e] = kap;
     }
     double* a = acc + t;
     if (BASES) {
@@ -712,13 +716,13 @@ __global__ void __launch_bounds__(kIntThreads) heat_t6_bases_k(int64_t nel, cons
                                                               const double* __restrict__ kappa, double Q, double P6,
                                                               double* __restrict__ bases,
                                                               const int32_t* __restrict__ dofs,
-                                                              double* __restrict__ fglob) {
+                                                              double* __restrict__ fglob, double* __restrict__ keep) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (e >= nel) return;
   // element e: coordinates and conductivity; element e + stride: vertex numbers and conductivity
   int32_t v0 = __ldg(conn + e * 6), v1 = __ldg(conn + e * 6 + 1), v2 = __ldg(conn + e * 6 + 2);
-  double kap = __ldg(kappa + e);
+  double kap = __ldcs(kappa + e);
   double2 p0 = __ldg(xy + v0), p1 = __ldg(xy + v1), p2 = __ldg(xy + v2);
   int64_t en = e + stride;
   double kapn = 0.0;
@@ -726,7 +730,7 @@ __global__ void __launch_bounds__(kIntThreads) heat_t6_bases_k(int64_t nel, cons
     v0 = __ldg(conn + en * 6);
     v1 = __ldg(conn + en * 6 + 1);
     v2 = __ldg(conn + en * 6 + 2);
-    kapn = __ldg(kappa + en);
+    kapn = __ldcs(kappa + en);
   }
   for (;;) {
     // the next element's coordinates, and the vertex numbers of the one after it
@@ -741,12 +745,13 @@ __global__ void __launch_bounds__(kIntThreads) heat_t6_bases_k(int64_t nel, cons
         v0 = __ldg(conn + enn * 6);
         v1 = __ldg(conn + enn * 6 + 1);
         v2 = __ldg(conn + enn * 6 + 2);
-        kapnn = __ldg(kappa + enn);
+        kapnn = __ldcs(kappa + enn);
       }
     }
     double bs[8];
     t6r_bases(__dsub_rn(p1.x, p0.x), __dsub_rn(p2.x, p0.x), __dsub_rn(p1.y, p0.y), __dsub_rn(p2.y, p0.y), kap, Q, P6,
               bs);
+    if (keep) keep[e] = kap;
     double2* o = reinterpret_cast<double2*>(bases + e * 8);
 #pragma unroll
     for (int k = 0; k < 4; ++k) o[k] = make_double2(bs[2 * k], bs[2 * k + 1]);
@@ -765,8 +770,15 @@ __global__ void __launch_bounds__(kIntThreads) heat_t6_bases_k(int64_t nel, cons
   }
 }
 
-int launch_heat_bases(Ctx* c, int64_t nel, const int32_t* conn, const double* xy, const double* kappa, double Q,
-                      const QPTab& tab, double* bases, double* fstore, const int32_t* dofs, double* fglob) {
+// The copy of host coefficients for a kernel that does not read them itself.
+static int copy_coef(Ctx* c, HostCoef host, int64_t n, double* dst) {
+  if (host.p) ELFEL_CUDA(c, cudaMemcpyAsync(dst, host.p, sizeof(double) * n, cudaMemcpyDefault, c->stream));
+  return ELFEL_OK;
+}
+
+int launch_heat_bases(Ctx* c, int64_t nel, const int32_t* conn, const double* xy, double* kappa, double Q,
+                      const QPTab& tab, double* bases, double* fstore, const int32_t* dofs, double* fglob,
+                      HostCoef host) {
   if (nel == 0) return ELFEL_OK;
   const unsigned grid = grid_for(nel, kIntThreads);
   const size_t sm = 11 * (kIntThreads + 1) * sizeof(double);
@@ -775,9 +787,10 @@ int launch_heat_bases(Ctx* c, int64_t nel, const int32_t* conn, const double* xy
     // 24 CTAs per SM (6 resident at 77 registers): 0.090 ms at 2M elements;
     // 8, 12, 16, 32, 64: 0.099, 0.095, 0.090, 0.090, 0.094 ms
     const unsigned g = grid_for(nel, kIntThreads, (int64_t)c->sm_count * 24);
-    heat_t6_bases_k<<<g, kIntThreads, 0, c->stream>>>(nel, conn, (const double2*)xy, kappa, Q, tab.P[3], bases, dofs,
-                                                     fglob);
+    heat_t6_bases_k<<<g, kIntThreads, 0, c->stream>>>(nel, conn, (const double2*)xy, host.p ? host.p : kappa, Q,
+                                                     tab.P[3], bases, dofs, fglob, host.p ? kappa : nullptr);
   } else {
+    ELFEL_TRY(copy_coef(c, host, nel, kappa));
     heat_t6s_k<kPatT6R, false, true><<<grid, kIntThreads, sm, c->stream>>>(nel, conn, (const double2*)xy, kappa, Q,
                                                                             tab, bases, fstore);
   }
@@ -789,9 +802,9 @@ bool heat_f_direct(int nn, int64_t ncurved, const QPTab& tab) {
   return nn == 6 && ncurved == 0 && heat_pattern(6, tab) == kPatT6R;
 }
 
-int launch_heat(Ctx* c, int nn, int64_t nel, const int32_t* conn, const double* xy, const double* kappa, double Q,
+int launch_heat(Ctx* c, int nn, int64_t nel, const int32_t* conn, const double* xy, double* kappa, double Q,
                 const uint8_t* straight, int64_t ncurved, const QPTab& tab, double* kstore, double* fstore,
-                const int32_t* dofs, double* fglob) {
+                const int32_t* dofs, double* fglob, HostCoef host) {
   if (nel == 0) return ELFEL_OK;
   const unsigned grid = grid_for(nel, kIntThreads);
   const double2* p = (const double2*)xy;
@@ -801,10 +814,11 @@ int launch_heat(Ctx* c, int nn, int64_t nel, const int32_t* conn, const double* 
     if (!heat_f_direct(nn, ncurved, tab) || !dofs)
       return fail(c, ELFEL_ERR_STATE, "heat: direct load-vector assembly needs the straight-sided exact T6 form");
     heat_t6s_k<kPatT6R, true><<<grid, kIntThreads, 11 * (kIntThreads + 1) * sizeof(double), c->stream>>>(
-        nel, conn, p, kappa, Q, tab, kstore, fstore, dofs, fglob);
+        nel, conn, p, host.p ? host.p : kappa, Q, tab, kstore, fstore, dofs, fglob, host.p ? kappa : nullptr);
     ELFEL_LAUNCH_CHECK(c);
     return ELFEL_OK;
   }
+  ELFEL_TRY(copy_coef(c, host, nel, kappa));
   if (nn == 3)
     heat_k<3, kPatGeneric><<<grid, kIntThreads, sm, c->stream>>>(nel, conn, p, kappa, Q, straight, tab, kstore, fstore);
   else if (ncurved == 0 && pat == kPatT6R)
@@ -980,11 +994,13 @@ __global__ void __launch_bounds__(kIntThreads) heat_q4_gauss2_k(int64_t nel, con
                                                                const double2* __restrict__ xy,
                                                                const double* __restrict__ kappa, double Q, double g,
                                                                double w, double* __restrict__ kstore,
-                                                               double* __restrict__ fstore) {
+                                                               double* __restrict__ fstore,
+                                                               double* __restrict__ keep) {
   constexpr int NT = kIntThreads, LD = NT + 1;
   __shared__ double acc[(kShapeNS + 4) * LD];
   __shared__ int32_t sconn[NT * 4];
   const int64_t e0 = (int64_t)blockIdx.x * NT;
+  const double kap = e0 + threadIdx.x < nel ? __ldcs(kappa + e0 + threadIdx.x) : 0.0;  // first: HostCoef
   load_conn4<NT>(conn, e0, nel, sconn);
   const int t = threadIdx.x;
   const int64_t e = e0 + t;
@@ -1004,7 +1020,8 @@ __global__ void __launch_bounds__(kIntThreads) heat_q4_gauss2_k(int64_t nel, con
       al[a] = fma(xt[a], xt[a], yt[a] * yt[a]);
       be[a] = fma(xs[a], xs[a], ys[a] * ys[a]);
     }
-    const double kw = kappa[e] * w;
+    const double kw = kap * w;
+    if (keep) keep[e] = kap;
 #pragma unroll
     for (int a = 0; a < 2; ++a)
 #pragma unroll
@@ -1101,12 +1118,14 @@ __global__ void __launch_bounds__(kIntThreads) heat_t4_k(int64_t nel, const int3
 }
 
 int launch_heat_shape(Ctx* c, const ShapeTab& tab, int64_t nel, const int32_t* conn, const double* xy,
-                      const double* kappa, double Q, double* kstore, double* fstore) {
+                      double* kappa, double Q, double* kstore, double* fstore, HostCoef host) {
   if (nel == 0) return ELFEL_OK;
   const unsigned grid = grid_for(nel, kIntThreads);
-  if (tab.shape == ELFEL_SHAPE_Q4 && tab.gauss2)
-    heat_q4_gauss2_k<<<grid, kIntThreads, 0, c->stream>>>(nel, conn, (const double2*)xy, kappa, Q, tab.g, tab.w[0], kstore,
-                                                          fstore);
+  const bool gauss2 = tab.shape == ELFEL_SHAPE_Q4 && tab.gauss2;
+  if (!gauss2) ELFEL_TRY(copy_coef(c, host, nel, kappa));
+  if (gauss2)
+    heat_q4_gauss2_k<<<grid, kIntThreads, 0, c->stream>>>(nel, conn, (const double2*)xy, host.p ? host.p : kappa, Q,
+                                                          tab.g, tab.w[0], kstore, fstore, host.p ? kappa : nullptr);
   else if (tab.shape == ELFEL_SHAPE_Q4)
     heat_q4_k<<<grid, kIntThreads, 0, c->stream>>>(nel, conn, (const double2*)xy, kappa, Q, tab, kstore, fstore);
   else if (tab.shape == ELFEL_SHAPE_T4)

@@ -31,6 +31,16 @@ struct Mat3 {
 
 int make_tables(int nn, int npts, const double* pc, const double* w, QPTab* t);
 
+// Conductivities that a kernel reads from the caller's page-locked array itself
+// (p, a device address) while it integrates, instead of a copy before it; it leaves
+// them in kappa as that copy would.  Kernels without this form get the copy.
+// Re-assembly to host CSC, 2M T6 elements: 2335 -> 2279 us, 491,000 Q4: 444 -> 425;
+// 500,000 T6 from tables to CSC 1717 -> 1593.  (The body forces of plane elasticity, two
+// per element, are copied: read by the kernel 250,000 elements took 1177 us, not 1167.)
+struct HostCoef {
+  const double* p = nullptr;
+};
+
 // straight: per-element straight-sided flags of the geometry (launch_straight;
 // unused for T3, whose elements always are); ncurved: the number of elements
 // without the flag (0 selects the straight-only T6 kernel).  fglob non-null:
@@ -38,17 +48,17 @@ int make_tables(int nn, int npts, const double* pc, const double* w, QPTab* t);
 // dofs) instead of being written to fstore; allowed only when
 // heat_f_direct() holds and no DOF is a midside node of more than two
 // elements.
-int launch_heat(Ctx* c, int nn, int64_t nel, const int32_t* conn, const double* xy, const double* kappa, double Q,
+int launch_heat(Ctx* c, int nn, int64_t nel, const int32_t* conn, const double* xy, double* kappa, double Q,
                 const uint8_t* straight, int64_t ncurved, const QPTab& tab, double* kstore, double* fstore,
-                const int32_t* dofs = nullptr, double* fglob = nullptr);
+                const int32_t* dofs = nullptr, double* fglob = nullptr, HostCoef host = HostCoef());
 // True when every element of a T6 mesh takes the exact-rule straight-sided
 // form, whose K record is determined by 8 bases (t6r_bases).
 bool heat_bases_ok(int nn, int64_t ncurved, const QPTab& tab);
 // The T6 heat integration writing the 8 bases per element (bases: nel x 8)
 // instead of the 21-entry K records; the load vector as in launch_heat.
-int launch_heat_bases(Ctx* c, int64_t nel, const int32_t* conn, const double* xy, const double* kappa, double Q,
+int launch_heat_bases(Ctx* c, int64_t nel, const int32_t* conn, const double* xy, double* kappa, double Q,
                       const QPTab& tab, double* bases, double* fstore, const int32_t* dofs = nullptr,
-                      double* fglob = nullptr);
+                      double* fglob = nullptr, HostCoef host = HostCoef());
 // True when the heat load vector of a T6 mesh takes the exact form (zero at
 // the vertices, Q det / 6 at the midside nodes) in the straight-only kernel.
 bool heat_f_direct(int nn, int64_t ncurved, const QPTab& tab);
@@ -95,7 +105,7 @@ int make_shape_tables(int shape, int npts, const double* pc, const double* w, Sh
 // Element records of the heat weak form on Q4 (xy: nnodes x 2) or T4 (xy:
 // nnodes x 3) meshes: kstore nel x 10 (upper triangle, column-packed), fstore nel x 4.
 int launch_heat_shape(Ctx* c, const ShapeTab& tab, int64_t nel, const int32_t* conn, const double* xy,
-                      const double* kappa, double Q, double* kstore, double* fstore);
+                      double* kappa, double Q, double* kstore, double* fstore, HostCoef host = HostCoef());
 
 // ncurved: curved elements of the geometry (0: the straight-sided tensor form).
 int launch_elasticity(Ctx* c, int nn, int64_t nel, const int32_t* conn, const double* xy, const Mat3& D,
