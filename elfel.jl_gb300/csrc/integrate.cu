@@ -987,9 +987,9 @@ __device__ __forceinline__ void q4_transform(const double (&X)[2][2], double p, 
 // values each), with them c = kappa w / det at the points and
 //   ke_ij = sum c [A_i A_j |x_eta|^2 + B_i B_j |x_xi|^2 - (A_i B_j + B_i A_j) x_xi.x_eta],
 // A_i = xi_i k_(eta_i)(eta), B_i = eta_i k_(xi_i)(xi) (k: q4_transform), the ten entries
-// are sums of three A A, three B B and four cross values.  About 165 FP64
+// are sums of three A A, three B B and four cross values.  About 140 FP64
 // operations per element instead of 330; the kernel is bound by them (491,401
-// elements: 285 -> 158 us).
+// elements: heat_q4_k 285 us, here 146, the conductivities read from the host included).
 __global__ void __launch_bounds__(kIntThreads) heat_q4_gauss2_k(int64_t nel, const int32_t* __restrict__ conn,
                                                                const double2* __restrict__ xy,
                                                                const double* __restrict__ kappa, double Q, double g,
@@ -1009,11 +1009,14 @@ __global__ void __launch_bounds__(kIntThreads) heat_q4_gauss2_k(int64_t nel, con
     const double2 n0 = __ldg(xy + sconn[t * 4]), n1 = __ldg(xy + sconn[t * 4 + 1]), n2 = __ldg(xy + sconn[t * 4 + 2]),
                   n3 = __ldg(xy + sconn[t * 4 + 3]);
     const double p = 0.25 * (1.0 + g), m = 0.25 * (1.0 - g);
-    // edge vectors: bottom, top (along xi), left, right (along eta)
-    const double bx = n1.x - n0.x, by = n1.y - n0.y, tx = n2.x - n3.x, ty = n2.y - n3.y;
-    const double lx = n3.x - n0.x, ly = n3.y - n0.y, rx = n2.x - n1.x, ry = n2.y - n1.y;
-    const double xs[2] = {fma(p, bx, m * tx), fma(p, tx, m * bx)}, ys[2] = {fma(p, by, m * ty), fma(p, ty, m * by)};
-    const double xt[2] = {fma(p, lx, m * rx), fma(p, rx, m * lx)}, yt[2] = {fma(p, ly, m * ry), fma(p, ry, m * ly)};
+    // twice the Jacobian's columns at the points: the bottom and left edges less
+    // (1 -+ g) / 2 of h = bottom - top = left - right (K does not change with that factor:
+    // products of two of them over their determinant)
+    const double bx = n1.x - n0.x, by = n1.y - n0.y, lx = n3.x - n0.x, ly = n3.y - n0.y;
+    const double hx = bx - (n2.x - n3.x), hy = by - (n2.y - n3.y);
+    const double m2 = 2.0 * m, p2 = 2.0 * p;
+    const double xs[2] = {fma(-m2, hx, bx), fma(-p2, hx, bx)}, ys[2] = {fma(-m2, hy, by), fma(-p2, hy, by)};
+    const double xt[2] = {fma(-m2, hx, lx), fma(-p2, hx, lx)}, yt[2] = {fma(-m2, hy, ly), fma(-p2, hy, ly)};
     double al[2], be[2], det[2][2], c[2][2], C[2][2];
 #pragma unroll
     for (int a = 0; a < 2; ++a) {
@@ -1034,11 +1037,11 @@ __global__ void __launch_bounds__(kIntThreads) heat_q4_gauss2_k(int64_t nel, con
     // S[b] = sum_a c |x_eta|^2, T[a] = sum_b c |x_xi|^2
     const double S0 = fma(c[0][0], al[0], c[1][0] * al[1]), S1 = fma(c[0][1], al[0], c[1][1] * al[1]);
     const double T0 = fma(c[0][0], be[0], c[0][1] * be[1]), T1 = fma(c[1][0], be[0], c[1][1] * be[1]);
-    const double Pb = fma(pp, S0, mm * S1), Pt = fma(mm, S0, pp * S1), Px = (S0 + S1) * pm;
-    const double Rl = fma(pp, T0, mm * T1), Rr = fma(mm, T0, pp * T1), Rx = (T0 + T1) * pm;
-    double G[2][2], D[2][2];
+    const double Ss = S0 + S1, Ts = T0 + T1, pq = pp + mm;
+    const double Pb = fma(pp, S0, mm * S1), Pt = fma(pq, Ss, -Pb), Px = Ss * pm;
+    const double Rl = fma(pp, T0, mm * T1), Rr = fma(pq, Ts, -Rl), Rx = Ts * pm;
+    double G[2][2];
     q4_transform(C, p, m, G);
-    q4_transform(det, p, m, D);
     double* k = acc + t;
     k[0 * LD] = fma(-2.0, G[0][0], Pb + Rl);        // 00
     k[1 * LD] = (Rx - Pb) + (G[0][0] - G[1][0]);    // 01
@@ -1050,11 +1053,14 @@ __global__ void __launch_bounds__(kIntThreads) heat_q4_gauss2_k(int64_t nel, con
     k[7 * LD] = -((Px + Rx) + (G[0][0] + G[1][1])); // 13
     k[8 * LD] = (Rx - Pt) + (G[1][1] - G[0][1]);    // 23
     k[9 * LD] = fma(2.0, G[0][1], Pt + Rl);         // 33
-    const double f = 4.0 * w * Q;
-    fa[0 * LD + t] = f * D[0][0];
-    fa[1 * LD + t] = f * D[1][0];
-    fa[2 * LD + t] = f * D[1][1];
-    fa[3 * LD + t] = f * D[0][1];
+    // load: det (four times it here) is linear in xi and eta
+    const double f = w * Q * 0.125, fg = f * g;
+    const double d0 = f * (det[0][0] + det[1][1]), du = fg * (det[1][0] - det[0][0]), dv = fg * (det[0][1] - det[0][0]);
+    const double lo = d0 - du, hi = d0 + du;
+    fa[0 * LD + t] = lo - dv;
+    fa[1 * LD + t] = hi - dv;
+    fa[2 * LD + t] = hi + dv;
+    fa[3 * LD + t] = lo + dv;
   }
   write_records_fixed<NT, kShapeNS, kShapeNS>(acc, 0, e0, nel, kstore);
   __syncthreads();
