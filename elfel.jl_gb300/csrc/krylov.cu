@@ -17,18 +17,19 @@
 //     (the same partials in the same order: the same bits in every block);
 //   - x is advanced between the arrival at and the wait for the second sum.
 // Per iteration, quadratic heat, FP64 and FP32 (graphs, then one launch):
-//       961 unknowns  21.3 ->  6.4 us   25.8 ->  9.5 us (12 replacements incl.)
-//     14161           21.1 ->  8.9      21.9 ->  6.5
-//    128881           26.2 -> 12.7      22.2 ->  8.6
-//    358801           40.2 -> 23.5      32.0 -> 11.9
-//    808201           62.7 -> 47.9      45.9 -> 16.2
-// MINRES (Taylor-Hood cavity) 27.2 -> 11.9 us at 9026 unknowns.  What is left
-// at 128881: the two sums over the grid (2.0 us each with their barriers), in
-// FP64 the FP64 unit (6 us).  Measured and not kept: the direction gathered
+//       961 unknowns  21.3 ->  6.0 us   25.8 ->  7.9 us (12 replacements incl.)
+//     14161           21.1 ->  8.0      21.9 ->  6.0
+//    128881           26.2 -> 11.9      22.2 ->  7.9
+//    358801           40.2 -> 22.7      32.0 -> 10.9
+//    808201           62.7 -> 46.7      45.9 -> 15.3
+// MINRES (Taylor-Hood cavity) 27.2 -> 11.0 us at 9026 unknowns.  What is left
+// at 128881: the two sums over the grid (1.5 us a barrier, 0.8 to collect), in
+// FP64 the FP64 unit (4.5 us).  Measured and not kept: the direction gathered
 // from global memory after a barrier of its own (FP32 9.4 us at 128881, 21.1 at
 // 808201: gathers that miss L1), 1024 threads a block (17.5 at 808201), the
-// next chunk of the matrix prefetched into registers (no change: the product
-// is bound by instruction issue).
+// next chunk of the matrix prefetched into registers (no change), the matrix
+// streamed through rings in shared memory with cp.async (19.0 at 808201), columns and
+// FP32 values in quads for 16-byte loads (15.6; 12.4 at 128881 in FP64).
 // Two groups are provided:
 //   ClusterGroup  one cluster of up to 16 blocks: sums through distributed
 //                 shared memory, the hardware cluster barrier (0.2-0.3 us);

@@ -29,8 +29,9 @@
 // the gathered vector stays in L2.
 //
 // All reductions are deterministic (per-block partials added in a fixed
-// order).  Iterations run as CUDA graphs of kGraphIters iterations; kernels
-// of a finished (or paused) iteration exit at once.
+// order).  The iterations of a system that fits run inside one kernel
+// (krylov.cu); others as CUDA graphs of kGraphIters iterations, whose kernels
+// exit at once in a finished (or paused) iteration.
 #include <math.h>
 
 #include <chrono>
