@@ -24,7 +24,7 @@ namespace {
 template <int NV, typename T>
 __device__ __forceinline__ void cluster_sum(ClusterGroup& grp, T (&v)[NV], double* part, double* wsum, double (&t)[NV]) {
   const int wid = threadIdx.x >> 5;
-  block_sums<NV>(v, part, wsum, t);
+  block_sums<NV>(v, part, wsum, t, kRW);
   if (wid == 0) grp.publish(t);
   grp.arrive(wid);
   grp.wait(wid);
@@ -113,7 +113,7 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
       if (IR) d2[N2 - 1] += zi * ro;
     }
     double t2[N2];
-    block_sums<N2>(d2, part, wsum, t2);
+    block_sums<N2>(d2, part, wsum, t2, kRW);
     if (wid == 0) grp.publish(t2);
     grp.arrive(wid);
     for (int i = tid; i < R.nloc; i += kRT) sx[i] += al * sp[i];

@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kRT, 1) cg_run_k(const CgRun<T> a, const RunGr
   const int ld = a.spb * 32;
   T *sr = sx + ld, *sq = sr + ld, *sd = sq + ld, *ss = sd + ld, *pw = ss + (a.own_sums ? ld : 0);
   const RunRows<T, D16, MS> R(a.A, a.v, (int)blockIdx.x, a.spb, a.room, reinterpret_cast<int2*>(pw + a.window));
-  const int r1 = (int)R.row0 + R.nloc;
+  const int r1 = (int)R.row0 + R.nloc, nw = run_warps(R.nsl);
   Window<T> W(pw, WIN ? a.win[blockIdx.x] : make_int4((int)R.row0, r1, r1, r1), false, (int)R.row0, R.nloc);
   T* const sp = pw + W.own;
   W.load(a.p);
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kRT, 1) cg_run_k(const CgRun<T> a, const RunGr
       }
     }
     double t1[N1];
-    block_sums<N1>(d1, part, wsum, t1);
+    block_sums<N1>(d1, part, wsum, t1, nw);
     if (wid == 0) grp.publish(t1);
     grp.arrive(wid);
     bool ok = grp.wait(wid);
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kRT, 1) cg_run_k(const CgRun<T> a, const RunGr
       if (IR) d2[N2 - 1] += zi * ro;
     }
     double t2[N2];
-    block_sums<N2>(d2, part, wsum, t2);
+    block_sums<N2>(d2, part, wsum, t2, nw);
     if (wid == 0) grp.publish(t2);
     grp.arrive(wid);
     for (int i = tid; i < R.nloc; i += kRT) sx[i] += al * sp[i];
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(kRT, 1) mr_run_k(const MrRun<T> a, const RunGr
   T *sq = sx + ld, *sm = sq + ld, *sv = sm + ld, *svm = sv + ld, *sw = svm + ld, *swm = sw + ld, *zw = swm + ld;
   const RunRows<T, D16, MS> R(a.A, a.v, (int)blockIdx.x, a.spb, a.room, reinterpret_cast<int2*>(zw + a.window));
   const int64_t r0 = R.row0;
-  const int r1 = (int)r0 + R.nloc;
+  const int r1 = (int)r0 + R.nloc, nw = run_warps(R.nsl);
   Window<T> W(zw, WIN ? a.win[blockIdx.x] : make_int4((int)r0, r1, r1, r1), true, (int)r0, R.nloc);
   T* const sz = zw + W.own;
   W.load(a.z);
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(kRT, 1) mr_run_k(const MrRun<T> a, const RunGr
       }
     }
     double t[1];
-    block_sums<1>(d1, part, wsum, t);
+    block_sums<1>(d1, part, wsum, t, nw);
     if (wid == 0) grp.publish(t);
     grp.arrive(wid);
     bool ok = grp.wait(wid);
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(kRT, 1) mr_run_k(const MrRun<T> a, const RunGr
       if (WIN) a.z[r0 + i] = zz;
       d2[0] += zz * vv;
     }
-    block_sums<1>(d2, part, wsum, t);
+    block_sums<1>(d2, part, wsum, t, nw);
     if (wid == 0) grp.publish(t);
     grp.arrive(wid);
     ok = grp.wait(wid);

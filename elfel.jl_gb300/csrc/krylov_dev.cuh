@@ -182,8 +182,11 @@ struct GridGroup {
 // The block's sums of the threads' values, in every lane of warp 0 (which
 // has room for 3 * kRT doubles in part and 16 in wsum).  FP32 values add
 // within the warp in FP32 first; FP64 values go to shared memory as they are.
+// nw: the warps that have values (the others' are zero): all, or fewer in a small
+// system's block, whose FP64 sums leave the zeros out (run_warps; a solve with 16 x 16 T6
+// elements 1119 -> 1076 us, 64 x 64 T3 1700 -> 1644).
 template <int NV, typename T>
-__device__ __forceinline__ void block_sums(T (&v)[NV], double* part, double* wsum, double (&tot)[NV]) {
+__device__ __forceinline__ void block_sums(T (&v)[NV], double* part, double* wsum, double (&tot)[NV], int nw) {
   constexpr int L = 32 / sum_groups(NV);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane / L, l = lane % L;
   if (sizeof(T) == 4) {
@@ -210,17 +213,32 @@ __device__ __forceinline__ void block_sums(T (&v)[NV], double* part, double* wsu
     for (int k = 0; k < NV; ++k) part[k * kRT + threadIdx.x] = (double)v[k];
     __syncthreads();
     if (wid < 4) {
+      // warp w adds the values of warps w, w + 4, ...
       double s = 0.0;
       if (g < NV) {
-        const double* p = part + g * kRT + wid * (kRT / 4) + l;
-        s = p[0];
+        const double* p = part + g * kRT + wid * 32 + l;
+        if (nw == kRW) {
+          s = p[0];
 #pragma unroll
-        for (int j = 1; j < kRT / 4 / L; ++j) s += p[j * L];
+          for (int j = 1; j < kRT / 4 / L; ++j) s += p[(j / (32 / L)) * 128 + (j % (32 / L)) * L];
+        } else if (wid < nw) {
+          s = p[0];
+#pragma unroll
+          for (int j = 1; j < 32 / L; ++j) s += p[j * L];
+          if (wid + 4 < nw) {
+#pragma unroll
+            for (int j = 0; j < 32 / L; ++j) s += p[128 + j * L];
+          }
+        }
       }
       quad_total<NV>(lanes_sum<L>(s), wsum, tot);
     }
   }
 }
+
+// Warps with values in a block of nsl slices: up to 8 slices go to as many warps
+// (RunRows::slice), rows beside one another too.
+__device__ __forceinline__ int run_warps(int nsl) { return nsl <= 8 ? nsl : kRW; }
 
 template <typename T>
 __device__ __forceinline__ T axpy(T b, T x, T z) {
