@@ -47,4 +47,13 @@ constexpr int kBRunIters = 64;
 int batch_run_launch(Ctx* c, cudaStream_t st, int ir, const BSys* sys, const int* list, int n, int blocks, size_t smem,
                      int iters);
 
+// One system's FP32 refinement inside a cluster kernel, replacements included
+// (elfel_solve): its descriptor, scalars and state on the device.
+struct IrOne {
+  BSys sys;
+  double sc[B_COUNT];
+  int st[I_COUNT];
+  int list;
+};
+
 }  // namespace elfel

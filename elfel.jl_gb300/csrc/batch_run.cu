@@ -22,9 +22,10 @@ namespace {
 
 // One sum over the cluster (all threads; the totals are valid in warp 0).
 template <int NV, typename T>
-__device__ __forceinline__ void cluster_sum(ClusterGroup& grp, T (&v)[NV], double* part, double* wsum, double (&t)[NV]) {
+__device__ __forceinline__ void cluster_sum(ClusterGroup& grp, T (&v)[NV], double* part, double* wsum, double (&t)[NV],
+                                            int nw = kRW) {
   const int wid = threadIdx.x >> 5;
-  block_sums<NV>(v, part, wsum, t, kRW);
+  block_sums<NV>(v, part, wsum, t, nw);
   if (wid == 0) grp.publish(t);
   grp.arrive(wid);
   grp.wait(wid);
@@ -48,6 +49,7 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
   const RunRows<T, D16, MS> R(S.A, IR ? (const T*)S.v32 : (const T*)S.v64, grp.rank, S.spb, S.room,
                               reinterpret_cast<int2*>(pw + S.window));
   const int64_t r0 = R.row0;
+  const int nw = run_warps(R.nsl);
   Window<T> W(pw, S.win[grp.rank], false, (int)r0, R.nloc);
   T* const sp = pw + W.own;
   W.load(gp);
@@ -90,7 +92,7 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
       }
     }
     double t1[N1];
-    cluster_sum<N1>(grp, d1, part, wsum, t1);
+    cluster_sum<N1>(grp, d1, part, wsum, t1, nw);
     if (wid == 0) {
       pq = t1[0];
       const double alpha = pos_finite(pq) ? fast_div(IR ? t1[N1 - 1] : rz, pq, fast_rcp(pq)) : 0.0;
@@ -113,7 +115,7 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
       if (IR) d2[N2 - 1] += zi * ro;
     }
     double t2[N2];
-    block_sums<N2>(d2, part, wsum, t2, kRW);
+    block_sums<N2>(d2, part, wsum, t2, nw);
     if (wid == 0) grp.publish(t2);
     grp.arrive(wid);
     for (int i = tid; i < R.nloc; i += kRT) sx[i] += al * sp[i];
@@ -314,6 +316,64 @@ int batch_run_launch(Ctx* c, cudaStream_t st, int ir, const BSys* sys, const int
   cfg.attrs = at;
   cfg.numAttrs = 1;
   ELFEL_CUDA(c, cudaLaunchKernelEx(&cfg, k, sys, list, iters));
+  return ELFEL_OK;
+}
+
+// The descriptor and the start of one system's refinement (run_ir_cluster).
+__global__ void ir_start_k(IrOne* one, BSys d, const double* scal, double tol2, double delta, double scale, double bn2,
+                           int maxit) {
+  const int t = threadIdx.x;
+  if (t < B_COUNT)
+    one->sc[t] = t == B_RZ      ? scal[S_RZ]
+                 : t == B_TOL2  ? tol2
+                 : t == B_DELTA ? delta
+                 : t == B_SCALE ? scale
+                 : t == B_BN2   ? bn2
+                 : t == B_RMAX  ? 1.0
+                                : 0.0;
+  if (t < I_COUNT) one->st[t] = t == I_MAXIT ? maxit : t == I_MODE ? M_CG : 0;
+  if (t == 0) {
+    d.sc = one->sc;
+    d.st = one->st;
+    one->sys = d;
+    one->list = 0;
+  }
+}
+
+int run_ir_cluster(Ctx* c, SolverData* S, const RunPlan& P, const int4* win, double tol2, double delta, double scale,
+                   double bn2, int maxit, IrResult* out) {
+  if (!S->ir_one.p) ELFEL_TRY(S->ir_one.alloc(c, sizeof(IrOne)));
+  IrOne* one = reinterpret_cast<IrOne*>(S->ir_one.p);
+  BSys d;
+  memset(&d, 0, sizeof(d));
+  d.A = S->view();
+  d.v32 = S->A.v32.p;
+  d.v64 = S->A.v64.p;
+  d.dinv32 = S->dinv32.p;
+  d.dinv64 = S->dinv64.p;
+  d.rowsum = S->rowsum32.p;
+  d.x32 = S->xa32.p;
+  d.r32 = S->r32.p;
+  d.z32 = S->z32.p;
+  d.p32 = S->p32.p;
+  d.x64 = S->x64.p;
+  d.r64 = S->r64.p;
+  d.b64 = S->b64.p;
+  d.spb = P.spb;
+  d.ms = P.ms;
+  d.window = P.window;
+  d.room = P.room;
+  d.win = win;
+  ir_start_k<<<1, 32, 0, c->stream>>>(one, d, S->scal.p, tol2, delta, scale, bn2, maxit);
+  ELFEL_LAUNCH_CHECK(c);
+  int st[I_COUNT];
+  do {
+    ELFEL_TRY(batch_run_launch(c, c->stream, 1, &one->sys, &one->list, 1, P.blocks, P.smem, kRunIters));
+    ELFEL_TRY(read_back(c, c->stream, {{st, one->st, sizeof(st)}}));
+  } while (st[I_MODE] == M_CG);
+  out->iterations = st[I_ITER];
+  out->replacements = st[I_REPL];
+  out->converged = st[I_CONV];
   return ELFEL_OK;
 }
 

@@ -532,33 +532,31 @@ RunPlan run_plan(Ctx* c, const SolverData* S, int elem, int vecs, int least_vecs
 // The window argument of a launch: the room for it (without one, for the own
 // rows of the direction), and the blocks' windows.
 static int run_window_arg(const RunPlan& P) { return P.window ? P.window : P.spb * 32; }
-static const int4* run_win_arg(const SolverData* S, const RunPlan& P) {
-  return S->run_win.p + (P.cluster ? 0 : kRunWinGrid);
-}
+const int4* run_windows(const SolverData* S, const RunPlan& P) { return S->run_win.p + (P.cluster ? 0 : kRunWinGrid); }
 
 int run_cg64(Ctx* c, SolverData* S, const RunPlan& P) {
   const CgRun<double> a{S->view(), S->A.v64.p, S->dinv64.p, nullptr, S->x64.p, S->r64.p, S->p64.p, S->z64.p,
-                        S->scal.p, S->flags.p, P.spb, run_window_arg(P), P.room, kRunIters, run_win_arg(S, P), P.vecs > 4};
+                        S->scal.p, S->flags.p, P.spb, run_window_arg(P), P.room, kRunIters, run_windows(S, P), P.vecs > 4};
   return S->A.d16 ? cg_launch<double, true, false>(c, S, P, a) : cg_launch<double, false, false>(c, S, P, a);
 }
 
 int run_cg32(Ctx* c, SolverData* S, const RunPlan& P) {
   const CgRun<float> a{S->view(), S->A.v32.p, S->dinv32.p, S->rowsum32.p, S->xa32.p, S->r32.p, S->p32.p, S->z32.p,
-                       S->scal.p, S->flags.p, P.spb, run_window_arg(P), P.room, kRunIters, run_win_arg(S, P), P.vecs > 4};
+                       S->scal.p, S->flags.p, P.spb, run_window_arg(P), P.room, kRunIters, run_windows(S, P), P.vecs > 4};
   return S->A.d16 ? cg_launch<float, true, true>(c, S, P, a) : cg_launch<float, false, true>(c, S, P, a);
 }
 
 int run_mr64(Ctx* c, SolverData* S, const RunPlan& P, double* x, double* z, double* vj, double* vjm, double* wj,
              double* wjm) {
   const MrRun<double> a{S->view(), S->A.v64.p, S->dinv64.p, x,     z,             vj,       vjm, wj, wjm,
-                        S->scal.p, S->flags.p, P.spb, run_window_arg(P), P.room, kRunIters, run_win_arg(S, P)};
+                        S->scal.p, S->flags.p, P.spb, run_window_arg(P), P.room, kRunIters, run_windows(S, P)};
   return S->A.d16 ? mr_launch<double, true>(c, S, P, a) : mr_launch<double, false>(c, S, P, a);
 }
 
 int run_mr32(Ctx* c, SolverData* S, const RunPlan& P, float* x, float* z, float* vj, float* vjm, float* wj,
              float* wjm) {
   const MrRun<float> a{S->view(), S->A.v32.p, S->dinv32.p, x,     z,             vj,       vjm, wj, wjm,
-                       S->scal.p, S->flags.p, P.spb, run_window_arg(P), P.room, kRunIters, run_win_arg(S, P)};
+                       S->scal.p, S->flags.p, P.spb, run_window_arg(P), P.room, kRunIters, run_windows(S, P)};
   return S->A.d16 ? mr_launch<float, true>(c, S, P, a) : mr_launch<float, false>(c, S, P, a);
 }
 

@@ -1262,7 +1262,7 @@ static int run_pcg64(elfel_sysmat* m, double rtol, int maxit, elfel_solve_stats*
   return ELFEL_OK;
 }
 
-static int run_pcg32(elfel_sysmat* m, double bn2, double rtol, int maxit, elfel_solve_stats* st, double* rr) {
+static int run_pcg32(elfel_sysmat* m, double bn2, double delta, double rtol, int maxit, elfel_solve_stats* st, double* rr) {
   Ctx* c = &m->h->c;
   SolverData* S = m->solver;
   const int64_t nu = S->nu;
@@ -1289,6 +1289,32 @@ static int run_pcg32(elfel_sysmat* m, double bn2, double rtol, int maxit, elfel_
   int refinements = 0, late = 0;
   int launches = 0;
   double hsc[S_COUNT];
+  if (run.blocks && run.cluster && run.window && run.ms && run.vecs == 5) {
+    IrResult ir;
+    ELFEL_TRY(run_ir_cluster(c, S, run, run_windows(S, run), rtol * rtol, delta, s, bn2, maxit, &ir));
+    hf[F_ITER] = ir.iterations;
+    refinements = ir.replacements;
+    bool all = false;
+    if (ir.converged) ELFEL_TRY(residual_converged(m, rtol, rr, &all));
+    if (c->trace)
+      fprintf(stderr, "[elfel pcg32] it %d, %d replacements in the kernel, converged %d (final residual: %d)\n",
+              ir.iterations, ir.replacements, ir.converged, (int)all);
+    if (all || !ir.converged || ir.iterations >= maxit) {
+      st->iterations = ir.iterations;
+      st->refinements = refinements;
+      return ELFEL_OK;
+    }
+    // the residual of the original system is above by a hair: restart from the permuted one
+    *rr = -1.0;
+    ++late;
+    ELFEL_TRY(read_back(c, c->stream, {{hsc, S->scal.p, sizeof(hsc)}}));
+    demote_k<<<vg, kBlk, 0, c->stream>>>(nu, S->r64.p, S->r32.p, 1.0 / s);
+    ELFEL_TRY(set_scal(c, S, ScalSet().set(S_RMAX, sqrt(hsc[S_RR]) / s).start(maxit)));
+    ELFEL_CUDA(c, cudaMemcpyAsync(S->flags.p + F_ITER, &hf[F_ITER], sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    cg_start_k<float><<<vg, kBlk, 0, c->stream>>>(nu, S->r32.p, S->z32.p, S->p32.p, S->dinv32.p, red_area(S, 0),
+                                                  S->scal.p, S->flags.p, 1, 1.0f);
+    ELFEL_LAUNCH_CHECK(c);
+  }
   while (true) {
     if (run.blocks) ELFEL_TRY(run_cg32(c, S, run));
     else ELFEL_CUDA(c, cudaGraphLaunch(S->g_pcg32, c->stream));
@@ -1422,7 +1448,7 @@ extern "C" int elfel_solve(elfel_sysmat* m, const double* Fh, double* T, int64_t
     rc = run_pcg64(m, rtol, maxit, &st, &rr);
   } else if (method == ELFEL_PCG32_IR) {
     Phase ph(c, "pcg32_ir");
-    rc = run_pcg32(m, bn2, rtol, maxit, &st, &rr);
+    rc = run_pcg32(m, bn2, delta, rtol, maxit, &st, &rr);
   } else if (method == ELFEL_MINRES64) {
     Phase ph(c, "minres64");
     for (int i = 0; i < 3; ++i) {

@@ -110,6 +110,7 @@ struct SolverData {
   DBuf<double> run_slots;
   DBuf<unsigned> run_bar;
   DBuf<int4> run_win;
+  DBuf<unsigned char> ir_one;  // IrOne (first use)
   cudaGraphExec_t g_pcg64 = nullptr, g_pcg32 = nullptr, g_minres64 = nullptr, g_minres32 = nullptr;
   SellView view() const {
     return SellView{A.nrows, A.nslices, A.sptr.p, A.sw.p, A.d16 ? A.dcol.p : nullptr, A.d16 ? nullptr : A.col.p};
@@ -137,7 +138,7 @@ struct SolverData {
     ff.release(c); fd.release(c); A.release(c);
     T64.release(c); slab64.release(c); slab32.release(c);
     for (int i = 0; i < 3; ++i) { v64[i].release(c); w64[i].release(c); v32[i].release(c); w32[i].release(c); }
-    scal.release(c); flags.release(c); red.release(c); tickets.release(c); run_slots.release(c); run_bar.release(c); run_win.release(c);
+    scal.release(c); flags.release(c); red.release(c); tickets.release(c); run_slots.release(c); run_bar.release(c); run_win.release(c); ir_one.release(c);
     for (cudaGraphExec_t* g : {&g_pcg64, &g_pcg32, &g_minres64, &g_minres32})
       if (*g) { cudaGraphExecDestroy(*g); *g = nullptr; }
   }
