@@ -47,7 +47,7 @@ constexpr int kBRunIters = 64;
 int batch_run_launch(Ctx* c, cudaStream_t st, int ir, const BSys* sys, const int* list, int n, int blocks, size_t smem,
                      int iters);
 
-// One system's FP32 refinement inside a cluster kernel, replacements included
+// One system's FP32 refinement inside one kernel, replacements included
 // (elfel_solve): its descriptor, scalars and state on the device.
 struct IrOne {
   BSys sys;

@@ -20,20 +20,30 @@ namespace elfel {
 
 namespace {
 
-// One sum over the cluster (all threads; the totals are valid in warp 0).
-template <int NV, typename T>
-__device__ __forceinline__ void cluster_sum(ClusterGroup& grp, T (&v)[NV], double* part, double* wsum, double (&t)[NV],
-                                            int nw = kRW) {
+// One sum over the group (all threads; the totals, and whether the wait ended, are valid in warp 0).
+template <int NV, typename T, class Group>
+__device__ __forceinline__ bool group_sum(Group& grp, T (&v)[NV], double* part, double* wsum, double (&t)[NV],
+                                          int nw = kRW) {
   const int wid = threadIdx.x >> 5;
   block_sums<NV>(v, part, wsum, t, nw);
   if (wid == 0) grp.publish(t);
   grp.arrive(wid);
-  grp.wait(wid);
+  const bool ok = grp.wait(wid);
   grp.collect(wid, wsum, t);
+  return ok;
 }
 
-template <bool IR, bool D16, bool MS>
-__device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint8_t* smem, RunMsg& msg, int iters) {
+// A grid group's wait is warp 0's: the block learns here that it ended (false: it ran out).
+template <class Group>
+__device__ __forceinline__ bool group_done(bool ok, RunMsg& msg) {
+  if (Group::kCluster) return true;
+  if (threadIdx.x == 0) msg.stop = ok ? M_CG : M_DONE;
+  __syncthreads();
+  return msg.stop == M_CG;
+}
+
+template <bool IR, bool D16, bool MS, class Group>
+__device__ __forceinline__ void batch_run(const BSys& S, Group& grp, int rank, uint8_t* smem, RunMsg& msg, int iters) {
   typedef typename std::conditional<IR, float, double>::type T;
   const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
   double* part = reinterpret_cast<double*>(smem);
@@ -46,11 +56,11 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
   T* const gp = IR ? (T*)S.p32 : (T*)S.p64;
   const T* const gd = IR ? (const T*)S.dinv32 : (const T*)S.dinv64;
   T* const gz = IR ? (T*)S.z32 : (T*)S.z64;
-  const RunRows<T, D16, MS> R(S.A, IR ? (const T*)S.v32 : (const T*)S.v64, grp.rank, S.spb, S.room,
+  const RunRows<T, D16, MS> R(S.A, IR ? (const T*)S.v32 : (const T*)S.v64, rank, S.spb, S.room,
                               reinterpret_cast<int2*>(pw + S.window));
   const int64_t r0 = R.row0;
   const int nw = run_warps(R.nsl);
-  Window<T> W(pw, S.win[grp.rank], false, (int)r0, R.nloc);
+  Window<T> W(pw, S.win[rank], false, (int)r0, R.nloc);
   T* const sp = pw + W.own;
   W.load(gp);
   for (int i = tid; i < R.nloc; i += kRT) {
@@ -92,13 +102,20 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
       }
     }
     double t1[N1];
-    cluster_sum<N1>(grp, d1, part, wsum, t1, nw);
+    bool ok = group_sum<N1>(grp, d1, part, wsum, t1, nw);
     if (wid == 0) {
       pq = t1[0];
       const double alpha = pos_finite(pq) ? fast_div(IR ? t1[N1 - 1] : rz, pq, fast_rcp(pq)) : 0.0;
-      if (lane == 0) msg.c[0] = alpha;
+      if (lane == 0) {
+        msg.c[0] = alpha;
+        if (!Group::kCluster) msg.stop = ok ? M_CG : M_DONE;
+      }
     }
     __syncthreads();
+    if (!Group::kCluster && msg.stop == M_DONE) {
+      mode = M_DONE;
+      break;
+    }
     // r -= alpha q, z = D r (kept in q); r.z, r.r (and z.r_old) -> beta
     constexpr int N2 = IR ? 3 : 2;
     const T al = (T)msg.c[0];
@@ -120,7 +137,7 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
     grp.arrive(wid);
     for (int i = tid; i < R.nloc; i += kRT) sx[i] += al * sp[i];
     if (wid == 0) inv_rz = fast_rcp(rz);
-    grp.wait(wid);
+    ok = grp.wait(wid);
     grp.collect(wid, wsum, t2);
     if (wid == 0) {
       const double beta = (IR ? t2[0] - t2[N2 - 1] : t2[0]) * inv_rz;
@@ -147,6 +164,10 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
         conv = conv && !bad;
         mode = M_DONE;
       }
+      if (!ok) {
+        conv = 0;
+        mode = M_DONE;
+      }
       if (lane == 0) {
         msg.c[0] = beta;
         msg.stop = mode;
@@ -168,8 +189,13 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
           S.x64[r0 + i] = (double)sx[i];
         }
       }
+      if (!Group::kCluster) __syncthreads();
       grp.arrive(wid);
-      grp.wait(wid);
+      ok = grp.wait(wid);
+      if (!group_done<Group>(ok, msg)) {
+        mode = M_DONE;
+        break;
+      }
       double d[1] = {0.0};
       for (int s = wid; s < R.nsl; s += kRW) {
         const int i = s * 32 + lane;
@@ -181,12 +207,13 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
         }
       }
       double t[1];
-      cluster_sum<1>(grp, d, part, wsum, t);
+      ok = group_sum<1>(grp, d, part, wsum, t);
       if (wid == 0) {
         const double rrt = t[0];
         ++repl;
         conv = (!(rrt > 0.0) && finite(rrt)) || rrt <= tol * bn2;
-        if (conv || !finite(rrt) || it >= maxit || (!IR && repl > 50)) {
+        conv = conv && ok;
+        if (conv || !ok || !finite(rrt) || it >= maxit || (!IR && repl > 50)) {
           mode = M_DONE;
         } else {
           // FP32: keep the direction unless the recurrence broke down or its
@@ -219,8 +246,12 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
         }
       }
       double t3[1];
-      cluster_sum<1>(grp, dz, part, wsum, t3);
+      ok = group_sum<1>(grp, dz, part, wsum, t3);
       if (wid == 0) rz = t3[0];
+      if (!group_done<Group>(ok, msg)) {
+        mode = M_DONE;
+        break;
+      }
       mode = M_CG;
       W.load(gp);  // the sum's barrier has made it visible
       keep = true;
@@ -233,7 +264,7 @@ __device__ __forceinline__ void batch_run(const BSys& S, ClusterGroup& grp, uint
     gr[r0 + i] = sr[i];
     if (mode == M_CG) gp[r0 + i] = keep ? sp[i] : axpy<T>(be, sp[i], sq[i]);
   }
-  if (grp.rank == 0 && tid == 0) {
+  if (rank == 0 && tid == 0) {
     S.sc[B_RZ] = rz;
     S.sc[B_RR] = rr;
     S.sc[B_PQ] = pq;
@@ -261,11 +292,11 @@ __global__ void __launch_bounds__(kRT, 1) batch_run_k(const BSys* __restrict__ s
   __syncthreads();
   if (S.st[I_MODE] == M_CG) {
     if (S.A.d16) {
-      if (S.ms) batch_run<IR, true, true>(S, grp, smem, msg, iters);
-      else batch_run<IR, true, false>(S, grp, smem, msg, iters);
+      if (S.ms) batch_run<IR, true, true>(S, grp, grp.rank, smem, msg, iters);
+      else batch_run<IR, true, false>(S, grp, grp.rank, smem, msg, iters);
     } else {
-      if (S.ms) batch_run<IR, false, true>(S, grp, smem, msg, iters);
-      else batch_run<IR, false, false>(S, grp, smem, msg, iters);
+      if (S.ms) batch_run<IR, false, true>(S, grp, grp.rank, smem, msg, iters);
+      else batch_run<IR, false, false>(S, grp, grp.rank, smem, msg, iters);
     }
   }
   grp.arrive(0);  // no block leaves while another may still write its shared memory
@@ -319,7 +350,41 @@ int batch_run_launch(Ctx* c, cudaStream_t st, int ir, const BSys* sys, const int
   return ELFEL_OK;
 }
 
-// The descriptor and the start of one system's refinement (run_ir_cluster).
+// One system's refinement over the whole grid (matrix in shared memory).
+template <bool D16>
+__global__ void __launch_bounds__(kRT, 1) ir_grid_k(const IrOne* __restrict__ one, RunGroup rg, int iters) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ GridGroup::Shared gsh;
+  __shared__ RunMsg msg;
+  __shared__ BSys S;
+  GridGroup grp(rg, &gsh);
+  if (threadIdx.x < sizeof(BSys) / 8)
+    reinterpret_cast<uint64_t*>(&S)[threadIdx.x] = reinterpret_cast<const uint64_t*>(&one->sys)[threadIdx.x];
+  __syncthreads();
+  batch_run<true, D16, true>(S, grp, (int)blockIdx.x, smem, msg, iters);
+}
+
+static int ir_grid_launch(Ctx* c, SolverData* S, const RunPlan& P, const IrOne* one) {
+  auto k = S->A.d16 ? ir_grid_k<true> : ir_grid_k<false>;
+  ELFEL_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem));
+  ELFEL_CUDA(c, cudaMemsetAsync(S->run_bar.p, 0, 2 * sizeof(unsigned), c->stream));
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)P.blocks);
+  cfg.blockDim = dim3(kRT);
+  cfg.dynamicSmemBytes = P.smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const RunGroup rg{S->run_slots.p, S->run_bar.p};
+  ELFEL_CUDA(c, cudaLaunchKernelEx(&cfg, k, one, rg, (int)kRunIters));
+  return ELFEL_OK;
+}
+
+// The descriptor and the start of one system's refinement (run_ir).
 __global__ void ir_start_k(IrOne* one, BSys d, const double* scal, double tol2, double delta, double scale, double bn2,
                            int maxit) {
   const int t = threadIdx.x;
@@ -340,7 +405,7 @@ __global__ void ir_start_k(IrOne* one, BSys d, const double* scal, double tol2, 
   }
 }
 
-int run_ir_cluster(Ctx* c, SolverData* S, const RunPlan& P, const int4* win, double tol2, double delta, double scale,
+int run_ir(Ctx* c, SolverData* S, const RunPlan& P, const int4* win, double tol2, double delta, double scale,
                    double bn2, int maxit, IrResult* out) {
   if (!S->ir_one.p) ELFEL_TRY(S->ir_one.alloc(c, sizeof(IrOne)));
   IrOne* one = reinterpret_cast<IrOne*>(S->ir_one.p);
@@ -368,8 +433,15 @@ int run_ir_cluster(Ctx* c, SolverData* S, const RunPlan& P, const int4* win, dou
   ELFEL_LAUNCH_CHECK(c);
   int st[I_COUNT];
   do {
-    ELFEL_TRY(batch_run_launch(c, c->stream, 1, &one->sys, &one->list, 1, P.blocks, P.smem, kRunIters));
-    ELFEL_TRY(read_back(c, c->stream, {{st, one->st, sizeof(st)}}));
+    unsigned bar[2] = {0, 0};
+    if (P.cluster) {
+      ELFEL_TRY(batch_run_launch(c, c->stream, 1, &one->sys, &one->list, 1, P.blocks, P.smem, kRunIters));
+      ELFEL_TRY(read_back(c, c->stream, {{st, one->st, sizeof(st)}}));
+    } else {
+      ELFEL_TRY(ir_grid_launch(c, S, P, one));
+      ELFEL_TRY(read_back(c, c->stream, {{st, one->st, sizeof(st)}, {bar, S->run_bar.p, sizeof(bar)}}));
+    }
+    if (bar[1]) return fail(c, ELFEL_ERR_TIMEOUT, "solve: a barrier of the iteration kernel timed out");
   } while (st[I_MODE] == M_CG);
   out->iterations = st[I_ITER];
   out->replacements = st[I_REPL];

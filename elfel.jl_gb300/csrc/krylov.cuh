@@ -102,16 +102,18 @@ int run_mr64(Ctx* c, SolverData* S, const RunPlan& P, double* x, double* z, doub
 int run_mr32(Ctx* c, SolverData* S, const RunPlan& P, float* x, float* z, float* vj, float* vjm, float* wj,
              float* wjm);
 
-// The FP32 refinement of a system with a cluster plan whose matrix and row sums
-// are in shared memory, to its end (batch_run.cu): the FP64 residual replacements
-// happen inside the kernel, where a host round trip each took 55 us (12 x 12 T3 elements,
-// 11 replacements: a solve 904 -> 408 us; 64 x 64: 2171 -> 1636).  The start is that of run_cg32 (x = 0, r, z, p, S_RZ).
-// Leaves x64, and r64 = b - K x64 of the last replacement.
+// The FP32 refinement of a system with a window whose matrix and row sums are in
+// shared memory, to its end (batch_run.cu): the FP64 residual replacements happen
+// inside the kernel, where a host round trip each took 55 us (a solve with
+// 12 x 12 T3 elements, 11 replacements: 904 -> 408 us; 64 x 64: 2171 -> 1636; over the
+// grid T4 40 x 40 x 40 2762 -> 2279).  A matrix from L2 stays with run_cg32: 808,000 unknowns
+// took 90.3 ms here, 88.7 there.  The start is that of run_cg32 (x = 0, r, z, p,
+// S_RZ).  Leaves x64, and r64 = b - K x64 of the last replacement.
 struct IrResult {
   int iterations, replacements, converged;
 };
 const int4* run_windows(const SolverData* S, const RunPlan& P);
-int run_ir_cluster(Ctx* c, SolverData* S, const RunPlan& P, const int4* win, double tol2, double delta, double scale,
+int run_ir(Ctx* c, SolverData* S, const RunPlan& P, const int4* win, double tol2, double delta, double scale,
                    double bn2, int maxit, IrResult* out);
 
 }  // namespace elfel

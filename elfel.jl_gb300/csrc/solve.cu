@@ -1289,9 +1289,9 @@ static int run_pcg32(elfel_sysmat* m, double bn2, double delta, double rtol, int
   int refinements = 0, late = 0;
   int launches = 0;
   double hsc[S_COUNT];
-  if (run.blocks && run.cluster && run.window && run.ms && run.vecs == 5) {
+  if (run.blocks && run.window && run.vecs == 5 && run.ms) {
     IrResult ir;
-    ELFEL_TRY(run_ir_cluster(c, S, run, run_windows(S, run), rtol * rtol, delta, s, bn2, maxit, &ir));
+    ELFEL_TRY(run_ir(c, S, run, run_windows(S, run), rtol * rtol, delta, s, bn2, maxit, &ir));
     hf[F_ITER] = ir.iterations;
     refinements = ir.replacements;
     bool all = false;

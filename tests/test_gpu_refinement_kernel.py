@@ -1,4 +1,4 @@
-"""The FP32 refinement of small systems with its residual replacements inside the cluster kernel (run_ir_cluster) (GPU).
+"""The FP32 refinement with its residual replacements inside the iteration kernel, cluster and grid (run_ir) (GPU).
 
 Against the graphs of three kernels with the replacements on the host
 (ELFEL_ONE_LAUNCH=0): both stop at a relative residual of 1e-10, so with
@@ -18,7 +18,7 @@ def laplacian(n):
     return (sp.identity(m * m) + sp.kron(sp.identity(m), L) + sp.kron(L, sp.identity(m))).tocsr()[:n, :n].tocsc()
 
 
-@pytest.mark.parametrize("n", [1, 32, 33, 257, 1025, 8193, 32768])
+@pytest.mark.parametrize("n", [1, 32, 33, 257, 1025, 8193, 32768, 32769, 70001, 400000])
 @pytest.mark.parametrize("scale", [1.0, 1e-30, 1e25])
 def test_against_graphs(E, gpu, monkeypatch, n, scale):
     A = laplacian(n)
