@@ -466,7 +466,9 @@ template <int NN, int NT, int PAT>
 __device__ __forceinline__ void heat_elems(int64_t e0, int64_t nel, const int32_t* __restrict__ conn,
                                            const double2* __restrict__ xy, const double* __restrict__ kappa, double Q,
                                            const uint8_t* __restrict__ straight, const QPTab& tab,
-                                           double* __restrict__ kstore, double* __restrict__ fstore) {
+                                           double* __restrict__ kstore, double* __restrict__ fstore,
+                                           double* __restrict__ keep) {
+  const double kap = e0 + threadIdx.x < nel ? __ldcs(kappa + e0 + threadIdx.x) : 0.0;  // first: HostCoef
   constexpr int NS = NN * (NN + 1) / 2;
   constexpr int LD = NT + 1;
   extern __shared__ double acc[];  // (NS + NN) * LD
@@ -481,7 +483,7 @@ __device__ __forceinline__ void heat_elems(int64_t e0, int64_t nel, const int32_
   const int64_t e = e0 + t;
   double* fa = acc + NS * LD;
   if (e < nel) {
-    const double kap = kappa[e];
+    if (keep) keep[e] = kap;
     if (NN == 3 || straight[e]) {
       straight_record<NN, LD, PAT>(g.x[0], g.y[0], g.x[1], g.y[1], g.x[2], g.y[2], kap, Q, sS, tab, acc, fa, t);
     } else {
@@ -677,9 +679,9 @@ __global__ void __launch_bounds__(kIntThreads) heat_k(int64_t nel, const int32_t
                                                      const double2* __restrict__ xy, const double* __restrict__ kappa,
                                                      double Q, const uint8_t* __restrict__ straight,
                                                      const __grid_constant__ QPTab tab, double* __restrict__ kstore,
-                                                     double* __restrict__ fstore) {
+                                                     double* __restrict__ fstore, double* __restrict__ keep) {
   heat_elems<NN, kIntThreads, PAT>((int64_t)blockIdx.x * kIntThreads, nel, conn, xy, kappa, Q, straight, tab, kstore,
-                                   fstore);
+                                   fstore, keep);
 }
 
 // Many meshes in one launch: CTA b works on mesh k with jobs[k].blk0 <= b <
@@ -694,7 +696,7 @@ __global__ void __launch_bounds__(NT) heat_batch_k(const HeatJob* __restrict__ j
   }
   const HeatJob J = jobs[lo];
   heat_elems<NN, NT, PAT>(((int64_t)blockIdx.x - J.blk0) * NT, J.nel, J.conn, (const double2*)J.xy, J.kappa, J.Q,
-                          J.straight, tab, J.kstore, J.fstore);
+                          J.straight, tab, J.kstore, J.fstore, nullptr);
 }
 
 static size_t heat_smem(int nn, int nt) { return (size_t)(nn == 3 ? 6 + 3 : 21 + 6) * (nt + 1) * sizeof(double); }
@@ -818,22 +820,30 @@ int launch_heat(Ctx* c, int nn, int64_t nel, const int32_t* conn, const double* 
     ELFEL_LAUNCH_CHECK(c);
     return ELFEL_OK;
   }
-  ELFEL_TRY(copy_coef(c, host, nel, kappa));
-  if (nn == 3)
-    heat_k<3, kPatGeneric><<<grid, kIntThreads, sm, c->stream>>>(nel, conn, p, kappa, Q, straight, tab, kstore, fstore);
-  else if (ncurved == 0 && pat == kPatT6R)
-    heat_t6s_k<kPatT6R><<<grid, kIntThreads, 11 * (kIntThreads + 1) * sizeof(double), c->stream>>>(
-        nel, conn, p, kappa, Q, tab, kstore, fstore);
-  else if (ncurved == 0 && pat == kPatT6)
-    heat_t6s_k<kPatT6><<<grid, kIntThreads, sm, c->stream>>>(nel, conn, p, kappa, Q, tab, kstore, fstore);
-  else if (ncurved == 0)
-    heat_t6s_k<kPatGeneric><<<grid, kIntThreads, sm, c->stream>>>(nel, conn, p, kappa, Q, tab, kstore, fstore);
-  else if (pat == kPatT6R)
-    heat_k<6, kPatT6R><<<grid, kIntThreads, sm, c->stream>>>(nel, conn, p, kappa, Q, straight, tab, kstore, fstore);
-  else if (pat == kPatT6)
-    heat_k<6, kPatT6><<<grid, kIntThreads, sm, c->stream>>>(nel, conn, p, kappa, Q, straight, tab, kstore, fstore);
-  else
-    heat_k<6, kPatGeneric><<<grid, kIntThreads, sm, c->stream>>>(nel, conn, p, kappa, Q, straight, tab, kstore, fstore);
+  // heat_k reads the host's conductivities itself, the straight-only T6 kernel without
+  // the load vector in place does not
+  const double* kin = host.p ? host.p : kappa;
+  double* keep = host.p ? kappa : nullptr;
+  if (nn == 3) {
+    heat_k<3, kPatGeneric><<<grid, kIntThreads, sm, c->stream>>>(nel, conn, p, kin, Q, straight, tab, kstore, fstore,
+                                                                keep);
+  } else if (ncurved == 0) {
+    ELFEL_TRY(copy_coef(c, host, nel, kappa));
+    if (pat == kPatT6R)
+      heat_t6s_k<kPatT6R><<<grid, kIntThreads, 11 * (kIntThreads + 1) * sizeof(double), c->stream>>>(
+          nel, conn, p, kappa, Q, tab, kstore, fstore);
+    else if (pat == kPatT6)
+      heat_t6s_k<kPatT6><<<grid, kIntThreads, sm, c->stream>>>(nel, conn, p, kappa, Q, tab, kstore, fstore);
+    else
+      heat_t6s_k<kPatGeneric><<<grid, kIntThreads, sm, c->stream>>>(nel, conn, p, kappa, Q, tab, kstore, fstore);
+  } else if (pat == kPatT6R) {
+    heat_k<6, kPatT6R><<<grid, kIntThreads, sm, c->stream>>>(nel, conn, p, kin, Q, straight, tab, kstore, fstore, keep);
+  } else if (pat == kPatT6) {
+    heat_k<6, kPatT6><<<grid, kIntThreads, sm, c->stream>>>(nel, conn, p, kin, Q, straight, tab, kstore, fstore, keep);
+  } else {
+    heat_k<6, kPatGeneric><<<grid, kIntThreads, sm, c->stream>>>(nel, conn, p, kin, Q, straight, tab, kstore, fstore,
+                                                                keep);
+  }
   ELFEL_LAUNCH_CHECK(c);
   return ELFEL_OK;
 }
@@ -1071,16 +1081,19 @@ __global__ void __launch_bounds__(kIntThreads) heat_t4_k(int64_t nel, const int3
                                                         const double* __restrict__ xyz,
                                                         const double* __restrict__ kappa, double Q,
                                                         const __grid_constant__ ShapeTab tab,
-                                                        double* __restrict__ kstore, double* __restrict__ fstore) {
+                                                        double* __restrict__ kstore, double* __restrict__ fstore,
+                                                        double* __restrict__ keep) {
   constexpr int NT = kIntThreads, LD = NT + 1;
   __shared__ double acc[(kShapeNS + 4) * LD];
   __shared__ int32_t sconn[NT * 4];
   const int64_t e0 = (int64_t)blockIdx.x * NT;
+  const double kap = e0 + threadIdx.x < nel ? __ldcs(kappa + e0 + threadIdx.x) : 0.0;  // first: HostCoef
   load_conn4<NT>(conn, e0, nel, sconn);
   const int t = threadIdx.x;
   const int64_t e = e0 + t;
   double* fa = acc + kShapeNS * LD;
   if (e < nel) {
+    if (keep) keep[e] = kap;
     double X[4][3];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -1108,7 +1121,7 @@ __global__ void __launch_bounds__(kIntThreads) heat_t4_k(int64_t nel, const int3
 #pragma unroll
     for (int k = 0; k < 3; ++k) A[0][k] = -(A[1][k] + A[2][k] + A[3][k]);
     const double det = d[0][0] * A[1][0] + d[0][1] * A[1][1] + d[0][2] * A[1][2];
-    const double c = kappa[e] * tab.W / det;
+    const double c = kap * tab.W / det;
     const double qd = Q * det;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -1127,16 +1140,17 @@ int launch_heat_shape(Ctx* c, const ShapeTab& tab, int64_t nel, const int32_t* c
                       double* kappa, double Q, double* kstore, double* fstore, HostCoef host) {
   if (nel == 0) return ELFEL_OK;
   const unsigned grid = grid_for(nel, kIntThreads);
-  const bool gauss2 = tab.shape == ELFEL_SHAPE_Q4 && tab.gauss2;
-  if (!gauss2) ELFEL_TRY(copy_coef(c, host, nel, kappa));
-  if (gauss2)
-    heat_q4_gauss2_k<<<grid, kIntThreads, 0, c->stream>>>(nel, conn, (const double2*)xy, host.p ? host.p : kappa, Q,
-                                                          tab.g, tab.w[0], kstore, fstore, host.p ? kappa : nullptr);
-  else if (tab.shape == ELFEL_SHAPE_Q4)
+  const double* kin = host.p ? host.p : kappa;
+  double* keep = host.p ? kappa : nullptr;
+  if (tab.shape == ELFEL_SHAPE_Q4 && tab.gauss2) {
+    heat_q4_gauss2_k<<<grid, kIntThreads, 0, c->stream>>>(nel, conn, (const double2*)xy, kin, Q, tab.g, tab.w[0], kstore,
+                                                          fstore, keep);
+  } else if (tab.shape == ELFEL_SHAPE_Q4) {
+    ELFEL_TRY(copy_coef(c, host, nel, kappa));
     heat_q4_k<<<grid, kIntThreads, 0, c->stream>>>(nel, conn, (const double2*)xy, kappa, Q, tab, kstore, fstore);
-  else if (tab.shape == ELFEL_SHAPE_T4)
-    heat_t4_k<<<grid, kIntThreads, 0, c->stream>>>(nel, conn, xy, kappa, Q, tab, kstore, fstore);
-  else
+  } else if (tab.shape == ELFEL_SHAPE_T4) {
+    heat_t4_k<<<grid, kIntThreads, 0, c->stream>>>(nel, conn, xy, kin, Q, tab, kstore, fstore, keep);
+  } else
     return fail(c, ELFEL_ERR_ARG, "heat: unknown element shape %d", tab.shape);
   ELFEL_LAUNCH_CHECK(c);
   return ELFEL_OK;

@@ -34,8 +34,8 @@ int make_tables(int nn, int npts, const double* pc, const double* w, QPTab* t);
 // Conductivities that a kernel reads from the caller's page-locked array itself
 // (p, a device address) while it integrates, instead of a copy before it; it leaves
 // them in kappa as that copy would.  Kernels without this form get the copy.
-// Re-assembly to host CSC, 2M T6 elements: 2335 -> 2279 us, 491,000 Q4: 444 -> 425;
-// 500,000 T6 from tables to CSC 1717 -> 1593.  (The body forces of plane elasticity, two
+// Re-assembly to host CSC, 2M T6 elements: 2335 -> 2279 us, 491,000 Q4: 444 -> 425, 2M T3
+// 683 -> 608, 750,000 T4 365 -> 336; 500,000 T6 from tables to CSC 1717 -> 1593.  (The body forces of plane elasticity, two
 // per element, are copied: read by the kernel 250,000 elements took 1177 us, not 1167.)
 struct HostCoef {
   const double* p = nullptr;

@@ -25,15 +25,20 @@ def system(E, kind, n):
     if kind == "elasticity":
         mesh, fesp, _, _ = elasticity_setup(E, n, max(1, n // 2))
         return mesh, fesp, {"npts": 3}
-    block = {"Q4": E.Q4block, "T3": E.T3block}.get(kind, E.T6block)
-    fe = {"Q4": E.FEH1_Q4, "T3": E.FEH1_T3}.get(kind, E.FEH1_T6)
+    if kind == "T4":
+        mesh = E.T4block(1.0, 1.0, 1.0, *(min(n, 20),) * 3)
+        fesp = E.FESpace(float, mesh, E.FEH1_T4())
+        E.numberdofs(fesp)
+        return mesh, fesp, {"npts": 1}
+    block = {"Q4": E.Q4block, "Q4x": E.Q4block, "T3": E.T3block}.get(kind, E.T6block)
+    fe = {"Q4": E.FEH1_Q4, "Q4x": E.FEH1_Q4, "T3": E.FEH1_T3}.get(kind, E.FEH1_T6)
     mesh = block(1.0, 1.0, n, n)
     if kind == "curved":  # one midside node off its edge
         mesh.xy[mesh.conn[0, 4] - 1] += 0.01 / n
-    return mesh, heat_space(E, mesh, fe()), {"kind": "Gauss", "order": 2} if kind == "Q4" else {"npts": 3}
+    return mesh, heat_space(E, mesh, fe()), {"kind": "Gauss", "order": 3 if kind == "Q4x" else 2} if kind[0] == "Q" else {"npts": 3}
 
 
-@pytest.mark.parametrize("kind", ["T6", "curved", "Q4", "T3", "elasticity"])
+@pytest.mark.parametrize("kind", ["T6", "curved", "Q4", "Q4x", "T3", "T4", "elasticity"])
 @pytest.mark.parametrize("n", [1, 8, 33, 130])
 @pytest.mark.parametrize("offset", [0, 1])
 def test_same_bits(E, gpu, kind, n, offset):
