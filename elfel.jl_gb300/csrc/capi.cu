@@ -12,19 +12,11 @@ using namespace elfel;
 
 namespace elfel {
 
-// Dense vector from a vector pattern: out[c] = 0 + the contributions of column c
-// in slot order, as SysvecAssembler adds element vectors into a zeroed vector
-// (Assemblers.jl:194-207; the leading +0 turns a sum of negative zeros into
-// +0, as there).
+// Dense vector from a vector pattern.
 __global__ void reduce_vector_k(const int32_t* __restrict__ cptr, const int32_t* __restrict__ contrib,
                                 const double* __restrict__ store, int64_t n, double* __restrict__ out) {
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t b = cptr[c], e = cptr[c + 1];
-    double s = 0.0;
-    if (b < e) s = __dadd_rn(0.0, store[contrib[b]]);
-    for (int32_t t = b + 1; t < e; ++t) s += store[contrib[t]];
-    out[c] = s;
-  }
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x)
+    out[c] = reduce_entry(cptr, contrib, store, c);
 }
 
 // *many = 1 when some DOF is a midside node (local nodes 3..5) of more than
@@ -923,20 +915,28 @@ static int head_of(elfel_sysmat* m, Head** h) {
   return ELFEL_OK;
 }
 
-// rhs_done: the integration kernel already added the load vector into rhs.
-static int finish_values(elfel_sysmat* m, bool rhs_done = false) {
+// K values and (fp, from fstore to out) a vector; together in one launch where
+// reduce_values does that, apart when phases are timed.
+static int reduce_both(elfel_sysmat* m, const Pattern* fp, const double* fstore, double* out, const char* name) {
   Ctx* c = &m->h->c;
+  VecRed v;
+  if (fp && !c->profiling) v = VecRed{fp->cptr.p, fp->contrib.p, fstore, fp->ncol, out};
   {
     Head* head;
     ELFEL_TRY(head_of(m, &head));
     Phase ph(c, "reduce_K");
-    ELFEL_TRY(reduce_values(c, m->P, m->F.kstore.p, m->vals.p, head));
+    ELFEL_TRY(reduce_values(c, m->P, m->F.kstore.p, m->vals.p, head, &v));
   }
-  if (!rhs_done) {
-    ELFEL_TRY(ensure_fpat(m));
-    Phase ph(c, "reduce_F");
-    ELFEL_TRY(reduce_dense(c, m->F.fpat, m->F.fstore.p, m->rhs.p));
-  }
+  if (!fp || (!c->profiling && v.n == 0)) return ELFEL_OK;
+  Phase ph(c, name);
+  return reduce_dense(c, *fp, fstore, out);
+}
+
+// rhs_done: the integration kernel already added the load vector into rhs.
+static int finish_values(elfel_sysmat* m, bool rhs_done = false) {
+  Fused& F = m->F;
+  if (!rhs_done) ELFEL_TRY(ensure_fpat(m));
+  ELFEL_TRY(reduce_both(m, rhs_done ? nullptr : &F.fpat, F.fstore.p, m->rhs.p, "reduce_F"));
   m->has_rhs = 1;
   m->finished = 1;
   m->values_version++;
@@ -1102,14 +1102,8 @@ extern "C" int elfel_fused_stokes(elfel_sysmat* m, double mu) {
     Phase ph(c, "integrate_stokes");
     ELFEL_TRY(launch_stokes(c, F.nel, F.conn_u.p, F.xy_u.p, mu, F.ncurved, F.tab, F.kstore.p, F.pmass_store.p));
   }
-  {
-    Head* head;
-    ELFEL_TRY(head_of(m, &head));
-    Phase ph(c, "reduce_K");
-    ELFEL_TRY(reduce_values(c, m->P, F.kstore.p, m->vals.p, head));
-  }
+  ELFEL_TRY(reduce_both(m, &F.pmpat, F.pmass_store.p, F.pmass_diag.p, "reduce_pmass"));
   ELFEL_CUDA(c, cudaMemsetAsync(m->rhs.p, 0, sizeof(double) * m->nrow, c->stream));
-  ELFEL_TRY(reduce_dense(c, F.pmpat, F.pmass_store.p, F.pmass_diag.p));
   m->has_rhs = 1;
   m->finished = 1;
   m->values_version++;

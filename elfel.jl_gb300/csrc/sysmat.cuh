@@ -279,8 +279,30 @@ struct Head {
   int64_t nnz = 0;  // nonzeros complete at ev (0: none was reduced apart)
 };
 
+// A vector to reduce beside a pattern's values (reduce_dense of pattern P).
+struct VecRed {
+  const int32_t* cptr = nullptr;
+  const int32_t* contrib = nullptr;
+  const double* store = nullptr;
+  int64_t n = 0;
+  double* out = nullptr;
+};
+// Entry k of a vector: 0 + its contributions in slot order, as SysvecAssembler
+// adds element vectors into a zeroed vector (Assemblers.jl:194-207; the leading
+// +0 turns a sum of negative zeros into +0, as there).
+__device__ __forceinline__ double reduce_entry(const int32_t* __restrict__ cptr, const int32_t* __restrict__ contrib,
+                                               const double* __restrict__ store, int64_t k) {
+  const int32_t b = cptr[k], e = cptr[k + 1];
+  double s = 0.0;
+  if (b < e) s = __dadd_rn(0.0, store[contrib[b]]);
+  for (int32_t t = b + 1; t < e; ++t) s += store[contrib[t]];
+  return s;
+}
+
 // vals_out[k] = sum of store[contrib[t]] over t in [cptr[k], cptr[k+1]), in order.
-int reduce_values(Ctx* c, Pattern& P, const double* store, double* vals_out, Head* head = nullptr);
+// vec: a vector that may go with the same launch (its n is 0 afterwards if it did).
+int reduce_values(Ctx* c, Pattern& P, const double* store, double* vals_out, Head* head = nullptr,
+                  VecRed* vec = nullptr);
 // Dense vector of a 1 x n pattern (the rhs): out[c] = contributions of column c.
 int reduce_dense(Ctx* c, const Pattern& P, const double* store, double* out);
 
