@@ -166,6 +166,13 @@ inline unsigned grid_for(int64_t n, int block, int64_t cap = 0) {
   return (unsigned)g;
 }
 
+// Programmatic dependent launch: a kernel lets the next one of its stream start
+// (its blocks' prologues) once all its blocks run; that one, launched with the
+// attribute, waits for the end of the first before it reads what it wrote.  Without
+// the attribute both do nothing.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ------------------------------------------------------------------ scan
 // Exclusive prefix sum of n int64 values in place: out[i] = sum_{j<i} in[j],
 // writes the total to out[n] (the buffer must hold n+1 entries).

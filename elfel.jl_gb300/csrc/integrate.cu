@@ -680,6 +680,7 @@ __global__ void __launch_bounds__(kIntThreads) heat_k(int64_t nel, const int32_t
                                                      double Q, const uint8_t* __restrict__ straight,
                                                      const __grid_constant__ QPTab tab, double* __restrict__ kstore,
                                                      double* __restrict__ fstore, double* __restrict__ keep) {
+  let_next_start();
   heat_elems<NN, kIntThreads, PAT>((int64_t)blockIdx.x * kIntThreads, nel, conn, xy, kappa, Q, straight, tab, kstore,
                                    fstore, keep);
 }
@@ -719,6 +720,7 @@ __global__ void __launch_bounds__(kIntThreads) heat_t6_bases_k(int64_t nel, cons
                                                               double* __restrict__ bases,
                                                               const int32_t* __restrict__ dofs,
                                                               double* __restrict__ fglob, double* __restrict__ keep) {
+  let_next_start();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (e >= nel) return;
@@ -1006,6 +1008,7 @@ __global__ void __launch_bounds__(kIntThreads) heat_q4_gauss2_k(int64_t nel, con
                                                                double w, double* __restrict__ kstore,
                                                                double* __restrict__ fstore,
                                                                double* __restrict__ keep) {
+  let_next_start();
   constexpr int NT = kIntThreads, LD = NT + 1;
   __shared__ double acc[(kShapeNS + 4) * LD];
   __shared__ int32_t sconn[NT * 4];
@@ -1083,6 +1086,7 @@ __global__ void __launch_bounds__(kIntThreads) heat_t4_k(int64_t nel, const int3
                                                         const __grid_constant__ ShapeTab tab,
                                                         double* __restrict__ kstore, double* __restrict__ fstore,
                                                         double* __restrict__ keep) {
+  let_next_start();
   constexpr int NT = kIntThreads, LD = NT + 1;
   __shared__ double acc[(kShapeNS + 4) * LD];
   __shared__ int32_t sconn[NT * 4];
@@ -1451,6 +1455,7 @@ __global__ void __launch_bounds__(kIntThreads) elast_t6_exact_k(int64_t nel, con
                                                                const double* __restrict__ bforce,
                                                                double* __restrict__ kstore,
                                                                double* __restrict__ fstore) {
+  let_next_start();
   constexpr int NS = 78, NT = kIntThreads, LD = NT + 1, NK = 13;
   __shared__ double acc[NK * LD];
   const int t = threadIdx.x;
@@ -1776,6 +1781,7 @@ __global__ void __launch_bounds__(kIntThreads) stokes_t6_exact_k(int64_t nel, co
                                                                 double Mp0, double Mp1, double Mp2,
                                                                 double* __restrict__ kstore,
                                                                 double* __restrict__ pmass) {
+  let_next_start();
   constexpr int NR = 114, NT = kIntThreads, LD = NT + 1, NK = 19;
   __shared__ double acc[NK * LD];
   const int t = threadIdx.x;
@@ -1846,12 +1852,7 @@ int launch_stokes(Ctx* c, int64_t nel, const int32_t* conn, const double* xy, do
     if (pat == kPatT6R && stokes_exact(tab)) {
       stokes_t6_exact_k<<<grid, kIntThreads, 0, c->stream>>>(nel, conn, (const double2*)xy, mu, tab.P[3], tab.Mp[0],
                                                              tab.Mp[1], tab.Mp[2], kstore, pmass);
-    } else if (pat == kPatT6R) {
-      ELFEL_CUDA(c, cudaFuncSetAttribute(stokes_straight_k<kPatT6R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)sm));
-      stokes_straight_k<kPatT6R><<<grid, kIntThreads, sm, c->stream>>>(nel, conn, (const double2*)xy, mu, tab,
-                                                                         kstore, pmass);
-    } else if (pat == kPatT6) {
+    } else if (pat != kPatGeneric) {
       ELFEL_CUDA(c, cudaFuncSetAttribute(stokes_straight_k<kPatT6>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)sm));
       stokes_straight_k<kPatT6><<<grid, kIntThreads, sm, c->stream>>>(nel, conn, (const double2*)xy, mu, tab,

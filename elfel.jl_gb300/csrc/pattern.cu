@@ -891,6 +891,7 @@ __global__ void reduce_k(const int32_t* __restrict__ cptr, const int32_t* __rest
 // however few of its lanes are active).  Each nonzero still adds its
 // contributions in slot order, and the window's values are written inside
 // its own 1 KB of the output.
+template <bool EARLY = false>
 __device__ __forceinline__ void reduce_windows(const int32_t* __restrict__ cptr, const int32_t* __restrict__ contrib,
                                                const uint8_t* __restrict__ perm, const double* __restrict__ store,
                                                int64_t nnz, double* __restrict__ out, unsigned blocks) {
@@ -914,6 +915,7 @@ __device__ __forceinline__ void reduce_windows(const int32_t* __restrict__ cptr,
         e[r] = cptr[base + j[r] + 1];
       }
     }
+    if (EARLY) wait_for_previous();
 #pragma unroll
     for (int r = 0; r < R; ++r) s[r] = b[r] < e[r] ? store[contrib[b[r]]] : 0.0;
 #pragma unroll
@@ -939,16 +941,21 @@ __global__ void __launch_bounds__(256) reduce_win_k(const int32_t* __restrict__ 
 // The same in the first `blocks` blocks, and a vector's entries (reduce_dense) in
 // the others: one launch instead of two for systems whose assembly is mostly
 // launches (re-assembly to the host: T3 12 x 12 47.2 -> 43.2 us, T4 4 x 4 x 4 49.8 -> 44.5, plane
-// elasticity 20 x 10 50.9 -> 48.1, Taylor-Hood 20 x 20 50.0 -> 45.7).
+// elasticity 20 x 10 50.9 -> 48.1, Taylor-Hood 20 x 20 50.0 -> 45.7).  EARLY: launched
+// beside the integration kernel, whose end is waited for after the first window's
+// lists are there (T3 12 x 12 43.8 -> 36.2 us, 60 x 60 46.2 -> 38.4; T4, Q4, elasticity and
+// Stokes 0 to 2 us less).
+template <bool EARLY>
 __global__ void __launch_bounds__(256) reduce_win_vec_k(const int32_t* __restrict__ cptr,
                                                        const int32_t* __restrict__ contrib,
                                                        const uint8_t* __restrict__ perm,
                                                        const double* __restrict__ store, int64_t nnz,
                                                        double* __restrict__ out, unsigned blocks, VecRed v) {
   if (blockIdx.x < blocks) {
-    reduce_windows(cptr, contrib, perm, store, nnz, out, blocks);
+    reduce_windows<EARLY>(cptr, contrib, perm, store, nnz, out, blocks);
     return;
   }
+  if (EARLY) wait_for_previous();
   const int64_t stride = (int64_t)(gridDim.x - blocks) * blockDim.x;
   for (int64_t k = (int64_t)(blockIdx.x - blocks) * blockDim.x + threadIdx.x; k < v.n; k += stride)
     v.out[k] = reduce_entry(v.cptr, v.contrib, v.store, k);
@@ -993,6 +1000,7 @@ int reduce_values(Ctx* c, Pattern& P, const double* store, double* vals_out, Hea
   // reduction on; a pattern reduced once (an end-to-end call) does without it.
   // Both kernels add every nonzero's contributions in slot order: same bits.
   // 1 x n patterns (vectors) are reduced by reduce_dense.
+  const bool ordered = P.perm.p != nullptr;  // the order is not being written by the launch before
   if (!P.perm.p && P.reductions >= 1 && P.nrow > 1) {
     const int64_t nwin = (P.nnz + kReduceWindow - 1) / kReduceWindow;
     ELFEL_TRY(P.perm.alloc(c, (size_t)(nwin * kReduceWindow)));
@@ -1020,8 +1028,20 @@ int reduce_values(Ctx* c, Pattern& P, const double* store, double* vals_out, Hea
     const int64_t nwin = (P.nnz + kReduceWindow - 1) / kReduceWindow;
     const unsigned gk = grid_for(nwin, 8, (int64_t)c->sm_count * 16);
     const unsigned gv = grid_for(vec->n, 256, (int64_t)c->sm_count * 16);
-    reduce_win_vec_k<<<gk + gv, 256, 0, c->stream>>>(P.cptr.p, P.contrib.p, P.perm.p, store, P.nnz, vals_out, gk, *vec);
-    ELFEL_LAUNCH_CHECK(c);
+    const bool early = ordered && P.nnz < kEarlyNnz;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(gk + gv);
+    cfg.blockDim = dim3(256);
+    cfg.stream = c->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = early ? 1 : 0;
+    ELFEL_CUDA(c, cudaLaunchKernelEx(&cfg, early ? reduce_win_vec_k<true> : reduce_win_vec_k<false>,
+                                     (const int32_t*)P.cptr.p, (const int32_t*)P.contrib.p, (const uint8_t*)P.perm.p,
+                                     store, P.nnz, vals_out, gk, *vec));
     vec->n = 0;
     return ELFEL_OK;
   }

@@ -274,6 +274,9 @@ int build_vector_pattern(Ctx* c, const SlotGen& g, int64_t ncol, Pattern* P);
 // whole reduction takes less than the extra launch saves.
 constexpr int64_t kHeadMinNnz = 1 << 22;
 inline int64_t values_head(int64_t nnz) { return nnz < kHeadMinNnz ? 0 : nnz / 8; }
+// Below this many nonzeros the reduction is launched while the integration still runs
+// (programmatic dependent launch) and waits for its end inside.
+constexpr int64_t kEarlyNnz = 1 << 18;
 struct Head {
   cudaEvent_t ev = nullptr;
   int64_t nnz = 0;  // nonzeros complete at ev (0: none was reduced apart)
