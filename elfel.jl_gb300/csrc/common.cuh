@@ -172,6 +172,20 @@ inline unsigned grid_for(int64_t n, int block, int64_t cap = 0) {
 // the attribute both do nothing.
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Loads of what the previous kernel wrote, by a kernel that started beside it: plain
+// ones, volatile so that they stay behind wait_for_previous().  The read-only path
+// (__ldg, const __restrict__) is for data that does not change while the kernel runs, and
+// its loads may be moved above the wait.
+__device__ __forceinline__ double load_after_wait(const double* p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double2 load_after_wait(const double2* p) {
+  double2 v;
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
 
 // ------------------------------------------------------------------ scan
 // Exclusive prefix sum of n int64 values in place: out[i] = sum_{j<i} in[j],

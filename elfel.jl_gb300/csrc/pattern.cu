@@ -893,7 +893,7 @@ __global__ void reduce_k(const int32_t* __restrict__ cptr, const int32_t* __rest
 // its own 1 KB of the output.
 template <bool EARLY = false>
 __device__ __forceinline__ void reduce_windows(const int32_t* __restrict__ cptr, const int32_t* __restrict__ contrib,
-                                               const uint8_t* __restrict__ perm, const double* __restrict__ store,
+                                               const uint8_t* __restrict__ perm, const double* store,
                                                int64_t nnz, double* __restrict__ out, unsigned blocks) {
   constexpr int R = kReduceWindow / 32;
   const int lane = threadIdx.x & 31;
@@ -917,13 +917,13 @@ __device__ __forceinline__ void reduce_windows(const int32_t* __restrict__ cptr,
     }
     if (EARLY) wait_for_previous();
 #pragma unroll
-    for (int r = 0; r < R; ++r) s[r] = b[r] < e[r] ? store[contrib[b[r]]] : 0.0;
+    for (int r = 0; r < R; ++r) s[r] = b[r] < e[r] ? stored<EARLY>(store + contrib[b[r]]) : 0.0;
 #pragma unroll
     for (int r = 0; r < R; ++r)
-      if (b[r] + 1 < e[r]) s[r] += store[contrib[b[r] + 1]];
+      if (b[r] + 1 < e[r]) s[r] += stored<EARLY>(store + contrib[b[r] + 1]);
 #pragma unroll
     for (int r = 0; r < R; ++r)
-      for (int32_t t = b[r] + 2; t < e[r]; ++t) s[r] += store[contrib[t]];
+      for (int32_t t = b[r] + 2; t < e[r]; ++t) s[r] += stored<EARLY>(store + contrib[t]);
 #pragma unroll
     for (int r = 0; r < R; ++r)
       if (j[r] < n) out[base + j[r]] = s[r];
@@ -949,8 +949,8 @@ template <bool EARLY>
 __global__ void __launch_bounds__(256) reduce_win_vec_k(const int32_t* __restrict__ cptr,
                                                        const int32_t* __restrict__ contrib,
                                                        const uint8_t* __restrict__ perm,
-                                                       const double* __restrict__ store, int64_t nnz,
-                                                       double* __restrict__ out, unsigned blocks, VecRed v) {
+                                                       const double* store, int64_t nnz, double* __restrict__ out,
+                                                       unsigned blocks, VecRed v) {
   if (blockIdx.x < blocks) {
     reduce_windows<EARLY>(cptr, contrib, perm, store, nnz, out, blocks);
     return;
@@ -958,7 +958,7 @@ __global__ void __launch_bounds__(256) reduce_win_vec_k(const int32_t* __restric
   if (EARLY) wait_for_previous();
   const int64_t stride = (int64_t)(gridDim.x - blocks) * blockDim.x;
   for (int64_t k = (int64_t)(blockIdx.x - blocks) * blockDim.x + threadIdx.x; k < v.n; k += stride)
-    v.out[k] = reduce_entry(v.cptr, v.contrib, v.store, k);
+    v.out[k] = reduce_entry<EARLY>(v.cptr, v.contrib, v.store, k);
 }
 
 // Many reductions in one launch: CTA b serves job k with jobs[k].blk0 <= b <

@@ -290,15 +290,23 @@ struct VecRed {
   int64_t n = 0;
   double* out = nullptr;
 };
+// A value of the element records: by a kernel beside the one that writes them (EARLY) or after it.
+template <bool EARLY>
+__device__ __forceinline__ double stored(const double* p) {
+  return EARLY ? load_after_wait(p) : __ldg(p);
+}
+
 // Entry k of a vector: 0 + its contributions in slot order, as SysvecAssembler
 // adds element vectors into a zeroed vector (Assemblers.jl:194-207; the leading
 // +0 turns a sum of negative zeros into +0, as there).
+// EARLY: store belongs to the previous kernel, whose end has been waited for.
+template <bool EARLY = false>
 __device__ __forceinline__ double reduce_entry(const int32_t* __restrict__ cptr, const int32_t* __restrict__ contrib,
-                                               const double* __restrict__ store, int64_t k) {
+                                               const double* store, int64_t k) {
   const int32_t b = cptr[k], e = cptr[k + 1];
   double s = 0.0;
-  if (b < e) s = __dadd_rn(0.0, store[contrib[b]]);
-  for (int32_t t = b + 1; t < e; ++t) s += store[contrib[t]];
+  if (b < e) s = __dadd_rn(0.0, stored<EARLY>(store + contrib[b]));
+  for (int32_t t = b + 1; t < e; ++t) s += stored<EARLY>(store + contrib[t]);
   return s;
 }
 

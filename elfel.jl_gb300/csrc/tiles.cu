@@ -31,6 +31,7 @@
 // its own first nonzero and smallest element and the blob of its program,
 // which stays in L2.
 #include <algorithm>
+#include <type_traits>
 #include <unordered_map>
 #include <vector>
 
@@ -331,13 +332,15 @@ struct RecFull {
   __device__ __forceinline__ double value(uint32_t st) const { return __ldg(store + st); }
 };
 
-// The 8 bases of the exact-rational T6 record (64 bytes per element).
+// The 8 bases of the exact-rational T6 record (64 bytes per element).  EARLY: of the
+// previous kernel, whose end has been waited for.
+template <bool EARLY = false>
 struct RecT6R {
   const double* bases;
   __device__ __forceinline__ void load(int64_t e, double2 (&x)[4]) const {
     const double2* p = reinterpret_cast<const double2*>(bases + e * 8);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) x[k] = __ldg(p + k);
+    for (int k = 0; k < 4; ++k) x[k] = EARLY ? load_after_wait(p + k) : __ldg(p + k);
   }
   __device__ __forceinline__ static void expand(const double2 (&x)[4], double* v, int ld) {
     double b[8];
@@ -358,7 +361,7 @@ struct RecT6R {
     const uint32_t e = st / 21u, s = st - e * 21u;
     double b[8], v[kT6RTable];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) b[k] = __ldg(bases + (int64_t)e * 8 + k);
+    for (int k = 0; k < 8; ++k) b[k] = stored<EARLY>(bases + (int64_t)e * 8 + k);
     t6r_table(b, v);
     return v[t6r_entry((int)s)];
   }
@@ -453,7 +456,7 @@ __global__ void __launch_bounds__(kRunThreads) tile_run_k(const TileHdr* __restr
                                                           const int2* __restrict__ runs, int maxnel, int maxblob,
                                                           const uint8_t* __restrict__ blob,
                                                           const int32_t* __restrict__ cptr,
-                                                          const int32_t* __restrict__ contrib, RecT6R rec,
+                                                          const int32_t* __restrict__ contrib, RecT6R<EARLY> rec,
                                                           double* __restrict__ vals) {
   constexpr int RT = kRunThreads;
   extern __shared__ uint4 smq[];  // program (maxblob bytes) | value table | values
@@ -491,7 +494,7 @@ __global__ void __launch_bounds__(kRunThreads) tile_run_k(const TileHdr* __restr
   double* out = tbl + (size_t)maxnel * kT6RTable;
   int64_t p0 = H0.p0;
   for (int t = 0; t < run.y; ++t) {
-    if (mine) RecT6R::expand(x, tbl + threadIdx.x, nel);
+    if (mine) RecT6R<EARLY>::expand(x, tbl + threadIdx.x, nel);
     int64_t pn = 0;
     if (t + 1 < run.y) {
       const TileHdr* hn = hdr + run.x + t + 1;
@@ -744,24 +747,26 @@ static int tile_reduce_runs(Ctx* c, const Pattern& P, const double* bases, doubl
   if (r0 < 0 || nr < 0 || r0 + nr > T.nruns) return fail(c, ELFEL_ERR_ARG, "tile runs outside the plan");
   if (nr == 0) return ELFEL_OK;
   const size_t sm = tile_smem(T);
-  RecT6R r{bases};
-  auto k = early ? tile_run_k<true> : tile_run_k<false>;
-  ELFEL_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3((unsigned)nr);
-  cfg.blockDim = dim3(kRunThreads);
-  cfg.dynamicSmemBytes = sm;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = early ? 1 : 0;
-  ELFEL_CUDA(c, cudaLaunchKernelEx(&cfg, k, (const TileHdr*)T.hdr.p, (const int2*)(T.runs.p + r0), T.maxnel, T.maxblob,
-                                   (const uint8_t*)T.blob.p, (const int32_t*)P.cptr.p, (const int32_t*)P.contrib.p, r,
-                                   vals));
-  return ELFEL_OK;
+  auto launch = [&](auto e) -> int {
+    constexpr bool EARLY = decltype(e)::value;
+    ELFEL_CUDA(c, cudaFuncSetAttribute(tile_run_k<EARLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)nr);
+    cfg.blockDim = dim3(kRunThreads);
+    cfg.dynamicSmemBytes = sm;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = EARLY ? 1 : 0;
+    ELFEL_CUDA(c, cudaLaunchKernelEx(&cfg, tile_run_k<EARLY>, (const TileHdr*)T.hdr.p, (const int2*)(T.runs.p + r0),
+                                     T.maxnel, T.maxblob, (const uint8_t*)T.blob.p, (const int32_t*)P.cptr.p,
+                                     (const int32_t*)P.contrib.p, RecT6R<EARLY>{bases}, vals));
+    return ELFEL_OK;
+  };
+  return early ? launch(std::true_type{}) : launch(std::false_type{});
 }
 
 int tile_reduce(Ctx* c, const Pattern& P, const double* src, int t6r_bases, double* vals, Head* head) {
@@ -772,7 +777,7 @@ int tile_reduce(Ctx* c, const Pattern& P, const double* src, int t6r_bases, doub
   const size_t sm = tile_smem(T);
   if (t6r_bases) {
     if (T.V != kT6RTable || T.S != 21) return fail(c, ELFEL_ERR_STATE, "tile plan is not for T6 bases");
-    RecT6R r{src};
+    RecT6R<> r{src};
     if (tile_runs_ok(T)) {
       const int64_t r0 = head ? T.head_runs : 0;
       if (!r0)
@@ -786,8 +791,8 @@ int tile_reduce(Ctx* c, const Pattern& P, const double* src, int t6r_bases, doub
       head->nnz = T.head_nnz;
       return ELFEL_OK;
     }
-    ELFEL_CUDA(c, cudaFuncSetAttribute(tile_reduce_k<RecT6R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    tile_reduce_k<RecT6R><<<(unsigned)T.ntiles, kRT, sm, c->stream>>>(T.hdr.p, T.maxnel, T.V, T.maxblob, T.blob.p,
+    ELFEL_CUDA(c, cudaFuncSetAttribute(tile_reduce_k<RecT6R<>>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    tile_reduce_k<RecT6R<>><<<(unsigned)T.ntiles, kRT, sm, c->stream>>>(T.hdr.p, T.maxnel, T.V, T.maxblob, T.blob.p,
                                                                        P.cptr.p, P.contrib.p, r, vals);
   } else {
     if (T.V != T.S) return fail(c, ELFEL_ERR_STATE, "tile plan is not for full records");
