@@ -315,7 +315,8 @@ extern "C" int elfel_sysmat_csc(elfel_sysmat* m, int64_t* colptr, int64_t* rowva
     // the values of a pattern the caller has already: no index arrays are formed
     // (2M quadratic triangles: 0.12 ms of a 2.6 ms re-assembly and download)
     int pin_v = 0;
-    const int64_t head = nzval && host_device_ptr(c, nzval, &pin_v) && pin_v ? std::min(m->head.nnz, nnz) : 0;
+    const bool direct = nzval && host_device_ptr(c, nzval, &pin_v) && pin_v && c->stream == c->own_stream;
+    const int64_t head = direct ? std::min(m->head.nnz, nnz) : 0;
     if (head) {
       // the head of the values leaves on the auxiliary stream as soon as it is
       // reduced, the rest behind it once the context stream has come so far
@@ -907,10 +908,18 @@ int elfel::ensure_fpat(elfel_sysmat* m) {
   return ELFEL_OK;
 }
 
-// The head of the system's next reduction (its event is created once).
+// The head of the system's next reduction (its event is created once), or null: small
+// systems; a caller's stream, whose order with the caller's own work the
+// copy on the auxiliary stream would not keep; a stream that is being captured.
 static int head_of(elfel_sysmat* m, Head** h) {
-  if (!m->head.ev) ELFEL_CUDA(&m->h->c, cudaEventCreateWithFlags(&m->head.ev, cudaEventDisableTiming));
+  Ctx* c = &m->h->c;
+  *h = nullptr;
   m->head.nnz = 0;
+  if (m->P.nnz < kHeadMinNnz || c->stream != c->own_stream) return ELFEL_OK;
+  cudaStreamCaptureStatus cs;
+  ELFEL_CUDA(c, cudaStreamIsCapturing(c->stream, &cs));
+  if (cs != cudaStreamCaptureStatusNone) return ELFEL_OK;
+  if (!m->head.ev) ELFEL_CUDA(c, cudaEventCreateWithFlags(&m->head.ev, cudaEventDisableTiming));
   *h = &m->head;
   return ELFEL_OK;
 }
