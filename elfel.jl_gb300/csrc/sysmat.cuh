@@ -280,6 +280,7 @@ constexpr int64_t kEarlyNnz = 1 << 18;
 struct Head {
   cudaEvent_t ev = nullptr;
   int64_t nnz = 0;  // nonzeros complete at ev (0: none was reduced apart)
+  int kept = 0;     // assemblies with a head since the last download that could use it
 };
 
 // A vector to reduce beside a pattern's values (reduce_dense of pattern P).
