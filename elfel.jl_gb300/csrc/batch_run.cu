@@ -379,7 +379,7 @@ static int ir_grid_launch(Ctx* c, SolverData* S, const RunPlan& P, const IrOne* 
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  const RunGroup rg{S->run_slots.p, S->run_bar.p};
+  const RunGroup rg{S->run_slots.p, S->run_bar.p, c->run_spins};
   ELFEL_CUDA(c, cudaLaunchKernelEx(&cfg, k, one, rg, (int)kRunIters));
   return ELFEL_OK;
 }

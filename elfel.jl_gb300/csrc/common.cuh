@@ -48,6 +48,9 @@ struct Ctx {
   int tiles = 1;
   // one-launch Krylov iterations: on unless ELFEL_ONE_LAUNCH=0
   int one_launch = 1;
+  // their waits give up after this many polls, about a second (ELFEL_RUN_SPINS); the
+  // solve then starts again in graphs
+  unsigned run_spins = 1u << 22;
   // autotuner: on unless ELFEL_TUNE=0; one line per tuned key
   int tune = 1;
   std::vector<std::string> tune_lines;

@@ -233,6 +233,7 @@ extern "C" int elfel_ctx_create(int device, int64_t mem_budget_bytes, elfel_ctx*
   h->c.tiles = (ti && ti[0] == '0') ? 0 : 1;
   const char* ol = getenv("ELFEL_ONE_LAUNCH");
   h->c.one_launch = (ol && ol[0] == '0') ? 0 : 1;
+  if (const char* rs = getenv("ELFEL_RUN_SPINS")) h->c.run_spins = (unsigned)strtoul(rs, nullptr, 10);
   *out = h;
   return ELFEL_OK;
 }

@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(kRT, 1) mr_run_k(const MrRun<T> a, const RunGr
 
 template <class Args>
 int run_launch(Ctx* c, SolverData* S, const RunPlan& P, void (*k)(const Args, const RunGroup), const Args& a) {
-  RunGroup rg{S->run_slots.p, S->run_bar.p};
+  RunGroup rg{S->run_slots.p, S->run_bar.p, c->run_spins};
   ELFEL_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem));
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
@@ -490,7 +490,7 @@ int run_spb_batch(int64_t nslices, int elem) {
 
 RunPlan run_plan(Ctx* c, const SolverData* S, int elem, int vecs, int least_vecs, int split) {
   const Sell& A = S->A;
-  if (!c->one_launch || S->nu < 1 || !S->run_slots.p) return RunPlan();
+  if (!c->one_launch || S->graphs || S->nu < 1 || !S->run_slots.p) return RunPlan();
   // A cluster saves about 5000 cycles an iteration at its barriers and sums; in
   // FP64 its 16 SMs take half a cycle over 16 per multiply-add (entries, and
   // about 8 per row for the vectors), which makes that up at 180k of them.

@@ -33,6 +33,7 @@ struct ColType<false> {
 struct RunGroup {
   double* slots;
   unsigned* words;
+  unsigned spins;  // polls of the arrival counter before a wait gives up
 };
 
 // Blocks' column windows in SolverData::run_win: of the cluster division, the

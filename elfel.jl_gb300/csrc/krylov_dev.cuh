@@ -14,7 +14,6 @@ namespace cg = cooperative_groups;
 constexpr int kRT = kRunThreads;
 constexpr int kRW = kRT / 32;
 constexpr int kRunPart = 3 * kRT + 16;  // doubles of shared memory for the block sums
-constexpr unsigned kRunSpins = 1u << 22;  // polls of the arrival counter, about a second
 
 // Sums.  The FP64 unit of an SM sub-partition takes a warp instruction every
 // 64 cycles whatever its active lanes, so what a sum costs is the number of
@@ -147,7 +146,7 @@ struct GridGroup {
       for (;;) {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(g.words) : "memory");
         if ((int)(v - target) >= 0) break;
-        if (++spins > kRunSpins || ((spins & 1023u) == 0 && *(volatile unsigned*)(g.words + 1))) {
+        if (++spins > g.spins || ((spins & 1023u) == 0 && *(volatile unsigned*)(g.words + 1))) {
           atomicExch(g.words + 1, 1u);
           ok = 0;
           break;

@@ -1368,6 +1368,20 @@ static int run_mr(Ctx* c, SolverData* S, const RunPlan& P, float* x, float* cons
   return run_mr32(c, S, P, x, h[3], h[0], h[2], h[6], h[8]);
 }
 
+// run(), and once more in graphs when a wait of its one-launch iterations ran out:
+// their grid needs every SM at once, and another kernel may hold some for longer than the
+// limit; the graphs get along with the SMs there are.  (Every driver starts from b.)
+template <class F>
+static int or_in_graphs(Ctx* c, SolverData* S, F run) {
+  int rc = run();
+  if (rc == ELFEL_ERR_TIMEOUT && !S->graphs) {
+    if (c->trace) fprintf(stderr, "[elfel solve] a wait of the iteration kernel ran out: starting again in graphs\n");
+    S->graphs = 1;
+    rc = run();
+  }
+  return rc;
+}
+
 // MINRES on A x = b (precision T, permuted order).  dp, hp: the nine
 // three-term buffers (v, z, w) as a device and as a host table.
 template <typename T>
@@ -1440,15 +1454,16 @@ extern "C" int elfel_solve(elfel_sysmat* m, const double* Fh, double* T, int64_t
   ELFEL_TRY(set_scal(c, S, ScalSet().set(S_TOL2, rtol * rtol).set(S_RMAX, sqrt(bn2)).set(S_DELTA, delta)));
   int rc = ELFEL_OK;
   double rr = -1.0;
+  S->graphs = 0;
   if (bn2 == 0.0) {
     ELFEL_CUDA(c, cudaMemsetAsync(S->x64.p, 0, sizeof(double) * nu, c->stream));
     st.converged = 1;
   } else if (method == ELFEL_PCG64) {
     Phase ph(c, "pcg64");
-    rc = run_pcg64(m, rtol, maxit, &st, &rr);
+    rc = or_in_graphs(c, S, [&]() { return run_pcg64(m, rtol, maxit, &st, &(rr = -1.0)); });
   } else if (method == ELFEL_PCG32_IR) {
     Phase ph(c, "pcg32_ir");
-    rc = run_pcg32(m, bn2, delta, rtol, maxit, &st, &rr);
+    rc = or_in_graphs(c, S, [&]() { return run_pcg32(m, bn2, delta, rtol, maxit, &st, &(rr = -1.0)); });
   } else if (method == ELFEL_MINRES64) {
     Phase ph(c, "minres64");
     for (int i = 0; i < 3; ++i) {
@@ -1465,8 +1480,10 @@ extern "C" int elfel_solve(elfel_sysmat* m, const double* Fh, double* T, int64_t
       S->g_minres64 = nullptr;
     }
     int it = 0, conv = 0;
-    rc = run_minres<double>(c, S, S->A.v64.p, S->dinv64.p, S->b64.p, S->x64.p, dptr.p, hp, S->q64.p, rtol, maxit,
-                            &S->g_minres64, &it, &conv);
+    rc = or_in_graphs(c, S, [&]() {
+      return run_minres<double>(c, S, S->A.v64.p, S->dinv64.p, S->b64.p, S->x64.p, dptr.p, hp, S->q64.p, rtol, maxit,
+                                &S->g_minres64, &it, &conv);
+    });
     ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
     dptr.release(c);
     st.iterations = it;
@@ -1497,8 +1514,10 @@ extern "C" int elfel_solve(elfel_sysmat* m, const double* Fh, double* T, int64_t
       if (!(s > 0.0)) break;
       demote_k<<<vg, kBlk, 0, c->stream>>>(nu, S->r64.p, S->b32.p, 1.0 / s);
       int it = 0, conv = 0;
-      rc = run_minres<float>(c, S, S->A.v32.p, S->dinv32.p, S->b32.p, S->x32.p, dptr.p, hp, S->q32.p, inner_tol,
-                             maxit - total, &S->g_minres32, &it, &conv);
+      rc = or_in_graphs(c, S, [&]() {
+        return run_minres<float>(c, S, S->A.v32.p, S->dinv32.p, S->b32.p, S->x32.p, dptr.p, hp, S->q32.p, inner_tol,
+                                 maxit - total, &S->g_minres32, &it, &conv);
+      });
       if (rc != ELFEL_OK) break;
       total += it;
       ++outer;

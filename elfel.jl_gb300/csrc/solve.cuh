@@ -111,6 +111,7 @@ struct SolverData {
   DBuf<unsigned> run_bar;
   DBuf<int4> run_win;
   DBuf<unsigned char> ir_one;  // IrOne (first use)
+  int graphs = 0;  // a wait of the one-launch form ran out in this solve: it goes on in graphs
   cudaGraphExec_t g_pcg64 = nullptr, g_pcg32 = nullptr, g_minres64 = nullptr, g_minres32 = nullptr;
   SellView view() const {
     return SellView{A.nrows, A.nslices, A.sptr.p, A.sw.p, A.d16 ? A.dcol.p : nullptr, A.d16 ? nullptr : A.col.p};
