@@ -1044,10 +1044,9 @@ int batch_add_dev(elfel_batch* b, elfel_sysmat* m, const double* F, const double
   return ELFEL_OK;
 }
 
-int batch_step(elfel_batch* b, int32_t graphs, int32_t* active) {
+// The launches of a step (batch_step joins the clusters' streams).
+static int step_launches(elfel_batch* b, int32_t graphs) {
   Ctx* c = ctx_of(b);
-  cudaSetDevice(c->device);
-  if (b->map_dirty) ELFEL_TRY(rebuild_map(b));
   if (b->nrun) ELFEL_TRY(run_clusters(b, graphs));
   for (int gi = 0; b->persist && gi < graphs && b->total_tiles > 0; ++gi) {
     // one cooperative launch of iters iterations (all blocks resident)
@@ -1085,7 +1084,18 @@ int batch_step(elfel_batch* b, int32_t graphs, int32_t* active) {
     b->launches++;
     b->kernel_launches += 3LL * b->iters;
   }
-  if (b->nrun) ELFEL_TRY(join_clusters(b));
+  return ELFEL_OK;
+}
+
+int batch_step(elfel_batch* b, int32_t graphs, int32_t* active) {
+  Ctx* c = ctx_of(b);
+  cudaSetDevice(c->device);
+  if (b->map_dirty) ELFEL_TRY(rebuild_map(b));
+  const int rc = step_launches(b, graphs);
+  // also after an error: what is freed on the context stream waits for the clusters
+  const int jc = b->nrun ? join_clusters(b) : ELFEL_OK;
+  ELFEL_TRY(rc);
+  ELFEL_TRY(jc);
   ELFEL_TRY(read_states(b));
   if (b->map_dirty) ELFEL_TRY(rebuild_map(b));
   int n = 0;
@@ -1285,6 +1295,8 @@ extern "C" int elfel_batch_destroy(elfel_batch* b) {
   Ctx* c = &b->h->c;
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
+  for (cudaStream_t st : b->run_stream)
+    if (st) cudaStreamSynchronize(st);
   for (Slot& s : b->slots) {
     s.part.release(c);
     if (s.m) s.m->busy = 0;

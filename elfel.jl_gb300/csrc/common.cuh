@@ -90,12 +90,15 @@ struct Phase {
 int fail(Ctx* c, int code, const char* fmt, ...);
 
 // Check a CUDA call; on failure record and return ELFEL_ERR_CUDA from the caller.
+// (an error is reported once: taken off the runtime's last one, which the next launch check reads)
 #define ELFEL_CUDA(ctx, call)                                                         \
   do {                                                                                \
     cudaError_t _e = (call);                                                          \
-    if (_e != cudaSuccess)                                                            \
+    if (_e != cudaSuccess) {                                                          \
+      cudaGetLastError();                                                             \
       return ::elfel::fail((ctx), ELFEL_ERR_CUDA, "%s:%d %s: %s", __FILE__, __LINE__, \
                            #call, cudaGetErrorString(_e));                            \
+    }                                                                                 \
   } while (0)
 
 #define ELFEL_TRY(expr)       \

@@ -1,0 +1,55 @@
+"""Batches that mix cluster systems and graph systems, and what happens when a step fails (GPU)."""
+import numpy as np
+import pytest
+
+from problems import heat_space
+
+pytestmark = pytest.mark.gpu
+
+
+def system(E, ctx, n, seed, etype="T6"):
+    """A resident heat system of n x n cells, its start vector and number of unknowns."""
+    mesh = E.jitter((E.T6block if etype == "T6" else E.T3block)(1.0, 1.0, n, n), 0.1 / n, seed=seed)
+    fesp = heat_space(E, mesh, E.FEH1_T6() if etype == "T6" else E.FEH1_T3())
+    nd, nu = E.ndofs(fesp), E.nunknowns(fesp)
+    kappa = np.random.default_rng(seed).uniform(0.5, 2.0, mesh.nel)
+    am = E.start(E.SysmatAssemblerGPU(ctx=ctx), nd, nd)
+    E.assemble_heat(am, E.FEIterator(fesp), E.QPIterator(fesp, {"npts": 3}), kappa, -6.0)
+    T = np.zeros(nd)
+    E.gathersysvec(T, fesp)
+    return am, T, nu
+
+
+def run(E, ctx, systems, method, capacity=8, rtol=1e-10):
+    b = E.BatchSolver(method, capacity=capacity, ctx=ctx)
+    slots = [b.add(am, T, nu, rtol=rtol) for am, T, nu in systems]
+    out = b.run(graphs=2)
+    b.close()
+    return [out[s] for s in slots]
+
+
+def test_failed_step(E, gpu, monkeypatch):
+    """A step fails after its clusters were launched: the graphs of the large system cannot
+    be captured on the legacy default stream (an error code, nothing runs).  The batch is
+    closed and its memory used again at once; a batch that is kept goes on, with the same bits."""
+    monkeypatch.setenv("ELFEL_TUNE", "0")
+    ctx = E.Context(0)
+    systems = [system(E, ctx, n, n) for n in (30, 20, 12, 104)]
+    want = run(E, ctx, systems, "pcg32_ir")
+    for keep in (False, True):
+        ctx.set_stream(1)  # cudaStreamLegacy
+        b = E.BatchSolver("pcg32_ir", capacity=8, ctx=ctx)
+        slots = [b.add(am, T, nu, rtol=1e-10) for am, T, nu in systems]
+        with pytest.raises(E.ElfelError):
+            b.step(50)
+        if keep:
+            ctx.set_stream(None)
+            out = b.run(graphs=2)
+            for s, (T, st) in zip(slots, want):
+                assert np.array_equal(out[s][0], T) and out[s][1]["iterations"] == st["iterations"]
+            b.close()
+        else:
+            b.close()
+            ctx.set_stream(None)
+            for (T, st), (T0, st0) in zip(run(E, ctx, systems, "pcg32_ir"), want):
+                assert np.array_equal(T, T0) and st["iterations"] == st0["iterations"]
