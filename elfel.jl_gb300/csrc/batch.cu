@@ -1158,32 +1158,46 @@ int batch_take(elfel_batch* b, int32_t k, double* T_out, int t_dev, elfel_solve_
   return ELFEL_OK;
 }
 
-// The results of the finished slots ks: into T[i] where want[i], stats[i].  Their
-// residuals and copies are issued together, through page-locked memory of at
-// most kStageDoubles (or one system's), one synchronisation each time it fills:
-// 65 us a slot one by one, 32 here (up to 24,000 unknowns each).
+// Page-locked memory for n doubles, or null where there is none to be had (ELFEL_STAGE=0).
+static double* stage_of(elfel_batch* b, size_t n) {
+  if (!ctx_of(b)->stage) return nullptr;
+  if (n > b->stage_n) {
+    if (b->stage) cudaFreeHost(b->stage);
+    b->stage = nullptr;
+    b->stage_n = 0;
+    if (cudaMallocHost((void**)&b->stage, sizeof(double) * n) != cudaSuccess) {
+      cudaGetLastError();
+      b->stage = nullptr;
+      return nullptr;
+    }
+    b->stage_n = n;
+  }
+  return b->stage;
+}
+
+// The results of the finished slots ks: into T[i] where want[i], stats[i], each with a
+// status of its own.  Their residuals and copies are issued together, through
+// page-locked memory of at most kStageDoubles (or one system's), one synchronisation
+// each time it fills: 65 us a slot one by one, 32 here (up to 24,000 unknowns each).
+// Where that fails the slots are taken one by one.
 constexpr size_t kStageDoubles = (size_t)4 << 20;
 
-int batch_take_many(elfel_batch* b, const std::vector<int32_t>& ks, const std::vector<char>& want,
-                    std::vector<std::vector<double>>* T, std::vector<elfel_solve_stats>* stats) {
+void batch_take_many(elfel_batch* b, const std::vector<int32_t>& ks, const std::vector<char>& want,
+                     std::vector<std::vector<double>>* T, std::vector<elfel_solve_stats>* stats,
+                     std::vector<int>* status) {
   Ctx* c = ctx_of(b);
   cudaSetDevice(c->device);
   T->resize(ks.size());
-  stats->resize(ks.size());
+  stats->assign(ks.size(), elfel_solve_stats());
+  status->assign(ks.size(), ELFEL_OK);
   auto need = [&](size_t i) { return 2 + (want[i] ? (size_t)b->slots[ks[i]].m->nrow : 0); };
-  for (int32_t k : ks) ELFEL_TRY(check_done(b, k));
-  for (size_t i0 = 0, i1 = 0; i0 < ks.size(); i0 = i1) {
-    size_t total = need(i0);
-    for (i1 = i0 + 1; i1 < ks.size() && total + need(i1) <= kStageDoubles; ++i1) total += need(i1);
-    if (total > b->stage_n) {
-      if (b->stage) cudaFreeHost(b->stage);
-      b->stage = nullptr;
-      b->stage_n = 0;
-      ELFEL_CUDA(c, cudaMallocHost((void**)&b->stage, sizeof(double) * total));
-      b->stage_n = total;
-    }
-    double* at = b->stage;
+  // the slots [i0, i1), whose results take `total` doubles
+  auto together = [&](size_t i0, size_t i1, size_t total) -> int {
+    double* const stage = stage_of(b, total);
+    if (!stage) return ELFEL_ERR_CUDA;
+    double* at = stage;
     for (size_t i = i0; i < i1; ++i) {
+      ELFEL_TRY(check_done(b, ks[i]));
       const Slot& s = b->slots[ks[i]];
       SolverData* S = s.m->solver;
       const int64_t n = s.m->nrow, nu = s.nu;
@@ -1201,15 +1215,24 @@ int batch_take_many(elfel_batch* b, const std::vector<int32_t>& ks, const std::v
       at += need(i);
     }
     ELFEL_CUDA(c, cudaStreamSynchronize(c->stream));
-    at = b->stage;
+    at = stage;
     for (size_t i = i0; i < i1; ++i) {
       const size_t len = need(i);
       if (want[i]) (*T)[i].assign(at + 2, at + len);
       free_slot(b, ks[i], at[0], at[1], &(*stats)[i]);
       at += len;
     }
+    return ELFEL_OK;
+  };
+  for (size_t i0 = 0, i1 = 0; i0 < ks.size(); i0 = i1) {
+    size_t total = need(i0);
+    for (i1 = i0 + 1; i1 < ks.size() && total + need(i1) <= kStageDoubles; ++i1) total += need(i1);
+    if (together(i0, i1, total) == ELFEL_OK) continue;
+    for (size_t i = i0; i < i1; ++i) {
+      if (want[i]) (*T)[i].resize((size_t)b->slots[ks[i]].m->nrow);
+      (*status)[i] = batch_take(b, ks[i], want[i] ? (*T)[i].data() : nullptr, 0, &(*stats)[i]);
+    }
   }
-  return ELFEL_OK;
 }
 
 int batch_counts(elfel_batch* b, int64_t* launches, int64_t* kernels) {

@@ -46,6 +46,8 @@ struct Ctx {
   std::vector<PhaseRec> phases;
   // tile reduction of resident T6 heat patterns: on unless ELFEL_TILES=0
   int tiles = 1;
+  // finished batch slots leave through page-locked memory: unless ELFEL_STAGE=0
+  int stage = 1;
   // one-launch Krylov iterations: on unless ELFEL_ONE_LAUNCH=0
   int one_launch = 1;
   // their waits give up after this many polls, about a second (ELFEL_RUN_SPINS); the

@@ -231,6 +231,8 @@ extern "C" int elfel_ctx_create(int device, int64_t mem_budget_bytes, elfel_ctx*
   h->c.tune = (tu && tu[0] == '0') ? 0 : 1;
   const char* ti = getenv("ELFEL_TILES");
   h->c.tiles = (ti && ti[0] == '0') ? 0 : 1;
+  const char* sg = getenv("ELFEL_STAGE");
+  h->c.stage = (sg && sg[0] == '0') ? 0 : 1;
   const char* ol = getenv("ELFEL_ONE_LAUNCH");
   h->c.one_launch = (ol && ol[0] == '0') ? 0 : 1;
   if (const char* rs = getenv("ELFEL_RUN_SPINS")) h->c.run_spins = (unsigned)strtoul(rs, nullptr, 10);

@@ -40,8 +40,9 @@ namespace elfel {
 int batch_add_dev(elfel_batch* b, elfel_sysmat* m, const double* F, const double* T, int t_dev, int64_t nu,
                   double rtol, int32_t maxit, int32_t* slot_out);
 int batch_step(elfel_batch* b, int32_t graphs, int32_t* active);
-int batch_take_many(elfel_batch* b, const std::vector<int32_t>& ks, const std::vector<char>& want,
-                    std::vector<std::vector<double>>* T, std::vector<elfel_solve_stats>* stats);
+void batch_take_many(elfel_batch* b, const std::vector<int32_t>& ks, const std::vector<char>& want,
+                     std::vector<std::vector<double>>* T, std::vector<elfel_solve_stats>* stats,
+                     std::vector<int>* status);
 int batch_counts(elfel_batch* b, int64_t* launches, int64_t* kernels);
 }  // namespace elfel
 
@@ -471,12 +472,13 @@ int step_batched(elfel_server* s, int32_t* active) {
   }
   std::vector<std::vector<double>> sols;
   std::vector<elfel_solve_stats> sst;
-  if (!slots.empty()) ELFEL_TRY(batch_take_many(s->batch, slots, want, &sols, &sst));
+  std::vector<int> status;
+  batch_take_many(s->batch, slots, want, &sols, &sst, &status);
   for (size_t i = 0; i < slots.size(); ++i) {
     auto it = s->by_slot.find(slots[i]);
     Sys* y = it->second;
     s->by_slot.erase(it);
-    ELFEL_TRY(finish_request(s, y, sst[i], ELFEL_OK, &sols[i]));
+    ELFEL_TRY(finish_request(s, y, sst[i], status[i], &sols[i]));
   }
   if (active) *active = (int32_t)s->by_slot.size();
   return ELFEL_OK;

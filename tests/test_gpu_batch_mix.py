@@ -53,3 +53,24 @@ def test_failed_step(E, gpu, monkeypatch):
             ctx.set_stream(None)
             for (T, st), (T0, st0) in zip(run(E, ctx, systems, "pcg32_ir"), want):
                 assert np.array_equal(T, T0) and st["iterations"] == st0["iterations"]
+
+
+def test_harvest_without_staging(E, gpu, monkeypatch):
+    """Without page-locked memory (ELFEL_STAGE=0 stands for none to be had) the finished requests
+    of a step are taken one by one: each has its own status, and the same solution."""
+    out = []
+    for on in ("1", "0"):
+        monkeypatch.setenv("ELFEL_STAGE", on)
+        ctx = E.Context(0)
+        srv = E.HeatServer("pcg32_ir", max_active=8, rtol=1e-10, ctx=ctx)
+        ids = [srv.submit(E.heat_request(et, n, kappa=k, Q=-3.0, keep_solution=i != 2))
+               for i, (et, n, k) in enumerate([("T3", 20, 1.0), ("T6", 12, 1.7), ("T3", 20, 0.6), ("T6", 105, 1.2),
+                                               ("T3", 9, 1.3)])]
+        res = {r["id"]: r for r in srv.drain()}
+        assert sorted(res) == sorted(ids) and all(r["status"] == 0 and r["converged"] for r in res.values())
+        out.append([(srv.solution(i), res[i]["iterations"], res[i]["relres"]) for k, i in enumerate(ids) if k != 2])
+        with pytest.raises(E.ElfelError):
+            srv.solution(ids[2])
+        srv.close()
+    for (T, it, rr), (T1, it1, rr1) in zip(*out):
+        assert np.array_equal(T, T1) and it == it1 and rr == rr1
