@@ -74,3 +74,23 @@ def test_harvest_without_staging(E, gpu, monkeypatch):
         srv.close()
     for (T, it, rr), (T1, it1, rr1) in zip(*out):
         assert np.array_equal(T, T1) and it == it1 and rr == rr1
+
+
+def test_tuning_is_not_timed_beside_clusters(E, gpu):
+    """The grid of the graphs is tuned on the graphs alone: with 20 cluster systems of the largest kind in
+    the same step the candidates' times stay within twice those without them (four times, timed beside them)."""
+    ms = []
+    for crowd in (0, 20):
+        ctx = E.Context(0)
+        big = system(E, ctx, 130, 1)
+        b = E.BatchSolver("pcg32_ir", capacity=64, ctx=ctx)
+        others = [system(E, ctx, 98, k) for k in range(crowd)]
+        for am, T, nu in [big] + others:
+            b.add(am, T, nu, rtol=1e-10)
+        b.step(8)
+        lines = [line for line, _ in ctx.tuning() if line.startswith("batch_pcg32_ir")]
+        assert len(lines) == 1
+        ms.append([float(w.split("=")[1].rstrip("*")[:-2]) for w in lines[0].split()[1:]])
+        b.run(graphs=2)
+        b.close()
+    assert min(ms[1]) <= 2.0 * min(ms[0]), ms
