@@ -849,7 +849,7 @@ int run_clusters(elfel_batch* b, int graphs) {
       ELFEL_CUDA(c, cudaStreamWaitEvent(st, b->run_fork, 0));
     }
     ELFEL_TRY(batch_run_launch(c, st, b->method == ELFEL_PCG32_IR, b->sys.p, list + R.off, R.n, R.blocks, R.smem,
-                               kBRunIters * graphs));
+                               (int)std::min<int64_t>((int64_t)kBRunIters * graphs, INT32_MAX)));
     if (!alone) ELFEL_CUDA(c, cudaEventRecord(b->run_join[k], st));
     b->launches++;
     b->kernel_launches++;

@@ -94,3 +94,14 @@ def test_tuning_is_not_timed_beside_clusters(E, gpu):
         b.run(graphs=2)
         b.close()
     assert min(ms[1]) <= 2.0 * min(ms[0]), ms
+
+
+def test_many_iterations_in_one_step(E, gpu):
+    """A step of 2^26 graphs: 2^32 iterations for a cluster system, more than an int holds; it ends when it has converged."""
+    ctx = E.Context(0)
+    am, T, nu = system(E, ctx, 6, 1, etype="T3")
+    b = E.BatchSolver("pcg32_ir", capacity=2, ctx=ctx)
+    s = b.add(am, T, nu, rtol=1e-10)
+    assert b.step(1 << 26) == 0 and b.done() == [s]
+    assert b.result(s)[1]["converged"]
+    b.close()
