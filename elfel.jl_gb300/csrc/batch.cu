@@ -1073,6 +1073,9 @@ static int step_launches(elfel_batch* b, int32_t graphs) {
   int32_t left = graphs;
   if (!b->persist && b->total_tiles > 0) ELFEL_TRY(choose_grid(b, &cfg, &left));
   if (b->nrun) ELFEL_TRY(run_clusters(b, graphs));
+  // the persistent form's grid barrier needs its blocks on every SM at once, within the
+  // limit of its wait: not beside clusters that may hold some for longer
+  if (b->nrun && b->persist && b->total_tiles > 0) ELFEL_TRY(join_clusters(b));
   for (int gi = 0; b->persist && gi < graphs && b->total_tiles > 0; ++gi) {
     // one cooperative launch of iters iterations (all blocks resident)
     const BSys* sy = b->sys.p;
