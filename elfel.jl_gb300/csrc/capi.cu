@@ -315,7 +315,7 @@ extern "C" int elfel_sysmat_csc(elfel_sysmat* m, int64_t* colptr, int64_t* rowva
     // the values of a pattern the caller has already: no index arrays are formed
     // (2M quadratic triangles: 0.12 ms of a 2.6 ms re-assembly and download)
     int pin_v = 0;
-    const bool direct = nzval && host_device_ptr(c, nzval, &pin_v) && pin_v && c->stream == c->own_stream;
+    const bool direct = nzval && host_device_ptr(c, nzval, sizeof(double) * nnz, &pin_v) && pin_v && c->stream == c->own_stream;
     const int64_t head = direct ? std::min(m->head.nnz, nnz) : 0;
     if (direct) m->head.kept = 0;
     if (head) {
@@ -334,8 +334,8 @@ extern "C" int elfel_sysmat_csc(elfel_sysmat* m, int64_t* colptr, int64_t* rowva
     return ELFEL_OK;
   }
   int pin_c = 0, pin_r = 0;
-  int64_t* cpd = colptr ? (int64_t*)host_device_ptr(c, colptr, &pin_c) : nullptr;
-  int64_t* rvd = rowval ? (int64_t*)host_device_ptr(c, rowval, &pin_r) : nullptr;
+  int64_t* cpd = colptr ? (int64_t*)host_device_ptr(c, colptr, sizeof(int64_t) * (ncol + 1), &pin_c) : nullptr;
+  int64_t* rvd = rowval ? (int64_t*)host_device_ptr(c, rowval, sizeof(int64_t) * nnz, &pin_r) : nullptr;
   if (colptr && rowval && cpd && rvd && pin_c && pin_r) {
     // pinned arrays: the 1-based indices are written straight into them (one
     // block per SM: more blocks writing across the host link run slower;
@@ -440,11 +440,17 @@ static int upload_space(Ctx* c, const elfel_space& s, int64_t ndofs, int sdim, D
 // before it uses them).  The index checks are deferred: bad[0..3] (primary
 // connectivity, primary DOFs, pressure connectivity, pressure DOFs) are read
 // once the work of both streams is done.
-static bool tables_readable(Ctx* c, const elfel_space& s) {
+static const void* conn_ptr(Ctx* c, const elfel_space& s) {
+  return host_device_ptr(c, s.conn, sizeof(int64_t) * s.nel * s.nodes_per_elem);
+}
+static const void* dofs_ptr(Ctx* c, const elfel_space& s) {
+  return host_device_ptr(c, s.eldofs, sizeof(int64_t) * s.nel * s.nodes_per_elem * s.ncomp);
+}
+static bool tables_readable(Ctx* c, const elfel_space& s, int sdim) {
   if (s.nel < 0 || s.nnodes < 0 || !s.conn || !s.eldofs || (s.nnodes > 0 && !s.xy))
     return false;  // upload_space reports the error
-  return (s.nel == 0 || (host_device_ptr(c, s.conn) && host_device_ptr(c, s.eldofs))) &&
-         (s.nnodes == 0 || host_device_ptr(c, s.xy));
+  return (s.nel == 0 || (conn_ptr(c, s) && dofs_ptr(c, s))) &&
+         (s.nnodes == 0 || host_device_ptr(c, s.xy, sizeof(double) * sdim * s.nnodes));
 }
 
 // Step 1 (context stream): the buffers, then the element DOFs.
@@ -454,19 +460,18 @@ static int upload_direct_dofs(Ctx* c, const elfel_space& s, int64_t ndofs, int s
   ELFEL_TRY(conn->alloc(c, (size_t)(nc > 0 ? nc : 1)));
   ELFEL_TRY(dofs->alloc(c, (size_t)(nd > 0 ? nd : 1)));
   if (xy) ELFEL_TRY(xy->alloc(c, (size_t)(s.nnodes > 0 ? sdim * s.nnodes : 1)));
-  return to_index32_direct(c, c->stream, (const int64_t*)host_device_ptr(c, s.eldofs), nd, ndofs, dofs->p,
-                           bad_dofs);
+  return to_index32_direct(c, c->stream, (const int64_t*)dofs_ptr(c, s), nd, ndofs, dofs->p, bad_dofs);
 }
 
 // Step 2 (auxiliary stream, forked after step 1's allocations): connectivity
 // and coordinates.
 static int upload_direct_rest(Ctx* c, const elfel_space& s, int sdim, DBuf<int32_t>* conn, DBuf<double>* xy,
                               int* bad_conn, cudaStream_t aux) {
-  ELFEL_TRY(to_index32_direct(c, aux, (const int64_t*)host_device_ptr(c, s.conn), s.nel * s.nodes_per_elem,
-                              s.nnodes, conn->p, bad_conn));
+  ELFEL_TRY(to_index32_direct(c, aux, (const int64_t*)conn_ptr(c, s), s.nel * s.nodes_per_elem, s.nnodes, conn->p,
+                              bad_conn));
   if (xy && s.nnodes) {
     int pinned = 0;
-    const double* src = (const double*)host_device_ptr(c, s.xy, &pinned);
+    const double* src = (const double*)host_device_ptr(c, s.xy, sizeof(double) * sdim * s.nnodes, &pinned);
     ELFEL_TRY(copy_host_f64(c, aux, pinned ? s.xy : src, pinned, sdim * s.nnodes, xy->p));
   }
   return ELFEL_OK;
@@ -544,7 +549,7 @@ extern "C" int elfel_fused_setup(elfel_sysmat* m, const elfel_fused_desc* d) {
   ELFEL_TRY(init_fused(m, d));
   Fused& F = m->F;
   const bool stokes = d->physics == ELFEL_STOKES;
-  if (!tables_readable(c, u) || (stokes && !tables_readable(c, d->p))) {
+  if (!tables_readable(c, u, sdim) || (stokes && !tables_readable(c, d->p, 2))) {
     ELFEL_TRY(upload_space(c, u, d->ndofs, sdim, &F.conn_u, &F.xy_u, &F.dofs_u, "primary"));
     if (stokes) ELFEL_TRY(upload_space(c, d->p, d->ndofs, 2, &F.conn_p, nullptr, &F.dofs_p, "pressure"));
     return fused_build(m, d->ndofs);
@@ -961,7 +966,7 @@ static int finish_values(elfel_sysmat* m, bool rhs_done = false) {
 static int host_coef(Ctx* c, const double* coef, int64_t n, double* dst, HostCoef* host) {
   if (!coef || n == 0) return ELFEL_OK;
   int pinned = 0;
-  const void* p = host_device_ptr(c, coef, &pinned);
+  const void* p = host_device_ptr(c, coef, sizeof(double) * n, &pinned);
   if (pinned) host->p = static_cast<const double*>(p);
   else ELFEL_CUDA(c, cudaMemcpyAsync(dst, coef, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
   return ELFEL_OK;

@@ -129,12 +129,12 @@ int read_back(Ctx* c, cudaStream_t st, std::initializer_list<HostRead> reads);
 // c->stream earlier); join with aux_join.
 int aux_after(Ctx* c, cudaEvent_t ev, cudaStream_t* aux);
 
-// A device-usable address of a host array: the device address of pinned
-// memory, the host address itself where kernels read pageable memory (ATS),
+// A device-usable address of a host array of so many bytes: the device address of
+// pinned memory (all of it: its first and its last byte), the host address itself where kernels read pageable memory (ATS),
 // else nullptr (the caller then copies with cudaMemcpyAsync).
 // *pinned (optional) = 1 for page-locked memory (copy engines work
 // asynchronously on it).
-const void* host_device_ptr(Ctx* c, const void* host, int* pinned = nullptr);
+const void* host_device_ptr(Ctx* c, const void* host, size_t bytes, int* pinned = nullptr);
 
 // Device allocation accounted against the context budget (stream-ordered).
 int dalloc(Ctx* c, void** p, size_t bytes);

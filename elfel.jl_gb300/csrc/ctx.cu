@@ -293,18 +293,25 @@ int read_back(Ctx* c, cudaStream_t st, std::initializer_list<HostRead> reads) {
   return ELFEL_OK;
 }
 
-const void* host_device_ptr(Ctx* c, const void* host, int* pinned) {
+const void* host_device_ptr(Ctx* c, const void* host, size_t bytes, int* pinned) {
   if (pinned) *pinned = 0;
   if (!host) return nullptr;
-  cudaPointerAttributes a;
+  cudaPointerAttributes a, z;
   if (cudaPointerGetAttributes(&a, host) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
   if (a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged) return host;
-  if (a.type == cudaMemoryTypeHost) {
-    if (pinned) *pinned = a.devicePointer != nullptr;
-    return a.devicePointer;
+  if (a.type == cudaMemoryTypeHost && a.devicePointer) {
+    // registered to the end?  (cudaHostRegister of a part: the rest is pageable)
+    const size_t last = bytes ? bytes - 1 : 0;
+    if (!last || (cudaPointerGetAttributes(&z, static_cast<const char*>(host) + last) == cudaSuccess &&
+                  z.type == cudaMemoryTypeHost &&
+                  z.devicePointer == static_cast<char*>(a.devicePointer) + last)) {
+      if (pinned) *pinned = 1;
+      return a.devicePointer;
+    }
+    cudaGetLastError();
   }
   return c->pageable_access ? host : nullptr;
 }
