@@ -105,7 +105,7 @@ __device__ __forceinline__ void batch_run(const BSys& S, Group& grp, int rank, u
     bool ok = group_sum<N1>(grp, d1, part, wsum, t1, nw);
     if (wid == 0) {
       pq = t1[0];
-      const double alpha = pos_finite(pq) ? fast_div(IR ? t1[N1 - 1] : rz, pq, fast_rcp(pq)) : 0.0;
+      const double alpha = pos_finite(pq) ? fast_div(IR ? t1[N1 - 1] : rz, pq) : 0.0;
       if (lane == 0) {
         msg.c[0] = alpha;
         if (!Group::kCluster) msg.stop = ok ? M_CG : M_DONE;

@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kRT, 1) cg_run_k(const CgRun<T> a, const RunGr
     grp.collect(wid, wsum, t1);
     if (wid == 0) {
       pq = t1[0];
-      alpha = pos_finite(pq) ? fast_div(IR ? t1[N1 - 1] : rz, pq, fast_rcp(pq)) : 0.0;
+      alpha = pos_finite(pq) ? fast_div(IR ? t1[N1 - 1] : rz, pq) : 0.0;
       if (lane == 0) {
         msg.c[0] = alpha;
         msg.stop = ok ? 0 : 2;
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kRT, 1) mr_run_k(const MrRun<T> a, const RunGr
     double delta = 0.0;
     if (wid == 0) {
       delta = t[0];
-      const double ca = fast_div(delta, gam, fast_rcp(gam));
+      const double ca = fast_div(delta, gam);
       if (lane == 0) {
         msg.c[0] = ca;
         msg.c[1] = bcoef;
