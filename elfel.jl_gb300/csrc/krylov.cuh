@@ -10,14 +10,20 @@ constexpr int kRunMaxBlocks = 160;  // blocks of a grid group (one per SM)
 // blocks), and the largest systems that run in one (FP64: entries + 8 rows).
 constexpr int kRunClusterSlices = 2;
 constexpr int64_t kRunClusterWork64 = 180000, kRunClusterRows32 = 32768;
-// Beyond this no grid group holds the vectors (20 bytes a row).
-constexpr int64_t kRunGridRows = (int64_t)kRunMaxBlocks * 12000;
 // A batched system takes the smallest cluster whose blocks hold this many rows each.
 constexpr int kRunBatchRows32 = 2048, kRunBatchRows64 = 1024;
 // Systems up to this size may run in a cluster (of the batch too).
 constexpr int64_t kRunSmallRows = 65536;
 constexpr int kRunIters = 4096;     // iterations of one launch at most
 constexpr int kRunSmem = 227 * 1024 - 2048;  // dynamic shared memory of a block (the kernels' static part apart)
+constexpr int kRunPart = 3 * kRunThreads + 16;  // doubles of it for the block sums
+// The largest system whose vectors the blocks of a grid group hold: a slice of 32 rows takes
+// its vectors, the gathered one, and 8 bytes (run_smem without a matrix and a window).
+constexpr int64_t run_most_rows(int blocks, int elem, int vecs) {
+  return (int64_t)blocks * ((kRunSmem - 8 * kRunPart) / (32 * (vecs + 1) * elem + 8)) * 32;
+}
+static_assert(run_most_rows(152, 4, 4) == 1634304 && run_most_rows(152, 8, 4) == 822016, "CG, FP32 and FP64");
+static_assert(run_most_rows(152, 4, 7) == 1026304 && run_most_rows(152, 8, 7) == 515584, "MINRES, FP32 and FP64");
 
 template <bool D16>
 struct ColType {

@@ -13,7 +13,6 @@ namespace cg = cooperative_groups;
 
 constexpr int kRT = kRunThreads;
 constexpr int kRW = kRT / 32;
-constexpr int kRunPart = 3 * kRT + 16;  // doubles of shared memory for the block sums
 
 // Sums.  The FP64 unit of an SM sub-partition takes a warp instruction every
 // 64 cycles whatever its active lanes, so what a sum costs is the number of

@@ -900,7 +900,7 @@ static int build_sell(Ctx* c, SolverData* S) {
   sell_fill_k<<<grid_for(nsl * 32, 256, (int64_t)c->sm_count * 16), 256, 0, c->stream>>>(
       nu, nsl, S->ff.rowptr.p, S->ff.col.p, S->ff.map.p, A.perm.p, iperm.p, A.sptr.p, A.sw.p, col.p, A.map.p, wide.p);
   ELFEL_LAUNCH_CHECK(c);
-  if (nu <= kRunGridRows) {
+  if (nu <= run_most_rows(std::min(c->sm_count, kRunMaxBlocks), 4, 4)) {
     // the cluster and batch divisions serve small systems only
     const bool small = nu <= kRunSmallRows;
     const WinArgs wa{{spbs.v[0], spbs.v[1], spbs.v[2], spbs.v[3]}, {kRunWinGrid, 0, kRunWinBatch32, kRunWinBatch64}};
