@@ -22,7 +22,7 @@ namespace {
 
 // One sum over the group (all threads; the totals, and whether the wait ended, are valid in warp 0).
 template <int NV, typename T, class Group>
-__device__ __forceinline__ bool group_sum(Group& grp, T (&v)[NV], double* part, double* wsum, double (&t)[NV],
+__device__ __forceinline__ bool group_sum(Group& grp, const Dot<T> (&v)[NV], double* part, double* wsum, double (&t)[NV],
                                           int nw = kRW) {
   const int wid = threadIdx.x >> 5;
   block_sums<NV>(v, part, wsum, t, nw);
@@ -88,7 +88,7 @@ __device__ __forceinline__ void batch_run(const BSys& S, Group& grp, int rank, u
     keep = false;
     // q = A p; p.q (and r.p) -> alpha
     constexpr int N1 = IR ? 2 : 1;
-    T d1[N1] = {};
+    Dot<T> d1[N1];
     for (int n = 0; n * kRW < R.nsl; ++n) {
       const int s = R.slice(wid, n);
       const int i = s * 32 + lane;
@@ -97,8 +97,8 @@ __device__ __forceinline__ void batch_run(const BSys& S, Group& grp, int rank, u
         T acc = R.template row<IR>(s, i, W.by_row(), pi);
         if (IR) acc += ss[i] * pi;
         sq[i] = acc;
-        d1[0] += acc * pi;
-        if (IR) d1[N1 - 1] += sr[i] * pi;
+        d1[0].add(acc, pi);
+        if (IR) d1[N1 - 1].add(sr[i], pi);
       }
     }
     double t1[N1];
@@ -119,7 +119,7 @@ __device__ __forceinline__ void batch_run(const BSys& S, Group& grp, int rank, u
     // r -= alpha q, z = D r (kept in q); r.z, r.r (and z.r_old) -> beta
     constexpr int N2 = IR ? 3 : 2;
     const T al = (T)msg.c[0];
-    T d2[N2] = {};
+    Dot<T> d2[N2];
     for (int i = tid; i < R.nloc; i += kRT) {
       const T ro = sr[i];
       const T ri = ro - al * sq[i];
@@ -127,9 +127,9 @@ __device__ __forceinline__ void batch_run(const BSys& S, Group& grp, int rank, u
       const T zi = sd[i] * ri;
       sq[i] = zi;
       gz[r0 + i] = zi;
-      d2[0] += ri * zi;
-      d2[1] += ri * ri;
-      if (IR) d2[N2 - 1] += zi * ro;
+      d2[0].add(ri, zi);
+      d2[1].add(ri, ri);
+      if (IR) d2[N2 - 1].add(zi, ro);
     }
     double t2[N2];
     block_sums<N2>(d2, part, wsum, t2, nw);
@@ -196,14 +196,14 @@ __device__ __forceinline__ void batch_run(const BSys& S, Group& grp, int rank, u
         mode = M_DONE;
         break;
       }
-      double d[1] = {0.0};
+      Dot<double> d[1];
       for (int s = wid; s < R.nsl; s += kRW) {
         const int i = s * 32 + lane;
         const double acc = sell_row_resid<D16, true>(S.A, S.v64, S.x64, r0 / 32 + s, lane);
         if (i < R.nloc) {
           const double rv = S.b64[r0 + i] - acc;
           S.r64[r0 + i] = rv;
-          d[0] += rv * rv;
+          d[0].add(rv, rv);
         }
       }
       double t[1];
@@ -234,7 +234,7 @@ __device__ __forceinline__ void batch_run(const BSys& S, Group& grp, int rank, u
       mode = msg.stop;
       if (mode == M_DONE) break;
       const double inv = 1.0 / scale;
-      T dz[1] = {0};
+      Dot<T> dz[1];
       for (int s = wid; s < R.nsl; s += kRW) {
         const int i = s * 32 + lane;
         if (i < R.nloc) {
@@ -242,7 +242,7 @@ __device__ __forceinline__ void batch_run(const BSys& S, Group& grp, int rank, u
           sr[i] = ri;
           const T zi = sd[i] * ri;
           gp[r0 + i] = mode == M_RESTART ? zi : sp[i];
-          dz[0] += ri * zi;
+          dz[0].add(ri, zi);
         }
       }
       double t3[1];

@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kRT, 1) cg_run_k(const CgRun<T> a, const RunGr
     }
     // q = A p; p.q (and r.p) -> alpha
     constexpr int N1 = IR ? 2 : 1;
-    T d1[N1] = {};
+    Dot<T> d1[N1];
     for (int n = 0; n * kRW < R.nsl; ++n) {
       const int s = R.slice(wid, n);
       const int i = s * 32 + lane;
@@ -121,8 +121,8 @@ __global__ void __launch_bounds__(kRT, 1) cg_run_k(const CgRun<T> a, const RunGr
         T acc = R.template row<IR>(s, i, WIN ? W.by_row() : (const T*)a.p, pi);
         if (IR) acc += rs[i] * pi;
         sq[i] = acc;
-        d1[0] += acc * pi;
-        if (IR) d1[N1 - 1] += sr[i] * pi;
+        d1[0].add(acc, pi);
+        if (IR) d1[N1 - 1].add(sr[i], pi);
       }
     }
     double t1[N1];
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(kRT, 1) cg_run_k(const CgRun<T> a, const RunGr
     // r -= alpha q, z = D r (kept in q); r.z, r.r (and z.r_old) -> beta
     constexpr int N2 = IR ? 3 : 2;
     const T al = (T)msg.c[0];
-    T d2[N2] = {};
+    Dot<T> d2[N2];
     for (int i = tid; i < R.nloc; i += kRT) {
       const T ro = sr[i];
       const T ri = ro - al * sq[i];
@@ -152,9 +152,9 @@ __global__ void __launch_bounds__(kRT, 1) cg_run_k(const CgRun<T> a, const RunGr
       const T zi = sd[i] * ri;
       sq[i] = zi;
       if (WIN) a.z[R.row0 + i] = zi;
-      d2[0] += ri * zi;
-      d2[1] += ri * ri;
-      if (IR) d2[N2 - 1] += zi * ro;
+      d2[0].add(ri, zi);
+      d2[1].add(ri, ri);
+      if (IR) d2[N2 - 1].add(zi, ro);
     }
     double t2[N2];
     block_sums<N2>(d2, part, wsum, t2, nw);
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(kRT, 1) mr_run_k(const MrRun<T> a, const RunGr
       }
     }
     // q = A z, delta = q.z
-    T d1[1] = {0};
+    Dot<T> d1[1];
     for (int n = 0; n * kRW < R.nsl; ++n) {
       const int sl = R.slice(wid, n);
       const int i = sl * 32 + lane;
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(kRT, 1) mr_run_k(const MrRun<T> a, const RunGr
         const T acc = WIN ? R.template row<false>(sl, i, W.by_row_split(), zi)
                           : R.template row<false>(sl, i, (const T*)a.z, zi);
         sq[i] = acc;
-        d1[0] += acc * zi;
+        d1[0].add(acc, zi);
       }
     }
     double t[1];
@@ -320,14 +320,14 @@ __global__ void __launch_bounds__(kRT, 1) mr_run_k(const MrRun<T> a, const RunGr
     if (msg.stop) break;
     // v' = q - (delta/gam) v_j - (gam/gamp) v_{j-1}, z' = M v' (in q), gamn^2 = z'.v'
     const T ca = (T)msg.c[0], cb = (T)msg.c[1];
-    T d2[1] = {0};
+    Dot<T> d2[1];
     for (int i = tid; i < R.nloc; i += kRT) {
       const T vv = sq[i] - ca * sv[i] - cb * svm[i];
       svm[i] = vv;
       const T zz = sm[i] * vv;
       sq[i] = zz;
       if (WIN) a.z[r0 + i] = zz;
-      d2[0] += zz * vv;
+      d2[0].add(zz, vv);
     }
     block_sums<1>(d2, part, wsum, t, nw);
     if (wid == 0) grp.publish(t);

@@ -177,6 +177,24 @@ struct GridGroup {
   static constexpr bool kCluster = false;
 };
 
+// A thread's part of a dot product.  FP32 terms are added with compensation (Kahan 1965), an
+// error of two units of rounding however many rows a thread has (up to 21 at the limit of a
+// grid group, five in a batched cluster; the graphs' threads had four rows and one); FP64 plainly.
+template <typename T>
+struct Dot {
+  T s = 0;
+  __device__ __forceinline__ void add(T a, T b) { s += a * b; }
+};
+template <>
+struct Dot<float> {
+  float s = 0.f, c = 0.f;
+  __device__ __forceinline__ void add(float a, float b) {
+    const float y = __fmaf_rn(a, b, -c), t = __fadd_rn(s, y);
+    c = __fsub_rn(__fsub_rn(t, s), y);
+    s = t;
+  }
+};
+
 // The block's sums of the threads' values, in every lane of warp 0 (which
 // has room for 3 * kRT doubles in part and 16 in wsum).  FP32 values add
 // within the warp in FP32 first; FP64 values go to shared memory as they are.
@@ -184,7 +202,10 @@ struct GridGroup {
 // system's block, whose FP64 sums leave the zeros out (run_warps; a solve with 16 x 16 T6
 // elements 1119 -> 1076 us, 64 x 64 T3 1700 -> 1644).
 template <int NV, typename T>
-__device__ __forceinline__ void block_sums(T (&v)[NV], double* part, double* wsum, double (&tot)[NV], int nw) {
+__device__ __forceinline__ void block_sums(const Dot<T> (&d)[NV], double* part, double* wsum, double (&tot)[NV], int nw) {
+  T v[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) v[k] = d[k].s;
   constexpr int L = 32 / sum_groups(NV);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane / L, l = lane % L;
   if (sizeof(T) == 4) {
