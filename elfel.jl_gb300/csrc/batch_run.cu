@@ -316,7 +316,11 @@ BRunPlan batch_run_plan(const Ctx* c, const SolverData* S, int ir) {
   const size_t sv = run_smem(spb, elem, ir ? 5 : 4, window, 0, S->A.d16);
   const size_t sm = run_smem(spb, elem, ir ? 5 : 4, window, entries, S->A.d16);
   // a system whose matrix does not fit iterates from L2 as long as its rows
-  // are few; larger ones are left to the graphs, which use the whole device
+  // are few (a quarter more than 16 full blocks); larger ones are left to the graphs, which
+  // use the whole device.  Ms in the cluster and in graphs, one system and 16: FP32 T6 38,025
+  // unknowns 7.3 and 17.1, 24.1 and 62.0; 47,961 (beyond) 8.8 and 20.4, 29.0 and 78.6.  FP64 18,769
+  // 6.8 and 11.9, 22.8 and 32.6; 25,281 (beyond) 10.6 and 13.7, 32.6 and 46.0; 62,001 30.8 and
+  // 24.4, 90.8 and 117.  So the line could lie further out.
   if (sv > (size_t)kRunSmem || spb * 32 > (ir ? kRunBatchRows32 : kRunBatchRows64) * 5 / 4) return P;
   P.ms = sm <= (size_t)kRunSmem;
   P.spb = spb;

@@ -17,14 +17,15 @@
 //     (the same partials in the same order: the same bits in every block);
 //   - x is advanced between the arrival at and the wait for the second sum.
 // Per iteration, quadratic heat, FP64 and FP32 (graphs, then one launch):
-//       961 unknowns  21.3 ->  6.0 us   25.8 ->  7.9 us (12 replacements incl.)
-//     14161           21.1 ->  8.0      21.9 ->  6.0
-//    128881           26.2 -> 11.9      22.2 ->  7.9
-//    358801           40.2 -> 22.7      32.0 -> 10.9
-//    808201           62.7 -> 46.7      45.9 -> 15.3
-// MINRES (Taylor-Hood cavity) 27.2 -> 11.0 us at 9026 unknowns.  What is left
-// at 128881: the two sums over the grid (1.5 us a barrier, 0.8 to collect), in
-// FP64 the FP64 unit (4.5 us).  Measured and not kept: the direction gathered
+//       961 unknowns  21.3 ->  5.4 us   25.8 ->  4.7 us
+//     14161           21.1 ->  7.7      21.9 ->  5.6
+//    128881           26.2 -> 12.0      22.2 ->  7.8
+//    358801           40.2 -> 22.6      32.0 -> 11.3
+//    808201           62.7 -> 47.2      45.9 -> 16.0
+// MINRES (Taylor-Hood cavity) 27.2 -> 11.1 us at 9026 unknowns.  What is left
+// at 128881: the two sums over the grid (1.5 us a barrier with the blocks' uneven
+// arrival, 0.8 to collect), in FP64 the FP64 unit (4.5 us), in FP32 at 808201 the
+// compensated sums (0.35).  Measured and not kept: the direction gathered
 // from global memory after a barrier of its own (FP32 9.4 us at 128881, 21.1 at
 // 808201: gathers that miss L1), 1024 threads a block (17.5 at 808201), the
 // next chunk of the matrix prefetched into registers (no change), the matrix
@@ -34,9 +35,10 @@
 //   ClusterGroup  one cluster of up to 16 blocks: sums through distributed
 //                 shared memory, the hardware cluster barrier (0.2-0.3 us);
 //   GridGroup     one block per SM, launched cooperatively: an arrival counter
-//                 in global memory (1.1 us per barrier at 152 blocks).  Every
-//                 wait is bounded; a wait that runs out marks the error word
-//                 and ends the kernel.
+//                 in global memory (1.1 to 1.25 us a barrier of 152 blocks by
+//                 itself).  Every wait is bounded; a wait that runs out marks the
+//                 error word and ends the kernel, and the solve starts again in
+//                 graphs (or_in_graphs in solve.cu).
 #include <algorithm>
 
 #include "krylov_dev.cuh"
@@ -507,7 +509,12 @@ RunPlan run_plan(Ctx* c, const SolverData* S, int elem, int vecs, int least_vecs
       P.blocks = (int)((A.nslices + P.spb - 1) / P.spb);
     // Every row of a window that is not the block's own costs a multiply-add a
     // product (FP64: half a cycle of the SM), which pays for the barrier that
-    // the window saves up to these widths.
+    // the window saves up to these widths.  Us an iteration with the window and without,
+    // by the rows beyond the own ones: FP64 cluster 1163 (T4 20^3) 7.5 and 7.6, 2468 (cavity
+    // 20 x 20) 8.6 and 8.5; FP64 grid 3519 (T4 40^3) 10.4 and 10.8, 6597 (56^3) 17.2 and 17.0,
+    // 9851 (70^3) 24.4 and 23.7; FP32 cluster 2468 6.2 and 6.9, 6447 (cavity 32 x 32) 8.7 and
+    // 8.6; FP32 grid 9851 23.8 and 26.3, 16426 (T4 90^3) 28.2 and 32.7, 23472 (cavity 128 x
+    // 128) 15.8 and 14.1.
     const int wide = S->run_window[split ? 4 + q : q];
     const int most = P.spb * 32 + (cluster ? 2000 : 8000) * (elem == 8 ? 1 : 2);
     P.window = wide > 0 && wide <= most ? wide + (wide & 1) : 0;  // even: 8-byte alignment of what follows

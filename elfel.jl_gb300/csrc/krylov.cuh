@@ -7,12 +7,21 @@ namespace elfel {
 constexpr int kRunThreads = 512;
 constexpr int kRunMaxBlocks = 160;  // blocks of a grid group (one per SM)
 // Cluster groups: slices per block that a cluster is grown for (up to 16
-// blocks), and the largest systems that run in one (FP64: entries + 8 rows).
+// blocks), and the largest systems that run in one (FP64: entries + 8 rows).  Us an
+// iteration in a grid and in a cluster, FP64: T6 6,241 unknowns (122,000 by that count) 7.5
+// and 6.8, 9,801 (191,000) 7.6 and 8.4; T3 3,481 7.1 and 4.9, 9,801 (147,000) 7.0 and 7.2,
+// 22,201 7.2 and 10.3.  FP32: T6 19,321 6.9 and 5.7, 32,041 7.0 and 6.4, from 39,601 on the
+// matrix is too large for 16 blocks; T3 32,041 6.9 and 5.9, 47,961 7.0 and 6.7.
 constexpr int kRunClusterSlices = 2;
 constexpr int64_t kRunClusterWork64 = 180000, kRunClusterRows32 = 32768;
 // A batched system takes the smallest cluster whose blocks hold this many rows each.
+// Fewer rows a block are faster alone (T6 3,481 unknowns FP32 with 512, 1024, 2048 rows:
+// 1.4, 1.5, 1.9 ms), more of them in a crowd (64 of them 14.1, 10.8, 10.0; 64 of 16,129
+// 53.6, 53.9, 40.1; a serving burst 12.2, 10.9, 9.3).  FP64 with 512 and 1024: alone 1.9 and
+// 2.6 ms, 64 of them 16.1 and 12.3.
 constexpr int kRunBatchRows32 = 2048, kRunBatchRows64 = 1024;
-// Systems up to this size may run in a cluster (of the batch too).
+// Up to here the windows of the cluster and batch divisions are formed: what 16 blocks can
+// hold at the rows above (with the quarter more of batch_run_plan, 40,960) and some room.
 constexpr int64_t kRunSmallRows = 65536;
 constexpr int kRunIters = 4096;     // iterations of one launch at most
 constexpr int kRunSmem = 227 * 1024 - 2048;  // dynamic shared memory of a block (the kernels' static part apart)

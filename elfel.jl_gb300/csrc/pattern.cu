@@ -46,7 +46,11 @@ struct Net {
 };
 constexpr int kNet = 48;    // block mode, on average at most kNetMean slots a column
 constexpr int kNetL = 96;   // block mode, more
-constexpr int kNet64 = 40;  // COO mode: 64-bit keys (48 spill)
+// COO mode: 64-bit keys (48 spill).  Triplets with longer columns (plane elasticity on T6, T4)
+// go on to sort_wide_k after a look at their lengths.  To CSC with a warp for every column
+// (and the values uploaded before the build) and here: T4 36^3 992 and 905 us, elasticity
+// 200 x 100 1420 and 1297, T6 200 x 200 807 and 706.
+constexpr int kNet64 = 40;
 // Slots per column: 16 to 18 on T3, T6 and Q4 meshes (vertices of a T6 mesh 36), 36 in
 // plane elasticity on T6 (24 and 72), 48 in Taylor-Hood, 96 on T4.  The larger form keeps
 // eight warps an SM instead of 16 and is taken where the other would leave most
