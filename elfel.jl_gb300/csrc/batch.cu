@@ -159,10 +159,6 @@ __device__ __forceinline__ bool item_finish(const BSys& S, const double* wsum, i
 }
 
 // ------------------------------------------------------------------ kernels
-// With programmatic dependent launch (launch_pdl, pdl_wait) the kernels stage
-// their first work item and its system descriptor before waiting on the
-// previous kernel.
-
 // Copy a system descriptor into shared memory (one 8-byte word per thread).
 __device__ __forceinline__ void stage_sys(const BSys* __restrict__ src, BSys* dst) {
   static_assert(sizeof(BSys) % 8 == 0 && sizeof(BSys) / 8 <= kBlk, "descriptor staging");
@@ -172,14 +168,11 @@ __device__ __forceinline__ void stage_sys(const BSys* __restrict__ src, BSys* ds
 }
 
 // body(it, S) for each work item it = (slot, first tile, tiles) of this
-// block, S its system's descriptor staged in shared memory.  The first
-// item's descriptor is staged before the wait on the previous kernel (the
-// item map and the descriptors are written before the graph runs).
+// block, S its system's descriptor staged in shared memory.
 template <typename F>
 __device__ __forceinline__ void for_items(const BSys* __restrict__ sys, const int4* __restrict__ items,
                                           const int* __restrict__ ntot, F&& body) {
   __shared__ BSys S;
-  pdl_launch_dependents();
   const int total = *ntot;
   int t = blockIdx.x;
   int4 it = make_int4(0, 0, 0, 0);
@@ -187,7 +180,6 @@ __device__ __forceinline__ void for_items(const BSys* __restrict__ sys, const in
     it = items[t];
     stage_sys(sys + it.x, &S);
   }
-  pdl_wait();
   while (t < total) {
     body(it, (const BSys&)S);
     t += gridDim.x;
@@ -742,9 +734,9 @@ void launch_iteration(cudaStream_t s, elfel_batch* b, const GridCfg& g, int sms)
   const BSys* sy = b->sys.p;
   const int4* it = b->items.p;
   const int* nt = b->ntot.p;
-  launch_pdl(b_spmv_k<IR>, g1, kBlk, s, sy, it, nt);
-  launch_pdl(b_update_k<IR>, g2, kBlk, s, sy, it, nt);
-  launch_pdl(b_p_k<IR>, g2, kBlk, s, sy, it, nt);
+  b_spmv_k<IR><<<g1, kBlk, 0, s>>>(sy, it, nt);
+  b_update_k<IR><<<g2, kBlk, 0, s>>>(sy, it, nt);
+  b_p_k<IR><<<g2, kBlk, 0, s>>>(sy, it, nt);
 }
 
 int graph_for(elfel_batch* b, int k, cudaGraphExec_t* out) {

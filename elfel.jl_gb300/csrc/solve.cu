@@ -153,8 +153,6 @@ template <typename T, bool D16, bool DIFF, bool FLEX>
 __global__ void __launch_bounds__(kBlk, sell_occ<T>()) sell_cg_spmv_k(SellView A, const T* __restrict__ v, const T* __restrict__ x,
                                                       T* __restrict__ y, const T* __restrict__ r, Red4 red,
                                                       double* scal, int slot, int* flags) {
-  pdl_launch_dependents();
-  pdl_wait();
   if (flags[F_DONE] || flags[F_RU]) {
     // F_RU = 1: requested by the previous update; p has been advanced once by
     // cg_p_k since.  Mark it 2 so the rest of the graph skips until the host
@@ -252,8 +250,6 @@ __global__ void __launch_bounds__(kBlk, kVecOcc) cg_update_k(int64_t n, T* __res
                                                    const T* __restrict__ p, const T* __restrict__ q,
                                                    T* __restrict__ z, const T* __restrict__ dinv, Red4 red,
                                                    double* scal, int* flags) {
-  pdl_launch_dependents();
-  pdl_wait();
   if (flags[F_DONE] || flags[F_RU]) return;
   // breakdown (p.Ap not positive or not finite): no update, report below
   const double pq = scal[S_PQ];
@@ -312,8 +308,6 @@ __global__ void __launch_bounds__(kBlk, kVecOcc) cg_p_k(int64_t n, T* __restrict
                                               const double* scal, const int* flags) {
   // runs once more after a replacement request (F_RU = 1), so that p is the
   // recurrence's next direction when the residual gets replaced
-  pdl_launch_dependents();
-  pdl_wait();
   if (flags[F_DONE] || flags[F_RU] == 2) return;
   const T beta = (T)scal[S_BETA];
   FOR4(i, n) p[i] = z[i] + beta * p[i];
@@ -1091,11 +1085,11 @@ template <typename T, bool DIFF, bool FLEX>
 static void launch_cg_spmv(Ctx* c, SolverData* S, const T* v, const T* x, T* y, const T* r, Red4 red, int slot) {
   const SellView V = S->view();
   if (S->A.d16)
-    launch_pdl(sell_cg_spmv_k<T, true, DIFF, FLEX>, sell_grid<T>(S), kBlk, c->stream, V, v, x, y, r, red, S->scal.p,
-               slot, S->flags.p);
+    sell_cg_spmv_k<T, true, DIFF, FLEX><<<sell_grid<T>(S), kBlk, 0, c->stream>>>(V, v, x, y, r, red,
+                                                                                       S->scal.p, slot, S->flags.p);
   else
-    launch_pdl(sell_cg_spmv_k<T, false, DIFF, FLEX>, sell_grid<T>(S), kBlk, c->stream, V, v, x, y, r, red, S->scal.p,
-               slot, S->flags.p);
+    sell_cg_spmv_k<T, false, DIFF, FLEX><<<sell_grid<T>(S), kBlk, 0, c->stream>>>(V, v, x, y, r, red,
+                                                                                       S->scal.p, slot, S->flags.p);
 }
 
 template <typename T>
@@ -1226,9 +1220,9 @@ static int run_pcg64(elfel_sysmat* m, double rtol, int maxit, elfel_solve_stats*
   const RunPlan run = run_plan(c, S, sizeof(double), 4, 4, 0);
   if (!run.blocks) ELFEL_TRY(capture(c, &S->g_pcg64, [&]() {
     launch_cg_spmv<double, false, false>(c, S, S->A.v64.p, S->p64.p, S->q64.p, nullptr, red_area(S, 0), S_PQ);
-    launch_pdl(cg_update_k<double, false>, vg, kBlk, c->stream, nu, S->x64.p, S->r64.p, S->p64.p, S->q64.p, S->z64.p,
-               S->dinv64.p, red_area(S, 1), S->scal.p, S->flags.p);
-    launch_pdl(cg_p_k<double>, vg, kBlk, c->stream, nu, S->p64.p, S->z64.p, S->scal.p, S->flags.p);
+    cg_update_k<double, false><<<vg, kBlk, 0, c->stream>>>(nu, S->x64.p, S->r64.p, S->p64.p, S->q64.p, S->z64.p,
+                                                           S->dinv64.p, red_area(S, 1), S->scal.p, S->flags.p);
+    cg_p_k<double><<<vg, kBlk, 0, c->stream>>>(nu, S->p64.p, S->z64.p, S->scal.p, S->flags.p);
   }));
   // When the recurrence residual says converged, the true residual b - K x is
   // checked in FP64; if the two have drifted apart (ill-conditioned systems
@@ -1282,9 +1276,9 @@ static int run_pcg32(elfel_sysmat* m, double bn2, double delta, double rtol, int
   const RunPlan run = run_plan(c, S, sizeof(float), 5, 4, 0);
   if (!run.blocks) ELFEL_TRY(capture(c, &S->g_pcg32, [&]() {
     launch_cg_spmv<float, true, true>(c, S, S->A.v32.p, S->p32.p, S->q32.p, S->r32.p, red_area(S, 0), S_PQ);
-    launch_pdl(cg_update_k<float, true>, vg, kBlk, c->stream, nu, S->xa32.p, S->r32.p, S->p32.p, S->q32.p, S->z32.p,
-               S->dinv32.p, red_area(S, 1), S->scal.p, S->flags.p);
-    launch_pdl(cg_p_k<float>, vg, kBlk, c->stream, nu, S->p32.p, S->z32.p, S->scal.p, S->flags.p);
+    cg_update_k<float, true><<<vg, kBlk, 0, c->stream>>>(nu, S->xa32.p, S->r32.p, S->p32.p, S->q32.p, S->z32.p,
+                                                         S->dinv32.p, red_area(S, 1), S->scal.p, S->flags.p);
+    cg_p_k<float><<<vg, kBlk, 0, c->stream>>>(nu, S->p32.p, S->z32.p, S->scal.p, S->flags.p);
   }));
   int refinements = 0, late = 0;
   int launches = 0;
