@@ -196,10 +196,8 @@ __device__ __forceinline__ double2 load_after_wait(const double2* p) {
 }
 
 // ------------------------------------------------------------------ scan
-// Exclusive prefix sum of n int64 values in place: out[i] = sum_{j<i} in[j],
-// writes the total to out[n] (the buffer must hold n+1 entries).
-int exclusive_scan_i64(Ctx* c, int64_t* data, int64_t n);
-// Exclusive scan of int32 counts into an int64 offsets array (n+1 entries).
+// Exclusive prefix sum of n int32 counts: offsets[i] = sum_{j<i} counts[j], the total
+// in offsets[n].
 int scan_counts_i32(Ctx* c, const int32_t* counts, int64_t n, int64_t* offsets);
 
 // ------------------------------------------------------------------ reductions

@@ -157,12 +157,6 @@ static int scan_impl(Ctx* c, const TIn* in, int64_t n, int64_t* out) {
   return ELFEL_OK;
 }
 
-int exclusive_scan_i64(Ctx* c, int64_t* data, int64_t n) {
-  // in-place: scan_tile reads its own items before writing them, and reads
-  // only its own tile, so in == out is safe.
-  return scan_impl<int64_t>(c, data, n, data);
-}
-
 int scan_counts_i32(Ctx* c, const int32_t* counts, int64_t n, int64_t* offsets) {
   return scan_impl<int32_t>(c, counts, n, offsets);
 }

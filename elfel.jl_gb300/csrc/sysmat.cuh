@@ -363,7 +363,6 @@ struct Fused {
   DBuf<int32_t> conn_u, conn_p;      // nel x nn, 0-based node ids
   DBuf<double> xy_u;                 // nnodes x sdim
   DBuf<int32_t> dofs_u, dofs_p;      // nel x nedof, 0-based DOFs
-  DBuf<int32_t> zero_rows;           // nel x nedof zeros (row table of the rhs "matrix")
   DBuf<double> coef;                 // per-element coefficients
   DBuf<double> kstore;               // element matrix records, nel x store_per_elem
   DBuf<double> fstore;               // element vector records, nel x nedof
@@ -387,7 +386,7 @@ struct Fused {
     ncurved = -1;
     straight.release(c);
     conn_u.release(c); conn_p.release(c); xy_u.release(c); dofs_u.release(c); dofs_p.release(c);
-    zero_rows.release(c); coef.release(c); kstore.release(c); fstore.release(c);
+    coef.release(c); kstore.release(c); fstore.release(c);
     fpat.release(c); pmass_store.release(c); pmpat.release(c); pmass_diag.release(c);
   }
 };
