@@ -1375,14 +1375,22 @@ __global__ void __launch_bounds__(kIntThreads) elast_straight_k(int64_t nel, con
 // 2 x 2 tensor Phi has closed-form entries: with m_ab = grad l_a^T Phi grad l_b of
 // the barycentric coordinates (rows and columns of m add up to zero),
 //   vertex a, vertex b       m_aa / 2, -m_ab / 6
-//   vertex p, edge (p, q)    2/3 m_pq (0 for an edge that p is not on)
+//   vertex p, edge (p, q)    2/3 m_pq (zero for an edge that p is not on)
 //   edge (p, q) with itself  4/3 (m_pp + m_qq) + 2/3 (m_pq + m_qp)
 //   edge (s, x), edge (s, y) 4/3 m_xy + 2/3 (m_sy - m_ys)
 // (integrals of l_a l_b over the triangle: area / 12 for a != b, area / 6 for a == b; edge
 // node 3 + p lies between vertices p and p + 1 mod 3).
+// zero: what entries that are zero whatever Phi is hold: 0, or NaN when an entry of m is
+// not finite (0 times it, as the sums over the rule's points give).
 struct BaryForm {
-  double m[3][3];
+  double m[3][3], zero;
 };
+
+// 0 for a finite x, else NaN (by integers: the FP64 unit bounds the kernels here).
+__device__ __forceinline__ double zero_of(double x) {
+  const int h = __double2hiint(x);
+  return __hiloint2double((h & 0x7ff00000) == 0x7ff00000 ? 0x7ff80000 : 0, 0);
+}
 
 template <bool SYM>
 __device__ __forceinline__ double t6_entry(const BaryForm& F, int a, int b) {
@@ -1391,7 +1399,7 @@ __device__ __forceinline__ double t6_entry(const BaryForm& F, int a, int b) {
   if (a < 3 && b < 3) return a == b ? __dmul_rn(0.5, m[a][a]) : __dmul_rn(k16, m[a][b]);
   if (a < 3 || b < 3) {
     const int v = a < 3 ? a : b, p = (a < 3 ? b : a) - 3, q = (p + 1) % 3;
-    if (v != p && v != q) return 0.0;
+    if (v != p && v != q) return F.zero;
     const int o = v == p ? q : p;
     return __dmul_rn(k23, a < 3 ? m[v][o] : m[o][v]);
   }
@@ -1419,6 +1427,7 @@ __device__ __forceinline__ BaryForm bary_form(double f00, double f01, double f10
   m[0][1] = -__dadd_rn(f00, f10);
   m[0][2] = -__dadd_rn(f01, f11);
   m[0][0] = __dadd_rn(r1, r2);
+  F.zero = zero_of(m[0][0]);
   return F;
 }
 
@@ -1498,7 +1507,10 @@ __global__ void __launch_bounds__(kIntThreads) elast_t6_exact_k(int64_t nel, con
   // load vector: 0 at the vertices, det b / 6 at the midside nodes
   if (in) {
 #pragma unroll
-    for (int k = 0; k < 12; ++k) acc[k * LD + t] = k < 6 ? 0.0 : (k & 1) ? f1 : f0;
+    for (int k = 0; k < 12; ++k) {
+      const double f = (k & 1) ? f1 : f0;
+      acc[k * LD + t] = k < 6 ? zero_of(f) : f;
+    }
   }
   write_records_fixed<NT, 12, 12>(acc, 0, e0, nel, fstore);
 }
