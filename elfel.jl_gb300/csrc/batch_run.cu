@@ -73,7 +73,7 @@ __device__ __forceinline__ void batch_run(const BSys& S, Group& grp, int rank, u
   const double scale = S.sc[B_SCALE], tol = S.sc[B_TOL2], bn2 = S.sc[B_BN2];
   const double thr = IR ? tol : tol * bn2, delta2 = S.sc[B_DELTA] * S.sc[B_DELTA];
   double rz = S.sc[B_RZ], rr = S.sc[B_RR], rmax2 = S.sc[B_RMAX] * S.sc[B_RMAX], pq = 0.0;
-  double inv_rz = 1.0 / rz, low2 = delta2 * rmax2;
+  double inv_rz = 0.0, low2 = delta2 * rmax2;
   int it = S.st[I_ITER], brk = S.st[I_BRK], repl = S.st[I_REPL], conv = 0, mode = M_CG;
   const int maxit = S.st[I_MAXIT];
   __syncthreads();
@@ -136,11 +136,12 @@ __device__ __forceinline__ void batch_run(const BSys& S, Group& grp, int rank, u
     if (wid == 0) grp.publish(t2);
     grp.arrive(wid);
     for (int i = tid; i < R.nloc; i += kRT) sx[i] += al * sp[i];
-    if (wid == 0) inv_rz = fast_rcp(rz);
+    if (wid == 0) inv_rz = IR ? fast_rcp(rz) : rcp_ahead(rz);
     ok = grp.wait(wid);
     grp.collect(wid, wsum, t2);
     if (wid == 0) {
-      const double beta = (IR ? t2[0] - t2[N2 - 1] : t2[0]) * inv_rz;
+      // (FP32: r.z is 0 or a normal double)
+      const double beta = IR ? (t2[0] - t2[N2 - 1]) * inv_rz : times_rcp(t2[0], rz, inv_rz);
       rz = t2[0];
       rr = t2[1];
       ++it;

@@ -24,6 +24,22 @@ __device__ __forceinline__ double fast_rcp(double x) {
   return newton_rcp(x);
 }
 
+// newton_rcp(x) here, ahead of where it is used (the compiler moves it there otherwise,
+// behind the barrier of a sum: FP64 CG on 129,000 unknowns 1 % longer).
+__device__ __forceinline__ double rcp_ahead(double x) {
+  double y = newton_rcp(x);
+  asm volatile("" : "+d"(y));
+  return y;
+}
+
+// a / x from y = newton_rcp(x), formed ahead of a: a y, within two units in the last place; where
+// the exponent of x is extreme the division (y is not used).
+__device__ __forceinline__ double times_rcp(double a, double x, double y) {
+  const int e = exponent_of(x);
+  if (e < 60 || e > 1980) return a / x;
+  return a * y;
+}
+
 // a / x: a y, y = newton_rcp(x), corrected by its remainder a - x q (Markstein 1990); at most one
 // unit in the last place from the rounded quotient.  Where an exponent is extreme (of a, x or the
 // quotient: a y overflows, the remainder underflows, zeros, infinities, NaN) the division.

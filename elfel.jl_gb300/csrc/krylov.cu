@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kRT, 1) cg_run_k(const CgRun<T> a, const RunGr
   }
   const T* const rs = IR && !a.own_sums ? a.rowsum + R.row0 : ss;  // row sums: of the own rows, or where they are
   // the loop's scalars (warp 0 uses them)
-  double rz = a.scal[S_RZ], rr = a.scal[S_RR], pq = 0.0, alpha = 0.0, beta = 0.0, inv_rz = 1.0 / rz;
+  double rz = a.scal[S_RZ], rr = a.scal[S_RR], pq = 0.0, alpha = 0.0, beta = 0.0, inv_rz = 0.0;
   const double thr = a.scal[S_TOL2] * (IR ? a.scal[S_BN2S] : a.scal[S_BN2]);
   const double delta2 = IR ? a.scal[S_DELTA] * a.scal[S_DELTA] : 0.0;
   double rmax2 = a.scal[S_RMAX] * a.scal[S_RMAX];  // the largest r.r since the last replacement
@@ -163,13 +163,14 @@ __global__ void __launch_bounds__(kRT, 1) cg_run_k(const CgRun<T> a, const RunGr
     if (wid == 0) grp.publish(t2);
     grp.arrive(wid);
     for (int i = tid; i < R.nloc; i += kRT) sx[i] += al * sp[i];
-    if (wid == 0) inv_rz = fast_rcp(rz);
+    if (wid == 0) inv_rz = IR ? fast_rcp(rz) : rcp_ahead(rz);
     ok = grp.wait(wid);
     grp.collect(wid, wsum, t2);
     if (wid == 0) {
       const double rzn = t2[0];
       rr = t2[1];
-      beta = (IR ? rzn - t2[N2 - 1] : rzn) * inv_rz;
+      // (FP32: r.z is 0 or a normal double)
+      beta = IR ? (rzn - t2[N2 - 1]) * inv_rz : times_rcp(rzn, rz, inv_rz);
       rz = rzn;
       ++it;
       conv = le_pos(rr, thr);

@@ -1,9 +1,10 @@
-"""fast_rcp and fast_div (fastdiv64.cuh) against the device's IEEE division (GPU).
+"""fast_rcp, fast_div and times_rcp (fastdiv64.cuh) against the device's IEEE division (GPU).
 
 A small program with the header is compiled and run.  Bounds, from the header:
 with y exact to 2^-40 after the first step, the second leaves 1 / x to 2^-80
 before its last rounding, so the result is the rounded quotient or its
-neighbour; the same for a quotient corrected by its remainder.  Arguments: random
+neighbour; the same for a quotient corrected by its remainder, one more rounding
+without the correction.  Arguments: random
 significands over all exponents and around the two exponents where the forms
 change, both signs; zeros, subnormals, infinities and NaN give what the division
 gives.
@@ -44,10 +45,10 @@ __device__ long long ulps(double got, double want) {
   if (isnan(got) || isnan(want) || (g ^ w) < 0) return -1;
   return g > w ? g - w : w - g;
 }
-// res: worst fast_rcp, worst fast_div, wrong specials, compared
+// res: worst fast_rcp, worst fast_div, wrong specials, compared, (specials), worst times_rcp
 __global__ void check(int n, long long* res) {
   const int stride = gridDim.x * blockDim.x;
-  long long wr = 0, wd = 0, bad = 0, cnt = 0;
+  long long wr = 0, wd = 0, wt = 0, bad = 0, cnt = 0;
   const int edges[8] = {58, 59, 60, 61, 1979, 1980, 1981, 1982};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     const uint64_t h = mix(2 * (uint64_t)i + 1), k = mix(2 * (uint64_t)i + 2);
@@ -65,12 +66,18 @@ __global__ void check(int n, long long* res) {
     } else {
       wd = max(wd, v);
     }
+    const double t = times_rcp(a, x, newton_rcp(x));
+    const long long w = ulps(t, d);
+    const int ex = (int)((__double_as_longlong(x) >> 52) & 0x7ff);
+    if (ex < 60 || ex > 1980) bad += w != 0;  // the division
+    else if (!special(d) && !special(t)) wt = max(wt, w < 0 ? 1000 : w);
     cnt += 2;
   }
   atomicMax(res, wr);
   atomicMax(res + 1, wd);
   atomicAdd((unsigned long long*)(res + 2), (unsigned long long)bad);
   atomicAdd((unsigned long long*)(res + 3), (unsigned long long)cnt);
+  atomicMax(res + 5, wt);
 }
 __global__ void specials(long long* res) {
   const double inf = __longlong_as_double(0x7ff0000000000000LL), nan = __longlong_as_double(0x7ff8000000000000LL);
@@ -91,14 +98,14 @@ __global__ void specials(long long* res) {
 }
 
 int main() {
-  long long *res, h[5];
+  long long *res, h[6];
   if (cudaMallocManaged(&res, sizeof(h))) return 2;
-  for (int k = 0; k < 5; ++k) res[k] = 0;
+  for (int k = 0; k < 6; ++k) res[k] = 0;
   check<<<304, 256>>>(1 << 24, res);
   specials<<<1, 1>>>(res);
   if (cudaDeviceSynchronize()) return 2;
-  for (int k = 0; k < 5; ++k) h[k] = res[k];
-  std::printf("%lld %lld %lld %lld %lld\n", h[0], h[1], h[2], h[3], h[4]);
+  for (int k = 0; k < 6; ++k) h[k] = res[k];
+  std::printf("%lld %lld %lld %lld %lld %lld\n", h[0], h[1], h[2], h[3], h[4], h[5]);
   return 0;
 }
 """
@@ -111,6 +118,33 @@ def test_against_the_division(gpu, tmp_path):
     subprocess.run([nvcc, "-std=c++17", "-O3", "-gencode", "arch=compute_103a,code=sm_103a", "-I", CSRC, str(src), "-o",
                     str(exe)], check=True, capture_output=True, timeout=300)
     out = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120, check=True)
-    rcp, div, wrong, compared, specials = map(int, out.stdout.split())
+    rcp, div, wrong, compared, specials, times = map(int, out.stdout.split())
     assert compared == 2 << 24
-    assert rcp <= 1 and div <= 1 and wrong == 0 and specials == 0, out.stdout
+    assert rcp <= 1 and div <= 1 and times <= 2 and wrong == 0 and specials == 0, out.stdout
+
+
+@pytest.mark.parametrize("method", ["pcg64", "batch"])
+@pytest.mark.parametrize("scale", [1.0, 1e-150, 1e-160, 1e140])
+def test_scalars_near_the_ends_of_the_range(E, gpu, method, scale):
+    """A right-hand side of 1e-160, whose dot products are subnormal: the steps divide by them.  Two
+    unknowns with condition number 7 / 3: a residual of 1e-9 leaves 3e-9; subnormal sums of 1e-320 have 11 bits,
+    so with them the answer is asked to 1 %."""
+    import numpy as np
+    import scipy.sparse as sp
+
+    A = sp.csr_matrix(np.array([[2.5, -1.0], [-1.0, 2.5]]))
+    F = scale * np.array([0.3, -1.1])
+    c = A.tocoo()
+    a = E.start(E.SysmatAssemblerSparse(0.0), 2, 2)
+    a._chunks.append((c.row.astype(np.int64) + 1, c.col.astype(np.int64) + 1, c.data.astype(np.float64)))
+    E.finish(a)
+    T = np.zeros(2)
+    if method == "batch":
+        b = E.BatchSolver("pcg64", capacity=1)
+        s = b.add(a, T, 2, F=F, rtol=1e-9)
+        T, st = b.run()[s]
+        b.close()
+    else:
+        st = E.solve(T, a, F, 2, method=method, rtol=1e-9)
+    want = np.linalg.solve(A.toarray(), F / scale)
+    assert st["converged"] and np.abs(T / scale - want).max() <= (0.01 if scale < 1e-155 else 3e-9)
