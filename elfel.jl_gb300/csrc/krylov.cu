@@ -20,12 +20,12 @@
 //       961 unknowns  21.3 ->  5.4 us   25.8 ->  4.7 us
 //     14161           21.1 ->  7.7      21.9 ->  5.6
 //    128881           26.2 -> 12.0      22.2 ->  7.8
-//    358801           40.2 -> 22.6      32.0 -> 11.3
-//    808201           62.7 -> 47.2      45.9 -> 16.0
+//    358801           40.2 -> 22.6      32.0 -> 11.2
+//    808201           62.7 -> 47.2      45.9 -> 15.8
 // MINRES (Taylor-Hood cavity) 27.2 -> 11.1 us at 9026 unknowns.  What is left
 // at 128881: the two sums over the grid (1.5 us a barrier with the blocks' uneven
 // arrival, 0.8 to collect), in FP64 the FP64 unit (4.5 us), in FP32 at 808201 the
-// compensated sums (0.35).  Measured and not kept: the direction gathered
+// compensated sums (0.1; 0.3 when a row is added at once).  Measured and not kept: the direction gathered
 // from global memory after a barrier of its own (FP32 9.4 us at 128881, 21.1 at
 // 808201: gathers that miss L1), 1024 threads a block (17.5 at 808201), the
 // next chunk of the matrix prefetched into registers (no change), the matrix
@@ -115,17 +115,31 @@ __global__ void __launch_bounds__(kRT, 1) cg_run_k(const CgRun<T> a, const RunGr
     // q = A p; p.q (and r.p) -> alpha
     constexpr int N1 = IR ? 2 : 1;
     Dot<T> d1[N1];
+    T la = 0, lp = 0, lr = 0;
     for (int n = 0; n * kRW < R.nsl; ++n) {
       const int s = R.slice(wid, n);
       const int i = s * 32 + lane;
       if (i < R.nloc) {
         const T pi = sp[i];
+        if (IR) {  // the row before, while this one's entries are on their way
+          d1[0].add(la, lp);
+          d1[N1 - 1].add(lr, lp);
+        }
         T acc = R.template row<IR>(s, i, WIN ? W.by_row() : (const T*)a.p, pi);
         if (IR) acc += rs[i] * pi;
         sq[i] = acc;
-        d1[0].add(acc, pi);
-        if (IR) d1[N1 - 1].add(sr[i], pi);
+        if (IR) {
+          la = acc;
+          lp = pi;
+          lr = sr[i];
+        } else {
+          d1[0].add(acc, pi);
+        }
       }
+    }
+    if (IR) {
+      d1[0].add(la, lp);
+      d1[N1 - 1].add(lr, lp);
     }
     double t1[N1];
     block_sums<N1>(d1, part, wsum, t1, nw);
